@@ -215,6 +215,7 @@ enum ScratchSlot : int {
     Q_AREA_EPOFF = 37,  // area: edge -> pixel index offsets (per ring position)
     Q_AREA_EPPIX = 38,  // area: edge -> pixel index entries
     Q_PAIR_ORDER = 39,  // intersect: the longest-first pair order
+    Q_SPILL = 48,       // intersect, contain: pixel pairs left to all warps
 };
 }  // namespace farm
 
@@ -238,7 +239,7 @@ struct farm_store {
     uint64_t tot_P = 0, tot_status = 0, tot_seq = 0;
     farm_raster_totals rtot = {};
     // scratch for the rasterizer and the queries
-    farm::DevBuf s[48];
+    farm::DevBuf s[49];
     farm::DevBuf cub_tmp;
     farm::DevBuf d_pairs, d_out, d_counters;
     farm::DevBuf d_check;  // pair-index validation counter
@@ -246,7 +247,7 @@ struct farm_store {
     void *h_stage[2] = {nullptr, nullptr};  // pinned staging of the .dt loader (farm_store_load_dt)
     size_t h_stage_cap = 0;
     cudaEvent_t ev_stage[2] = {};
-    cudaEvent_t ev[8] = {};
+    cudaEvent_t ev[9] = {};
     uint64_t launches = 0;  // engine kernels launched through this store
     void *mlp = nullptr;    // learned scorer state (mlp.cu)
     uint64_t raster_epoch = 0;     // bumped by every rasterization (plans check it)

@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "segments.cuh"
+#include "spill.cuh"
 
 namespace farm {
 
@@ -132,18 +133,40 @@ __device__ bool edges_cross_box(const StoreView &sv, const PolyHdr &T, uint32_t 
     return false;
 }
 
+// An entry of the queue: source pixel, target pixel; kOutBorder marks an OUT
+// source pixel over a BORDER target pixel (the others are BORDER x BORDER).
+constexpr uint32_t kOutBorder = 0x80000000u;
+
+// Whether pixel pair e says "no"; part / nparts as in refine_pixel_pair.
+__device__ __forceinline__ bool pixel_pair_violates(const StoreView &sv, const PolyHdr &S, const PolyHdr &T, uint2 e,
+                                                    float4 *tb, unsigned long long &tests, uint32_t part,
+                                                    uint32_t nparts) {
+    if (!(e.x & kOutBorder)) return refine_pixel_pair(sv, S, T, e.x, e.y, tb, tests, part, nparts);
+    if (part) return false;
+    const int i = (int)((e.x & ~kOutBorder) % (uint32_t)S.dimx), j = (int)((e.x & ~kOutBorder) / (uint32_t)S.dimx);
+    return edges_cross_box(sv, T, e.y, S.mbr[0] + i * S.step_x, S.mbr[1] + j * S.step_y,
+                           S.mbr[0] + (i + 1) * S.step_x, S.mbr[1] + (j + 1) * S.step_y, tests);
+}
+
+// One warp per candidate pair up to its budget; what is left of a pair goes to
+// k_contain_spill. A pair's result is written here as if no spilled pixel pair
+// said "no".
 __global__ void __launch_bounds__(kContainWarps * 32)
     k_contain(const StoreView sv, const uint32_t *__restrict__ pairs, uint64_t n, uint64_t tgt_base,
-              unsigned long long *__restrict__ next, uint8_t *__restrict__ out, ContainCounters *__restrict__ ctr) {
-    __shared__ float4 tbufs[kContainWarps][32];
+              unsigned long long *__restrict__ next, uint8_t *__restrict__ out, ContainCounters *__restrict__ ctr,
+              SpillPool sp) {
+    __shared__ uint2 queue[kContainWarps][kQueue];
+    __shared__ float4 tbufs[kContainWarps][2 * kStage];
+    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    uint2 *q = queue[wib];
     float4 *tb = tbufs[wib];
     const int cc = sv.category_count;
     unsigned long long my_found = 0, my_pp = 0, my_tests = 0;
     for (;;) {
         unsigned long long pid = 0;
         if (lane == 0) pid = atomicAdd(next, 1ull);
-        pid = __shfl_sync(0xffffffffu, pid, 0);
+        pid = __shfl_sync(full, pid, 0);
         if (pid >= n) break;
         const uint32_t s = pairs[2 * pid], t = pairs[2 * pid + 1];
         const PolyHdr &S = sv.hdr[s];
@@ -167,53 +190,67 @@ __global__ void __launch_bounds__(kContainWarps * 32)
             const long k = base + lane;
             int st = 1;
             if (k < nw) st = show_status(sst[(w.sy + (int)(k % wh)) * S.dimx + w.sx + (int)(k / wh)], cc);
-            n_out += __popc(__ballot_sync(0xffffffffu, k < nw && st == 0));
-            n_in += __popc(__ballot_sync(0xffffffffu, k < nw && st == 2));
+            n_out += __popc(__ballot_sync(full, k < nw && st == 0));
+            n_in += __popc(__ballot_sync(full, k < nw && st == 2));
         }
         int result;
+        bool spilled = false;
+        uint32_t head = 0;
         if (n_out == nw) {
             result = 0;
         } else if (n_in == nw) {
             result = 1;
         } else {
-            bool violated = false;
-            for (long base = 0; base < nw && !violated; base += 32) {
-                // one source window pixel per lane (x outer, y inner); IN
-                // pixels are skipped
-                const long k = base + lane;
-                int tw_sx = 0, tw_sy = 0, tw_ey = -1;
-                uint32_t pa = 0, cnt = 0;
-                int pa_st = 2;
-                double b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-                if (k < nw) {
-                    const int i = w.sx + (int)(k / wh), j = w.sy + (int)(k % wh);
-                    pa = (uint32_t)(j * S.dimx + i);
-                    pa_st = show_status(sst[pa], cc);
-                    if (pa_st != 2) {
-                        b0 = S.mbr[0] + i * S.step_x;
-                        b1 = S.mbr[1] + j * S.step_y;
-                        b2 = S.mbr[0] + (i + 1) * S.step_x;
-                        b3 = S.mbr[1] + (j + 1) * S.step_y;
-                        const Window tw = retrieve(T.mbr, T.step_x, T.step_y, T.dimx, T.dimy, b0, b1, b2, b3);
-                        if (tw.ex >= tw.sx && tw.ey >= tw.sy) {
-                            tw_sx = tw.sx;
-                            tw_sy = tw.sy;
-                            tw_ey = tw.ey;
-                            cnt = (uint32_t)((tw.ex - tw.sx + 1) * (tw.ey - tw.sy + 1));
+            bool violated = false, may_spill = sp.cap > 0;
+            const float pp_cost = pixel_pair_cost(S, T);
+            float spent = 0.f;
+            int qn = 0;
+            // one source window pixel per lane (x outer, y inner; IN pixels are
+            // skipped), its target window flattened across the warp
+            long base = 0;
+            int tw_sx = 0, tw_sy = 0, tw_ey = -1, pa_st = 2;
+            uint32_t pa = 0, excl = 0, total = 0, f = 0;
+            for (bool more = true; more && !violated;) {
+                while (qn + 32 <= kQueue) {
+                    if (f >= total) {
+                        if (base >= nw) {
+                            more = false;
+                            break;
                         }
+                        const long k = base + lane;
+                        uint32_t cnt = 0;
+                        pa_st = 2;
+                        if (k < nw) {
+                            const int i = w.sx + (int)(k / wh), j = w.sy + (int)(k % wh);
+                            pa = (uint32_t)(j * S.dimx + i);
+                            pa_st = show_status(sst[pa], cc);
+                            if (pa_st != 2) {
+                                const double b0 = S.mbr[0] + i * S.step_x, b1 = S.mbr[1] + j * S.step_y;
+                                const double b2 = S.mbr[0] + (i + 1) * S.step_x, b3 = S.mbr[1] + (j + 1) * S.step_y;
+                                const Window tw = retrieve(T.mbr, T.step_x, T.step_y, T.dimx, T.dimy, b0, b1, b2, b3);
+                                if (tw.ex >= tw.sx && tw.ey >= tw.sy) {
+                                    tw_sx = tw.sx;
+                                    tw_sy = tw.sy;
+                                    tw_ey = tw.ey;
+                                    cnt = (uint32_t)((tw.ex - tw.sx + 1) * (tw.ey - tw.sy + 1));
+                                }
+                            }
+                        }
+                        excl = warp_excl_scan(cnt, lane, total);
+                        base += 32;
+                        f = 0;
+                        continue;
                     }
-                }
-                uint32_t total;
-                const uint32_t excl = warp_excl_scan(cnt, lane, total);
-                for (uint32_t f = 0; f < total && !violated; f += 32) {
                     const uint32_t item = f + lane;
+                    f += 32;
                     const int owner = warp_owner(excl, item);
-                    const uint32_t o_excl = __shfl_sync(0xffffffffu, excl, owner);
-                    const int o_sx = __shfl_sync(0xffffffffu, tw_sx, owner);
-                    const int o_sy = __shfl_sync(0xffffffffu, tw_sy, owner);
-                    const int o_ey = __shfl_sync(0xffffffffu, tw_ey, owner);
-                    const int o_st = __shfl_sync(0xffffffffu, pa_st, owner);
-                    bool out_in = false, ob = false, bb = false;
+                    const uint32_t o_excl = __shfl_sync(full, excl, owner);
+                    const int o_sx = __shfl_sync(full, tw_sx, owner);
+                    const int o_sy = __shfl_sync(full, tw_sy, owner);
+                    const int o_ey = __shfl_sync(full, tw_ey, owner);
+                    const int o_st = __shfl_sync(full, pa_st, owner);
+                    const uint32_t o_pa = __shfl_sync(full, pa, owner);
+                    bool out_in = false, edges = false;
                     uint32_t pb = 0;
                     if (item < total) {
                         const uint32_t r = item - o_excl;
@@ -222,30 +259,32 @@ __global__ void __launch_bounds__(kContainWarps * 32)
                         pb = (uint32_t)(v * T.dimx + u);
                         const int pb_st = show_status(tst[pb], cc);
                         out_in = o_st == 0 && pb_st == 2;
-                        ob = o_st == 0 && pb_st == 1;
-                        bb = o_st == 1 && pb_st == 1;
+                        edges = pb_st == 1;  // the source pixel is OUT or BORDER
                     }
-                    if (__any_sync(0xffffffffu, out_in)) {
+                    if (__any_sync(full, out_in)) {
                         violated = true;
                         break;
                     }
-                    // pixel pairs that need edges: the whole warp takes one at a time
-                    for (unsigned m = __ballot_sync(0xffffffffu, ob || bb); m && !violated; m &= m - 1) {
-                        const int src = __ffs(m) - 1;
-                        const uint32_t qb = __shfl_sync(0xffffffffu, pb, src);
-                        const bool q_ob = __shfl_sync(0xffffffffu, ob, src);
-                        const int ow = __shfl_sync(0xffffffffu, owner, src);
-                        const uint32_t qa = __shfl_sync(0xffffffffu, pa, ow);
-                        if (lane == 0) my_pp++;
-                        if (q_ob) {
-                            const double e0 = __shfl_sync(0xffffffffu, b0, ow), e1 = __shfl_sync(0xffffffffu, b1, ow);
-                            const double e2 = __shfl_sync(0xffffffffu, b2, ow), e3 = __shfl_sync(0xffffffffu, b3, ow);
-                            violated = edges_cross_box(sv, T, qb, e0, e1, e2, e3, my_tests);
-                        } else {
-                            violated = refine_pixel_pair(sv, S, T, qa, qb, tb, my_tests);
-                        }
-                    }
+                    const unsigned m = __ballot_sync(full, edges);
+                    if (edges) q[qn + __popc(m & ((1u << lane) - 1))] = make_uint2(o_pa | (o_st == 0 ? kOutBorder : 0u), pb);
+                    qn += __popc(m);
                 }
+                if (violated || qn == 0) continue;
+                __syncwarp();
+                for (int k = 0; k < qn && !violated; k++) {
+                    if (may_spill && spent > sp.budget) {
+                        if (spill_rest(sp, pid, q, k, qn, pp_cost, lane, &head, &spilled)) {
+                            if (lane == 0) my_pp += qn - k;
+                            break;
+                        }
+                        may_spill = false;  // the pool is full
+                    }
+                    if (lane == 0) my_pp++;
+                    violated = pixel_pair_violates(sv, S, T, q[k], tb, my_tests, 0, 1);
+                    spent += pp_cost;
+                }
+                qn = 0;
+                __syncwarp();
             }
             if (violated) {
                 result = 0;
@@ -256,20 +295,47 @@ __global__ void __launch_bounds__(kContainWarps * 32)
                     const float2 p0 = sv.ring[T.ring];
                     in = contain_point(sv, S, p0.x, p0.y);
                 }
-                result = __shfl_sync(0xffffffffu, in, 0) ? 1 : 0;
+                result = __shfl_sync(full, in, 0) ? 1 : 0;
             }
         }
         if (lane == 0) {
             out[pid] = (uint8_t)result;
             my_found += result == 1;
+            if (spilled && result == 0) sp.flag[head] = 1u;  // nothing left to find out
         }
         __syncwarp();
     }
-    for (int o = 16; o; o >>= 1) my_tests += __shfl_xor_sync(0xffffffffu, my_tests, o);
+    for (int o = 16; o; o >>= 1) my_tests += __shfl_xor_sync(full, my_tests, o);
     if (lane == 0) {
         atomicAdd(&ctr->found, my_found);
         atomicAdd(&ctr->pixel_pairs, my_pp);
         atomicAdd(&ctr->segment_tests, my_tests);
+    }
+}
+
+// The pixel pairs that k_contain spilled, over all warps: a "no" takes back
+// the result that k_contain wrote (1, or the pair's flag were set).
+__global__ void __launch_bounds__(kContainWarps * 32, 3)
+    k_contain_spill(const StoreView sv, const uint32_t *__restrict__ pairs, uint64_t tgt_base, SpillPool sp,
+                    uint8_t *__restrict__ out, ContainCounters *__restrict__ ctr) {
+    __shared__ float4 tbufs[kContainWarps][2 * kStage];
+    float4 *tb = tbufs[threadIdx.x >> 5];
+    unsigned long long lost = 0, my_tests = 0;
+    spill_units(
+        sp,
+        [&](unsigned long long p, uint2 e, uint32_t part, uint32_t nparts) {
+            const PolyHdr &S = sv.hdr[pairs[2 * p]];
+            const PolyHdr &T = sv.hdr[tgt_base + pairs[2 * p + 1]];
+            return pixel_pair_violates(sv, S, T, e, tb, my_tests, part, nparts);
+        },
+        [&](unsigned long long p) {
+            out[p] = 0;
+            lost++;
+        });
+    for (int o = 16; o; o >>= 1) my_tests += __shfl_xor_sync(0xffffffffu, my_tests, o);
+    if ((threadIdx.x & 31) == 0) {
+        if (lost) atomicAdd(&ctr->found, 0ull - lost);
+        if (my_tests) atomicAdd(&ctr->segment_tests, my_tests);
     }
 }
 
@@ -307,13 +373,19 @@ extern "C" int farm_contain(farm_store *s, const uint32_t *pairs, uint64_t n, in
     FARM_TRY(s->d_counters.ensure(256));
     unsigned long long *next = s->d_counters.as<unsigned long long>();
     ContainCounters *ctr = reinterpret_cast<ContainCounters *>(next + 1);
-    FARM_CUDA(cudaMemsetAsync(next, 0, 8 + sizeof(ContainCounters), stream));
+    static_assert(8 + sizeof(ContainCounters) <= 64, "the spill counters follow at [8]");
+    FARM_CUDA(cudaMemsetAsync(next, 0, 88, stream));
+    SpillPool sp;
+    if (n) FARM_TRY(spill_pool(s, n, next + 8, 512.f, 4096.f, &sp));
     FARM_CUDA(cudaEventRecord(s->ev[6], stream));
     if (n) {
-        k_contain<<<sm_count() * 8, kContainWarps * 32, 0, stream>>>(s->view(), dpairs, n, s->n_side[0], next, dout,
-                                                                     ctr);
+        const uint64_t most = (uint64_t)sm_count() * 8;
+        k_contain<<<(unsigned)(n < most ? n : most), kContainWarps * 32, 0, stream>>>(s->view(), dpairs, n,
+                                                                                      s->n_side[0], next, dout, ctr, sp);
+        k_contain_spill<<<3 * sm_count(), kContainWarps * 32, 0, stream>>>(s->view(), dpairs, s->n_side[0], sp, dout,
+                                                                           ctr);
         FARM_CUDA(cudaGetLastError());
-        s->launches++;
+        s->launches += 2;
     }
     FARM_CUDA(cudaEventRecord(s->ev[7], stream));
     ContainCounters h{};
@@ -331,7 +403,7 @@ extern "C" int farm_contain(farm_store *s, const uint32_t *pairs, uint64_t n, in
         cudaEventElapsedTime(&ms, s->ev[6], s->ev[7]);
         st->ms_total = ms;
         st->ms_stage[2] = ms;
-        st->kernel_launches = n ? 1 : 0;
+        st->kernel_launches = n ? 2 : 0;
     }
     return FARM_OK;
 }

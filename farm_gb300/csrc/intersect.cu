@@ -20,11 +20,11 @@
 
 #include "common.cuh"
 #include "segments.cuh"
+#include "spill.cuh"
 
 namespace farm {
 
 constexpr int kWarpsPerBlock = 8;
-constexpr int kQueue = 256;  // BORDER x BORDER pixel pairs buffered per warp
 
 struct PairView {
     const uint32_t *pairs;
@@ -86,10 +86,10 @@ enum { K_EXACT = 0, K_APPROX = 1, K_FILTER = 2 };
 template <int kMode>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_intersect(const StoreView sv, PairView pv, unsigned long long *__restrict__ next, uint8_t *__restrict__ out,
-                IxCounters *__restrict__ ctr) {
+                IxCounters *__restrict__ ctr, SpillPool sp) {
     __shared__ uint2 queue[kWarpsPerBlock][kQueue];
     __shared__ float qkeys[kWarpsPerBlock][kQueue];
-    __shared__ float4 tbufs[kWarpsPerBlock][32];
+    __shared__ float4 tbufs[kWarpsPerBlock][2 * kStage];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     uint2 *q = queue[wib];
     float *qk = qkeys[wib];
@@ -118,90 +118,87 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         bool decided = false, has_bb = false;
         uint32_t pair_bb = 0;
         int qn = 0;  // warp-uniform queue fill
-        auto flush = [&]() {
-            // the warp refines the queued pixel pairs one after another, most
-            // probable first, and stops at the first hit
-            if (qn > 1) sort_queue_desc(qk, q, qn, lane);
-            bool hit = false;
-            for (int k = 0; k < qn && !hit; k++) {
-                const uint2 pp = q[k];
-                hit = refine_pixel_pair(sv, S, T, pp.x, pp.y, tb, my_tests);
-            }
-            qn = 0;
-            __syncwarp();
-            return hit;
-        };
-        for (long base = 0; base < nw && !decided; base += 32) {
-            // one source window pixel per lane (x outer, y inner)
-            long k = base + lane;
-            int tw_sx = 0, tw_ex = -1, tw_sy = 0, tw_ey = -1;
-            uint32_t pa = 0;
-            int pa_st = 0;
-            uint32_t cnt = 0;
-            if (k < nw) {
-                int i = w.sx + (int)(k / wh), j = w.sy + (int)(k % wh);
-                pa = (uint32_t)(j * S.dimx + i);
-                pa_st = show_status(sst[pa], cc);
-                if (pa_st != 0) {
-                    double b0 = S.mbr[0] + i * S.step_x, b1 = S.mbr[1] + j * S.step_y;
-                    double b2 = S.mbr[0] + (i + 1) * S.step_x, b3 = S.mbr[1] + (j + 1) * S.step_y;
-                    Window tw = retrieve(T.mbr, T.step_x, T.step_y, T.dimx, T.dimy, b0, b1, b2, b3);
-                    tw_sx = tw.sx;
-                    tw_ex = tw.ex;
-                    tw_sy = tw.sy;
-                    tw_ey = tw.ey;
-                    cnt = (uint32_t)((tw.ex - tw.sx + 1) * (tw.ey - tw.sy + 1));
+        // the pixels' areas over the larger of them, for the fill probability
+        // (it only orders the refinement, so float will do)
+        const float spa = (float)S.step_x * (float)S.step_y, tpa = (float)T.step_x * (float)T.step_y;
+        const float srel = spa > tpa ? 1.f : spa / tpa, trel = spa > tpa ? tpa / spa : 1.f;
+        const float pp_cost = pixel_pair_cost(S, T);
+        float spent = 0.f;
+        bool may_spill = kMode == K_EXACT && sp.cap > 0, spilled = false;
+        uint32_t head = 0;
+        // one source window pixel per lane (x outer, y inner), its target window
+        // flattened across the warp; a batch's state lives here so that the
+        // queue can be refined in the middle of it
+        long base = 0;
+        int tw_sx = 0, tw_sy = 0, tw_ey = -1;
+        uint32_t pa = 0, excl = 0, total = 0, f = 0;
+        int pa_st = 0;
+        for (bool more = true; more && !decided;) {
+            while (qn + 32 <= kQueue) {
+                if (f >= total) {
+                    if (base >= nw) {
+                        more = false;
+                        break;
+                    }
+                    const long k = base + lane;
+                    uint32_t cnt = 0;
+                    tw_sx = 0;
+                    tw_sy = 0;
+                    tw_ey = -1;
+                    pa = 0;
+                    pa_st = 0;
+                    if (k < nw) {
+                        int i = w.sx + (int)(k / wh), j = w.sy + (int)(k % wh);
+                        pa = (uint32_t)(j * S.dimx + i);
+                        pa_st = show_status(sst[pa], cc);
+                        if (pa_st != 0) {
+                            double b0 = S.mbr[0] + i * S.step_x, b1 = S.mbr[1] + j * S.step_y;
+                            double b2 = S.mbr[0] + (i + 1) * S.step_x, b3 = S.mbr[1] + (j + 1) * S.step_y;
+                            Window tw = retrieve(T.mbr, T.step_x, T.step_y, T.dimx, T.dimy, b0, b1, b2, b3);
+                            tw_sx = tw.sx;
+                            tw_sy = tw.sy;
+                            tw_ey = tw.ey;
+                            cnt = (uint32_t)((tw.ex - tw.sx + 1) * (tw.ey - tw.sy + 1));
+                        }
+                    }
+                    excl = warp_excl_scan(cnt, lane, total);
+                    if (lane == 0) {
+                        my_ws += (unsigned long long)min((long)32, nw - base);
+                        my_wt += total;
+                    }
+                    base += 32;
+                    f = 0;
+                    continue;
                 }
-            }
-            // flatten the lanes' target windows across the warp
-            uint32_t incl = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-            uint32_t excl = incl - cnt;
-            if (lane == 0) {
-                my_ws += (unsigned long long)min((long)32, nw - base);
-                my_wt += total;
-            }
-            for (uint32_t f = 0; f < total && !decided; f += 32) {
-                uint32_t item = f + lane;
-                bool valid = item < total;
-                // owner lane: the last lane whose exclusive prefix <= item
-                int owner = 0;
-                for (int b = 16; b; b >>= 1) {
-                    int cand = owner + b;
-                    uint32_t ex = __shfl_sync(0xffffffffu, excl, cand);
-                    if (cand < 32 && ex <= item) owner = cand;
-                }
-                uint32_t o_excl = __shfl_sync(0xffffffffu, excl, owner);
-                int o_sx = __shfl_sync(0xffffffffu, tw_sx, owner), o_sy = __shfl_sync(0xffffffffu, tw_sy, owner);
-                int o_ey = __shfl_sync(0xffffffffu, tw_ey, owner);
-                uint32_t o_pa = __shfl_sync(0xffffffffu, pa, owner);
-                int o_st = __shfl_sync(0xffffffffu, pa_st, owner);
+                const uint32_t item = f + lane;
+                f += 32;
+                const int owner = warp_owner(excl, item);
+                const uint32_t o_excl = __shfl_sync(0xffffffffu, excl, owner);
+                const int o_sx = __shfl_sync(0xffffffffu, tw_sx, owner), o_sy = __shfl_sync(0xffffffffu, tw_sy, owner);
+                const int o_ey = __shfl_sync(0xffffffffu, tw_ey, owner);
+                const uint32_t o_pa = __shfl_sync(0xffffffffu, pa, owner);
+                const int o_st = __shfl_sync(0xffffffffu, pa_st, owner);
                 bool in_hit = false, bb = false;
                 float prob = 0.f;  // fill probability of a BORDER x BORDER pair (refinement order)
                 uint32_t pb = 0;
-                if (valid) {
+                if (item < total) {
                     uint32_t r = item - o_excl;
                     int th = o_ey - o_sy + 1;
                     int u = o_sx + (int)(r / (uint32_t)th), v = o_sy + (int)(r % (uint32_t)th);
                     pb = (uint32_t)(v * T.dimx + u);
-                    int pb_st = show_status(tst[pb], cc);
+                    const uint8_t tb_st = tst[pb];
+                    int pb_st = show_status(tb_st, cc);
                     if (pb_st != 0) {
                         if (o_st == 2 || pb_st == 2) {
                             in_hit = true;
                         } else if (kMode == K_APPROX) {
-                            const double spa = S.step_x * S.step_y, tpa = T.step_x * T.step_y;
-                            const double pr = (apx_area(sst[o_pa], spa, cc) + apx_area(tst[pb], tpa, cc)) /
-                                              (spa > tpa ? spa : tpa);
+                            const double dspa = S.step_x * S.step_y, dtpa = T.step_x * T.step_y;
+                            const double pr = (apx_area(sst[o_pa], dspa, cc) + apx_area(tb_st, dtpa, cc)) /
+                                              (dspa > dtpa ? dspa : dtpa);
                             in_hit = pr > 1.0;
                             bb = true;
                         } else {
-                            const double spa = S.step_x * S.step_y, tpa = T.step_x * T.step_y;
-                            prob = (float)((apx_area(sst[o_pa], spa, cc) + apx_area(tst[pb], tpa, cc)) /
-                                           (spa > tpa ? spa : tpa));
+                            if (kMode == K_EXACT) prob = (float)(2 * sst[o_pa] - 1) * srel + (float)(2 * tb_st - 1) * trel;
                             bb = true;
                         }
                     }
@@ -211,36 +208,37 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
                     if (lane == 0) my_in++;
                     break;
                 }
-                unsigned m = __ballot_sync(0xffffffffu, bb);
+                const unsigned m = __ballot_sync(0xffffffffu, bb);
+                if (lane == 0) my_bb += __popc(m);
                 if (kMode != K_EXACT) {  // nothing to refine
-                    if (lane == 0) my_bb += __popc(m);
                     has_bb |= m != 0;
                     pair_bb += __popc(m);
-                    m = 0;
-                }
-                if (m) {
-                    int nb = __popc(m);
-                    if (qn + nb > kQueue) {
-                        __syncwarp();
-                        if (flush()) {
-                            decided = true;
-                            break;
-                        }
-                    }
+                } else {
                     if (bb) {
                         const int at = qn + __popc(m & ((1u << lane) - 1));
                         q[at] = make_uint2(o_pa, pb);
                         qk[at] = prob;
                     }
-                    qn += nb;
-                    if (lane == 0) my_bb += nb;
-                    __syncwarp();
+                    qn += __popc(m);
                 }
             }
-        }
-        if (!decided && qn > 0) {
+            if (kMode != K_EXACT || decided || qn == 0) continue;
+            // the warp refines the queued pixel pairs one after another, most
+            // probable first, and stops at the first hit; past its budget it
+            // leaves the rest to k_refine_spill, as long as the pool has room
             __syncwarp();
-            decided = flush();
+            if (qn > 1) sort_queue_desc(qk, q, qn, lane);
+            for (int k = 0; k < qn && !decided; k++) {
+                if (may_spill && spent > sp.budget) {
+                    if (spill_rest(sp, pid, q, k, qn, pp_cost, lane, &head, &spilled)) break;
+                    may_spill = false;  // the pool is full
+                }
+                const uint2 pp = q[k];
+                decided = refine_pixel_pair(sv, S, T, pp.x, pp.y, tb, my_tests);
+                spent += pp_cost;
+            }
+            qn = 0;
+            __syncwarp();
         }
         if (lane == 0) {
             if (out) out[pid] = decided ? 1 : (kMode == K_FILTER && has_bb ? 3 : 0);
@@ -252,6 +250,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
                 pv.bb[pid] = __float_as_uint(c);
             }
             my_found += decided;
+            if (spilled && decided) sp.flag[head] = 1u;  // an IN overlap met after the spill
         }
         __syncwarp();
     }
@@ -264,6 +263,31 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
         atomicAdd(&ctr->segment_tests, my_tests);
         atomicAdd(&ctr->src_window, my_ws);
         atomicAdd(&ctr->tgt_window, my_wt);
+    }
+}
+
+// The pixel pairs that k_intersect spilled, over all warps.
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 3)
+    k_refine_spill(const StoreView sv, PairView pv, SpillPool sp, uint8_t *__restrict__ out,
+                   IxCounters *__restrict__ ctr) {
+    __shared__ float4 tbufs[kWarpsPerBlock][2 * kStage];
+    float4 *tb = tbufs[threadIdx.x >> 5];
+    unsigned long long my_found = 0, my_tests = 0;
+    spill_units(
+        sp,
+        [&](unsigned long long p, uint2 pp, uint32_t part, uint32_t nparts) {
+            const PolyHdr &S = sv.hdr[pv.pairs[2 * p]];
+            const PolyHdr &T = sv.hdr[pv.tgt_base + pv.pairs[2 * p + 1]];
+            return refine_pixel_pair(sv, S, T, pp.x, pp.y, tb, my_tests, part, nparts);
+        },
+        [&](unsigned long long p) {
+            if (out) out[p] = 1;
+            my_found++;
+        });
+    for (int o = 16; o; o >>= 1) my_tests += __shfl_xor_sync(0xffffffffu, my_tests, o);
+    if ((threadIdx.x & 31) == 0) {
+        if (my_found) atomicAdd(&ctr->found, my_found);
+        if (my_tests) atomicAdd(&ctr->segment_tests, my_tests);
     }
 }
 
@@ -280,7 +304,7 @@ int intersect_filter(farm_store *s, const uint32_t *dpairs, uint64_t n, uint8_t 
     IxCounters *ctr = reinterpret_cast<IxCounters *>(next + 1);
     FARM_CUDA(cudaMemsetAsync(next, 0, 8 + sizeof(IxCounters), stream));
     PairView pv{dpairs, n, s->n_side[0], bb};
-    k_intersect<K_FILTER><<<sm_count() * 8, kWarpsPerBlock * 32, 0, stream>>>(s->view(), pv, next, dout, ctr);
+    k_intersect<K_FILTER><<<sm_count() * 8, kWarpsPerBlock * 32, 0, stream>>>(s->view(), pv, next, dout, ctr, SpillPool{});
     s->launches++;
     FARM_CUDA(cudaGetLastError());
     IxCounters h{};
@@ -311,7 +335,8 @@ static bool pair_order_on() {
 
 static int pair_order(farm_store *s, const uint32_t *dpairs, uint64_t n, const uint32_t **order) {
     *order = nullptr;
-    if (n < 2 || n > 0xFFFFFFFFull) return FARM_OK;
+    // up to a warp per pair all pairs start at once, in any order
+    if (n <= 16ull * sm_count() || n > 0xFFFFFFFFull) return FARM_OK;
     cudaStream_t stream = s->stream;
     FARM_TRY(s->s[Q_PAIR_ORDER].ensure(16 * n + 64));
     uint32_t *key = s->s[Q_PAIR_ORDER].as<uint32_t>(), *key_s = key + n, *idx = key_s + n, *idx_s = idx + n;
@@ -326,6 +351,27 @@ static int pair_order(farm_store *s, const uint32_t *dpairs, uint64_t n, const u
     FARM_CUDA(cub::DeviceRadixSort::SortPairs(s->cub_tmp.p, bytes, key, key_s, idx, idx_s, (int64_t)n, 0, 32,
                                               stream));
     *order = idx_s;
+    return FARM_OK;
+}
+
+// Blocks of the persistent pair kernels: every SM filled, or for a short list
+// one block per pair, so that its pairs spread over the SMs.
+static int query_blocks(uint64_t n) {
+    const uint64_t most = (uint64_t)sm_count() * 8;
+    return (int)(n < 1 ? 1 : (n < most ? n : most));
+}
+
+int spill_pool(farm_store *s, uint64_t n, unsigned long long *ctr, float few, float many, SpillPool *sp) {
+    const uint32_t cap = (uint32_t)(n < 4096 ? 4096 : (n > 65536 ? 65536 : n));
+    DevBuf &b = s->s[Q_SPILL];
+    FARM_TRY(b.ensure((uint64_t)cap * (kQueue * sizeof(uint2) + sizeof(SpillChunk) + 4) + 64));
+    sp->items = b.as<uint2>();
+    sp->chunk = reinterpret_cast<SpillChunk *>(sp->items + (uint64_t)cap * kQueue);
+    sp->flag = reinterpret_cast<uint32_t *>(sp->chunk + cap);
+    sp->ctr = ctr;
+    sp->cap = cap;
+    const char *v = getenv("FARM_SPILL_BUDGET");
+    sp->budget = v && *v ? (float)atof(v) : (n <= 16ull * sm_count() ? few : many);
     return FARM_OK;
 }
 
@@ -355,17 +401,28 @@ int intersect(farm_store *s, const uint32_t *pairs, uint64_t n, int mode, int me
     FARM_TRY(s->d_counters.ensure(256));
     unsigned long long *next = s->d_counters.as<unsigned long long>();
     IxCounters *ctr = reinterpret_cast<IxCounters *>(next + 1);
-    FARM_CUDA(cudaMemsetAsync(next, 0, 8 + sizeof(IxCounters), stream));
+    static_assert(8 + sizeof(IxCounters) <= 64, "the spill counters follow at [8]");
+    FARM_CUDA(cudaMemsetAsync(next, 0, 88, stream));
     PairView pv{dpairs, n, s->n_side[0]};
     StoreView sv = s->view();
+    SpillPool sp;
+    // A warp's budget per pair in segment tests. A pair kept in place ends at its
+    // first crossing, a spilled one has company; measured (512 / 4,096 / 32,768):
+    // 48 pairs 45 / 55 / 51 us, 19,375 pairs of configuration 1 589 / 344 / 600 us
+    // (a smaller pool), 150,001 heavy pairs 26.8 / 26.8 / 24.2 ms.
+    if (mode == FARM_MODE_EXACT && n) FARM_TRY(spill_pool(s, n, next + 8, 512.f, 4096.f, &sp));
     FARM_CUDA(cudaEventRecord(s->ev[6], stream));
     if (mode == FARM_MODE_EXACT && pair_order_on()) FARM_TRY(pair_order(s, dpairs, n, &pv.order));
-    int blocks = sm_count() * 8;
+    const int blocks = query_blocks(n);
     if (mode == FARM_MODE_APPROX)
-        k_intersect<K_APPROX><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(sv, pv, next, dout, ctr);
+        k_intersect<K_APPROX><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(sv, pv, next, dout, ctr, SpillPool{});
     else
-        k_intersect<K_EXACT><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(sv, pv, next, dout, ctr);
+        k_intersect<K_EXACT><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(sv, pv, next, dout, ctr, sp);
     s->launches++;
+    if (sp.cap) {
+        k_refine_spill<<<3 * sm_count(), kWarpsPerBlock * 32, 0, stream>>>(sv, pv, sp, dout, ctr);
+        s->launches++;
+    }
     FARM_CUDA(cudaGetLastError());
     FARM_CUDA(cudaEventRecord(s->ev[7], stream));
     IxCounters h{};
@@ -386,7 +443,7 @@ int intersect(farm_store *s, const uint32_t *pairs, uint64_t n, int mode, int me
         cudaEventElapsedTime(&ms, s->ev[6], s->ev[7]);
         st->ms_total = ms;
         st->ms_stage[1] = ms;
-        st->kernel_launches = 1;
+        st->kernel_launches = sp.cap ? 2 : 1;
     }
     return FARM_OK;
 }
@@ -524,7 +581,7 @@ extern "C" int farm_intersect_static(farm_store *s, const uint32_t *pairs, uint6
         if (e == cudaSuccess && n) e = cudaMemcpyAsync(dpairs, pairs, 8 * n, cudaMemcpyHostToDevice, stream);
         if (e == cudaSuccess && n) {
             PairView pv{dpairs, n, s->n_side[0]};
-            k_intersect<K_EXACT><<<sm_count() * 8, kWarpsPerBlock * 32, 0, stream>>>(s->view(), pv, next, dout, ctr);
+            k_intersect<K_EXACT><<<sm_count() * 8, kWarpsPerBlock * 32, 0, stream>>>(s->view(), pv, next, dout, ctr, SpillPool{});
             e = cudaGetLastError();
             if (e == cudaSuccess) s->launches++;
         }
