@@ -15,18 +15,26 @@
 // pixels it holds (the children of its members), so each level here keeps
 // two pixel sets instead of an explicit pair queue.
 //
-// Kernels: k_within_descend (one warp per pair) writes the finest level's
-// candidate pairs; a merge sort orders them by pair and the reference's tuple;
-// k_within_refine (one warp per pair) runs the ordered refinement, with the
-// point-segment distances of each edge-sequence pair spread over the lanes.
-#include <cub/cub.cuh>
-
+// The ordered refinement has an order-free form. Every candidate but the last
+// in order is followed by one whose lower bound is at most d, so "false" can
+// only be decided at the last candidate, after its first sequence pair: the
+// answer is "true" iff some point-segment distance of some candidate before
+// the last is below d, or one of the last candidate's first sequence pair (and
+// further ones only while no distance so far was below 100000, the minimum's
+// start value). So nothing is sorted, any warp may test any candidate, and a
+// point-segment test only has to tell whether its FP64 distance is below d,
+// which FP32 with an error bound decides for all but a few.
+//
+// Kernels: k_within (one warp per pair) descends, tests the finest level's
+// candidates a lane each, and spills what is past its budget; k_within_spill
+// tests those over all warps.
 #include <cstring>
 #include <mutex>
 #include <string>
 #include <vector>
 
 #include "common.cuh"
+#include "spill.cuh"
 
 namespace farm {
 
@@ -118,15 +126,15 @@ __device__ __forceinline__ float4 box_corners_f(const Box &a) {
     return make_float4((float)a.lo0, (float)a.lo1, (float)a.hi0, (float)a.hi1);
 }
 
-// the same from the boxes' float corners (box_corners_f) and a's lo1
+// the same from the boxes' float corners (box_corners_f) and a's lo1. Of a box
+// lo <= hi, so the largest |x difference| is one of hi - lo either way.
+__device__ __forceinline__ float2 corner_spans(const float4 &fa, const float4 &ft) {
+    return make_float2(fmaxf(__fsub_rn(fa.z, ft.x), __fsub_rn(ft.z, fa.x)),
+                       fmaxf(__fsub_rn(fa.w, ft.y), __fsub_rn(ft.w, fa.y)));
+}
 __device__ double box_max_distance_f(const float4 &fa, const float4 &ft, double a_lo1, bool geo) {
-    const float ax0 = fa.x, ax1 = fa.z, ay0 = fa.y, ay1 = fa.w;
-    const float tx0 = ft.x, tx1 = ft.z, ty0 = ft.y, ty1 = ft.w;
-    const float mx = fmaxf(fmaxf(fabsf(__fsub_rn(ax0, tx0)), fabsf(__fsub_rn(ax0, tx1))),
-                           fmaxf(fabsf(__fsub_rn(ax1, tx0)), fabsf(__fsub_rn(ax1, tx1))));
-    const float my = fmaxf(fmaxf(fabsf(__fsub_rn(ay0, ty0)), fabsf(__fsub_rn(ay0, ty1))),
-                           fmaxf(fabsf(__fsub_rn(ay1, ty0)), fabsf(__fsub_rn(ay1, ty1))));
-    double dx = mx, dy = my;
+    const float2 m = corner_spans(fa, ft);
+    double dx = m.x, dy = m.y;
     if (geo) {
         dy = dy / DEG_LAT;
         dx = dx / deg_lon(a_lo1);
@@ -134,23 +142,8 @@ __device__ double box_max_distance_f(const float4 &fa, const float4 &ft, double 
     return sqrt(dx * dx + dy * dy);
 }
 
-__device__ double box_max_distance(const Box &a, const Box &t, bool geo) {
-    const float ax0 = (float)a.lo0, ax1 = (float)a.hi0, ay0 = (float)a.lo1, ay1 = (float)a.hi1;
-    const float tx0 = (float)t.lo0, tx1 = (float)t.hi0, ty0 = (float)t.lo1, ty1 = (float)t.hi1;
-    const float mx = fmaxf(fmaxf(fabsf(__fsub_rn(ax0, tx0)), fabsf(__fsub_rn(ax0, tx1))),
-                           fmaxf(fabsf(__fsub_rn(ax1, tx0)), fabsf(__fsub_rn(ax1, tx1))));
-    const float my = fmaxf(fmaxf(fabsf(__fsub_rn(ay0, ty0)), fabsf(__fsub_rn(ay0, ty1))),
-                           fmaxf(fabsf(__fsub_rn(ay1, ty0)), fabsf(__fsub_rn(ay1, ty1))));
-    double dx = mx, dy = my;
-    if (geo) {
-        dy = dy / DEG_LAT;
-        dx = dx / deg_lon(a.lo1);
-    }
-    return sqrt(dx * dx + dy * dy);
-}
-
 // geometry_computation.h:49-89
-__device__ double pt_seg_dist(float2 p, float2 p1, float2 p2, bool geo) {
+__device__ __noinline__ double pt_seg_dist(float2 p, float2 p1, float2 p2, bool geo) {
     double A = __fsub_rn(p.x, p1.x), B = __fsub_rn(p.y, p1.y);
     double C = __fsub_rn(p2.x, p1.x), D = __fsub_rn(p2.y, p1.y);
     double dot = A * C + B * D;
@@ -176,110 +169,299 @@ __device__ double pt_seg_dist(float2 p, float2 p1, float2 p2, bool geo) {
     return sqrt(dx * dx + dy * dy);
 }
 
-// FP32 first pass of pt_seg_dist, with a bound on its distance from the FP64
-// value pt_seg_dist returns. It works relative to p1 — the reference's own
-// float differences A, B, C, D and the projection parameter clamped to
-// [0, 1] — so absolute coordinates never enter its rounding:
-//   |d32 - d64| <= 20 u32 (M + L) S + 7 u32 d32 + 8 u64 (|p| + |p1| + M + L) S
-// (taken about 3x wider below)
+// The FP32 screen of pt_seg_dist(...) < thr. It works relative to p1 (the
+// reference's own float differences A, B, C, D and the projection parameter
+// clamped to [0, 1]), so absolute coordinates never enter its rounding:
+//   |d32 - d64| <= 22 u32 (M + L) S + 7 u32 d32 + 8 u64 (|p| + |p1| + M + L) S
 // with M = |A| + |B|, L = |C| + |D|, S the geography scale (1 when planar).
-// The first term covers the FP32 dot/length/parameter/projection rounding
-// and the float roundings of the differences the reference keeps in double;
-// the second the sqrt, scaling and squares; the third the reference's own
+// The first term covers the FP32 dot / reciprocal / parameter / projection
+// rounding and the float roundings of the differences the reference keeps in
+// double; the second the scaling and squares; the third the reference's own
 // FP64 rounding (its projection is taken in absolute coordinates). The
 // distance to a segment is 1-Lipschitz in the clamped parameter times the
-// segment length, so branch flips at the clamp stay inside the bound.
-__device__ __forceinline__ float pt_seg_dist32(float2 p, float2 p1, float2 p2, bool geo, float &err) {
-    const float A = __fsub_rn(p.x, p1.x), B = __fsub_rn(p.y, p1.y);
-    const float C = __fsub_rn(p2.x, p1.x), D = __fsub_rn(p2.y, p1.y);
-    const float dot = __fadd_rn(__fmul_rn(A, C), __fmul_rn(B, D));
-    const float len = __fadd_rn(__fmul_rn(C, C), __fmul_rn(D, D));
-    float t = len != 0.f ? __fdiv_rn(dot, len) : 0.f;
-    t = fminf(fmaxf(t, 0.f), 1.f);
-    float dx = __fsub_rn(A, __fmul_rn(t, C)), dy = __fsub_rn(B, __fmul_rn(t, D));
-    float S = 1.f;
-    if (geo) {
-        float a = fabsf(p.y);
-        if (a == 90.f) a = 89.9f;
-        int idx = (int)(a * 10.f);
-        if (idx < 0 || idx >= 900) idx = 899;
-        // the table index may differ from the FP64 one at a boundary; taking
-        // the larger neighbouring scale keeps the bound valid either way
-        const float s0 = c_inv_deg_lon_f[idx];
-        const float s1 = c_inv_deg_lon_f[idx + 1 < 900 ? idx + 1 : 899];
-        const float s2 = c_inv_deg_lon_f[idx > 0 ? idx - 1 : 0];
-        const float sy = (float)(40076.0 / 360.0);
-        dx = __fmul_rn(dx, s0);
-        dy = __fmul_rn(dy, sy);
-        S = fmaxf(fmaxf(fmaxf(s0, s1), s2), sy);
-        // a neighbouring table entry changes dx's scale: widen by that difference
-        err = fabsf(__fsub_rn(A, __fmul_rn(t, C))) * fmaxf(fabsf(s1 - s0), fabsf(s2 - s0));
-    } else {
-        err = 0.f;
-    }
-    const float d = sqrtf(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)));
-    const float M = fabsf(A) + fabsf(B), L = fabsf(C) + fabsf(D);
-    const float absx = fabsf(p.x) + fabsf(p.y) + fabsf(p1.x) + fabsf(p1.y);
-    // the derivation's constants (20 u32, 7 u32, 8 u64), widened about 3x
-    err += 4e-6f * (M + L) * S + 1.2e-6f * d + 3e-15f * (absx + M + L) * S;
-    return d;
+// segment length, so branch flips at the clamp stay inside the bound. The
+// constants below are about 3x wider, as c0 (the threshold, the third term
+// over the pair's largest coordinate) and k1 (the first); the relative term
+// is in the final comparison. A test that is not clearly at or past the
+// threshold is evaluated in FP64, so the answer is pt_seg_dist's.
+struct Near {
+    double thr;
+    float c0, k1;
+};
+constexpr float kScaleGeo = 111.5f;  // no degree is longer: 40076 / 360 km
+
+__device__ __forceinline__ Near near_of(const PolyHdr &S, const PolyHdr &T, double thr, bool geo) {
+    double m = 0;
+    for (int k = 0; k < 4; k++) m = fmax(m, fmax(fabs(S.mbr[k]), fabs(T.mbr[k])));
+    const float sc = geo ? kScaleGeo : 1.f;
+    Near w;
+    // the running minimum of the reference starts at 100000: any test is below a larger threshold
+    w.thr = thr > 100000.0 ? (double)INFINITY : thr;
+    w.c0 = (float)w.thr * 1.000001f + 5e-14f * (float)m * sc;
+    w.k1 = 4e-6f * sc;
+    return w;
 }
 
-struct WCand {
-    double apx, lo, hi;
-    uint32_t pair;
-    int32_t id1, id2;
-    uint32_t pad;
-};
+// Longitude scale of a point by its latitude's table entry: x the scale, y the
+// largest step to a neighbouring entry (the index may differ from the FP64
+// one at a boundary).
+__device__ __forceinline__ float2 lon_entry(int idx) {
+    const float s0 = c_inv_deg_lon_f[idx];
+    const float s1 = c_inv_deg_lon_f[idx + 1 < 900 ? idx + 1 : 899], s2 = c_inv_deg_lon_f[idx > 0 ? idx - 1 : 0];
+    return make_float2(s0, 1.001f * fmaxf(fabsf(s1 - s0), fabsf(s2 - s0)));
+}
+__device__ __forceinline__ int lat_index(float lat) {
+    float a = fabsf(lat);
+    if (a == 90.f) a = 89.9f;
+    const int idx = (int)(a * 10.f);
+    return idx < 0 || idx >= 900 ? 899 : idx;
+}
 
-struct WCandLess {
-    __device__ bool operator()(const WCand &a, const WCand &b) const {
-        if (a.pair != b.pair) return a.pair < b.pair;
-        if (a.apx != b.apx) return a.apx < b.apx;
-        if (a.lo != b.lo) return a.lo < b.lo;
-        if (a.hi != b.hi) return a.hi < b.hi;
-        if (a.id1 != b.id1) return a.id1 < b.id1;
-        return a.id2 < b.id2;
+struct Seg {
+    float2 p1, p2;
+    float C, D, inv, L;
+};
+__device__ __forceinline__ Seg make_seg(float2 p1, float2 p2) {
+    Seg g;
+    g.p1 = p1;
+    g.p2 = p2;
+    g.C = __fsub_rn(p2.x, p1.x);
+    g.D = __fsub_rn(p2.y, p1.y);
+    const float len = __fmaf_rn(g.C, g.C, __fmul_rn(g.D, g.D));
+    g.inv = len != 0.f ? __frcp_rn(len) : 0.f;
+    g.L = fabsf(g.C) + fabsf(g.D);
+    return g;
+}
+
+template <bool kGeo>
+__device__ __forceinline__ bool near_test(float2 p, const Seg &g, const Near &w, const float2 *tab, uint32_t &rechk) {
+    const float A = __fsub_rn(p.x, g.p1.x), B = __fsub_rn(p.y, g.p1.y);
+    const float t = __saturatef(__fmul_rn(__fmaf_rn(A, g.C, __fmul_rn(B, g.D)), g.inv));
+    float dx = __fmaf_rn(-t, g.C, A), dy = __fmaf_rn(-t, g.D, B);
+    float lim = __fmaf_rn(w.k1, fabsf(A) + fabsf(B) + g.L, w.c0);
+    if (kGeo) {
+        const float2 e = tab[lat_index(p.y)];
+        lim = __fmaf_rn(fabsf(dx), e.y, lim);
+        dx = __fmul_rn(dx, e.x);
+        dy = __fmul_rn(dy, (float)(40076.0 / 360.0));
     }
+    if (__fmaf_rn(dx, dx, __fmul_rn(dy, dy)) > lim * lim * 1.00001f) return false;
+    rechk++;
+    return pt_seg_dist(p, g.p1, g.p2, kGeo) < w.thr;
+}
+
+// One side of a candidate pixel pair: its pixel's edge sequences.
+struct SeqSet {
+    const uint2 *seq;
+    const float2 *ring;
+    uint32_t a, b;  // sequences [a, b)
+};
+__device__ __forceinline__ SeqSet seq_set(const StoreView &sv, const PolyHdr &h, uint32_t id) {
+    const uint32_t *o = sv.offset + h.off;
+    return {sv.seq + h.seq, sv.ring + h.ring, o[id], o[id + 1]};
+}
+
+// Sequences of fewer than 2 points are skipped, and a sequence (start, len)
+// reads points [start, start + len) and the len - 1 segments between them
+// (segment_to_segment_within_batch). Over all sequence pairs of a pixel pair
+// that is every point of one side against every segment of the other.
+template <bool kGeo>
+__device__ bool points_near_segments(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
+                                     uint32_t &rechk) {
+    for (uint32_t i = G.a; i < G.b; i++) {
+        const uint2 e = G.seq[i];
+        if (e.y < 2) continue;
+        float2 p1 = G.ring[e.x];
+        for (uint32_t k = 1; k < e.y; k++) {
+            const float2 p2 = G.ring[e.x + k];
+            const Seg g = make_seg(p1, p2);
+            for (uint32_t j = P.a; j < P.b; j++) {
+                const uint2 f = P.seq[j];
+                if (f.y < 2) continue;
+                for (uint32_t q = 0; q < f.y; q++)
+                    if (near_test<kGeo>(P.ring[f.x + q], g, w, tab, rechk)) return true;
+            }
+            p1 = p2;
+        }
+    }
+    return false;
+}
+
+// The same with the warp on one pixel pair: segments over the lanes, points read by all.
+template <bool kGeo>
+__device__ bool points_near_segments_warp(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
+                                          int lane, uint32_t &rechk) {
+    const unsigned full = 0xffffffffu;
+    for (uint32_t i0 = G.a; i0 < G.b; i0 += 32) {
+        const uint2 e = i0 + lane < G.b ? G.seq[i0 + lane] : make_uint2(0u, 0u);
+        const uint32_t mine = e.y >= 2 ? e.y - 1 : 0u;
+        uint32_t incl = mine;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(full, incl, o);
+            if (lane >= o) incl += u;
+        }
+        const uint32_t total = __shfl_sync(full, incl, 31), excl = incl - mine;
+        for (uint32_t s0 = 0; s0 < total; s0 += 32) {
+            const uint32_t s = s0 + lane;
+            int owner = 0;
+            for (int b = 16; b; b >>= 1)
+                if (__shfl_sync(full, excl, owner + b) <= s) owner += b;
+            const uint32_t start = __shfl_sync(full, e.x, owner), ex = __shfl_sync(full, excl, owner);
+            const bool valid = s < total;
+            Seg g{};
+            if (valid) g = make_seg(G.ring[start + (s - ex)], G.ring[start + (s - ex) + 1]);
+            for (uint32_t j = P.a; j < P.b; j++) {
+                const uint2 f = P.seq[j];
+                if (f.y < 2) continue;
+                bool hit = false;
+                for (uint32_t q = 0; q < f.y && !hit; q++) {
+                    const float2 p = P.ring[f.x + q];
+                    if (valid) hit = near_test<kGeo>(p, g, w, tab, rechk);
+                }
+                if (__any_sync(full, hit)) return true;
+            }
+        }
+    }
+    return false;
+}
+
+// Point-segment tests a lane takes on a candidate by itself; a larger one gets the warp.
+constexpr uint32_t kLaneTests = 1024;
+
+struct WithinTally {
+    unsigned long long cand = 0, box = 0, tests = 0, rechk = 0, seqp = 0;
 };
 
-// out codes of the descent: 0 / 1 decided, 4 refine candidates, 2 polygon
-// failed rasterization, 3 did not fit the candidate buffer (retried)
-enum : uint8_t { W_FALSE = 0, W_TRUE = 1, W_BADPOLY = 2, W_RETRY = 3, W_REFINE = 4 };
+// Candidates (one per lane, valid lanes) against the threshold: the mask of
+// lanes whose pixel pair holds a point-segment distance below it.
+__device__ unsigned test_candidates(const StoreView &sv, const PolyHdr &S, const PolyHdr &T, bool valid, uint32_t id1,
+                                    uint32_t id2, const Near &w, bool geo, const float2 *tab, int lane,
+                                    WithinTally &my) {
+    const unsigned full = 0xffffffffu;
+    SeqSet A{}, B{};
+    uint32_t tests = 0, rechk = 0;
+    if (valid) {
+        A = seq_set(sv, S, id1);
+        B = seq_set(sv, T, id2);
+        uint32_t pa = 0, ga = 0, pb = 0, gb = 0;
+        for (uint32_t i = A.a; i < A.b; i++) {
+            const uint32_t y = A.seq[i].y;
+            if (y >= 2) pa += y, ga += y - 1;
+        }
+        for (uint32_t i = B.a; i < B.b; i++) {
+            const uint32_t y = B.seq[i].y;
+            if (y >= 2) pb += y, gb += y - 1;
+        }
+        tests = pa * gb + pb * ga;
+        my.tests += tests;
+        my.seqp += (unsigned long long)(A.b - A.a) * (B.b - B.a);
+    }
+    bool hit = false;
+    if (tests && tests <= kLaneTests) {
+        hit = geo ? points_near_segments<true>(B, A, w, tab, rechk) || points_near_segments<true>(A, B, w, tab, rechk)
+                  : points_near_segments<false>(B, A, w, tab, rechk) ||
+                        points_near_segments<false>(A, B, w, tab, rechk);
+    }
+    __syncwarp();
+    unsigned hits = __ballot_sync(full, hit);
+    for (unsigned m = __ballot_sync(full, tests > kLaneTests); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const SeqSet a = seq_set(sv, S, __shfl_sync(full, id1, src)), b = seq_set(sv, T, __shfl_sync(full, id2, src));
+        const bool h = geo ? points_near_segments_warp<true>(b, a, w, tab, lane, rechk) ||
+                                 points_near_segments_warp<true>(a, b, w, tab, lane, rechk)
+                           : points_near_segments_warp<false>(b, a, w, tab, lane, rechk) ||
+                                 points_near_segments_warp<false>(a, b, w, tab, lane, rechk);
+        if (h) hits |= 1u << src;
+    }
+    my.rechk += rechk;
+    return hits;
+}
+
+enum : uint8_t { W_FALSE = 0, W_TRUE = 1, W_BADPOLY = 2 };
 
 struct WithinArgs {
     const uint32_t *pairs;
     uint64_t n;
     uint64_t tgt_base;
     double thr;
-    int geo;
+    bool geo, approx;
     uint32_t cap_pix;  // per-side pixel capacity of a warp's scratch
-    uint32_t *scratch; // per warp: 2 sides x (bitmap words + 2 lists)
+    uint32_t *scratch; // per warp (within_scratch_words)
     uint64_t scratch_words;
-    WCand *cand;
-    unsigned long long *ncand;
-    uint64_t cand_cap;
     uint8_t *out;
     unsigned long long *next;
-    unsigned long long *stats;  // candidates, box pairs
+    unsigned long long *stats;  // candidates, box pairs, tests, FP64 tests, sequence pairs
+    SpillPool sp;
 };
+
+// A layer of a polygon's hierarchy (layer_geom), the parts the descent reads.
+struct Layer {
+    double mbr[2], step_x, step_y;
+    int32_t dimx, dimy;
+    uint32_t offset, pad;
+};
+constexpr int kMaxLayers = 32;
+
+// All layers of a polygon into L, a lane each: every layer's box and dims come
+// from the finest raster directly (its step is the finest one doubled, which
+// is exact), and its status offset is the finer layers' sizes added up.
+__device__ void load_layers(const PolyHdr &h, Layer *L, int lane) {
+    const unsigned full = 0xffffffffu;
+    const int nl = (int)h.num_layers, up = nl - 1 - lane;
+    Layer g{};
+    uint32_t size = 0;
+    if (up == 0) {
+        g.mbr[0] = h.mbr[0];
+        g.mbr[1] = h.mbr[1];
+        g.step_x = h.step_x;
+        g.step_y = h.step_y;
+        g.dimx = h.dimx;
+        g.dimy = h.dimy;
+    } else if (up > 0) {
+        g.step_x = ldexp(h.step_x, up);
+        g.step_y = ldexp(h.step_y, up);
+        g.mbr[0] = floor(h.mbr[0] / g.step_x) * g.step_x;
+        g.mbr[1] = floor(h.mbr[1] / g.step_y) * g.step_y;
+        const double hx = ceil(h.mbr[2] / g.step_x) * g.step_x, hy = ceil(h.mbr[3] / g.step_y) * g.step_y;
+        g.dimx = (int)round((hx - g.mbr[0]) / g.step_x);
+        g.dimy = (int)round((hy - g.mbr[1]) / g.step_y);
+        size = (uint32_t)(g.dimx * g.dimy);
+    }
+    uint32_t incl = size;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(full, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (up > 0) g.offset = h.P + (__shfl_sync(full, incl, 31) - incl);
+    else __shfl_sync(full, incl, 31);
+    if (lane < nl) L[lane] = g;
+}
+
+__device__ __forceinline__ Box layer_box(const Layer &g, int id) {
+    const int x = id % g.dimx, y = id / g.dimx;
+    Box b;
+    b.lo0 = g.mbr[0] + x * g.step_x;
+    b.lo1 = g.mbr[1] + y * g.step_y;
+    b.hi0 = g.mbr[0] + (x + 1) * g.step_x;
+    b.hi1 = g.mbr[1] + (y + 1) * g.step_y;
+    return b;
+}
 
 struct SideScratch {
     uint32_t *bits;  // cap_pix/32 + 1 words
     uint32_t *q;     // current queued set
     uint32_t *p;     // next level set
-    Box *box;        // the boxes of the pixels in p, and their corners as floats
-    float4 *fbox;    // (lo0, lo1, hi0, hi1)
+    float4 *fbox;    // float corners (lo0, lo1, hi0, hi1) of the pixels in p
+    float *lon;      // geography, source side: longitude scale at lo1
 };
 
-// u32 words of one warp's scratch: per side the boxes (8 words each) and
-// float corners (4) of up to cap pixels, then per side a bitmap and two lists
+// u32 words of one warp's scratch: per side the float corners (4 words each)
+// of up to cap pixels, the source side's scales, per side a bitmap and two lists
 __host__ __device__ inline uint64_t within_scratch_words(uint32_t cap) {
-    const uint64_t w = 24ull * cap + 2 * (((uint64_t)cap >> 5) + 1 + 2ull * cap);
+    const uint64_t w = 9ull * cap + 2 * (((uint64_t)cap >> 5) + 1 + 2ull * cap);
     return (w + 3) & ~3ull;
 }
 
-// set bit, return whether newly set
 __device__ __forceinline__ void set_bit(uint32_t *bits, uint32_t id) { atomicOr(&bits[id >> 5], 1u << (id & 31)); }
 
 // Compact the set bits of [0, nbits) into list (ascending) and clear them.
@@ -308,20 +490,16 @@ __device__ uint32_t compact_bits(uint32_t *bits, uint32_t nbits, uint32_t *list,
     return total;
 }
 
-// Children of the queued pixels at layer `li` (their box at the coarser
-// layer, shrunk by 1e-6, then retrieve_pixels' own 1e-6) or the queued pixels
+// Children of the queued pixels at layer g (their box at the coarser layer pg,
+// shrunk by 1e-6, then retrieve_pixels' own 1e-6) or the queued pixels
 // themselves; BORDER ones only (Ideal.cpp:2513-2551).
-__device__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, bool advance, uint32_t li, const uint32_t *q,
-                             uint32_t nq, SideScratch &sc, int lane, int cc) {
-    LayerGeom g;
-    layer_geom(h, li, g);
-    LayerGeom pg;
-    if (advance) layer_geom(h, li - 1, pg);
+__device__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, const Layer &g, const Layer *pg, uint32_t nq,
+                             SideScratch &sc, int lane, int cc) {
     const uint8_t *st = status + h.st + g.offset;
     for (uint32_t k = lane; k < nq; k += 32) {
-        uint32_t id = q[k];
-        if (advance) {
-            Box b = pixel_box(pg, (int)id);
+        uint32_t id = sc.q[k];
+        if (pg) {
+            Box b = layer_box(*pg, (int)id);
             b.lo0 += 1e-6;
             b.lo1 += 1e-6;
             b.hi0 -= 1e-6;
@@ -343,56 +521,172 @@ __device__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, bool advan
     return compact_bits(sc.bits, (uint32_t)(g.dimx * g.dimy), sc.p, lane);
 }
 
-__global__ void __launch_bounds__(256) k_within_descend(const StoreView sv, WithinArgs a) {
-    const int lane = threadIdx.x & 31;
+// f(k1, k2, valid) over [0, ns) x [0, nt), all lanes at a time, until it
+// returns true (warp-uniform). The longer list runs over the lanes; two short
+// ones are flattened.
+template <typename F>
+__device__ __forceinline__ bool for_product(uint32_t ns, uint32_t nt, int lane, F f) {
+    if (nt >= ns && nt >= 24) {
+        for (uint32_t a = 0; a < ns; a++)
+            for (uint32_t b = 0; b < nt; b += 32)
+                if (f(a, b + lane, b + lane < nt)) return true;
+    } else if (ns >= 24) {
+        for (uint32_t b = 0; b < nt; b++)
+            for (uint32_t a = 0; a < ns; a += 32)
+                if (f(a + lane, b, a + lane < ns)) return true;
+    } else {
+        for (uint32_t k0 = 0; k0 < ns * nt; k0 += 32) {
+            const uint32_t k = k0 + lane;
+            if (f(k / nt, k % nt, k < ns * nt)) return true;
+        }
+    }
+    return false;
+}
+
+// FP32 view of one level's box pairs. Float corners are off by half an ulp of
+// the coordinate, so a box distance computed from them is off by at most
+// slack(k1) plus 4e-6 of itself; max-distances use the reference's own float
+// corners and are off by 4e-6 of themselves (scales and squares).
+struct Level {
+    float ex, ey;  // coordinate roundings, x and y
+    bool geo;
+    const float *lon;
+    __device__ __forceinline__ float sx(uint32_t k1) const { return geo ? lon[k1] : 1.f; }
+    __device__ __forceinline__ float sy() const { return geo ? (float)(40076.0 / 360.0) : 1.f; }
+    __device__ __forceinline__ float slack(float sx_) const { return 1.5f * (ex * sx_ + ey * sy()); }
+    __device__ __forceinline__ float dist(const float4 &a, const float4 &t, float sx_) const {
+        const float dx = fmaxf(0.f, fmaxf(t.x - a.z, a.x - t.z)) * sx_;
+        const float dy = fmaxf(0.f, fmaxf(t.y - a.w, a.y - t.w)) * sy();
+        return sqrtf(__fmaf_rn(dx, dx, dy * dy));
+    }
+    __device__ __forceinline__ float max2(const float4 &a, const float4 &t, float sx_) const {
+        const float2 m = corner_spans(a, t);
+        const float dx = m.x * sx_, dy = m.y * sy();
+        return __fmaf_rn(dx, dx, dy * dy);
+    }
+    // below every value the distance can have
+    __device__ __forceinline__ float low(float d, float sx_) const { return d * (1.f - 4e-6f) - slack(sx_); }
+    __device__ __forceinline__ float high(float d, float sx_) const { return d * (1.f + 4e-6f) + slack(sx_); }
+};
+
+__device__ __forceinline__ float warp_min(float v) {
+    for (int o = 16; o; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Keep the pixels of a side whose box may lie within `cut` of box bb.
+__device__ uint32_t prune_side(SideScratch &sc, uint32_t n, const float4 &bb, const Level &lv, bool source,
+                               float sx_low, float cut, int lane) {
+    uint32_t at = 0;
+    for (uint32_t b = 0; b < n; b += 32) {
+        const uint32_t k = b + lane;
+        bool keep = false;
+        uint32_t id = 0;
+        float4 fb = make_float4(0, 0, 0, 0);
+        float lo = 0;
+        if (k < n) {
+            id = sc.p[k];
+            fb = sc.fbox[k];
+            if (source && lv.geo) lo = sc.lon[k];
+            const float sx_ = source ? (lv.geo ? lo : 1.f) : sx_low;
+            keep = !(lv.low(lv.dist(fb, bb, sx_), source ? sx_ : (lv.geo ? kScaleGeo : 1.f)) > cut);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+            const uint32_t w = at + __popc(m & ((1u << lane) - 1));
+            sc.p[w] = id;
+            sc.fbox[w] = fb;
+            if (source && lv.geo) sc.lon[w] = lo;
+        }
+        at += __popc(m);
+        __syncwarp();
+    }
+    return at;
+}
+
+// The reference's order of candidates (Ideal.cpp:2612).
+struct CandKey {
+    double apx, lo, hi;
+    int32_t id1, id2;
+};
+__device__ __forceinline__ bool key_less(const CandKey &a, const CandKey &b) {
+    if (a.apx != b.apx) return a.apx < b.apx;
+    if (a.lo != b.lo) return a.lo < b.lo;
+    if (a.hi != b.hi) return a.hi < b.hi;
+    if (a.id1 != b.id1) return a.id1 < b.id1;
+    return a.id2 < b.id2;
+}
+
+// resident blocks of k_within per SM (its grid, and so its scratch)
+constexpr int kWithinBlocks = 2;
+// box pairs of a level above which its pixel sets are pruned first
+constexpr uint32_t kPrunePairs = 256;
+
+// One warp per pair.
+//
+// Descent: what bounds it is the FP64 pipe (2 lanes per clock per SM against
+// 128 for FP32), so the box distances of a level are screened in FP32 with
+// error bounds, and the reference's FP64 expressions decide only what the
+// screen leaves open: the smallest max-distance among the pairs within 1e-5
+// of the FP32 smallest, and the kept pairs within the rounding of the cut. A
+// large level first drops pixels that lie farther from the other polygon's
+// box than a max-distance already found: they can be in neither the smallest
+// max-distance nor a kept pair.
+//
+// Refinement: a lane per candidate (they have 28 point-segment tests on
+// average in configuration 3, far too few for a warp each), first the closest
+// one each lane met, then all, up to the budget; the rest is spilled.
+//
+// 60,001 pairs of configuration 3: 794 ms refinement and 55 ms descent with an
+// ordered refinement, a warp per pair.
+__global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView sv, WithinArgs a) {
+    __shared__ uint2 queue[8][kQueue];
+    __shared__ Layer layers[8][2][kMaxLayers];
+    __shared__ float2 tab[900];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int cc = sv.category_count;
-    const bool geo = a.geo != 0;
+    const bool geo = a.geo;
+    uint2 *q = queue[wib];
+    Layer *LS = layers[wib][0], *LT = layers[wib][1];
+    if (geo)
+        for (int k = threadIdx.x; k < 900; k += blockDim.x) tab[k] = lon_entry(k);
+    const uint32_t cap = a.cap_pix, bw = (cap >> 5) + 1;
     uint32_t *wbase = a.scratch + warp * a.scratch_words;
-    const uint32_t cap = a.cap_pix;
-    Box *boxes = reinterpret_cast<Box *>(wbase);
-    float4 *fboxes = reinterpret_cast<float4 *>(wbase + 16ull * cap);
-    uint32_t *base = wbase + 24ull * cap;
-    const uint32_t bw = (cap >> 5) + 1;
-    SideScratch ss{base, base + bw, base + bw + cap, boxes, fboxes};
-    SideScratch ts{base + bw + 2 * cap, base + 2 * bw + 2 * cap, base + 2 * bw + 3 * cap, boxes + cap, fboxes + cap};
-    unsigned long long my_cand = 0, my_box = 0;
+    float4 *fboxes = reinterpret_cast<float4 *>(wbase);
+    uint32_t *base = wbase + 9ull * cap;
+    SideScratch ss{base, base + bw, base + bw + cap, fboxes, reinterpret_cast<float *>(wbase + 8ull * cap)};
+    SideScratch ts{base + bw + 2 * cap, base + 2 * bw + 2 * cap, base + 2 * bw + 3 * cap, fboxes + cap, nullptr};
+    for (uint32_t w = lane; w < bw; w += 32) ss.bits[w] = ts.bits[w] = 0u;
+    __syncthreads();
+    WithinTally my;
     for (;;) {
         unsigned long long pid = 0;
         if (lane == 0) pid = atomicAdd(a.next, 1ull);
-        pid = __shfl_sync(0xffffffffu, pid, 0);
+        pid = __shfl_sync(full, pid, 0);
         if (pid >= a.n) break;
-        const uint32_t s = a.pairs[2 * pid], t = a.pairs[2 * pid + 1];
-        const PolyHdr &S = sv.hdr[s];
-        const PolyHdr &T = sv.hdr[a.tgt_base + t];
+        const PolyHdr &S = sv.hdr[a.pairs[2 * pid]];
+        const PolyHdr &T = sv.hdr[a.tgt_base + a.pairs[2 * pid + 1]];
         if (S.err || T.err) {
             if (lane == 0) a.out[pid] = W_BADPOLY;
             continue;
         }
-        if (S.num_layers == 0 || T.num_layers == 0) {
-            if (lane == 0) a.out[pid] = W_RETRY;
-            continue;
-        }
+        __syncwarp();
+        load_layers(S, LS, lane);
+        load_layers(T, LT, lane);
+        __syncwarp();
         const uint32_t sL = S.num_layers - 1, tL = T.num_layers - 1;
         // initial queue: every layer-0 pixel pair (Ideal.cpp:2483-2488)
-        uint32_t nqs, nqt;
-        {
-            LayerGeom g0;
-            layer_geom(S, 0, g0);
-            nqs = (uint32_t)(g0.dimx * g0.dimy);
-            for (uint32_t k = lane; k < nqs; k += 32) ss.q[k] = k;
-            layer_geom(T, 0, g0);
-            nqt = (uint32_t)(g0.dimx * g0.dimy);
-            for (uint32_t k = lane; k < nqt; k += 32) ts.q[k] = k;
-            __syncwarp();
-        }
+        uint32_t nqs = (uint32_t)(LS[0].dimx * LS[0].dimy), nqt = (uint32_t)(LT[0].dimx * LT[0].dimy);
+        for (uint32_t k = lane; k < nqs; k += 32) ss.q[k] = k;
+        for (uint32_t k = lane; k < nqt; k += 32) ts.q[k] = k;
+        __syncwarp();
         uint32_t i = 0, j = 0;
-        uint8_t result = W_FALSE;
+        bool yes = false, spilled = false;
+        uint32_t head = 0;
         for (;;) {
-            LayerGeom gs, gt;
-            layer_geom(S, i, gs);
-            layer_geom(T, j, gt);
-            const double s_step = gs.step_x, t_step = gt.step_x;
+            const double s_step = LS[i].step_x, t_step = LT[j].step_x;
             bool s_next = false, t_next = false;
             if (i < sL && (s_step >= t_step || j >= tL)) {
                 i++;
@@ -403,106 +697,326 @@ __global__ void __launch_bounds__(256) k_within_descend(const StoreView sv, With
                 t_next = true;
             }
             if (nqs == 0 || nqt == 0) break;  // empty queue
-            uint32_t np_s = next_set(S, sv.status, s_next, i, ss.q, nqs, ss, lane, cc);
-            uint32_t np_t = next_set(T, sv.status, t_next, j, ts.q, nqt, ts, lane, cc);
-            layer_geom(S, i, gs);
-            layer_geom(T, j, gt);
-            // each pixel's box and float corners once per level, for all the
-            // box pairs it is in (the same values as computed per pair)
-            for (uint32_t k = lane; k < np_s; k += 32) {
-                const Box b = pixel_box(gs, (int)ss.p[k]);
-                ss.box[k] = b;
+            const Layer &gs = LS[i], &gt = LT[j];
+            uint32_t ns = next_set(S, sv.status, gs, s_next ? &LS[i - 1] : nullptr, nqs, ss, lane, cc);
+            uint32_t nt = next_set(T, sv.status, gt, t_next ? &LT[j - 1] : nullptr, nqt, ts, lane, cc);
+            if (ns == 0 || nt == 0) break;
+            if (lane == 0) my.box += (uint64_t)ns * nt;
+            for (uint32_t k = lane; k < ns; k += 32) {
+                const Box b = layer_box(gs, (int)ss.p[k]);
                 ss.fbox[k] = box_corners_f(b);
-            }
-            for (uint32_t k = lane; k < np_t; k += 32) {
-                const Box b = pixel_box(gt, (int)ts.p[k]);
-                ts.box[k] = b;
-                ts.fbox[k] = box_corners_f(b);
-            }
-            __syncwarp();
-            // smallest box max-distance; any <= d decides (Ideal.cpp:2557-2570)
-            const uint64_t tot = (uint64_t)np_s * np_t;
-            double mbd = 100000.0;
-            bool hit = false;
-            for (uint64_t k = lane; k < tot; k += 32) {
-                const uint32_t k1 = (uint32_t)(k / np_t), k2 = (uint32_t)(k % np_t);
-                double md = box_max_distance_f(ss.fbox[k1], ts.fbox[k2], ss.box[k1].lo1, geo);
-                if (md <= a.thr) {
-                    hit = true;
-                    break;
+                if (geo) {
+                    double l = fabs(b.lo1);
+                    if (l == 90) l = 89.9;
+                    const int idx = (int)(l * 10);
+                    ss.lon[k] = c_inv_deg_lon_f[idx < 0 || idx >= 900 ? 899 : idx];
                 }
-                mbd = mbd < md ? mbd : md;
             }
-            if (lane == 0) my_box += tot;
-            if (__any_sync(0xffffffffu, hit)) {
-                result = W_TRUE;
+            for (uint32_t k = lane; k < nt; k += 32) ts.fbox[k] = box_corners_f(layer_box(gt, (int)ts.p[k]));
+            __syncwarp();
+            const float4 sbb = make_float4((float)gs.mbr[0], (float)gs.mbr[1], (float)(gs.mbr[0] + gs.dimx * gs.step_x),
+                                           (float)(gs.mbr[1] + gs.dimy * gs.step_y));
+            const float4 tbb = make_float4((float)gt.mbr[0], (float)gt.mbr[1], (float)(gt.mbr[0] + gt.dimx * gt.step_x),
+                                           (float)(gt.mbr[1] + gt.dimy * gt.step_y));
+            Level lv;
+            lv.ex = 2.4e-7f * (fmaxf(fabsf(sbb.x), fabsf(sbb.z)) + fmaxf(fabsf(tbb.x), fabsf(tbb.z)));
+            lv.ey = 2.4e-7f * (fmaxf(fabsf(sbb.y), fabsf(sbb.w)) + fmaxf(fabsf(tbb.y), fabsf(tbb.w)));
+            lv.geo = geo;
+            lv.lon = ss.lon;
+            float sx_low = 1.f;  // the smallest longitude scale of the source pixels
+            if (geo) {
+                sx_low = INFINITY;
+                for (uint32_t k = lane; k < ns; k += 32) sx_low = fminf(sx_low, ss.lon[k]);
+                sx_low = warp_min(sx_low);
+            }
+            const bool large = (uint64_t)ns * nt > kPrunePairs;
+            if (large) {
+                // the source pixel nearest T's box and the target pixel nearest
+                // S's: the smallest max-distance of either is a first cut
+                float best = INFINITY;
+                uint32_t bk = 0;
+                for (uint32_t k = lane; k < ns; k += 32) {
+                    const float d = lv.dist(ss.fbox[k], tbb, lv.sx(k));
+                    if (d < best) best = d, bk = k;
+                }
+                float w = warp_min(best);
+                bk = __shfl_sync(full, bk, __ffs(__ballot_sync(full, best == w)) - 1);
+                const float4 near_s = ss.fbox[bk];
+                const float near_sx = lv.sx(bk);
+                best = INFINITY;
+                bk = 0;
+                for (uint32_t k = lane; k < nt; k += 32) {
+                    const float d = lv.dist(ts.fbox[k], sbb, sx_low);
+                    if (d < best) best = d, bk = k;
+                }
+                w = warp_min(best);
+                bk = __shfl_sync(full, bk, __ffs(__ballot_sync(full, best == w)) - 1);
+                const float4 near_t = ts.fbox[bk];
+                float ub2 = INFINITY;
+                for (uint32_t k = lane; k < nt; k += 32) ub2 = fminf(ub2, lv.max2(near_s, ts.fbox[k], near_sx));
+                for (uint32_t k = lane; k < ns; k += 32) ub2 = fminf(ub2, lv.max2(ss.fbox[k], near_t, lv.sx(k)));
+                const float cut = sqrtf(warp_min(ub2)) * 1.00001f;
+                ns = prune_side(ss, ns, tbb, lv, true, sx_low, cut, lane);
+                nt = prune_side(ts, nt, sbb, lv, false, sx_low, cut, lane);
+            }
+            // smallest box max-distance; any <= d decides (Ideal.cpp:2557-2570)
+            float m2 = INFINITY;
+            for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                if (v) m2 = fminf(m2, lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)));
+                return false;
+            });
+            m2 = warp_min(m2);
+            if (sqrtf(m2) * 1.00001f < (float)a.thr * 0.999999f) {
+                yes = true;
                 break;
             }
+            const float m2_lim = m2 * 1.00002f;
+            double mbd = INFINITY;
+            for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                if (v && !(lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)) > m2_lim)) {
+                    const double lo1 = gs.mbr[1] + (int)(ss.p[k1] / (uint32_t)gs.dimx) * gs.step_y;
+                    const double md = box_max_distance_f(ss.fbox[k1], ts.fbox[k2], lo1, geo);
+                    mbd = md < mbd ? md : mbd;
+                }
+                return false;
+            });
             for (int o = 16; o; o >>= 1) {
-                double v = __shfl_xor_sync(0xffffffffu, mbd, o);
+                const double v = __shfl_xor_sync(full, mbd, o);
                 mbd = mbd < v ? mbd : v;
             }
-            const bool last = !s_next && !t_next;
-            // keep pairs with box distance <= d and < the smallest max-distance
-            bool overflow = false;
-            unsigned long long nc = 0;
-            for (uint64_t k0 = 0; k0 < tot; k0 += 32) {
-                uint64_t k = k0 + lane;
-                bool keep = false;
-                uint32_t id1 = 0, id2 = 0;
-                Box b1, b2;
-                double lo = 0;
-                if (k < tot) {
-                    const uint32_t k1 = (uint32_t)(k / np_t), k2 = (uint32_t)(k % np_t);
-                    id1 = ss.p[k1];
-                    id2 = ts.p[k2];
-                    b1 = ss.box[k1];
-                    b2 = ts.box[k2];
-                    lo = box_distance(b1, b2, geo);
-                    keep = !(lo > a.thr) && lo < mbd;
-                }
-                if (!last) {
-                    if (keep) {
-                        set_bit(ss.bits, id1);
-                        set_bit(ts.bits, id2);
-                    }
-                    continue;
-                }
-                unsigned m = __ballot_sync(0xffffffffu, keep);
-                if (!m) continue;
-                unsigned long long at = 0;
-                if (lane == 0) at = atomicAdd(a.ncand, (unsigned long long)__popc(m));
-                at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1));
-                nc += __popc(m);
-                if (keep) {
-                    if (at < a.cand_cap) {
-                        // Ideal.cpp:2587-2606
-                        double hi = box_max_distance(b1, b2, geo);
-                        int pf = classify(sv.areas[S.pix + id1] + sv.areas[T.pix + id2],
-                                          S.step_x * S.step_y + T.step_x * T.step_y, 20);
-                        WCand c;
-                        c.apx = lo + (double)c_mean20[pf] * (hi - lo);
-                        c.lo = lo;
-                        c.hi = hi;
-                        c.pair = (uint32_t)pid;
-                        c.id1 = (int32_t)id1;
-                        c.id2 = (int32_t)id2;
-                        c.pad = 0;
-                        a.cand[at] = c;
-                    } else {
-                        overflow = true;
-                    }
-                }
-            }
-            if (last) {
-                overflow = __any_sync(0xffffffffu, overflow);
-                result = overflow ? W_RETRY : (nc ? W_REFINE : W_FALSE);
-                if (lane == 0) my_cand += nc;
+            if (mbd <= a.thr) {
+                yes = true;
                 break;
             }
-            __syncwarp();
-            nqs = compact_bits(ss.bits, (uint32_t)(gs.dimx * gs.dimy), ss.q, lane);
-            nqt = compact_bits(ts.bits, (uint32_t)(gt.dimx * gt.dimy), ts.q, lane);
+            mbd = mbd < 100000.0 ? mbd : 100000.0;  // the reference's start value
+            // keep pairs with box distance <= d and < the smallest max-distance
+            const float lim = (float)(a.thr < mbd ? a.thr : mbd);
+            const float lim_up = lim * 1.000001f, lim_dn = lim * 0.999999f;
+            if (large && (uint64_t)ns * nt > kPrunePairs) {
+                ns = prune_side(ss, ns, tbb, lv, true, sx_low, lim_up, lane);
+                nt = prune_side(ts, nt, sbb, lv, false, sx_low, lim_up, lane);
+            }
+            auto exact_lo = [&](uint32_t k1, uint32_t k2) {
+                return box_distance(layer_box(gs, (int)ss.p[k1]), layer_box(gt, (int)ts.p[k2]), geo);
+            };
+            auto keep_pair = [&](uint32_t k1, uint32_t k2, float &d) {
+                const float sx_ = lv.sx(k1);
+                d = lv.dist(ss.fbox[k1], ts.fbox[k2], sx_);
+                if (lv.low(d, sx_) > lim_up) return false;
+                if (lv.high(d, sx_) < lim_dn) return true;
+                const double lo = exact_lo(k1, k2);
+                return !(lo > a.thr) && lo < mbd;
+            };
+            if (s_next || t_next) {
+                for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                    float d;
+                    if (v && keep_pair(k1, k2, d)) {
+                        set_bit(ss.bits, ss.p[k1]);
+                        set_bit(ts.bits, ts.p[k2]);
+                    }
+                    return false;
+                });
+                __syncwarp();
+                nqs = compact_bits(ss.bits, (uint32_t)(gs.dimx * gs.dimy), ss.q, lane);
+                nqt = compact_bits(ts.bits, (uint32_t)(gt.dimx * gt.dimy), ts.q, lane);
+                continue;
+            }
+            // ---- the finest level: its kept pairs are the candidates
+            auto max_d = [&](uint32_t k1, uint32_t k2) {
+                const double lo1 = gs.mbr[1] + (int)(ss.p[k1] / (uint32_t)gs.dimx) * gs.step_y;
+                return box_max_distance_f(ss.fbox[k1], ts.fbox[k2], lo1, geo);
+            };
+            if (a.approx) {
+                // Within "-a" (query_within_polygon.cu:332-375): a pair left
+                // undecided is within when one of its surviving finest pixel
+                // pairs has apxDist = minDist + mean (maxDist - minDist) <= the
+                // distance, in float. mean is (1.0 - pf / category_count) * 0.5
+                // with both operands 8-bit integers (:352), so the quotient is 0
+                // and mean is 0.5; 0.5 (max - min) is exact in float, so
+                // contracting the sum into an FMA rounds the same.
+                unsigned nc = 0;
+                yes = for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                    float d;
+                    bool h = false;
+                    if (v && keep_pair(k1, k2, d)) {
+                        const float lo = (float)exact_lo(k1, k2), hi = (float)max_d(k1, k2);
+                        h = (double)(lo + 0.5f * (hi - lo)) <= a.thr;
+                        nc++;
+                    }
+                    return __any_sync(full, h) != 0;
+                });
+                my.cand += nc;
+                break;
+            }
+            const Near w = near_of(S, T, a.thr, geo);
+            auto cand_key = [&](uint32_t k1, uint32_t k2) {  // Ideal.cpp:2587-2606
+                CandKey c;
+                c.id1 = (int32_t)ss.p[k1];
+                c.id2 = (int32_t)ts.p[k2];
+                c.lo = exact_lo(k1, k2);
+                c.hi = max_d(k1, k2);
+                const int pf = classify(sv.areas[S.pix + c.id1] + sv.areas[T.pix + c.id2],
+                                        S.step_x * S.step_y + T.step_x * T.step_y, 20);
+                c.apx = c.lo + (double)c_mean20[pf] * (c.hi - c.lo);
+                return c;
+            };
+            // the candidates counted, and the closest one each lane meets
+            uint32_t cnt = 0;
+            float bestd = INFINITY;
+            uint32_t b1 = 0, b2 = 0;
+            for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                float d;
+                if (v && keep_pair(k1, k2, d)) {
+                    cnt++;
+                    d += sqrtf(lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)));
+                    if (d < bestd) bestd = d, b1 = k1, b2 = k2;
+                }
+                return false;
+            });
+            my.cand += cnt;
+            for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(full, cnt, o);
+            if (cnt == 0) break;
+            // the last candidate in order, once known: only its first sequence
+            // pair counts, and last_hit has seen to that
+            bool know_last = false;
+            uint32_t last1 = 0, last2 = 0;
+            // the first sequence pair of candidate (id1, id2), the last in order
+            auto last_hit = [&](uint32_t id1, uint32_t id2) {
+                const SeqSet A = seq_set(sv, S, id1), B = seq_set(sv, T, id2);
+                for (uint32_t ia = A.a; ia < A.b; ia++) {
+                    const uint2 e1 = A.seq[ia];
+                    for (uint32_t jb = B.a; jb < B.b; jb++) {
+                        const uint2 e2 = B.seq[jb];
+                        if (e1.y < 2 || e2.y < 2) continue;
+                        const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
+                        double m = 1.7976931348623157e308;
+                        for (uint32_t k = lane; k < n1 + n2; k += 32) {
+                            const uint32_t r = k < n1 ? k : k - n1, len = k < n1 ? e1.y - 1 : e2.y - 1;
+                            const uint32_t pi = r / len, si = r % len;
+                            const float2 *pr = k < n1 ? B.ring + e2.x : A.ring + e1.x;
+                            const float2 *gr = k < n1 ? A.ring + e1.x : B.ring + e2.x;
+                            const double d = pt_seg_dist(pr[pi], gr[si], gr[si + 1], geo);
+                            m = m < d ? m : d;
+                        }
+                        for (int o = 16; o; o >>= 1) {
+                            const double v = __shfl_xor_sync(full, m, o);
+                            m = m < v ? m : v;
+                        }
+                        if (lane == 0) my.rechk += n1 + n2;
+                        if (m < w.thr) return true;
+                        if (m < 100000.0) return false;
+                        // the running minimum still at its start value: any
+                        // earlier distance below it ends the search here
+                        Near far = w;
+                        far.thr = 100000.0;
+                        far.c0 += 100100.f;
+                        const bool below = for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                            float d;
+                            v = v && keep_pair(k1, k2, d) && !(ss.p[k1] == id1 && ts.p[k2] == id2);
+                            return test_candidates(sv, S, T, v, v ? ss.p[k1] : 0, v ? ts.p[k2] : 0, far, geo, tab,
+                                                   lane, my) != 0;
+                        });
+                        if (below) return false;
+                    }
+                }
+                return false;
+            };
+            // lanes' candidates tested; true when one that counts has a hit
+            auto tested = [&](bool v, uint32_t id1, uint32_t id2, uint32_t k1, uint32_t k2) {
+                if (know_last && id1 == last1 && id2 == last2) v = false;
+                for (unsigned m = test_candidates(sv, S, T, v, id1, id2, w, geo, tab, lane, my); m; m &= m - 1) {
+                    if (know_last) return true;  // the last candidate was left out above
+                    // a hit counts unless its candidate is the last in order
+                    const int src = __ffs(m) - 1;
+                    const uint32_t h1 = __shfl_sync(full, k1, src), h2 = __shfl_sync(full, k2, src);
+                    const CandKey c = cand_key(h1, h2);
+                    const bool later = cnt > 1 && for_product(ns, nt, lane, [&](uint32_t a1, uint32_t a2, bool vv) {
+                        float d;
+                        return __any_sync(full, vv && keep_pair(a1, a2, d) && key_less(c, cand_key(a1, a2))) != 0;
+                    });
+                    if (later) return true;
+                    know_last = true;
+                    last1 = (uint32_t)c.id1;
+                    last2 = (uint32_t)c.id2;
+                    if (last_hit(last1, last2)) return true;
+                }
+                return false;
+            };
+            const bool probe = bestd < INFINITY;
+            yes = tested(probe, probe ? ss.p[b1] : 0, probe ? ts.p[b2] : 0, b1, b2);
+            if (!yes && cnt > (uint32_t)__popc(__ballot_sync(full, probe))) {
+                // queue entries are (k1, k2) until they are spilled as pixel ids
+                bool may_spill = a.sp.cap > 0;
+                uint32_t spent = 0;
+                int qn = 0;
+                auto flush = [&]() {
+                    for (int k = 0; k < qn; k += 32) {
+                        if (may_spill && (float)spent >= a.sp.budget) {
+                            if (!know_last) {  // the largest key of all
+                                CandKey top{-1.0, 0, 0, 0, 0};
+                                for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                                    float d;
+                                    if (v && keep_pair(k1, k2, d)) {
+                                        const CandKey c = cand_key(k1, k2);
+                                        if (key_less(top, c)) top = c;
+                                    }
+                                    return false;
+                                });
+                                for (int o = 16; o; o >>= 1) {
+                                    CandKey c;
+                                    c.apx = __shfl_xor_sync(full, top.apx, o);
+                                    c.lo = __shfl_xor_sync(full, top.lo, o);
+                                    c.hi = __shfl_xor_sync(full, top.hi, o);
+                                    c.id1 = __shfl_xor_sync(full, top.id1, o);
+                                    c.id2 = __shfl_xor_sync(full, top.id2, o);
+                                    if (key_less(top, c)) top = c;
+                                }
+                                know_last = true;
+                                last1 = (uint32_t)top.id1;
+                                last2 = (uint32_t)top.id2;
+                                if (last_hit(last1, last2)) return true;
+                            }
+                            // the last candidate stays out of the pool
+                            for (int e = k + lane; e < qn; e += 32) {
+                                uint2 c = make_uint2(ss.p[q[e].x], ts.p[q[e].y]);
+                                if (c.x == last1 && c.y == last2) c.x = ~0u;
+                                q[e] = c;
+                            }
+                            __syncwarp();
+                            if (spill_rest(a.sp, pid, q, k, qn, 0.f, lane, &head, &spilled)) return false;
+                            may_spill = false;  // the pool is full: back to this warp
+                            for (; k < qn; k += 32) {
+                                const bool v = k + lane < qn && q[k + lane].x != ~0u;
+                                const uint2 c = v ? q[k + lane] : make_uint2(0u, 0u);
+                                if (tested(v, c.x, c.y, 0, 0)) return true;
+                            }
+                            return false;
+                        }
+                        const bool v = k + lane < qn;
+                        const uint2 c = v ? q[k + lane] : make_uint2(0u, 0u);
+                        spent += 32;
+                        if (tested(v, ss.p[c.x], ts.p[c.y], c.x, c.y)) return true;
+                    }
+                    return false;
+                };
+                yes = for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+                    float d;
+                    const bool keep = v && keep_pair(k1, k2, d);
+                    const unsigned m = __ballot_sync(full, keep);
+                    if (keep) q[qn + __popc(m & ((1u << lane) - 1))] = make_uint2(k1, k2);
+                    qn += __popc(m);
+                    if (qn + 32 <= kQueue) return false;
+                    __syncwarp();
+                    const bool h = flush();
+                    qn = 0;
+                    __syncwarp();
+                    return h;
+                });
+                __syncwarp();
+                if (!yes && qn) yes = flush();
+                __syncwarp();
+            }
+            break;
         }
         // leave the scratch bitmaps clean for the next pair
         __syncwarp();
@@ -511,390 +1025,91 @@ __global__ void __launch_bounds__(256) k_within_descend(const StoreView sv, With
             ts.bits[w] = 0u;
         }
         __syncwarp();
-        if (lane == 0) a.out[pid] = result;
-    }
-    if (lane == 0) {
-        atomicAdd(&a.stats[0], my_cand);
-        atomicAdd(&a.stats[1], my_box);
-    }
-}
-
-// first candidate of each pair (candidates sorted by pair)
-__global__ void k_cand_bounds(const WCand *__restrict__ c, uint64_t n, uint64_t *__restrict__ first) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-        if (k == 0 || c[k - 1].pair != c[k].pair) first[c[k].pair] = k;
-    }
-}
-
-// Work order of the refinement: the pairs with the most candidates first
-// (longest-first scheduling, so that the pass does not end on a long pair
-// that started last). key[p] = ~(candidates of p) at p's last candidate;
-// pairs without candidates keep the all-ones key and come last. Results are
-// written by pair index, so the order is invisible.
-__global__ void k_within_cost(const WCand *__restrict__ c, uint64_t n, const uint64_t *__restrict__ first,
-                              uint32_t *__restrict__ key) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-        if (k + 1 == n || c[k + 1].pair != c[k].pair) {
-            const uint64_t cnt = k + 1 - first[c[k].pair];
-            key[c[k].pair] = ~(uint32_t)(cnt < 0xFFFFFFFEull ? cnt : 0xFFFFFFFEull);
-        }
-    }
-}
-
-__global__ void k_iota32(uint32_t *__restrict__ v, uint64_t n) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
-        v[k] = (uint32_t)k;
-}
-
-// FARM_PAIR_ORDER=0 takes the pairs in index order
-static bool within_order_on() {
-    const char *v = getenv("FARM_PAIR_ORDER");
-    return !(v && *v == '0');
-}
-
-// suf[k] = the smallest lo of the pair's candidates after k (100000 after the
-// last), the bound Ideal.cpp:2615-2621 recomputes for every candidate; one
-// warp per refined pair scans its candidates backwards 32 at a time.
-__global__ void k_cand_sufmin(const WCand *__restrict__ c, uint64_t ncand, const uint64_t *__restrict__ first,
-                              const uint8_t *__restrict__ out, uint64_t n, double *__restrict__ suf) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t w0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t pid = w0; pid < n; pid += nw) {
-        if (out[pid] != W_REFINE) continue;
-        const uint64_t b = first[pid];
-        uint64_t e = b;
-        while (e < ncand && c[e].pair == pid) e++;
-        double carry = 100000.0;
-        for (uint64_t hi = e; hi > b;) {
-            const uint64_t cnt = hi - b < 32 ? hi - b : 32;
-            const bool v = (uint64_t)lane < cnt;
-            const uint64_t k = hi - 1 - lane;
-            double incl = v ? c[k].lo : 100000.0;
-            // inclusive min over lanes 0..lane (indices hi-1 down to k)
-            for (int o = 1; o < 32; o <<= 1) {
-                double x = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl = incl < x ? incl : x;
-            }
-            double before = __shfl_up_sync(0xffffffffu, incl, 1);  // indices after k in this chunk
-            double r = lane == 0 ? carry : (carry < before ? carry : before);
-            if (v) suf[k] = r;
-            double last = __shfl_sync(0xffffffffu, incl, 31);
-            carry = carry < last ? carry : last;
-            hi -= cnt;
-        }
-    }
-}
-
-struct RefineArgs {
-    const uint32_t *pairs;
-    uint64_t n;
-    uint64_t tgt_base;
-    double thr;
-    int geo;
-    const WCand *cand;
-    uint64_t ncand;
-    const uint64_t *first;
-    const double *suf;  // per candidate: smallest lo of the later candidates
-    uint8_t *out;
-    unsigned long long *next;
-    unsigned long long *stats;  // seq pairs, point-segment tests
-    const uint32_t *order;      // pairs taken in this order (most candidates first), or index order
-};
-
-// Ideal.cpp:2612-2643 in the candidates' order.
-// exclusive warp scan of v; the warp's total in `total`
-__device__ __forceinline__ uint32_t warp_scan_excl(uint32_t v, int lane, uint32_t &total) {
-    uint32_t incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    total = __shfl_sync(0xffffffffu, incl, 31);
-    return incl - v;
-}
-
-// float <-> int keys whose signed order is the floats' order (no NaNs)
-__device__ __forceinline__ int ord_key(float v) {
-    const int i = __float_as_int(v);
-    return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float ord_val(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
-
-// Sequence pairs of one candidate pixel pair refined together (see below)
-// when there are at most this many.
-constexpr uint32_t kFlatSP = 64;
-
-__global__ void __launch_bounds__(256) k_within_refine(const StoreView sv, RefineArgs a) {
-    const int lane = threadIdx.x & 31;
-    const bool geo = a.geo != 0;
-    const int cc = sv.category_count;
-    unsigned long long my_seq = 0, my_tests = 0, my_rechk = 0;
-    __shared__ uint2 s_seq[8][2 * kFlatSP];
-    __shared__ uint32_t s_off[8][kFlatSP + 1];
-    __shared__ int s_lb[8][kFlatSP];
-    const int wib = threadIdx.x >> 5;
-    uint2 *sa = s_seq[wib], *sb = s_seq[wib] + kFlatSP;
-    uint32_t *off = s_off[wib];
-    int *lbk = s_lb[wib];
-    for (;;) {
-        unsigned long long pid = 0;
         if (lane == 0) {
-            pid = atomicAdd(a.next, 1ull);
-            if (a.order && pid < a.n) pid = a.order[pid];
+            a.out[pid] = yes ? W_TRUE : W_FALSE;
+            if (spilled && yes) a.sp.flag[head] = 1u;  // found after the spill
         }
-        pid = __shfl_sync(0xffffffffu, pid, 0);
-        if (pid >= a.n) break;
-        if (a.out[pid] != W_REFINE) continue;
-        const uint32_t s = a.pairs[2 * pid], t = a.pairs[2 * pid + 1];
-        const PolyHdr &S = sv.hdr[s];
-        const PolyHdr &T = sv.hdr[a.tgt_base + t];
-        const uint64_t b = a.first[pid];
-        uint64_t e = b;
-        while (e < a.ncand && a.cand[e].pair == pid) e++;
-        const uint32_t *so = sv.offset + S.off, *to = sv.offset + T.off;
-        const uint2 *sseq = sv.seq + S.seq, *tseq = sv.seq + T.seq;
-        const float2 *sr = sv.ring + S.ring, *tr = sv.ring + T.ring;
-        double min_dist = 100000.0;
-        int decided = -1;
-        for (uint64_t k = b; k < e && decided < 0; k++) {
-            // lower bound of every later candidate
-            const double ref = a.suf[k];
-            const int id1 = a.cand[k].id1, id2 = a.cand[k].id2;
-            uint32_t a0 = 0, a1 = 0, b0 = 0, b1 = 0;
-            if (show_status(sv.status[S.st + id1], cc) == 1) {
-                a0 = so[id1];
-                a1 = so[id1 + 1];
-            }
-            if (show_status(sv.status[T.st + id2], cc) == 1) {
-                b0 = to[id2];
-                b1 = to[id2 + 1];
-            }
-            const uint32_t na = a1 - a0, nb = b1 - b0;
-            if (na * nb <= kFlatSP) {
-                // All sequence pairs of the pixel pair at once: the FP32
-                // lower bounds of every (point, segment) test of every
-                // sequence pair are spread over the lanes, with a minimum per
-                // sequence pair; then the reference's sequential rule is
-                // replayed on them in its order (source sequence outer,
-                // target inner), with the FP64 minimum of a sequence pair
-                // computed where its bound may lower the running minimum.
-                // The bounds are those of the loop below, so the decisions
-                // are the same.
-                const uint32_t nsp = na * nb;
-                for (uint32_t i = lane; i < na; i += 32) sa[i] = sseq[a0 + i];
-                for (uint32_t j = lane; j < nb; j += 32) sb[j] = tseq[b0 + j];
-                __syncwarp();
-                // tests of sequence pairs lane and lane + 32
-                auto sp_tests = [&](uint32_t sp) -> uint32_t {
-                    if (sp >= nsp) return 0u;
-                    const uint2 e1 = sa[sp / nb], e2 = sb[sp % nb];
-                    return (e1.y >= 2 && e2.y >= 2) ? e2.y * (e1.y - 1) + e1.y * (e2.y - 1) : 0u;
-                };
-                const uint32_t sz0 = sp_tests((uint32_t)lane), sz1 = sp_tests((uint32_t)lane + 32u);
-                uint32_t tot0, tot1;
-                const uint32_t ex0 = warp_scan_excl(sz0, lane, tot0);
-                const uint32_t ex1 = warp_scan_excl(sz1, lane, tot1);
-                const uint32_t total = tot0 + tot1;
-                if ((uint32_t)lane < nsp) {
-                    off[lane] = ex0;
-                    lbk[lane] = ord_key(3.4e38f);
-                }
-                if ((uint32_t)lane + 32u < nsp) {
-                    off[lane + 32] = tot0 + ex1;
-                    lbk[lane + 32] = ord_key(3.4e38f);
-                }
-                if (lane == 0) off[nsp] = total;
-                __syncwarp();
-                for (uint32_t t0 = 0; t0 < total; t0 += 32) {
-                    const uint32_t t = t0 + lane;
-                    if (t < total) {
-                        uint32_t lo = 0, hi = nsp;  // the last sp with off[sp] <= t
-                        while (hi - lo > 1) {
-                            const uint32_t mid = (lo + hi) >> 1;
-                            if (off[mid] <= t) lo = mid; else hi = mid;
-                        }
-                        const uint32_t sp = lo, k2 = t - off[sp];
-                        const uint2 e1 = sa[sp / nb], e2 = sb[sp % nb];
-                        const uint32_t n1 = e2.y * (e1.y - 1);
-                        float d, er;
-                        if (k2 < n1) {
-                            const uint32_t pi = k2 / (e1.y - 1), si = k2 % (e1.y - 1);
-                            d = pt_seg_dist32(tr[e2.x + pi], sr[e1.x + si], sr[e1.x + si + 1], geo, er);
-                        } else {
-                            const uint32_t r = k2 - n1;
-                            const uint32_t pi = r / (e2.y - 1), si = r % (e2.y - 1);
-                            d = pt_seg_dist32(sr[e1.x + pi], tr[e2.x + si], tr[e2.x + si + 1], geo, er);
-                        }
-                        atomicMin(&lbk[sp], ord_key(d - er));
-                    }
-                }
-                __syncwarp();
-                for (uint32_t sp = 0; sp < nsp && decided < 0; sp++) {
-                    const uint32_t nsz = off[sp + 1] - off[sp];
-                    if (nsz == 0) continue;  // a sequence of fewer than 2 points
-                    const uint2 e1 = sa[sp / nb], e2 = sb[sp % nb];
-                    const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
-                    const float lb = ord_val(lbk[sp]);
-                    if (lane == 0) {
-                        my_seq++;
-                        my_tests += nsz;
-                    }
-                    if ((double)lb < min_dist) {
-                        double m = 1.7976931348623157e308;
-                        for (uint32_t k2 = lane; k2 < n1 + n2; k2 += 32) {
-                            double dd;
-                            if (k2 < n1) {
-                                uint32_t pi = k2 / (e1.y - 1), si = k2 % (e1.y - 1);
-                                dd = pt_seg_dist(tr[e2.x + pi], sr[e1.x + si], sr[e1.x + si + 1], geo);
-                            } else {
-                                uint32_t r = k2 - n1;
-                                uint32_t pi = r / (e2.y - 1), si = r % (e2.y - 1);
-                                dd = pt_seg_dist(sr[e1.x + pi], tr[e2.x + si], tr[e2.x + si + 1], geo);
-                            }
-                            m = m < dd ? m : dd;
-                        }
-                        for (int o = 16; o; o >>= 1) {
-                            double v = __shfl_xor_sync(0xffffffffu, m, o);
-                            m = m < v ? m : v;
-                        }
-                        if (lane == 0) my_rechk++;
-                        min_dist = min_dist < m ? min_dist : m;
-                    }
-                    if (min_dist < a.thr) {
-                        decided = 1;
-                    } else if (min_dist < ref) {
-                        decided = 0;
-                    }
-                }
-                __syncwarp();
-                continue;
-            }
-            for (uint32_t ia = a0; ia < a1 && decided < 0; ia++) {
-                uint2 e1 = sseq[ia];
-                for (uint32_t jb = b0; jb < b1; jb++) {
-                    uint2 e2 = tseq[jb];
-                    if (e1.y < 2 || e2.y < 2) continue;
-                    // segment_to_segment_within_batch(target seq, source seq):
-                    // e2.y target points vs e1.y - 1 source segments, and back
-                    const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
-                    // FP32 first: a lower bound on this sequence pair's minimum
-                    float lb = 3.4e38f;
-                    for (uint32_t k2 = lane; k2 < n1 + n2; k2 += 32) {
-                        float d, er;
-                        if (k2 < n1) {
-                            uint32_t pi = k2 / (e1.y - 1), si = k2 % (e1.y - 1);
-                            d = pt_seg_dist32(tr[e2.x + pi], sr[e1.x + si], sr[e1.x + si + 1], geo, er);
-                        } else {
-                            uint32_t r = k2 - n1;
-                            uint32_t pi = r / (e2.y - 1), si = r % (e2.y - 1);
-                            d = pt_seg_dist32(sr[e1.x + pi], tr[e2.x + si], tr[e2.x + si + 1], geo, er);
-                        }
-                        lb = fminf(lb, d - er);
-                    }
-                    for (int o = 16; o; o >>= 1) lb = fminf(lb, __shfl_xor_sync(0xffffffffu, lb, o));
-                    if (lane == 0) {
-                        my_seq++;
-                        my_tests += n1 + n2;
-                    }
-                    // FP64 only when this pair may lower the exact running
-                    // minimum, so min_dist is always the reference's value
-                    if ((double)lb < min_dist) {
-                        double m = 1.7976931348623157e308;
-                        for (uint32_t k2 = lane; k2 < n1 + n2; k2 += 32) {
-                            double d;
-                            if (k2 < n1) {
-                                uint32_t pi = k2 / (e1.y - 1), si = k2 % (e1.y - 1);
-                                d = pt_seg_dist(tr[e2.x + pi], sr[e1.x + si], sr[e1.x + si + 1], geo);
-                            } else {
-                                uint32_t r = k2 - n1;
-                                uint32_t pi = r / (e2.y - 1), si = r % (e2.y - 1);
-                                d = pt_seg_dist(sr[e1.x + pi], tr[e2.x + si], tr[e2.x + si + 1], geo);
-                            }
-                            m = m < d ? m : d;
-                        }
-                        for (int o = 16; o; o >>= 1) {
-                            double v = __shfl_xor_sync(0xffffffffu, m, o);
-                            m = m < v ? m : v;
-                        }
-                        if (lane == 0) my_rechk++;
-                        min_dist = min_dist < m ? min_dist : m;
-                    }
-                    if (min_dist < a.thr) {
-                        decided = 1;
-                        break;
-                    } else if (min_dist < ref) {
-                        decided = 0;
-                        break;
-                    }
-                }
-            }
-        }
-        if (lane == 0) a.out[pid] = decided == 1 ? W_TRUE : W_FALSE;
-    }
-    if (lane == 0) {
-        atomicAdd(&a.stats[0], my_seq);
-        atomicAdd(&a.stats[1], my_tests);
-        atomicAdd(&a.stats[2], my_rechk);
-    }
-}
-
-__global__ void k_within_count(const uint8_t *__restrict__ out, uint64_t n, unsigned long long *found,
-                               unsigned long long *retry) {
-    unsigned long long f = 0, r = 0;
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-        f += out[k] == W_TRUE;
-        r += out[k] == W_RETRY;
     }
     for (int o = 16; o; o >>= 1) {
-        f += __shfl_xor_sync(0xffffffffu, f, o);
-        r += __shfl_xor_sync(0xffffffffu, r, o);
+        my.cand += __shfl_xor_sync(full, my.cand, o);
+        my.tests += __shfl_xor_sync(full, my.tests, o);
+        my.rechk += __shfl_xor_sync(full, my.rechk, o);
+        my.seqp += __shfl_xor_sync(full, my.seqp, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(found, f);
-        atomicAdd(retry, r);
-    }
-}
-
-__global__ void k_gather_retry(const uint32_t *__restrict__ pairs, const uint8_t *__restrict__ out, uint64_t n,
-                               uint32_t *__restrict__ rp, uint64_t *__restrict__ ridx,
-                               unsigned long long *__restrict__ cnt) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-        if (out[k] != W_RETRY) continue;
-        unsigned long long at = atomicAdd(cnt, 1ull);
-        rp[2 * at] = pairs[2 * k];
-        rp[2 * at + 1] = pairs[2 * k + 1];
-        ridx[at] = k;
+    if (lane == 0) {
+        atomicAdd(&a.stats[0], my.cand);
+        atomicAdd(&a.stats[1], my.box);
+        atomicAdd(&a.stats[2], my.tests);
+        atomicAdd(&a.stats[3], my.rechk);
+        atomicAdd(&a.stats[4], my.seqp);
     }
 }
 
-__global__ void k_scatter_retry(const uint8_t *__restrict__ rout, const uint64_t *__restrict__ ridx, uint64_t n,
-                                uint8_t *__restrict__ out) {
+// The candidates that k_within spilled, a warp's worth of one chunk at a time,
+// slice by slice across the chunks (as spill_units, a lane per entry).
+__global__ void __launch_bounds__(256, 3) k_within_spill(const StoreView sv, WithinArgs a) {
+    __shared__ float2 tab[900];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned long long n = min(a.sp.ctr[0], (unsigned long long)a.sp.cap);
+    if (n == 0) return;
+    if (a.geo)
+        for (int k = threadIdx.x; k < 900; k += blockDim.x) tab[k] = lon_entry(k);
+    __syncthreads();
+    const unsigned long long total = n * ((a.sp.ctr[2] + 31) / 32);
+    WithinTally my;
+    for (;;) {
+        unsigned long long u = 0;
+        if (lane == 0) u = atomicAdd(&a.sp.ctr[1], 1ull);
+        u = __shfl_sync(full, u, 0);
+        if (u >= total) break;
+        const uint64_t c = u % n;
+        const SpillChunk h = a.sp.chunk[c];
+        const uint32_t e = (uint32_t)(u / n) * 32;
+        if (e >= h.count) continue;
+        if (__shfl_sync(full, *(volatile uint32_t *)&a.sp.flag[h.head], 0)) continue;
+        const PolyHdr &S = sv.hdr[a.pairs[2 * h.pid]];
+        const PolyHdr &T = sv.hdr[a.tgt_base + a.pairs[2 * h.pid + 1]];
+        const uint2 cd = e + lane < h.count ? a.sp.items[c * kQueue + e + lane] : make_uint2(~0u, 0u);
+        const bool v = cd.x != ~0u;
+        if (test_candidates(sv, S, T, v, cd.x, cd.y, near_of(S, T, a.thr, a.geo), a.geo, tab, lane, my) && lane == 0) {
+            a.sp.flag[h.head] = 1u;
+            a.out[h.pid] = W_TRUE;
+        }
+    }
+    for (int o = 16; o; o >>= 1) {
+        my.tests += __shfl_xor_sync(full, my.tests, o);
+        my.rechk += __shfl_xor_sync(full, my.rechk, o);
+        my.seqp += __shfl_xor_sync(full, my.seqp, o);
+    }
+    if (lane == 0) {
+        atomicAdd(&a.stats[2], my.tests);
+        atomicAdd(&a.stats[3], my.rechk);
+        atomicAdd(&a.stats[4], my.seqp);
+    }
+}
+
+// The largest layer of any polygon, in pixels: a warp per polygon, a lane per layer.
+__global__ void k_within_cap(const PolyHdr *__restrict__ hdr, uint32_t npoly, unsigned long long *__restrict__ most) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long mine = 0;
+    for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < npoly; p += (gridDim.x * blockDim.x) >> 5) {
+        const PolyHdr &h = hdr[p];
+        if (h.err || lane >= (int)h.num_layers) continue;
+        LayerGeom g;
+        layer_geom(h, (uint32_t)lane, g);
+        mine = max(mine, (unsigned long long)(uint32_t)(g.dimx * g.dimy));
+    }
+    for (int o = 16; o; o >>= 1) mine = max(mine, __shfl_xor_sync(0xffffffffu, mine, o));
+    if (lane == 0 && mine) atomicMax(most, mine);
+}
+
+__global__ void k_within_count(const uint8_t *__restrict__ out, uint64_t n, unsigned long long *found) {
+    unsigned long long f = 0;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
-        out[ridx[k]] = rout[k];
-}
-
-// Within "-a" (query_within_polygon.cu:332-375): a pair the descent left
-// undecided is within when one of its surviving finest pixel pairs has
-// apxDist = minDist + mean (maxDist - minDist) <= the distance, in float.
-// mean is (1.0 - pf / category_count) * 0.5 with both operands 8-bit
-// integers (:352), so the quotient is 0 and mean is 0.5; 0.5 (max - min) is
-// exact in float, so contracting the sum into an FMA rounds the same.
-__global__ void k_within_apx(const WCand *__restrict__ c, uint64_t nc, const uint8_t *__restrict__ out, double thr,
-                             uint8_t *__restrict__ hit) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nc; k += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t p = c[k].pair;
-        if (out[p] != W_REFINE) continue;
-        const float lo = (float)c[k].lo, hi = (float)c[k].hi;
-        const float apx = lo + 0.5f * (hi - lo);
-        if ((double)apx <= thr) hit[p] = 1;
-    }
-}
-
-__global__ void k_within_apx_final(const uint8_t *__restrict__ hit, uint64_t n, uint8_t *__restrict__ out) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
-        if (out[k] == W_REFINE) out[k] = hit[k] ? W_TRUE : W_FALSE;
+        f += out[k] == W_TRUE;
+    for (int o = 16; o; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+    if ((threadIdx.x & 31) == 0 && f) atomicAdd(found, f);
 }
 
 static unsigned gbw(uint64_t n) {
@@ -902,126 +1117,6 @@ static unsigned gbw(uint64_t n) {
     uint64_t cap = 32ull * sm_count();
     if (g > cap) g = cap;
     return (unsigned)(g ? g : 1);
-}
-
-// One descend + sort + refine round over n device pairs with out in device memory.
-static int within_round(farm_store *s, const uint32_t *dpairs, uint64_t n, uint8_t *dout, double thr, int geo,
-                        int mode, uint64_t tgt_base, uint32_t cap_pix, int nwarps, uint64_t cand_cap,
-                        farm_stats *acc, int &launches) {
-    cudaStream_t st = s->stream;
-    StoreView sv = s->view();
-    const uint64_t words = within_scratch_words(cap_pix);
-    DevBuf &scr = s->s[Q_SCR0], &cand = s->s[Q_SCR1], &tmp = s->s[Q_SCR2], &first = s->s[Q_SCR3];
-    FARM_TRY(scr.ensure(4 * words * (uint64_t)nwarps + 64));
-    FARM_CUDA(cudaMemsetAsync(scr.p, 0, 4 * words * (uint64_t)nwarps, st));
-    FARM_TRY(cand.ensure(sizeof(WCand) * cand_cap + 64));
-    FARM_TRY(s->d_counters.ensure(256));
-    unsigned long long *ctr = s->d_counters.as<unsigned long long>();
-    FARM_CUDA(cudaMemsetAsync(ctr, 0, 256, st));
-    WithinArgs wa;
-    wa.pairs = dpairs;
-    wa.n = n;
-    wa.tgt_base = tgt_base;
-    wa.thr = thr;
-    wa.geo = geo;
-    wa.cap_pix = cap_pix;
-    wa.scratch = scr.as<uint32_t>();
-    wa.scratch_words = words;
-    wa.cand = cand.as<WCand>();
-    wa.ncand = ctr + 1;
-    wa.cand_cap = cand_cap;
-    wa.out = dout;
-    wa.next = ctr + 0;
-    wa.stats = ctr + 2;
-    // device time of the descent and of the ordered refinement (events on the
-    // store's stream, read after the synchronisations below)
-    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    for (auto &e : ev) cudaEventCreate(&e);
-    struct EvFree {
-        cudaEvent_t *e;
-        ~EvFree() {
-            for (int k = 0; k < 3; k++)
-                if (e[k]) cudaEventDestroy(e[k]);
-        }
-    } ev_free{ev};
-    if (ev[0]) cudaEventRecord(ev[0], st);
-    k_within_descend<<<nwarps / 8, 256, 0, st>>>(sv, wa);
-    launches++;
-    if (ev[1]) cudaEventRecord(ev[1], st);
-    unsigned long long hc[4];
-    FARM_CUDA(cudaMemcpyAsync(hc, ctr, 32, cudaMemcpyDeviceToHost, st));
-    FARM_CUDA(cudaStreamSynchronize(st));
-    {
-        float ms = 0;
-        if (ev[0] && ev[1] && cudaEventElapsedTime(&ms, ev[0], ev[1]) == cudaSuccess) acc->ms_stage[1] += ms;
-    }
-    uint64_t nc = hc[1] < cand_cap ? hc[1] : cand_cap;
-    acc->border_pairs += hc[3];
-    acc->in_hits += hc[2];  // candidate pixel pairs
-    if (nc && mode == FARM_MODE_APPROX) {
-        // no order and no refinement: one pass over the candidates
-        FARM_TRY(first.ensure(n + 64));
-        uint8_t *hit = first.as<uint8_t>();
-        FARM_CUDA(cudaMemsetAsync(hit, 0, n, st));
-        k_within_apx<<<gbw(nc), 256, 0, st>>>(cand.as<WCand>(), nc, dout, thr, hit);
-        k_within_apx_final<<<gbw(n), 256, 0, st>>>(hit, n, dout);
-        launches += 2;
-    } else if (nc) {
-        // order by pair, then the reference's tuple (Ideal.cpp:2612)
-        size_t bytes = 0;
-        FARM_CUDA(cub::DeviceMergeSort::SortKeys(nullptr, bytes, cand.as<WCand>(), (int64_t)nc, WCandLess(), st));
-        FARM_TRY(tmp.ensure(bytes + 64));
-        FARM_CUDA(cub::DeviceMergeSort::SortKeys(tmp.p, bytes, cand.as<WCand>(), (int64_t)nc, WCandLess(), st));
-        FARM_TRY(first.ensure(8 * n + 64));
-        k_cand_bounds<<<gbw(nc), 256, 0, st>>>(cand.as<WCand>(), nc, first.as<uint64_t>());
-        RefineArgs ra;
-        ra.pairs = dpairs;
-        ra.n = n;
-        ra.tgt_base = tgt_base;
-        ra.thr = thr;
-        ra.geo = geo;
-        ra.cand = cand.as<WCand>();
-        ra.ncand = nc;
-        ra.first = first.as<uint64_t>();
-        DevBuf &suf = s->s[Q_WITHIN_SUF];
-        FARM_TRY(suf.ensure(8 * nc + 64));
-        k_cand_sufmin<<<sm_count() * 8, 256, 0, st>>>(cand.as<WCand>(), nc, first.as<uint64_t>(), dout, n,
-                                                      suf.as<double>());
-        launches++;
-        ra.suf = suf.as<double>();
-        ra.out = dout;
-        ra.next = ctr + 4;
-        ra.stats = ctr + 5;
-        ra.order = nullptr;
-        if (within_order_on() && n > 1 && n < 0xFFFFFFFFull) {
-            FARM_TRY(s->s[Q_PAIR_ORDER].ensure(16 * n + 64));
-            uint32_t *key = s->s[Q_PAIR_ORDER].as<uint32_t>(), *key_s = key + n, *idx = key_s + n, *idx_s = idx + n;
-            FARM_CUDA(cudaMemsetAsync(key, 0xFF, 4 * n, st));
-            k_within_cost<<<gbw(nc), 256, 0, st>>>(cand.as<WCand>(), nc, first.as<uint64_t>(), key);
-            k_iota32<<<gbw(n), 256, 0, st>>>(idx, n);
-            launches += 2;
-            size_t ob = 0;
-            FARM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, ob, key, key_s, idx, idx_s, (int64_t)n, 0, 32, st));
-            FARM_TRY(s->cub_tmp.ensure(ob + 64));
-            FARM_CUDA(cub::DeviceRadixSort::SortPairs(s->cub_tmp.p, ob, key, key_s, idx, idx_s, (int64_t)n, 0, 32,
-                                                      st));
-            ra.order = idx_s;
-        }
-        k_within_refine<<<sm_count() * 8, 256, 0, st>>>(sv, ra);
-        launches += 2;
-        if (ev[2]) cudaEventRecord(ev[2], st);
-        unsigned long long hs[3];
-        FARM_CUDA(cudaMemcpyAsync(hs, ctr + 5, 24, cudaMemcpyDeviceToHost, st));
-        FARM_CUDA(cudaStreamSynchronize(st));
-        {
-            float ms = 0;
-            if (ev[1] && ev[2] && cudaEventElapsedTime(&ms, ev[1], ev[2]) == cudaSuccess) acc->ms_stage[2] += ms;
-        }
-        acc->sequence_pairs += hs[0];
-        acc->segment_tests += hs[1];
-        acc->fp64_rechecks += hs[2];
-    }
-    return FARM_OK;
 }
 
 int within(farm_store *s, const uint32_t *pairs, uint64_t n, double distance, int geography, int self, int mode,
@@ -1053,90 +1148,77 @@ int within(farm_store *s, const uint32_t *pairs, uint64_t n, double distance, in
         FARM_TRY(s->d_out.ensure(n + 64));
         dout = s->d_out.as<uint8_t>();
     }
-    // the largest finest raster bounds a warp's pixel sets
+    FARM_TRY(s->d_counters.ensure(256));
+    unsigned long long *ctr = s->d_counters.as<unsigned long long>();
+    FARM_CUDA(cudaMemsetAsync(ctr, 0, 128, stream));
+    int launches = 0;
+    // the largest layer of any polygon bounds a warp's pixel sets
     uint32_t cap = 64;
     {
-        std::vector<PolyHdr> hh(s->n_poly);
-        FARM_CUDA(cudaMemcpyAsync(hh.data(), s->d_hdr.p, sizeof(PolyHdr) * s->n_poly, cudaMemcpyDeviceToHost, stream));
+        k_within_cap<<<gbw(32ull * s->n_poly), 256, 0, stream>>>(s->d_hdr.as<PolyHdr>(), (uint32_t)s->n_poly, ctr + 15);
+        FARM_CUDA(cudaGetLastError());
+        launches++;
+        unsigned long long most = 0;
+        FARM_CUDA(cudaMemcpyAsync(&most, ctr + 15, 8, cudaMemcpyDeviceToHost, stream));
         FARM_CUDA(cudaStreamSynchronize(stream));
-        for (auto &h : hh) {
-            if (h.err) continue;
-            for (uint32_t li = 0; li < h.num_layers; li++) {
-                LayerGeom g;
-                layer_geom(h, li, g);
-                uint32_t np = (uint32_t)(g.dimx * g.dimy);
-                if (np > cap) cap = np;
-            }
-        }
+        if (most > cap) cap = (uint32_t)most;
         cap = (cap + 31) & ~31u;
     }
-    farm_stats acc;
-    memset(&acc, 0, sizeof acc);
-    int launches = 0;
     FARM_CUDA(cudaEventRecord(s->ev[6], stream));
-    int nwarps = sm_count() * 8 * 2;
-    size_t freeb = 0, totb = 0;
-    cudaMemGetInfo(&freeb, &totb);
-    const uint64_t words = within_scratch_words(cap);
-    while (nwarps > 64 && 4ull * words * (uint64_t)nwarps > freeb / 4) nwarps /= 2;
-    uint64_t cand_cap = 1ull << 24;
-    if (n) FARM_TRY(within_round(s, dpairs, n, dout, distance, geography, mode, tgt_base, cap, nwarps, cand_cap,
-                                 &acc, launches));
-    // pairs whose candidates did not fit: gather and rerun with a larger buffer
-    for (int round = 0; round < 8 && n; round++) {
-        FARM_TRY(s->d_counters.ensure(256));
-        unsigned long long *ctr = s->d_counters.as<unsigned long long>() + 16;
-        FARM_CUDA(cudaMemsetAsync(ctr, 0, 16, stream));
-        k_within_count<<<gbw(n), 256, 0, stream>>>(dout, n, ctr, ctr + 1);
-        launches++;
-        unsigned long long hc[2];
-        FARM_CUDA(cudaMemcpyAsync(hc, ctr, 16, cudaMemcpyDeviceToHost, stream));
-        FARM_CUDA(cudaStreamSynchronize(stream));
-        if (hc[1] == 0) break;
-        DevBuf &rp = s->s[Q_SCR4], &ro = s->s[Q_SCR5];
-        FARM_TRY(rp.ensure((8 + 8) * hc[1] + 64));
-        FARM_TRY(ro.ensure(hc[1] + 64));
-        uint32_t *rpairs = rp.as<uint32_t>();
-        uint64_t *ridx = reinterpret_cast<uint64_t *>(rpairs + 2 * hc[1] + 2);
-        FARM_CUDA(cudaMemsetAsync(ctr, 0, 8, stream));
-        k_gather_retry<<<gbw(n), 256, 0, stream>>>(dpairs, dout, n, rpairs, ridx, ctr);
-        launches++;
-        cand_cap *= 4;
-        int rw = nwarps > 256 ? 256 : nwarps;
-        FARM_TRY(within_round(s, rpairs, hc[1], ro.as<uint8_t>(), distance, geography, mode, tgt_base, cap, rw,
-                              cand_cap, &acc, launches));
-        k_scatter_retry<<<gbw(hc[1]), 256, 0, stream>>>(ro.as<uint8_t>(), ridx, hc[1], dout);
-        launches++;
+    if (n) {
+        const uint64_t words = within_scratch_words(cap);
+        uint64_t blocks = (uint64_t)sm_count() * kWithinBlocks;
+        if (blocks > n) blocks = n;
+        size_t freeb = 0, totb = 0;
+        cudaMemGetInfo(&freeb, &totb);
+        while (blocks > 8 && 4ull * words * 8 * blocks > freeb / 4) blocks /= 2;
+        DevBuf &scr = s->s[Q_SCR0];
+        FARM_TRY(scr.ensure(4 * words * 8 * blocks + 64));
+        WithinArgs wa;
+        wa.pairs = dpairs;
+        wa.n = n;
+        wa.tgt_base = tgt_base;
+        wa.thr = distance;
+        wa.geo = geography != 0;
+        wa.approx = mode == FARM_MODE_APPROX;
+        wa.cap_pix = cap;
+        wa.scratch = scr.as<uint32_t>();
+        wa.scratch_words = words;
+        wa.out = dout;
+        wa.next = ctr;
+        wa.stats = ctr + 1;
+        FARM_TRY(spill_pool(s, n, ctr + 8, 64.f, 512.f, &wa.sp));
+        k_within<<<(unsigned)blocks, 256, 0, stream>>>(s->view(), wa);
+        FARM_CUDA(cudaGetLastError());
+        FARM_CUDA(cudaEventRecord(s->ev[8], stream));
+        k_within_spill<<<3 * sm_count(), 256, 0, stream>>>(s->view(), wa);
+        FARM_CUDA(cudaGetLastError());
+        launches += 2;
     }
     FARM_CUDA(cudaEventRecord(s->ev[7], stream));
-    unsigned long long *fc = s->d_counters.as<unsigned long long>() + 20;
-    FARM_CUDA(cudaMemsetAsync(fc, 0, 16, stream));
-    k_within_count<<<gbw(n), 256, 0, stream>>>(dout, n, fc, fc + 1);
+    k_within_count<<<gbw(n), 256, 0, stream>>>(dout, n, ctr + 14);
     launches++;
-    unsigned long long hf[2] = {0, 0};
-    FARM_CUDA(cudaMemcpyAsync(hf, fc, 16, cudaMemcpyDeviceToHost, stream));
+    unsigned long long h[16];
+    FARM_CUDA(cudaMemcpyAsync(h, ctr, sizeof h, cudaMemcpyDeviceToHost, stream));
     if (mem == FARM_MEM_HOST && out && n) FARM_CUDA(cudaMemcpyAsync(out, dout, n, cudaMemcpyDeviceToHost, stream));
     FARM_CUDA(cudaStreamSynchronize(stream));
     s->launches += (uint64_t)launches;
-    if (hf[1]) {
-        set_error("farm_within: some pairs exceeded the candidate buffer after retries");
-        return FARM_ENOMEM;
-    }
-    if (found) *found = hf[0];
+    if (found) *found = h[14];
     if (st) {
         memset(st, 0, sizeof *st);
         st->pairs = n;
-        st->found = hf[0];
-        st->border_pairs = acc.border_pairs;
-        st->segment_tests = acc.segment_tests;
-        st->fp64_rechecks = acc.fp64_rechecks;
-        st->sequence_pairs = acc.sequence_pairs;
-        st->in_hits = acc.in_hits;
-        float ms = 0;
+        st->found = h[14];
+        st->in_hits = h[1];  // candidate pixel pairs
+        st->border_pairs = h[2];
+        st->segment_tests = h[3];
+        st->fp64_rechecks = h[4];
+        st->sequence_pairs = h[5];
+        float ms = 0, ms1 = 0;
         cudaEventElapsedTime(&ms, s->ev[6], s->ev[7]);
+        if (n) cudaEventElapsedTime(&ms1, s->ev[6], s->ev[8]);
         st->ms_total = ms;
-        st->ms_stage[1] = acc.ms_stage[1];  // the hierarchical descent (filter)
-        st->ms_stage[2] = acc.ms_stage[2];  // candidate order and the ordered refinement
+        st->ms_stage[1] = ms1;       // the descent and the tests kept with it
+        st->ms_stage[2] = ms - ms1;  // the spilled tests
         st->kernel_launches = launches;
     }
     return FARM_OK;

@@ -42,3 +42,28 @@ def test_gpu_spilled_pairs_match_oracle(gpu_lib, monkeypatch, seed, n_lo, n_hi, 
     exp = np.array([O.contain(RS[s], RT[t]) for s, t in pairs], np.uint8)
     assert np.array_equal(con, exp), f"{int((con != exp).sum())} of {len(exp)} differ"
     assert held == int(exp.sum())
+
+
+@pytest.mark.parametrize("budget", ["0", None, "1e30"])
+@pytest.mark.parametrize("seed,n_hi,vpr,geo,distance", [(81, 700, 10, False, 0.02), (82, 700, 4, False, 0.3),
+                                                        (83, 1500, 700, False, 0.1), (84, 900, 10, True, 10.0),
+                                                        (85, 300, 4, True, 150.0), (86, 200, 10, False, 1.5e5)])
+def test_gpu_within_spilled_candidates_match_oracle(gpu_lib, monkeypatch, seed, n_hi, vpr, geo, distance, budget):
+    if budget is None:
+        monkeypatch.delenv("FARM_SPILL_BUDGET", raising=False)
+    else:
+        monkeypatch.setenv("FARM_SPILL_BUDGET", budget)
+    prm = P.StarParams(dom_hi=9.0, n_hi=n_hi)
+    S = P.generate(prm, seed, 40)
+    pairs = np.array([(i, j) for i in range(40) for j in range(40) if i != j], np.uint32)
+    RS = O.rasterize_set(S, vpr, True)
+    with Store() as st:
+        st.load_sets(S)
+        st.rasterize(vpr=vpr, hierarchy=True)
+        out, found = st.within(pairs, distance=distance, geography=geo, self_join=True)
+        apx, _ = st.within(pairs, distance=distance, geography=geo, self_join=True, mode=1)
+    exp = np.array([O.within(RS[s], RS[t], distance, geo) for s, t in pairs], np.uint8)
+    assert np.array_equal(out, exp), f"{int((out != exp).sum())} of {len(exp)} differ"
+    assert found == int(exp.sum())
+    exp = np.array([O.within_heuristic(RS[s], RS[t], distance, geo) for s, t in pairs], np.uint8)
+    assert np.array_equal(apx, exp), f"{int((apx != exp).sum())} of {len(exp)} differ (-a)"
