@@ -7,8 +7,10 @@
 // (8 x 16-byte core matrices; LBO = distance between K-adjacent cores, SBO =
 // distance between M/N-adjacent 8-row groups), one elected thread issues
 // tcgen05.mma.cta_group::1.kind::f16 (K = 16 per instruction) into a TMEM
-// accumulator, and tcgen05.commit arrives on an mbarrier per stage (two
-// stages, so loading chunk k+1 overlaps the MMAs of chunk k). The epilogue
+// accumulator, and tcgen05.commit arrives on an mbarrier per stage. Row-major
+// operands come by cp.async, three chunks ahead of the MMAs; operands given
+// transposed ([K x M], a product over rows) are loaded as 8 x 8 blocks and
+// turned in registers, so that no transposed copy is made. The epilogue
 // reads TMEM with tcgen05.ld (warp w owns lanes 32w..32w+31 = tile rows) and
 // hands 16 columns at a time to a functor. Every mbarrier wait is bounded;
 // on timeout the CTA records an error, still frees its TMEM, and returns.
@@ -30,15 +32,17 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// shared memory matrix descriptor (no swizzle, descriptor version 1)
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
+// shared memory matrix descriptor (no swizzle, descriptor version 1); sbo: the
+// distance between 8-row groups
+__device__ __forceinline__ uint64_t make_desc_sbo(uint32_t saddr, uint32_t sbo) {
     uint64_t d = 0;
     d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
     d |= (uint64_t)((kLBO >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((kSBO >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
     d |= 1ull << 46;
     return d;
 }
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) { return make_desc_sbo(saddr, kSBO); }
 
 // instruction descriptor: D f32, A/B bf16, both K-major, M x N
 __host__ __device__ constexpr uint32_t make_idesc(int M, int N) {
@@ -112,38 +116,73 @@ __device__ __forceinline__ uint32_t tile_off(uint32_t row, uint32_t k) {
     return (row >> 3) * kSBO + (k >> 3) * kLBO + (row & 7) * 16 + (k & 7) * 2;
 }
 
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid = true) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");  // not valid: zeros
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kLeft>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLeft) : "memory");
+}
+
 // Stage a [rows x 64] slice of a row-major bf16 matrix (ld elements per row)
 // into the core-matrix layout, 16 bytes per access; rows >= nrows and columns
 // >= ncols read as zero.
 __device__ __forceinline__ void stage_tile(unsigned char *dst, const __nv_bfloat16 *src, int ld, int row0, int nrows,
                                            int k0, int ncols, int rows) {
     const int vecs = rows * 8;  // 8 x 16 B per row of 64 bf16
+    const uint32_t d = smem_addr(dst);
     for (int v = threadIdx.x; v < vecs; v += kThreads) {
-        int r = v >> 3, kc = v & 7;
-        int gr = row0 + r, gk = k0 + kc * 8;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (gr < nrows && gk < ncols) val = *reinterpret_cast<const uint4 *>(src + (size_t)gr * ld + gk);
-        *reinterpret_cast<uint4 *>(dst + tile_off((uint32_t)r, (uint32_t)(kc * 8))) = val;
+        const int r = v >> 3, kc = v & 7;
+        const int gr = row0 + r, gk = k0 + kc * 8;
+        const bool valid = gr < nrows && gk < ncols;
+        cp_async16(d + tile_off((uint32_t)r, (uint32_t)(kc * 8)), valid ? src + (size_t)gr * ld + gk : src, valid);
     }
 }
 
-// Tile GEMM body. smem: 2 stages x (A 16 KB + B BN x 128 B) + barriers.
+// The same of a matrix given as [K x rows] (ld elements per k): each thread
+// turns 8 x 8 blocks. Rows and k are in range (multiples of 8 and 64).
+__device__ __forceinline__ void stage_tile_t(unsigned char *dst, const __nv_bfloat16 *src, int ld, int row0, int k0,
+                                             int rows) {
+    for (int v = threadIdx.x; v < rows; v += kThreads) {  // rows / 8 x 8 blocks
+        const int rb = v % (rows >> 3), kb = v / (rows >> 3);
+        const __nv_bfloat16 *g = src + (size_t)(k0 + kb * 8) * ld + row0 + rb * 8;
+        uint4 in[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) in[k] = *reinterpret_cast<const uint4 *>(g + (size_t)k * ld);
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(in);  // w[4 k + i]: rows 2i, 2i + 1 of column k
+        unsigned char *d = dst + tile_off((uint32_t)(rb * 8), (uint32_t)(kb * 8));
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            uint32_t a[4], b[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                a[q] = __byte_perm(w[8 * q + i], w[8 * q + 4 + i], 0x5410);
+                b[q] = __byte_perm(w[8 * q + i], w[8 * q + 4 + i], 0x7632);
+            }
+            *reinterpret_cast<uint4 *>(d + (2 * i) * 16) = make_uint4(a[0], a[1], a[2], a[3]);
+            *reinterpret_cast<uint4 *>(d + (2 * i + 1) * 16) = make_uint4(b[0], b[1], b[2], b[3]);
+        }
+    }
+}
+
+constexpr int kStages = 4;
+
+// Tile GEMM body over k in [kb, ke) (kb a multiple of 64). smem: kStages x
+// (A 16 KB + B BN x 128 B) + barriers. kT: both operands transposed.
 // epi(row, col0, v[16]) is called for every row < M and 16-column group < N.
-template <int BN, typename Epi>
-__device__ void gemm_tile(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ldb, int M, int N, int K,
-                          int m0, int n0, unsigned char *smem, int *err, Epi epi) {
+template <int BN, bool kT, typename Epi>
+__device__ void gemm_tile(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *B, int ldb, int M, int N, int kb,
+                          int ke, int m0, int n0, unsigned char *smem, int *err, Epi epi) {
     static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "MMA N");
     constexpr uint32_t kTmemCols = BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
     constexpr uint32_t kA = kBM * kBK * 2, kB = BN * kBK * 2;
-    unsigned char *sA[2] = {smem, smem + kA + kB};
-    unsigned char *sB[2] = {smem + kA, smem + 2 * kA + kB};
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 2 * (kA + kB));  // [0],[1] stages, [2] final
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 3);
+    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + kStages * (kA + kB));  // a stage each, then the final one
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + kStages + 1);
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_init(&bar[2], 1);
+        for (int k = 0; k <= kStages; k++) mbar_init(&bar[k], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) tmem_alloc(tslot, kTmemCols);
@@ -152,35 +191,45 @@ __device__ void gemm_tile(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *
     fence_after_sync();
     const uint32_t tmem = *tslot;
     const uint32_t idesc = make_idesc(kBM, BN);
-    const int nk = (K + kBK - 1) / kBK;
-    uint32_t phase[2] = {0, 0};
+    const int nk = (ke - kb + kBK - 1) / kBK;
     bool ok = true;
-    for (int kc = 0; kc < nk; kc++) {
-        int s = kc & 1;
-        if (kc >= 2) {  // the MMAs that read this stage two chunks ago must be done
-            ok = ok && mbar_wait(&bar[s], phase[s]);
-            phase[s] ^= 1;
+    auto load = [&](int kc) {
+        unsigned char *sA = smem + (kc % kStages) * (kA + kB), *sB = sA + kA;
+        if (kT) {
+            stage_tile_t(sA, A, lda, m0, kb + kc * kBK, kBM);
+            stage_tile_t(sB, B, ldb, n0, kb + kc * kBK, BN);
+        } else {
+            stage_tile(sA, A, lda, m0, M, kb + kc * kBK, ke, kBM);
+            stage_tile(sB, B, ldb, n0, N, kb + kc * kBK, ke, BN);
         }
-        stage_tile(sA[s], A, lda, m0, M, kc * kBK, K, kBM);
-        stage_tile(sB[s], B, ldb, n0, N, kc * kBK, K, BN);
+    };
+    for (int kc = 0; kc < kStages - 1; kc++) {
+        if (kc < nk) load(kc);
+        cp_async_commit();
+    }
+    for (int kc = 0; kc < nk; kc++) {
+        cp_async_wait<kStages - 2>();
         fence_async_smem();
         fence_before_sync();
         __syncthreads();
         fence_after_sync();
         if (threadIdx.x == 0 && ok) {
+            const uint32_t sA = smem_addr(smem + (kc % kStages) * (kA + kB)), sB = sA + kA;
 #pragma unroll
-            for (int kk = 0; kk < kBK / 16; kk++) {
-                uint64_t ad = make_desc(smem_addr(sA[s]) + kk * 2 * kLBO);
-                uint64_t bd = make_desc(smem_addr(sB[s]) + kk * 2 * kLBO);
-                mma_bf16(tmem, ad, bd, idesc, (kc > 0 || kk > 0) ? 1u : 0u);
-            }
-            mma_commit(&bar[s]);
+            for (int kk = 0; kk < kBK / 16; kk++)
+                mma_bf16(tmem, make_desc(sA + kk * 2 * kLBO), make_desc(sB + kk * 2 * kLBO), idesc,
+                         (kc > 0 || kk > 0) ? 1u : 0u);
+            mma_commit(&bar[kc % kStages]);
         }
+        // the chunk three ahead goes where the previous one's MMAs read from
+        if (kc > 0) ok = ok && mbar_wait(&bar[(kc - 1) % kStages], ((kc - 1) / kStages) & 1);
+        if (kc + kStages - 1 < nk) load(kc + kStages - 1);
+        cp_async_commit();
     }
     // the final commit tracks every MMA issued before it: once it arrives no
     // MMA can still write the accumulator, so TMEM may be read and freed
-    if (threadIdx.x == 0) mma_commit(&bar[2]);
-    bool fin = mbar_wait(&bar[2], 0) && ok;
+    if (threadIdx.x == 0) mma_commit(&bar[kStages]);
+    bool fin = mbar_wait(&bar[kStages], 0) && ok;
     fence_after_sync();
     __syncthreads();
     if (!fin) {
@@ -193,6 +242,7 @@ __device__ void gemm_tile(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *
             if (m0 + row < M && n0 + c < N) epi(m0 + row, n0 + c, v);
         }
     }
+    cp_async_wait<0>();
     fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, kTmemCols);
@@ -200,7 +250,7 @@ __device__ void gemm_tile(const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *
 
 template <int BN>
 constexpr int smem_bytes() {
-    return 2 * (kBM * kBK * 2 + BN * kBK * 2) + 64;
+    return kStages * (kBM * kBK * 2 + BN * kBK * 2) + 64;
 }
 
 }  // namespace tc
