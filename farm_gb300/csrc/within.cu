@@ -94,7 +94,7 @@ __device__ __forceinline__ Box pixel_box(const LayerGeom &g, int id) {
 }
 
 // Box.cpp:90-118
-__device__ double box_distance(const Box &a, const Box &t, bool geo) {
+__device__ __noinline__ double box_distance(const Box &a, const Box &t, bool geo) {
     if (!(t.lo0 > a.hi0 || t.hi0 < a.lo0 || t.lo1 > a.hi1 || t.hi1 < a.lo1)) return 0;
     double dx = 0, dy = 0;
     if (t.lo1 > a.hi1)
@@ -132,7 +132,7 @@ __device__ __forceinline__ float2 corner_spans(const float4 &fa, const float4 &f
     return make_float2(fmaxf(__fsub_rn(fa.z, ft.x), __fsub_rn(ft.z, fa.x)),
                        fmaxf(__fsub_rn(fa.w, ft.y), __fsub_rn(ft.w, fa.y)));
 }
-__device__ double box_max_distance_f(const float4 &fa, const float4 &ft, double a_lo1, bool geo) {
+__device__ __noinline__ double box_max_distance_f(const float4 &fa, const float4 &ft, double a_lo1, bool geo) {
     const float2 m = corner_spans(fa, ft);
     double dx = m.x, dy = m.y;
     if (geo) {
@@ -266,7 +266,7 @@ __device__ __forceinline__ SeqSet seq_set(const StoreView &sv, const PolyHdr &h,
 // (segment_to_segment_within_batch). Over all sequence pairs of a pixel pair
 // that is every point of one side against every segment of the other.
 template <bool kGeo>
-__device__ bool points_near_segments(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
+__device__ __noinline__ bool points_near_segments(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
                                      uint32_t &rechk) {
     for (uint32_t i = G.a; i < G.b; i++) {
         const uint2 e = G.seq[i];
@@ -289,7 +289,7 @@ __device__ bool points_near_segments(const SeqSet &P, const SeqSet &G, const Nea
 
 // The same with the warp on one pixel pair: segments over the lanes, points read by all.
 template <bool kGeo>
-__device__ bool points_near_segments_warp(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
+__device__ __noinline__ bool points_near_segments_warp(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
                                           int lane, uint32_t &rechk) {
     const unsigned full = 0xffffffffu;
     for (uint32_t i0 = G.a; i0 < G.b; i0 += 32) {
@@ -334,7 +334,7 @@ struct WithinTally {
 
 // Candidates (one per lane, valid lanes) against the threshold: the mask of
 // lanes whose pixel pair holds a point-segment distance below it.
-__device__ unsigned test_candidates(const StoreView &sv, const PolyHdr &S, const PolyHdr &T, bool valid, uint32_t id1,
+__device__ __noinline__ unsigned test_candidates(const StoreView &sv, const PolyHdr &S, const PolyHdr &T, bool valid, uint32_t id1,
                                     uint32_t id2, const Near &w, bool geo, const float2 *tab, int lane,
                                     WithinTally &my) {
     const unsigned full = 0xffffffffu;
@@ -405,7 +405,7 @@ constexpr int kMaxLayers = 32;
 // All layers of a polygon into L, a lane each: every layer's box and dims come
 // from the finest raster directly (its step is the finest one doubled, which
 // is exact), and its status offset is the finer layers' sizes added up.
-__device__ void load_layers(const PolyHdr &h, Layer *L, int lane) {
+__device__ __noinline__ void load_layers(const PolyHdr &h, Layer *L, int lane) {
     const unsigned full = 0xffffffffu;
     const int nl = (int)h.num_layers, up = nl - 1 - lane;
     Layer g{};
@@ -432,8 +432,8 @@ __device__ void load_layers(const PolyHdr &h, Layer *L, int lane) {
         const uint32_t u = __shfl_up_sync(full, incl, o);
         if (lane >= o) incl += u;
     }
-    if (up > 0) g.offset = h.P + (__shfl_sync(full, incl, 31) - incl);
-    else __shfl_sync(full, incl, 31);
+    const uint32_t all = __shfl_sync(full, incl, 31);
+    if (up > 0) g.offset = h.P + (all - incl);
     if (lane < nl) L[lane] = g;
 }
 
@@ -465,7 +465,7 @@ __host__ __device__ inline uint64_t within_scratch_words(uint32_t cap) {
 __device__ __forceinline__ void set_bit(uint32_t *bits, uint32_t id) { atomicOr(&bits[id >> 5], 1u << (id & 31)); }
 
 // Compact the set bits of [0, nbits) into list (ascending) and clear them.
-__device__ uint32_t compact_bits(uint32_t *bits, uint32_t nbits, uint32_t *list, int lane) {
+__device__ __noinline__ uint32_t compact_bits(uint32_t *bits, uint32_t nbits, uint32_t *list, int lane) {
     uint32_t nw = (nbits + 31) >> 5;
     uint32_t total = 0;
     for (uint32_t w0 = 0; w0 < nw; w0 += 32) {
@@ -493,7 +493,7 @@ __device__ uint32_t compact_bits(uint32_t *bits, uint32_t nbits, uint32_t *list,
 // Children of the queued pixels at layer g (their box at the coarser layer pg,
 // shrunk by 1e-6, then retrieve_pixels' own 1e-6) or the queued pixels
 // themselves; BORDER ones only (Ideal.cpp:2513-2551).
-__device__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, const Layer &g, const Layer *pg, uint32_t nq,
+__device__ __noinline__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, const Layer &g, const Layer *pg, uint32_t nq,
                              SideScratch &sc, int lane, int cc) {
     const uint8_t *st = status + h.st + g.offset;
     for (uint32_t k = lane; k < nq; k += 32) {
@@ -521,27 +521,34 @@ __device__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, const Laye
     return compact_bits(sc.bits, (uint32_t)(g.dimx * g.dimy), sc.p, lane);
 }
 
-// f(k1, k2, valid) over [0, ns) x [0, nt), all lanes at a time, until it
-// returns true (warp-uniform). The longer list runs over the lanes; two short
-// ones are flattened.
-template <typename F>
-__device__ __forceinline__ bool for_product(uint32_t ns, uint32_t nt, int lane, F f) {
-    if (nt >= ns && nt >= 24) {
-        for (uint32_t a = 0; a < ns; a++)
-            for (uint32_t b = 0; b < nt; b += 32)
-                if (f(a, b + lane, b + lane < nt)) return true;
-    } else if (ns >= 24) {
-        for (uint32_t b = 0; b < nt; b++)
-            for (uint32_t a = 0; a < ns; a += 32)
-                if (f(a + lane, b, a + lane < ns)) return true;
-    } else {
-        for (uint32_t k0 = 0; k0 < ns * nt; k0 += 32) {
-            const uint32_t k = k0 + lane;
-            if (f(k / nt, k % nt, k < ns * nt)) return true;
-        }
+// The pairs (k1, k2) of [0, ns) x [0, nt) in batches of 32 lanes: the longer
+// list over the lanes, the other in the outer loop; two short ones are
+// flattened. One loop body serves all three (k_within's code would otherwise
+// not stay in the instruction cache).
+struct Product {
+    uint32_t ns, nt, outer, inner, o = 0, b = 0;
+    int way;  // 0 flat, 1 targets over the lanes, 2 sources over the lanes
+    __device__ __forceinline__ Product(uint32_t ns_, uint32_t nt_) : ns(ns_), nt(nt_) {
+        way = nt >= ns && nt >= 24 ? 1 : (ns >= 24 ? 2 : 0);
+        outer = way == 0 ? 1u : (way == 1 ? ns : nt);
+        inner = way == 0 ? ns * nt : (way == 1 ? nt : ns);
+        if (ns == 0 || nt == 0) outer = 0;
     }
-    return false;
-}
+    // this lane's pair of the next batch; false past the last
+    __device__ __forceinline__ bool next(int lane, uint32_t &k1, uint32_t &k2, bool &valid) {
+        if (o >= outer) return false;
+        const uint32_t k = b + lane;
+        valid = k < inner;
+        k1 = way == 0 ? k / nt : (way == 1 ? o : k);
+        k2 = way == 0 ? k - k1 * nt : (way == 1 ? k : o);
+        b += 32;
+        if (b >= inner) {
+            b = 0;
+            o++;
+        }
+        return true;
+    }
+};
 
 // FP32 view of one level's box pairs. Float corners are off by half an ulp of
 // the coordinate, so a box distance computed from them is off by at most
@@ -575,7 +582,7 @@ __device__ __forceinline__ float warp_min(float v) {
 }
 
 // Keep the pixels of a side whose box may lie within `cut` of box bb.
-__device__ uint32_t prune_side(SideScratch &sc, uint32_t n, const float4 &bb, const Level &lv, bool source,
+__device__ __noinline__ uint32_t prune_side(SideScratch &sc, uint32_t n, const float4 &bb, const Level &lv, bool source,
                                float sx_low, float cut, int lane) {
     uint32_t at = 0;
     for (uint32_t b = 0; b < n; b += 32) {
@@ -615,6 +622,69 @@ __device__ __forceinline__ bool key_less(const CandKey &a, const CandKey &b) {
     if (a.hi != b.hi) return a.hi < b.hi;
     if (a.id1 != b.id1) return a.id1 < b.id1;
     return a.id2 < b.id2;
+}
+
+// A pair's finest level, for the candidates' FP64 expressions.
+struct Finest {
+    const StoreView *sv;
+    const PolyHdr *S, *T;
+    const Layer *gs, *gt;
+    bool geo;
+};
+__device__ __noinline__ double exact_lo(const Finest &f, uint32_t id1, uint32_t id2) {
+    return box_distance(layer_box(*f.gs, (int)id1), layer_box(*f.gt, (int)id2), f.geo);
+}
+__device__ __noinline__ double exact_hi(const Finest &f, uint32_t id1, uint32_t id2) {
+    const Box b = layer_box(*f.gs, (int)id1);
+    return box_max_distance_f(box_corners_f(b), box_corners_f(layer_box(*f.gt, (int)id2)), b.lo1, f.geo);
+}
+__device__ __noinline__ CandKey cand_key(const Finest &f, uint32_t id1, uint32_t id2) {  // Ideal.cpp:2587-2606
+    CandKey c;
+    c.id1 = (int32_t)id1;
+    c.id2 = (int32_t)id2;
+    c.lo = exact_lo(f, id1, id2);
+    c.hi = exact_hi(f, id1, id2);
+    const PolyHdr &S = *f.S, &T = *f.T;
+    const int pf = classify(f.sv->areas[S.pix + id1] + f.sv->areas[T.pix + id2],
+                            S.step_x * S.step_y + T.step_x * T.step_y, 20);
+    c.apx = c.lo + (double)c_mean20[pf] * (c.hi - c.lo);
+    return c;
+}
+
+// The sequence pairs of candidate (id1, id2), the last in order, from the
+// *from-th on (skipped ones not counted): 1 when the next one holds a distance
+// below the threshold, 0 when it ends the search (its minimum is below the
+// running minimum's start value, or there is none), 2 when it does neither.
+__device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id2, double thr, uint32_t *from, int lane,
+                                      unsigned long long &rechk) {
+    const SeqSet A = seq_set(*f.sv, *f.S, id1), B = seq_set(*f.sv, *f.T, id2);
+    uint32_t at = 0;
+    for (uint32_t ia = A.a; ia < A.b; ia++) {
+        const uint2 e1 = A.seq[ia];
+        for (uint32_t jb = B.a; jb < B.b; jb++) {
+            const uint2 e2 = B.seq[jb];
+            if (e1.y < 2 || e2.y < 2) continue;
+            if (at++ < *from) continue;
+            (*from)++;
+            const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
+            double m = 1.7976931348623157e308;
+            for (uint32_t k = lane; k < n1 + n2; k += 32) {
+                const uint32_t r = k < n1 ? k : k - n1, len = k < n1 ? e1.y - 1 : e2.y - 1;
+                const uint32_t pi = r / len, si = r % len;
+                const float2 *pr = k < n1 ? B.ring + e2.x : A.ring + e1.x;
+                const float2 *gr = k < n1 ? A.ring + e1.x : B.ring + e2.x;
+                const double d = pt_seg_dist(pr[pi], gr[si], gr[si + 1], f.geo);
+                m = m < d ? m : d;
+            }
+            for (int o = 16; o; o >>= 1) {
+                const double v = __shfl_xor_sync(0xffffffffu, m, o);
+                m = m < v ? m : v;
+            }
+            if (lane == 0) rechk += n1 + n2;
+            return m < thr ? 1 : (m < 100000.0 ? 0 : 2);
+        }
+    }
+    return 0;
 }
 
 // resident blocks of k_within per SM (its grid, and so its scratch)
@@ -760,29 +830,27 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                 nt = prune_side(ts, nt, sbb, lv, false, sx_low, cut, lane);
             }
             // smallest box max-distance; any <= d decides (Ideal.cpp:2557-2570)
+            uint32_t k1, k2;
+            bool v;
             float m2 = INFINITY;
-            for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+            for (Product p(ns, nt); p.next(lane, k1, k2, v);)
                 if (v) m2 = fminf(m2, lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)));
-                return false;
-            });
             m2 = warp_min(m2);
             if (sqrtf(m2) * 1.00001f < (float)a.thr * 0.999999f) {
                 yes = true;
                 break;
             }
+            const Finest fin{&sv, &S, &T, &gs, &gt, geo};
             const float m2_lim = m2 * 1.00002f;
             double mbd = INFINITY;
-            for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
+            for (Product p(ns, nt); p.next(lane, k1, k2, v);)
                 if (v && !(lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)) > m2_lim)) {
-                    const double lo1 = gs.mbr[1] + (int)(ss.p[k1] / (uint32_t)gs.dimx) * gs.step_y;
-                    const double md = box_max_distance_f(ss.fbox[k1], ts.fbox[k2], lo1, geo);
+                    const double md = exact_hi(fin, ss.p[k1], ts.p[k2]);
                     mbd = md < mbd ? md : mbd;
                 }
-                return false;
-            });
             for (int o = 16; o; o >>= 1) {
-                const double v = __shfl_xor_sync(full, mbd, o);
-                mbd = mbd < v ? mbd : v;
+                const double u = __shfl_xor_sync(full, mbd, o);
+                mbd = mbd < u ? mbd : u;
             }
             if (mbd <= a.thr) {
                 yes = true;
@@ -796,224 +864,152 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                 ns = prune_side(ss, ns, tbb, lv, true, sx_low, lim_up, lane);
                 nt = prune_side(ts, nt, sbb, lv, false, sx_low, lim_up, lane);
             }
-            auto exact_lo = [&](uint32_t k1, uint32_t k2) {
-                return box_distance(layer_box(gs, (int)ss.p[k1]), layer_box(gt, (int)ts.p[k2]), geo);
-            };
             auto keep_pair = [&](uint32_t k1, uint32_t k2, float &d) {
                 const float sx_ = lv.sx(k1);
                 d = lv.dist(ss.fbox[k1], ts.fbox[k2], sx_);
                 if (lv.low(d, sx_) > lim_up) return false;
                 if (lv.high(d, sx_) < lim_dn) return true;
-                const double lo = exact_lo(k1, k2);
+                const double lo = exact_lo(fin, ss.p[k1], ts.p[k2]);
                 return !(lo > a.thr) && lo < mbd;
             };
+            float d;
             if (s_next || t_next) {
-                for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
-                    float d;
+                for (Product p(ns, nt); p.next(lane, k1, k2, v);)
                     if (v && keep_pair(k1, k2, d)) {
                         set_bit(ss.bits, ss.p[k1]);
                         set_bit(ts.bits, ts.p[k2]);
                     }
-                    return false;
-                });
                 __syncwarp();
                 nqs = compact_bits(ss.bits, (uint32_t)(gs.dimx * gs.dimy), ss.q, lane);
                 nqt = compact_bits(ts.bits, (uint32_t)(gt.dimx * gt.dimy), ts.q, lane);
                 continue;
             }
-            // ---- the finest level: its kept pairs are the candidates
-            auto max_d = [&](uint32_t k1, uint32_t k2) {
-                const double lo1 = gs.mbr[1] + (int)(ss.p[k1] / (uint32_t)gs.dimx) * gs.step_y;
-                return box_max_distance_f(ss.fbox[k1], ts.fbox[k2], lo1, geo);
-            };
-            if (a.approx) {
-                // Within "-a" (query_within_polygon.cu:332-375): a pair left
-                // undecided is within when one of its surviving finest pixel
-                // pairs has apxDist = minDist + mean (maxDist - minDist) <= the
-                // distance, in float. mean is (1.0 - pf / category_count) * 0.5
-                // with both operands 8-bit integers (:352), so the quotient is 0
-                // and mean is 0.5; 0.5 (max - min) is exact in float, so
-                // contracting the sum into an FMA rounds the same.
-                unsigned nc = 0;
-                yes = for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
-                    float d;
-                    bool h = false;
-                    if (v && keep_pair(k1, k2, d)) {
-                        const float lo = (float)exact_lo(k1, k2), hi = (float)max_d(k1, k2);
-                        h = (double)(lo + 0.5f * (hi - lo)) <= a.thr;
-                        nc++;
-                    }
-                    return __any_sync(full, h) != 0;
-                });
-                my.cand += nc;
-                break;
-            }
-            const Near w = near_of(S, T, a.thr, geo);
-            auto cand_key = [&](uint32_t k1, uint32_t k2) {  // Ideal.cpp:2587-2606
-                CandKey c;
-                c.id1 = (int32_t)ss.p[k1];
-                c.id2 = (int32_t)ts.p[k2];
-                c.lo = exact_lo(k1, k2);
-                c.hi = max_d(k1, k2);
-                const int pf = classify(sv.areas[S.pix + c.id1] + sv.areas[T.pix + c.id2],
-                                        S.step_x * S.step_y + T.step_x * T.step_y, 20);
-                c.apx = c.lo + (double)c_mean20[pf] * (c.hi - c.lo);
-                return c;
-            };
-            // the candidates counted, and the closest one each lane meets
-            uint32_t cnt = 0;
+            // ---- the finest level: its kept pairs are the candidates. First
+            // they are counted, and each lane keeps the closest one it meets.
+            uint32_t cnt = 0, b1 = 0, b2 = 0;
             float bestd = INFINITY;
-            uint32_t b1 = 0, b2 = 0;
-            for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
-                float d;
+            bool apx_hit = false;
+            for (Product p(ns, nt); p.next(lane, k1, k2, v);)
                 if (v && keep_pair(k1, k2, d)) {
                     cnt++;
-                    d += sqrtf(lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)));
-                    if (d < bestd) bestd = d, b1 = k1, b2 = k2;
+                    if (a.approx) {
+                        // Within "-a" (query_within_polygon.cu:332-375): a pair left
+                        // undecided is within when one of its surviving finest pixel
+                        // pairs has apxDist = minDist + mean (maxDist - minDist) <=
+                        // the distance, in float. mean is (1.0 - pf /
+                        // category_count) * 0.5 with both operands 8-bit integers
+                        // (:352), so the quotient is 0 and mean is 0.5; 0.5 (max -
+                        // min) is exact in float, so contracting the sum into an FMA
+                        // rounds the same.
+                        const float lo = (float)exact_lo(fin, ss.p[k1], ts.p[k2]);
+                        const float hi = (float)exact_hi(fin, ss.p[k1], ts.p[k2]);
+                        apx_hit |= (double)(lo + 0.5f * (hi - lo)) <= a.thr;
+                    } else {
+                        d += sqrtf(lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)));
+                        if (d < bestd) bestd = d, b1 = ss.p[k1], b2 = ts.p[k2];
+                    }
                 }
-                return false;
-            });
             my.cand += cnt;
             for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(full, cnt, o);
+            if (a.approx) {
+                yes = __any_sync(full, apx_hit);
+                break;
+            }
             if (cnt == 0) break;
+            const Near w = near_of(S, T, a.thr, geo);
+            // queue of candidates (pixel ids): the closest ones, then all
+            const unsigned pm = __ballot_sync(full, bestd < INFINITY);
+            if (bestd < INFINITY) q[__popc(pm & ((1u << lane) - 1))] = make_uint2(b1, b2);
+            int qn = __popc(pm);
             // the last candidate in order, once known: only its first sequence
-            // pair counts, and last_hit has seen to that
-            bool know_last = false;
-            uint32_t last1 = 0, last2 = 0;
-            // the first sequence pair of candidate (id1, id2), the last in order
-            auto last_hit = [&](uint32_t id1, uint32_t id2) {
-                const SeqSet A = seq_set(sv, S, id1), B = seq_set(sv, T, id2);
-                for (uint32_t ia = A.a; ia < A.b; ia++) {
-                    const uint2 e1 = A.seq[ia];
-                    for (uint32_t jb = B.a; jb < B.b; jb++) {
-                        const uint2 e2 = B.seq[jb];
-                        if (e1.y < 2 || e2.y < 2) continue;
-                        const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
-                        double m = 1.7976931348623157e308;
-                        for (uint32_t k = lane; k < n1 + n2; k += 32) {
-                            const uint32_t r = k < n1 ? k : k - n1, len = k < n1 ? e1.y - 1 : e2.y - 1;
-                            const uint32_t pi = r / len, si = r % len;
-                            const float2 *pr = k < n1 ? B.ring + e2.x : A.ring + e1.x;
-                            const float2 *gr = k < n1 ? A.ring + e1.x : B.ring + e2.x;
-                            const double d = pt_seg_dist(pr[pi], gr[si], gr[si + 1], geo);
-                            m = m < d ? m : d;
-                        }
-                        for (int o = 16; o; o >>= 1) {
-                            const double v = __shfl_xor_sync(full, m, o);
-                            m = m < v ? m : v;
-                        }
-                        if (lane == 0) my.rechk += n1 + n2;
-                        if (m < w.thr) return true;
-                        if (m < 100000.0) return false;
-                        // the running minimum still at its start value: any
-                        // earlier distance below it ends the search here
-                        Near far = w;
-                        far.thr = 100000.0;
-                        far.c0 += 100100.f;
-                        const bool below = for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
-                            float d;
-                            v = v && keep_pair(k1, k2, d) && !(ss.p[k1] == id1 && ts.p[k2] == id2);
-                            return test_candidates(sv, S, T, v, v ? ss.p[k1] : 0, v ? ts.p[k2] : 0, far, geo, tab,
-                                                   lane, my) != 0;
-                        });
-                        if (below) return false;
-                    }
-                }
-                return false;
-            };
-            // lanes' candidates tested; true when one that counts has a hit
-            auto tested = [&](bool v, uint32_t id1, uint32_t id2, uint32_t k1, uint32_t k2) {
-                if (know_last && id1 == last1 && id2 == last2) v = false;
-                for (unsigned m = test_candidates(sv, S, T, v, id1, id2, w, geo, tab, lane, my); m; m &= m - 1) {
-                    if (know_last) return true;  // the last candidate was left out above
-                    // a hit counts unless its candidate is the last in order
-                    const int src = __ffs(m) - 1;
-                    const uint32_t h1 = __shfl_sync(full, k1, src), h2 = __shfl_sync(full, k2, src);
-                    const CandKey c = cand_key(h1, h2);
-                    const bool later = cnt > 1 && for_product(ns, nt, lane, [&](uint32_t a1, uint32_t a2, bool vv) {
-                        float d;
-                        return __any_sync(full, vv && keep_pair(a1, a2, d) && key_less(c, cand_key(a1, a2))) != 0;
-                    });
-                    if (later) return true;
-                    know_last = true;
-                    last1 = (uint32_t)c.id1;
-                    last2 = (uint32_t)c.id2;
-                    if (last_hit(last1, last2)) return true;
-                }
-                return false;
-            };
-            const bool probe = bestd < INFINITY;
-            yes = tested(probe, probe ? ss.p[b1] : 0, probe ? ts.p[b2] : 0, b1, b2);
-            if (!yes && cnt > (uint32_t)__popc(__ballot_sync(full, probe))) {
-                // queue entries are (k1, k2) until they are spilled as pixel ids
-                bool may_spill = a.sp.cap > 0;
-                uint32_t spent = 0;
-                int qn = 0;
-                auto flush = [&]() {
-                    for (int k = 0; k < qn; k += 32) {
-                        if (may_spill && (float)spent >= a.sp.budget) {
-                            if (!know_last) {  // the largest key of all
-                                CandKey top{-1.0, 0, 0, 0, 0};
-                                for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
-                                    float d;
-                                    if (v && keep_pair(k1, k2, d)) {
-                                        const CandKey c = cand_key(k1, k2);
-                                        if (key_less(top, c)) top = c;
-                                    }
-                                    return false;
-                                });
-                                for (int o = 16; o; o >>= 1) {
-                                    CandKey c;
-                                    c.apx = __shfl_xor_sync(full, top.apx, o);
-                                    c.lo = __shfl_xor_sync(full, top.lo, o);
-                                    c.hi = __shfl_xor_sync(full, top.hi, o);
-                                    c.id1 = __shfl_xor_sync(full, top.id1, o);
-                                    c.id2 = __shfl_xor_sync(full, top.id2, o);
-                                    if (key_less(top, c)) top = c;
-                                }
-                                know_last = true;
-                                last1 = (uint32_t)top.id1;
-                                last2 = (uint32_t)top.id2;
-                                if (last_hit(last1, last2)) return true;
-                            }
-                            // the last candidate stays out of the pool
-                            for (int e = k + lane; e < qn; e += 32) {
-                                uint2 c = make_uint2(ss.p[q[e].x], ts.p[q[e].y]);
-                                if (c.x == last1 && c.y == last2) c.x = ~0u;
-                                q[e] = c;
-                            }
+            // pair counts, and it is left out of everything else
+            bool know_last = false, may_spill = a.sp.cap > 0, more = cnt > (uint32_t)qn;
+            uint32_t last1 = ~0u, last2 = ~0u, spent = 0;
+            Product all(ns, nt);
+            __syncwarp();
+            for (;;) {
+                for (int k = 0; k < qn && !yes;) {
+                    bool check_last = false;
+                    if (may_spill && (float)spent >= a.sp.budget) {
+                        if (know_last) {
+                            for (int e = k + lane; e < qn; e += 32)
+                                if (q[e].x == last1 && q[e].y == last2) q[e].x = ~0u;
                             __syncwarp();
-                            if (spill_rest(a.sp, pid, q, k, qn, 0.f, lane, &head, &spilled)) return false;
-                            may_spill = false;  // the pool is full: back to this warp
-                            for (; k < qn; k += 32) {
-                                const bool v = k + lane < qn && q[k + lane].x != ~0u;
-                                const uint2 c = v ? q[k + lane] : make_uint2(0u, 0u);
-                                if (tested(v, c.x, c.y, 0, 0)) return true;
-                            }
-                            return false;
+                            if (spill_rest(a.sp, pid, q, k, qn, 0.f, lane, &head, &spilled)) break;
+                            may_spill = false;  // the pool is full
+                            continue;
                         }
-                        const bool v = k + lane < qn;
-                        const uint2 c = v ? q[k + lane] : make_uint2(0u, 0u);
+                        CandKey top{-1.0, 0, 0, 0, 0};  // the largest key of all
+                        for (Product p(ns, nt); p.next(lane, k1, k2, v);)
+                            if (v && keep_pair(k1, k2, d)) {
+                                const CandKey c = cand_key(fin, ss.p[k1], ts.p[k2]);
+                                if (key_less(top, c)) top = c;
+                            }
+                        for (int o = 16; o; o >>= 1) {
+                            CandKey c;
+                            c.apx = __shfl_xor_sync(full, top.apx, o);
+                            c.lo = __shfl_xor_sync(full, top.lo, o);
+                            c.hi = __shfl_xor_sync(full, top.hi, o);
+                            c.id1 = __shfl_xor_sync(full, top.id1, o);
+                            c.id2 = __shfl_xor_sync(full, top.id2, o);
+                            if (key_less(top, c)) top = c;
+                        }
+                        last1 = (uint32_t)top.id1;
+                        last2 = (uint32_t)top.id2;
+                        check_last = true;
+                    } else {
+                        const uint2 c = k + lane < qn ? q[k + lane] : make_uint2(~0u, ~0u);
+                        const bool ok = c.x != ~0u && !(know_last && c.x == last1 && c.y == last2);
+                        const unsigned hits = test_candidates(sv, S, T, ok, c.x, c.y, w, geo, tab, lane, my);
+                        k += 32;
                         spent += 32;
-                        if (tested(v, ss.p[c.x], ts.p[c.y], c.x, c.y)) return true;
+                        if (hits == 0) continue;
+                        yes = know_last || (hits & (hits - 1)) != 0;
+                        if (yes) break;
+                        // one hit: it counts unless its candidate is the last in order
+                        const int src = __ffs(hits) - 1;
+                        const uint32_t h1 = __shfl_sync(full, c.x, src), h2 = __shfl_sync(full, c.y, src);
+                        const CandKey key = cand_key(fin, h1, h2);
+                        for (Product p(ns, nt); !yes && p.next(lane, k1, k2, v);)
+                            yes = __any_sync(full, v && keep_pair(k1, k2, d) &&
+                                                       key_less(key, cand_key(fin, ss.p[k1], ts.p[k2])));
+                        if (yes) break;
+                        last1 = h1;
+                        last2 = h2;
+                        check_last = true;
                     }
-                    return false;
-                };
-                yes = for_product(ns, nt, lane, [&](uint32_t k1, uint32_t k2, bool v) {
-                    float d;
+                    if (check_last) {
+                        know_last = true;
+                        uint32_t from = 0;
+                        int r = last_pair(fin, last1, last2, w.thr, &from, lane, my.rechk);
+                        while (r == 2) {
+                            // the running minimum still at its start value unless
+                            // an earlier candidate holds a distance below it
+                            Near far = w;
+                            far.thr = 100000.0;
+                            far.c0 += 100100.f;
+                            unsigned below = 0;
+                            for (Product p(ns, nt); !below && p.next(lane, k1, k2, v);) {
+                                const bool ok = v && keep_pair(k1, k2, d) && !(ss.p[k1] == last1 && ts.p[k2] == last2);
+                                below = test_candidates(sv, S, T, ok, ok ? ss.p[k1] : 0, ok ? ts.p[k2] : 0, far, geo,
+                                                        tab, lane, my);
+                            }
+                            r = below ? 0 : last_pair(fin, last1, last2, w.thr, &from, lane, my.rechk);
+                        }
+                        yes = r == 1;
+                    }
+                }
+                if (yes || !more) break;
+                __syncwarp();
+                qn = 0;
+                while (qn + 32 <= kQueue) {
+                    more = all.next(lane, k1, k2, v);
+                    if (!more) break;
                     const bool keep = v && keep_pair(k1, k2, d);
                     const unsigned m = __ballot_sync(full, keep);
-                    if (keep) q[qn + __popc(m & ((1u << lane) - 1))] = make_uint2(k1, k2);
+                    if (keep) q[qn + __popc(m & ((1u << lane) - 1))] = make_uint2(ss.p[k1], ts.p[k2]);
                     qn += __popc(m);
-                    if (qn + 32 <= kQueue) return false;
-                    __syncwarp();
-                    const bool h = flush();
-                    qn = 0;
-                    __syncwarp();
-                    return h;
-                });
-                __syncwarp();
-                if (!yes && qn) yes = flush();
+                }
                 __syncwarp();
             }
             break;
