@@ -75,6 +75,8 @@ enum Scratch {
     S_XTILE = 44,   // bucketing (k_bucket): per-polygon tile and counter offsets
     S_XSLOT = 45,   // bucketing: (bucket, tile) counters and their scan
     S_XSTART = 34,  // column clip: first point of each polygon
+    S_SMALLP = 49,  // small polygons: counters, list, finished flags
+    S_SMALLSCR = 50, // small polygons: a scratch slice per block
 };
 
 // ------------------------------------------------------------ headers ----
@@ -919,6 +921,8 @@ struct Chunk {
     uint64_t col0, ncol; // fill sweep columns
     uint64_t row0, nrow; // scanline rows
     uint64_t hn0, vn0;   // global node bases of the chunk's first polygon
+    uint64_t nhn, nvn;   // nodes of all its polygons
+    const uint8_t *done; // polygons already rasterized (raster_small.cuh): nothing of theirs is touched
 };
 
 // Walk order: an FP32 estimate of the pixels an edge crosses, so that the
@@ -990,20 +994,6 @@ __global__ void k_tot_sizes(const unsigned long long *__restrict__ tot, const Po
     }
 }
 
-__global__ void k_set_node_bases(PolyHdr *__restrict__ hdr, uint32_t npoly, const uint64_t *__restrict__ sz,
-                                 const uint64_t *__restrict__ sc) {
-    uint64_t n1 = (uint64_t)npoly + 1;
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npoly; p += gridDim.x * blockDim.x) {
-        PolyHdr &h = hdr[p];
-        h.seq = sc[p];
-        h.n_seq = (uint32_t)sz[p];
-        h.hnode = sc[n1 + p];
-        h.n_hnodes = (uint32_t)sz[n1 + p];
-        h.vnode = sc[2 * n1 + p];
-        h.n_vnodes = (uint32_t)sz[2 * n1 + p];
-    }
-}
-
 __global__ void k_walk_count(const StoreView sv, PolyHdr *__restrict__ hdr, const WalkF *__restrict__ wf,
                              const uint64_t *__restrict__ off, Chunk ch, const uint32_t *__restrict__ perm, uint32_t *__restrict__ cnt) {
     uint64_t n1 = ch.ne + 1;
@@ -1038,7 +1028,7 @@ __global__ void k_load_counts(const PolyHdr *__restrict__ hdr, const uint64_t *_
          k += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t e = ch.e0 + k;
         uint32_t p = ch.p0 + find_segment(off + ch.p0, ch.np, e);
-        const bool ok = hdr[p].err == 0;
+        const bool ok = hdr[p].err == 0 && !ch.done[p];
         cnt[k] = ok ? c16[e] : 0u;
         cnt[n1 + k] = ok ? c16[ne_all + e] : 0u;
         cnt[2 * n1 + k] = ok ? c16[2 * ne_all + e] : 0u;
@@ -1151,7 +1141,7 @@ __global__ void k_seq_single(const PolyHdr *__restrict__ hdr, Chunk ch, const ui
                              uint2 *__restrict__ seq, uint32_t *__restrict__ pixcnt) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < ch.np; q += gridDim.x * blockDim.x) {
         const PolyHdr &h = hdr[ch.p0 + q];
-        if (h.err == 0 && cbase[q + 1] == cbase[q]) {
+        if (h.err == 0 && !ch.done[ch.p0 + q] && cbase[q + 1] == cbase[q]) {
             seq[h.seq] = make_uint2(0u, h.nv);
             pixcnt[h.pix - ch.pix0] += 1;
         }
@@ -1165,6 +1155,7 @@ __global__ void k_offsets(const PolyHdr *__restrict__ hdr, const uint64_t *__res
     for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ch.npix;
          g += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t p = ch.p0 + find_segment(pixbase + ch.p0, ch.np, g + ch.pix0);
+        if (ch.done[p]) continue;
         const PolyHdr &h = hdr[p];
         uint64_t lb = h.pix - ch.pix0;
         uint32_t i = (uint32_t)(g - lb);
@@ -1176,6 +1167,18 @@ __global__ void k_offsets(const PolyHdr *__restrict__ hdr, const uint64_t *__res
 __global__ void k_line_count(const uint64_t *__restrict__ key, uint64_t n, uint32_t *__restrict__ cnt) {
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
         atomicAdd(&cnt[key[k]], 1u);
+}
+
+// The nodes of finished polygons (Chunk::done) keep their places among the
+// chunk's: each such polygon's last line is given their number on top of its
+// own count of zero. The sorts go by the counts, so they pass them over.
+__global__ void k_line_gaps(const PolyHdr *__restrict__ hdr, Chunk ch, int vertical, uint64_t *__restrict__ lc64) {
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < ch.np; q += gridDim.x * blockDim.x) {
+        if (!ch.done[ch.p0 + q]) continue;
+        const PolyHdr &h = hdr[ch.p0 + q];
+        const uint64_t last = vertical ? h.vline - ch.v0 + (uint64_t)h.dimx + 1 : h.hline - ch.h0 + (uint64_t)h.dimy + 1;
+        lc64[last] += vertical ? h.n_vnodes : h.n_hnodes;
+    }
 }
 
 __global__ void k_line_scatter(const uint64_t *__restrict__ key, const double *__restrict__ val, uint64_t n,
@@ -1209,12 +1212,12 @@ __device__ inline double dval(uint64_t k) {
 // Lines of at most 32 nodes, most of them: one warp per line, a bitonic
 // network across the lanes (shuffles, no block barrier).
 __global__ void k_line_sort_warp(const double *__restrict__ in, double *__restrict__ out,
-                                 const uint64_t *__restrict__ start, uint64_t nseg) {
+                                 const uint64_t *__restrict__ start, const uint32_t *__restrict__ cnt, uint64_t nseg) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < nseg; l += nw) {
-        const uint64_t b = start[l], n = start[l + 1] - b;
+        const uint64_t b = start[l], n = cnt[l];
         if (n == 0 || n > 32) continue;
         uint64_t k = (uint64_t)lane < n ? dkey(in[b + lane]) : ~0ull;
         for (int size = 2; size <= 32; size <<= 1)
@@ -1231,13 +1234,14 @@ __global__ void k_line_sort_warp(const double *__restrict__ in, double *__restri
 // line in the warp's slice of shared memory (warp barriers only).
 constexpr int kLineMid = 256;
 __global__ void __launch_bounds__(256) k_line_sort_mid(const double *__restrict__ in, double *__restrict__ out,
-                                                       const uint64_t *__restrict__ start, uint64_t nseg) {
+                                                       const uint64_t *__restrict__ start,
+                                                       const uint32_t *__restrict__ cnt, uint64_t nseg) {
     __shared__ uint64_t sks[8][kLineMid];
     const int lane = threadIdx.x & 31;
     uint64_t *sk = sks[threadIdx.x >> 5];
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t l = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; l < nseg; l += nw) {
-        const uint64_t b = start[l], n = start[l + 1] - b;
+        const uint64_t b = start[l], n = cnt[l];
         if (n <= 32 || n > (uint64_t)kLineMid) continue;
         uint32_t N = 64;
         while (N < n) N <<= 1;
@@ -1263,12 +1267,13 @@ __global__ void __launch_bounds__(256) k_line_sort_mid(const double *__restrict_
 }
 
 __global__ void __launch_bounds__(256) k_line_sort(const double *__restrict__ in, double *__restrict__ out,
-                                                   const uint64_t *__restrict__ start, uint64_t nseg,
+                                                   const uint64_t *__restrict__ start,
+                                                   const uint32_t *__restrict__ cnt, uint64_t nseg,
                                                    uint64_t *__restrict__ big_b, uint64_t *__restrict__ big_e,
                                                    unsigned long long *__restrict__ nbig) {
     __shared__ uint64_t sk[kLineSortMax];
     for (uint64_t l = blockIdx.x; l < nseg; l += gridDim.x) {
-        const uint64_t b = start[l], n = start[l + 1] - b;
+        const uint64_t b = start[l], n = cnt[l];
         if (n <= (uint64_t)kLineMid) continue;  // k_line_sort_warp, k_line_sort_mid
         if (n > (uint64_t)kLineSortMax) {
             if (threadIdx.x == 0) {
@@ -1306,6 +1311,7 @@ __global__ void __launch_bounds__(256) k_line_sort(const double *__restrict__ in
 __global__ void k_line_offsets(PolyHdr *__restrict__ hdr, Chunk ch, int vertical, const uint32_t *__restrict__ cnt,
                                const uint64_t *__restrict__ start, uint32_t *__restrict__ loff) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < ch.np; q += gridDim.x * blockDim.x) {
+        if (ch.done[ch.p0 + q]) continue;
         PolyHdr &h = hdr[ch.p0 + q];
         uint64_t gl = vertical ? h.vline : h.hline;
         uint64_t lb = gl - (vertical ? ch.v0 : ch.h0);
@@ -1321,65 +1327,104 @@ __global__ void k_line_offsets(PolyHdr *__restrict__ hdr, Chunk ch, int vertical
     }
 }
 
-// Ideal.cpp:540-573: the scanline fill of the non-BORDER pixels.
+// Ideal.cpp:540-573: the scanline fill of one row's non-BORDER pixels, by a
+// warp, 32 pixels at a time; st: the row's classes, [i0, j0) its nodes. The
+// reference's sweep consumes, at each BORDER pixel x, the row's nodes up to
+// its right border start_x + step_x * (x + 1), and sets every other pixel from
+// the parity of the nodes consumed so far. The nodes are sorted, so the nodes
+// consumed before pixel x are those <= the right border of the last BORDER
+// pixel left of x: each pixel finds that pixel by a warp max-scan and counts
+// the nodes by binary search.
+__device__ __forceinline__ void scan_row(const PolyHdr &h, uint8_t *st, uint32_t i0, uint32_t j0, const double *nodes,
+                                         int cc, int lane) {
+    const unsigned full = 0xffffffffu;
+    const double start_x = h.mbr[0];
+    int carry = -1;  // last BORDER pixel of the earlier batches
+    for (int x0 = 0; x0 < h.dimx; x0 += 32) {
+        const int x = x0 + lane;
+        const bool v = x < h.dimx;
+        const uint8_t sx = v ? st[x] : 0;
+        const bool border = v && show_status(sx, cc) == 1;
+        int last = border ? x : -1;  // inclusive max-scan of BORDER positions
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(full, last, o);
+            if (lane >= o && t > last) last = t;
+        }
+        int before = __shfl_up_sync(full, last, 1);  // last BORDER pixel strictly left of x
+        if (lane == 0) before = -1;
+        if (before < carry) before = carry;
+        if (v && !border) {
+            bool isin = false;
+            if (before >= 0) {
+                const double rb = start_x + h.step_x * (before + 1);
+                uint32_t lo = i0, hi = j0;  // first node > rb
+                while (lo < hi) {
+                    const uint32_t mid = (lo + hi) >> 1;
+                    if (nodes[mid] <= rb) lo = mid + 1;
+                    else hi = mid;
+                }
+                isin = ((lo - i0) & 1u) != 0;
+            }
+            st[x] = isin ? 2 : 0;
+        }
+        const int tail = __shfl_sync(full, last, 31);
+        if (tail > carry) carry = tail;
+    }
+}
+
 __global__ void k_scanline(const PolyHdr *__restrict__ hdr, const uint64_t *__restrict__ rowbase, Chunk ch,
                            uint8_t *__restrict__ status, const uint32_t *__restrict__ hoff,
                            const double *__restrict__ hnodes, int cc) {
-    // One warp per row, 32 pixels at a time. The reference's sweep consumes,
-    // at each BORDER pixel x, the row's nodes up to its right border
-    // start_x + step_x * (x + 1), and sets every other pixel from the parity
-    // of the nodes consumed so far. The nodes are sorted, so the nodes
-    // consumed before pixel x are those <= the right border of the last
-    // BORDER pixel left of x: each pixel finds that pixel by a warp max-scan
-    // and counts the nodes by binary search.
-    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
     for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < ch.nrow; g += nw) {
         const uint32_t p = ch.p0 + find_segment(rowbase + ch.p0, ch.np, g + ch.row0);
         const PolyHdr &h = hdr[p];
         const int y = (int)(g + ch.row0 - rowbase[p]);
-        if (y < 1 || y >= h.dimy || h.err) continue;
-        const double start_x = h.mbr[0];
-        const uint32_t i0 = hoff[h.hline + y], j0 = hoff[h.hline + y + 1];
-        const double *nodes = hnodes + h.hnode;
-        uint8_t *st = status + h.st + (uint64_t)y * h.dimx;
-        int carry = -1;  // last BORDER pixel of the earlier batches
-        for (int x0 = 0; x0 < h.dimx; x0 += 32) {
-            const int x = x0 + lane;
-            const bool v = x < h.dimx;
-            const uint8_t sx = v ? st[x] : 0;
-            const bool border = v && show_status(sx, cc) == 1;
-            int last = border ? x : -1;  // inclusive max-scan of BORDER positions
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(full, last, o);
-                if (lane >= o && t > last) last = t;
-            }
-            int before = __shfl_up_sync(full, last, 1);  // last BORDER pixel strictly left of x
-            if (lane == 0) before = -1;
-            if (before < carry) before = carry;
-            if (v && !border) {
-                bool isin = false;
-                if (before >= 0) {
-                    const double rb = start_x + h.step_x * (before + 1);
-                    uint32_t lo = i0, hi = j0;  // first node > rb
-                    while (lo < hi) {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if (nodes[mid] <= rb) lo = mid + 1;
-                        else hi = mid;
-                    }
-                    isin = ((lo - i0) & 1u) != 0;
-                }
-                st[x] = isin ? 2 : 0;
-            }
-            const int tail = __shfl_sync(full, last, 31);
-            if (tail > carry) carry = tail;
-        }
+        if (y < 1 || y >= h.dimy || h.err || ch.done[p]) continue;
+        scan_row(h, status + h.st + (uint64_t)y * h.dimx, hoff[h.hline + y], hoff[h.hline + y + 1], hnodes + h.hnode,
+                 cc, lane);
     }
 }
 
+// Points the edge A -> B contributes to every column; their number. kEmit:
+// written from `at` on, with keys key0 + column. Both forms run the same
+// arithmetic, so they agree point for point. emitA: the ring's first edge.
+template <bool kEmit, typename K>
+__device__ __forceinline__ uint32_t clip_x_edge(const PolyHdr &h, const double *colx, const LineF *colf, int cert,
+                                                float2 A, float2 B, bool emitA, uint64_t at, K *okey, K key0,
+                                                float2 *opt) {
+    const float mnx = A.x < B.x ? A.x : B.x, mxx = A.x < B.x ? B.x : A.x;
+    const float mg = fmargin_f(mnx, mxx);
+    const float vstart = __fsub_rn(mnx, mg), vend = __fadd_rn(mxx, mg);
+    const double *lines = colx + h.col;
+    const LineF *lf = colf + h.col;
+    int c = first_line_f(lf, h.ncols, vstart);
+    uint32_t total = 0;
+    float2 buf[4];
+    const ClipXEdge E(A, B);
+    LineF L0 = lf[c];
+    float2 pi = make_float2(L0.rn, c < h.ncols ? E.ordf(lines[c], L0, cert) : 0.f);
+    for (; c < h.ncols && L0.dn <= vend; c++) {
+        const LineF L1 = lf[c + 1];  // the line Xi + step_x
+        const float2 pi1 = make_float2(L1.rn, E.ordf(lines[c + 1], L1, cert));
+        int m = clip_x_points(A, B, L0, L1, pi, pi1, emitA, kEmit ? buf : nullptr);
+        if (kEmit) {
+            for (int q = 0; q < m; q++) {
+                okey[at] = key0 + (K)c;
+                opt[at] = buf[q];
+                at++;
+            }
+        }
+        total += (uint32_t)m;
+        L0 = L1;
+        pi = pi1;
+    }
+    return total;
+}
+
 // Per edge: points contributed to every column (count pass or emit pass).
-// Both passes run the same arithmetic, so they agree point for point.
+template <bool kEmit>
 __global__ void __launch_bounds__(256, 4) k_clipx(const StoreView sv, const PolyHdr *__restrict__ hdr, const uint64_t *__restrict__ off,
                         Chunk ch, const uint32_t *__restrict__ perm, const double *__restrict__ colx,
                         const LineF *__restrict__ colf, int cert, uint32_t *__restrict__ cnt,
@@ -1390,41 +1435,15 @@ __global__ void __launch_bounds__(256, 4) k_clipx(const StoreView sv, const Poly
         uint64_t e = ch.e0 + k;
         uint32_t p = ch.p0 + find_segment(off + ch.p0, ch.np, e);
         const PolyHdr &h = hdr[p];
-        if (h.err) {
-            if (cnt) cnt[k] = 0;
+        if (h.err || ch.done[p]) {
+            if (!kEmit) cnt[k] = 0;
             continue;
         }
         uint32_t i = (uint32_t)(e - h.edge);
         const float2 *r = sv.ring + h.ring;
-        float2 A = r[i], B = r[i + 1];
-        const float mnx = A.x < B.x ? A.x : B.x, mxx = A.x < B.x ? B.x : A.x;
-        const float mg = fmargin_f(mnx, mxx);
-        const float vstart = __fsub_rn(mnx, mg), vend = __fadd_rn(mxx, mg);
-        const double *lines = colx + h.col;
-        const LineF *lf = colf + h.col;
-        int c = first_line_f(lf, h.ncols, vstart);
-        uint32_t total = 0;
-        uint64_t at = scan ? scan[k] : 0;
-        float2 buf[4];
-        const ClipXEdge E(A, B);
-        LineF L0 = lf[c];
-        float2 pi = make_float2(L0.rn, c < h.ncols ? E.ordf(lines[c], L0, cert) : 0.f);
-        for (; c < h.ncols && L0.dn <= vend; c++) {
-            const LineF L1 = lf[c + 1];  // the line Xi + step_x
-            const float2 pi1 = make_float2(L1.rn, E.ordf(lines[c + 1], L1, cert));
-            int m = clip_x_points(A, B, L0, L1, pi, pi1, i == 0, okey ? buf : nullptr);
-            if (okey) {
-                for (int q = 0; q < m; q++) {
-                    okey[at] = (h.col - ch.col0) + (uint64_t)c;
-                    opt[at] = buf[q];
-                    at++;
-                }
-            }
-            total += (uint32_t)m;
-            L0 = L1;
-            pi = pi1;
-        }
-        if (cnt) cnt[k] = total;
+        const uint32_t n = clip_x_edge<kEmit>(h, colx, colf, cert, r[i], r[i + 1], i == 0, kEmit ? scan[k] : 0, okey,
+                                              h.col - ch.col0, opt);
+        if (!kEmit) cnt[k] = n;
     }
 }
 
@@ -1752,8 +1771,56 @@ __global__ void k_cp_cost(const PolyHdr *__restrict__ hdr, const uint64_t *__res
     }
 }
 
+// Points the column-polygon edge A -> B contributes to each row; their number.
+// kEmit: written from `at` on with their rows. Both forms run the same
+// arithmetic, so they agree point for point.
+template <bool kEmit>
+__device__ __forceinline__ uint32_t clip_y_edge(const PolyHdr &h, const double *rowy, const LineF *rowf, int cert,
+                                                float2 A, float2 B, uint64_t at, uint32_t *okey, float2 *opt) {
+    const float mny = A.y < B.y ? A.y : B.y, mxy = A.y < B.y ? B.y : A.y;
+    const float mg = fmargin_f(mny, mxy);
+    const float vstart = __fsub_rn(mny, mg), vend = __fadd_rn(mxy, mg);
+    const double *lines = rowy + h.row;
+    const LineF *lf = rowf + h.row;
+    int r = first_line_f(lf, h.nrows, vstart);
+    uint32_t total = 0;
+    float2 buf[4];
+    const ClipYEdge E(A, B);
+    LineF L0 = lf[r];
+    // the point on line Yi, carried from the previous row's Yi1
+    // (horizontal edges take per-row abscissae instead)
+    float2 pc = make_float2(E.vert ? A.x : (E.general() && r < h.nrows ? E.abscf(lines[r], L0, cert) : 0.f), L0.rn);
+    for (; r < h.nrows && L0.dn <= vend; r++) {
+        const LineF L1 = lf[r + 1];  // the line Yi + step_y
+        float2 pi, pi1;
+        bool par = false;
+        if (E.horiz) {
+            // the edge lies on a row line only if A.y equals that double exactly
+            const bool on0 = L0.up == L0.dn && A.y == L0.rn, on1 = L1.up == L1.dn && A.y == L1.rn;
+            pi = make_float2(on0 ? A.x : (on1 ? -INFINITY : 0.f), L0.rn);
+            pi1 = make_float2(on0 ? -INFINITY : (on1 ? A.x : 0.f), L1.rn);
+            par = !on0 && !on1;
+        } else {
+            pi = pc;
+            pi1 = make_float2(E.vert ? A.x : E.abscf(lines[r + 1], L1, cert), L1.rn);
+            pc = pi1;
+        }
+        int k = clip_y_points(A, B, L0, L1, pi, pi1, par, kEmit ? buf : nullptr);
+        if (kEmit) {
+            for (int q = 0; q < k; q++) {  // the row within the column; the column is the edge's
+                okey[at] = (uint32_t)r;
+                opt[at] = buf[q];
+                at++;
+            }
+        }
+        total += (uint32_t)k;
+        L0 = L1;
+    }
+    return total;
+}
+
 // Per column-polygon edge: points contributed to each row (count or emit).
-// Both passes run the same arithmetic, so they agree point for point.
+template <bool kEmit>
 __global__ void __launch_bounds__(256, 4) k_clipy(const PolyHdr *__restrict__ hdr, Chunk ch, const uint32_t *__restrict__ perm,
                         const uint64_t *__restrict__ cpstart, const float2 *__restrict__ cpoly,
                         const uint32_t *__restrict__ cpcol, const uint32_t *__restrict__ colpoly, uint64_t ncp,
@@ -1764,51 +1831,10 @@ __global__ void __launch_bounds__(256, 4) k_clipy(const PolyHdr *__restrict__ hd
         const uint64_t j = perm[t];
         const uint64_t c = cpcol[j];
         uint32_t total = 0;
-        if (j + 1 < cpstart[c + 1]) {
-            const PolyHdr &h = hdr[colpoly[c]];
-            float2 A = cpoly[j], B = cpoly[j + 1];
-            const float mny = A.y < B.y ? A.y : B.y, mxy = A.y < B.y ? B.y : A.y;
-            const float mg = fmargin_f(mny, mxy);
-            const float vstart = __fsub_rn(mny, mg), vend = __fadd_rn(mxy, mg);
-            const double *lines = rowy + h.row;
-            const LineF *lf = rowf + h.row;
-            int r = first_line_f(lf, h.nrows, vstart);
-            uint64_t at = scan ? scan[j] : 0;
-            float2 buf[4];
-            const ClipYEdge E(A, B);
-            LineF L0 = lf[r];
-            // the point on line Yi, carried from the previous row's Yi1
-            // (horizontal edges take per-row abscissae instead)
-            float2 pc = make_float2(E.vert ? A.x : (E.general() && r < h.nrows ? E.abscf(lines[r], L0, cert) : 0.f),
-                                    L0.rn);
-            for (; r < h.nrows && L0.dn <= vend; r++) {
-                const LineF L1 = lf[r + 1];  // the line Yi + step_y
-                float2 pi, pi1;
-                bool par = false;
-                if (E.horiz) {
-                    // the edge lies on a row line only if A.y equals that double exactly
-                    const bool on0 = L0.up == L0.dn && A.y == L0.rn, on1 = L1.up == L1.dn && A.y == L1.rn;
-                    pi = make_float2(on0 ? A.x : (on1 ? -INFINITY : 0.f), L0.rn);
-                    pi1 = make_float2(on0 ? -INFINITY : (on1 ? A.x : 0.f), L1.rn);
-                    par = !on0 && !on1;
-                } else {
-                    pi = pc;
-                    pi1 = make_float2(E.vert ? A.x : E.abscf(lines[r + 1], L1, cert), L1.rn);
-                    pc = pi1;
-                }
-                int k = clip_y_points(A, B, L0, L1, pi, pi1, par, okey ? buf : nullptr);
-                if (okey && k) {
-                    for (int q = 0; q < k; q++) {  // the row within the column; the column is the edge's
-                        okey[at] = (uint32_t)r;
-                        opt[at] = buf[q];
-                        at++;
-                    }
-                }
-                total += (uint32_t)k;
-                L0 = L1;
-            }
-        }
-        if (cnt) cnt[j] = total;
+        if (j + 1 < cpstart[c + 1])
+            total = clip_y_edge<kEmit>(hdr[colpoly[c]], rowy, rowf, cert, cpoly[j], cpoly[j + 1], kEmit ? scan[j] : 0,
+                                       okey, opt);
+        if (!kEmit) cnt[j] = total;
     }
 }
 
@@ -1971,11 +1997,43 @@ __global__ void k_iota_u32(uint32_t *__restrict__ a, uint64_t n) {
         a[k] = (uint32_t)k;
 }
 
-// Per pixel: cell area (geometry_computation.h:275-297 over the cell's clip,
-// closed as Ideal.cpp:805-808 does) and the fill class (Ideal.cpp:880-914).
-// Each term is (double)p1.x * p2.y - (double)p2.x * p1.y: the two exact
-// products come from exact_fmul, so the FP64 pipe only takes the difference and
-// the running sum, in the reference's order.
+// Pixel id's cell: its area (geometry_computation.h:275-297 over the cell's n
+// clip points pt, closed as Ideal.cpp:805-808 does) and fill class
+// (Ideal.cpp:880-914). Each term is (double)p1.x * p2.y - (double)p2.x * p1.y:
+// the two exact products come from exact_fmul, so the FP64 pipe only takes the
+// difference and the running sum, in the reference's order.
+__device__ __forceinline__ void cell_area_class(const PolyHdr &h, uint32_t id, const float2 *pt, uint64_t n,
+                                                uint8_t *status, double *areas, int cc) {
+    const bool close = n > 0 && pt_ne(pt[0], pt[n - 1]);
+    const uint64_t m = n + (close ? 1 : 0);
+    double area = 0.0;
+    if (m >= 3) {
+        float2 p1 = pt[0];
+        for (uint64_t k = 0; k + 1 < m; k++) {
+            const float2 p2 = (k + 1 < n) ? pt[k + 1] : pt[0];
+            area += exact_fmul(p1.x, p2.y) - exact_fmul(p2.x, p1.y);
+            p1 = p2;
+        }
+        area = fabs(area) / 2.0;
+    }
+    const double pa = h.step_x * h.step_y;
+    const int type = classify(area, pa, cc);
+    uint8_t *st = status + id;
+    const uint8_t raw = *st;
+    if (raw == 1) {
+        int t2 = type < cc - 2 ? type : cc - 2;
+        *st = (uint8_t)(t2 > 1 ? t2 : 1);
+        areas[h.pix + id] = area;
+    } else if (raw == 2) {
+        *st = (uint8_t)(cc - 1);
+        areas[h.pix + id] = pa;
+    } else {
+        *st = 0;
+        areas[h.pix + id] = 0.0;
+    }
+}
+
+// Per pixel of the chunk: cell area and class.
 __global__ void k_cells(PolyHdr *__restrict__ hdr, const uint64_t *__restrict__ pixbase, Chunk ch,
                         const uint32_t *__restrict__ order, const uint32_t *__restrict__ cellend,
                         const uint64_t *__restrict__ yscan, const float2 *__restrict__ cpt,
@@ -1986,7 +2044,7 @@ __global__ void k_cells(PolyHdr *__restrict__ hdr, const uint64_t *__restrict__ 
         const uint64_t g = order ? order[t] : t;
         uint32_t p = ch.p0 + find_segment(pixbase + ch.p0, ch.np, g + ch.pix0);
         const PolyHdr &h = hdr[p];
-        if (h.err) continue;
+        if (h.err || ch.done[p]) continue;
         uint32_t id = (uint32_t)(g + ch.pix0 - h.pix);
         int x = (int)(id % (uint32_t)h.dimx), y = (int)(id / (uint32_t)h.dimx);
         if (x >= h.ncols || y >= h.nrows) continue;
@@ -1994,36 +2052,11 @@ __global__ void k_cells(PolyHdr *__restrict__ hdr, const uint64_t *__restrict__ 
         if (cpstart[cidx + 1] == cpstart[cidx]) continue;  // empty column: not visited
         const uint64_t colbase = yscan[cpstart[cidx]];  // the column's points (k_cell_bucket)
         const uint64_t b = colbase + (y ? cellend[g - (uint64_t)h.dimx] : 0u), e = colbase + cellend[g];
-        uint64_t n = e - b;
-        bool close = n > 0 && pt_ne(cpt[b], cpt[e - 1]);
-        uint64_t m = n + (close ? 1 : 0);
-        double area = 0.0;
-        if (m >= 3) {
-            float2 p1 = cpt[b];
-            for (uint64_t k = 0; k + 1 < m; k++) {
-                const float2 p2 = (k + 1 < n) ? cpt[b + k + 1] : cpt[b];
-                area += exact_fmul(p1.x, p2.y) - exact_fmul(p2.x, p1.y);
-                p1 = p2;
-            }
-            area = fabs(area) / 2.0;
-        }
-        double pa = h.step_x * h.step_y;
-        int type = classify(area, pa, cc);
-        uint8_t *st = status + h.st + id;
-        uint8_t raw = *st;
-        if (raw == 1) {
-            int t2 = type < cc - 2 ? type : cc - 2;
-            *st = (uint8_t)(t2 > 1 ? t2 : 1);
-            areas[h.pix + id] = area;
-        } else if (raw == 2) {
-            *st = (uint8_t)(cc - 1);
-            areas[h.pix + id] = pa;
-        } else {
-            *st = 0;
-            areas[h.pix + id] = 0.0;
-        }
+        cell_area_class(h, id, cpt + b, e - b, status + h.st, areas, cc);
     }
 }
+
+#include "raster_small.cuh"
 
 // ---------------------------------------------------------- hierarchy --
 // Ideal.cpp:1008-1059: each coarse pixel sums the finest areas under it. The
@@ -2076,9 +2109,44 @@ __global__ void k_merge(const PolyHdr *__restrict__ hdr, Chunk ch, uint8_t *__re
     }
 }
 
-__global__ void k_fill_u32(uint32_t *a, uint64_t n, uint32_t v) {
-    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x)
-        a[k] = v;
+// up to five buffers zeroed in one launch, 16 bytes at a time
+struct ZeroArgs {
+    uint4 *p[5];
+    uint64_t n[5];
+};
+__global__ void k_zero(ZeroArgs a) {
+    for (int t = 0; t < 5; t++)
+        for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < a.n[t];
+             k += (uint64_t)gridDim.x * blockDim.x)
+            a.p[t][k] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Exclusive prefix sums of short rows, a block each (row blockIdx.x of n).
+__global__ void __launch_bounds__(1024) k_scan_rows(const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
+                                                    uint64_t n) {
+    __shared__ uint64_t sums[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint64_t *row = in + blockIdx.x * n;
+    uint64_t *dst = out + blockIdx.x * n, run = 0;
+    for (uint64_t b = 0; b < n; b += 1024) {
+        const uint64_t i = b + threadIdx.x, v = i < n ? row[i] : 0;
+        uint64_t incl = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) sums[w] = incl;
+        __syncthreads();
+        uint64_t all = sums[lane];  // every warp scans the 32 sums
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t u = __shfl_up_sync(0xffffffffu, all, o);
+            if (lane >= o) all += u;
+        }
+        const uint64_t before = w ? __shfl_sync(0xffffffffu, all, w - 1) : 0;
+        if (i < n) dst[i] = run + before + incl - v;
+        run += __shfl_sync(0xffffffffu, all, 31);
+        __syncthreads();
+    }
 }
 
 __global__ void k_u32_to_u64(const uint32_t *__restrict__ a, uint64_t n, uint64_t *__restrict__ b) {
@@ -2207,9 +2275,100 @@ struct RasterCtx {
     int cc;
     int launches = 0;
     KTimer timer;
-    std::vector<uint64_t> hoff;  // per-polygon first edge (host copy of doff)
+    const uint64_t *hoff = nullptr;  // per-polygon first edge (the host's copy of doff)
     bool counts_kept = false;    // phase 1's per-edge counts are valid for phase 2
+    SmallInfo *info = nullptr;   // small polygons: counters, list, flags of the finished ones
+    uint32_t *list = nullptr;
+    uint8_t *done = nullptr;
 };
+
+// Exclusive prefix sums of `rows` rows of n. Up to 32,768 entries a block per
+// row in one launch (a block takes about 1.3 us per 1,024 entries), longer
+// rows by the library's scan (two launches a row).
+static int scan_rows(RasterCtx &R, const uint64_t *in, uint64_t *out, uint64_t n, int rows) {
+    if (n <= 32768) {
+        k_scan_rows<<<rows, 1024, 0, R.s->stream>>>(in, out, n);
+        R.launches++;
+        FARM_CUDA(cudaGetLastError());
+        return FARM_OK;
+    }
+    for (int t = 0; t < rows; t++) FARM_TRY(excl_scan(R.s, in + t * n, out + t * n, n));
+    return FARM_OK;
+}
+
+// FARM_RASTER_SMALL=0 sends every polygon through the pipeline, as the
+// variables that size its chunks do.
+static int small_on() {
+    const char *v = getenv("FARM_RASTER_SMALL");
+    return !(v && *v == '0') && !getenv("FARM_CHUNK_EDGES") && !getenv("FARM_CHUNK_CROSS") &&
+           !getenv("FARM_CHUNK_PIX");
+}
+
+// Phase 2 of the small polygons (raster_small.cuh). The scratch holds, per
+// block, the largest polygon's walk and, for the clips, twice its vertical
+// crossings (each lies in two columns) and its vertices, the cell clip four
+// times those; a polygon that needs more is left to the pipeline.
+static int raster_small(RasterCtx &R, const SmallInfo &info) {
+    farm_store *s = R.s;
+    SmallArgs a;
+    a.sv = s->view();
+    a.hdr = R.hdr;
+    a.wf = R.wf;
+    a.list = R.list;
+    a.off = R.doff;
+    a.c16 = s->s[S_ECNT16].as<uint16_t>();
+    a.ne_all = s->n_edges;
+    a.colx = R.colx;
+    a.rowy = R.rowy;
+    a.colf = R.colf;
+    a.rowf = R.rowf;
+    a.status = s->d_status.as<uint8_t>();
+    a.offset = s->d_offset.as<uint32_t>();
+    a.hoff = s->d_hoff.as<uint32_t>();
+    a.voff = s->d_voff.as<uint32_t>();
+    a.seq = s->d_seq.as<uint2>();
+    a.hnodes = s->d_hnodes.as<double>();
+    a.vnodes = s->d_vnodes.as<double>();
+    a.areas = s->d_areas.as<double>();
+    a.done = R.done;
+    a.info = R.info;
+    a.cap_e = (uint32_t)info.edges;
+    a.cap_c = (uint32_t)info.cross;
+    a.cap_h = (uint32_t)info.hn;
+    a.cap_v = (uint32_t)info.vn;
+    a.cap_x = (uint32_t)(2 * info.vn + info.edges + info.edges / 4 + 64);
+    a.cap_cp = a.cap_x + (uint32_t)info.lines;
+    a.cap_y = 4 * a.cap_x;
+    a.hash = 64;
+    while (a.hash < 2 * a.cap_x) a.hash <<= 1;
+    a.pix = (uint32_t)info.pix;
+    a.lines = (uint32_t)info.lines;
+    a.n = (uint32_t)info.n;
+    a.cert = R.cert;
+    a.cc = R.cc;
+    a.slice = small_scratch(a, nullptr, nullptr);
+    const bool many = a.n >= kSmallMany;
+    const uint64_t sms = (uint64_t)sm_count();
+    uint64_t wb = sms * (many ? kWalkBlocks64 : kBlocks256), fb = sms * (many ? kFillBlocks64 : kBlocks256);
+    if (wb > a.n) wb = a.n;
+    if (fb > a.n) fb = a.n;
+    FARM_TRY(s->s[S_SMALLSCR].ensure(a.slice * (wb > fb ? wb : fb) + 256));
+    a.scratch = s->s[S_SMALLSCR].as<unsigned char>();
+    const uint32_t warps = many ? 2 : 8, most = a.pix > a.lines ? a.pix : a.lines;
+    const int wsm = (int)(4 * (most + 1 + most * warps + 1));
+    const int fsm = (int)(4 * (a.pix + 1 + 3 * (a.lines + 1) + a.lines * warps + 1));
+    auto launch = [&](auto walk, auto fill, int threads) -> int {
+        FARM_CUDA(cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, wsm));
+        FARM_CUDA(cudaFuncSetAttribute(fill, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+        walk<<<(unsigned)wb, threads, wsm, s->stream>>>(a);
+        fill<<<(unsigned)fb, threads, fsm, s->stream>>>(a);
+        FARM_CUDA(cudaGetLastError());
+        R.launches += 2;
+        return FARM_OK;
+    };
+    return many ? launch(k_small_walk<64, kWalkBlocks64>, k_small_fill<64, kFillBlocks64>, 64)
+                : launch(k_small_walk<256, kBlocks256>, k_small_fill<256, kBlocks256>, 256);
+}
 
 // perm = items [0, n) ordered by key within tiles (k_local_order)
 static int local_order(RasterCtx &R, const uint8_t *key, uint64_t n, uint32_t *perm) {
@@ -2376,9 +2535,11 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
             L++;
         }
         k_u32_to_u64<<<gb(nl + 1), 256, 0, st>>>(lcnt, nl + 1, lc64);
-        L++;
+        k_line_gaps<<<gb(ch.np), 256, 0, st>>>(R.hdr, ch, vert, lc64);
+        L += 2;
         FARM_TRY(excl_scan(s, lc64, lstart, nl + 1));
-        FARM_TRY(s->s[S_TMP_B].ensure(8 * nn + 16));
+        const uint64_t room = vert ? ch.nvn : ch.nhn;  // the chunk's nodes, finished polygons' among them
+        FARM_TRY(s->s[S_TMP_B].ensure(8 * room + 16));
         double *unsorted = s->s[S_TMP_B].as<double>();
         if (nn) {
             k_line_scatter<<<gb(nn), 256, 0, st>>>(key, val, nn, lstart, lfill, unsorted);
@@ -2388,15 +2549,16 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
             unsigned long long *nbig = reinterpret_cast<unsigned long long *>(big_e + (nl + 1));
             FARM_CUDA(cudaMemsetAsync(nbig, 0, 8, st));
             unsigned lb = (unsigned)std::min<uint64_t>(nl, 8ull * sm_count());
-            k_line_sort_warp<<<warp_blocks(nl), 256, 0, st>>>(unsorted, nodes_out, lstart, nl);
-            k_line_sort_mid<<<warp_blocks(nl), 256, 0, st>>>(unsorted, nodes_out, lstart, nl);
-            k_line_sort<<<lb ? lb : 1, 256, 0, st>>>(unsorted, nodes_out, lstart, nl, big_b, big_e, nbig);
+            k_line_sort_warp<<<warp_blocks(nl), 256, 0, st>>>(unsorted, nodes_out, lstart, lcnt, nl);
+            k_line_sort_mid<<<warp_blocks(nl), 256, 0, st>>>(unsorted, nodes_out, lstart, lcnt, nl);
+            k_line_sort<<<lb ? lb : 1, 256, 0, st>>>(unsorted, nodes_out, lstart, lcnt, nl, big_b,
+                                                       big_e, nbig);
             L += 3;
             unsigned long long hbig = 0;
             FARM_TRY(d2h(s, &hbig, nbig, 8));
             if (hbig) {  // lines beyond the shared-memory sort: the library's segmented sort
                 FARM_TRY(cub_call(s, [&](void *t, size_t &b) {
-                    return cub::DeviceSegmentedSort::SortKeys(t, b, unsorted, nodes_out, (int64_t)nn, (int64_t)hbig,
+                    return cub::DeviceSegmentedSort::SortKeys(t, b, unsorted, nodes_out, (int64_t)room, (int64_t)hbig,
                                                               big_b, big_e, st);
                 }));
             }
@@ -2417,7 +2579,7 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
     FARM_CUDA(cudaMemsetAsync(xcnt, 0, 4 * ne1, st));
     const uint32_t *xperm = nullptr;
     FARM_TRY(edge_order(R, ch.p0, ch.np, ch.e0, ne, &xperm, 1));
-    R.timer.time(T_CLIPX, st, [&] { k_clipx<<<gb(ne), 256, 0, st>>>(sv, R.hdr, R.doff, ch, xperm, R.colx, R.colf, R.cert, xcnt, nullptr, nullptr, nullptr); });
+    R.timer.time(T_CLIPX, st, [&] { k_clipx<false><<<gb(ne), 256, 0, st>>>(sv, R.hdr, R.doff, ch, xperm, R.colx, R.colf, R.cert, xcnt, nullptr, nullptr, nullptr); });
     FARM_TRY(s->s[S_TMP_A].ensure(8 * ne1 + 16));
     uint64_t *x64 = s->s[S_TMP_A].as<uint64_t>();
     k_u32_to_u64<<<gb(ne1), 256, 0, st>>>(xcnt, ne1, x64);
@@ -2435,7 +2597,7 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
     uint64_t *xkey = s->s[S_VKEY].as<uint64_t>(), *xkey_s = s->s[S_VKEY2].as<uint64_t>();
     float2 *xpt = s->s[S_VVAL].as<float2>(), *xpt_s = s->s[S_VVAL2].as<float2>();
     if (nX) {
-        R.timer.time(T_CLIPX, st, [&] { k_clipx<<<gb(ne), 256, 0, st>>>(sv, R.hdr, R.doff, ch, xperm, R.colx, R.colf, R.cert, nullptr, xscan, xkey, xpt); });
+        R.timer.time(T_CLIPX, st, [&] { k_clipx<true><<<gb(ne), 256, 0, st>>>(sv, R.hdr, R.doff, ch, xperm, R.colx, R.colf, R.cert, nullptr, xscan, xkey, xpt); });
         L++;
         // group the points by column (k_bucket), in clip order within each
         FARM_TRY(s->s[S_XSTART].ensure(8 * ((uint64_t)ch.np + 1) + 64));
@@ -2570,7 +2732,7 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
     uint32_t *ycnt = s->s[S_CNT_E].as<uint32_t>();
     FARM_CUDA(cudaMemsetAsync(ycnt, 0, 4 * (nCP + 1), st));
     if (nCP) {
-        R.timer.time(T_CLIPY, st, [&] { k_clipy<<<gb(nCP), 256, 0, st>>>(R.hdr, ch, yperm, cpstart, cpoly, cpcol, colpoly, nCP, R.rowy, R.rowf, R.cert, ycnt,
+        R.timer.time(T_CLIPY, st, [&] { k_clipy<false><<<gb(nCP), 256, 0, st>>>(R.hdr, ch, yperm, cpstart, cpoly, cpcol, colpoly, nCP, R.rowy, R.rowf, R.cert, ycnt,
                                          nullptr, nullptr, nullptr); });
         L++;
     }
@@ -2596,7 +2758,7 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
     uint32_t *cellend = s->s[S_TMP_A].as<uint32_t>();
     FARM_CUDA(cudaMemsetAsync(cellend, 0, 4 * (ch.npix + 1), st));
     if (nY) {
-        R.timer.time(T_CLIPY, st, [&] { k_clipy<<<gb(nCP), 256, 0, st>>>(R.hdr, ch, yperm, cpstart, cpoly, cpcol, colpoly, nCP, R.rowy, R.rowf,
+        R.timer.time(T_CLIPY, st, [&] { k_clipy<true><<<gb(nCP), 256, 0, st>>>(R.hdr, ch, yperm, cpstart, cpoly, cpcol, colpoly, nCP, R.rowy, R.rowf,
                                          R.cert, nullptr, yscan, ykb, ypb); });
         L++;
     }
@@ -2626,17 +2788,6 @@ static int raster_chunk(RasterCtx &R, const Chunk &ch) {
                                          cpstart, s->d_status.as<uint8_t>(), s->d_areas.as<double>(), R.cc); });
     L++;
 
-    // ---- hierarchy
-    if (s->ropts.hierarchy) {
-        FARM_TRY(s->s[S_TMP_B].ensure(4ull * 32 * ch.np + 16));
-        uint32_t *fb = s->s[S_TMP_B].as<uint32_t>();
-        k_fill_u32<<<gb(32ull * ch.np), 256, 0, st>>>(fb, 32ull * ch.np, 0xFFFFFFFFu);
-        k_merge<<<gb(32ull * ch.np), 256, 0, st>>>(R.hdr, ch, s->d_status.as<uint8_t>(), s->d_areas.as<double>(), R.cc,
-                                                  0, fb);
-        k_merge<<<gb(32ull * ch.np), 256, 0, st>>>(R.hdr, ch, s->d_status.as<uint8_t>(), s->d_areas.as<double>(), R.cc,
-                                                  1, fb);
-        L += 3;
-    }
     FARM_CUDA(cudaGetLastError());
     return FARM_OK;
 }
@@ -2672,9 +2823,11 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
     R.n1 = (uint64_t)np + 1;
     R.cc = o->category_count;
     R.doff = s->d_off.as<uint64_t>();
-    R.hoff.resize((size_t)np + 1);
-    FARM_CUDA(cudaMemcpyAsync(R.hoff.data(), R.doff, 8 * ((size_t)np + 1), cudaMemcpyDeviceToHost, st));
-    FARM_CUDA(cudaStreamSynchronize(st));
+    if (s->h_cat.size() != (size_t)np + 1) {
+        set_error("the last load of the store failed");
+        return FARM_EINVAL;
+    }
+    R.hoff = s->h_cat.data();
     const uint64_t n1 = R.n1;
     FARM_TRY(s->d_hdr.ensure(sizeof(PolyHdr) * np));
     FARM_TRY(s->s[S_SIZES].ensure(9 * n1 * 8));
@@ -2685,9 +2838,9 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
     R.scan = scan;
     k_header<<<gb(32ull * np), 256, 0, st>>>(s->d_ring.as<float2>(), R.doff, np, rp, R.hdr, sizes);
     R.launches++;
-    for (int t = 0; t < 8; t++) FARM_TRY(excl_scan(s, sizes + t * n1, scan + t * n1, n1));
+    FARM_TRY(scan_rows(R, sizes, scan, n1, 8));
     uint64_t tot[8];
-    for (int t = 0; t < 8; t++) FARM_CUDA(cudaMemcpyAsync(&tot[t], scan + t * n1 + np, 8, cudaMemcpyDeviceToHost, st));
+    FARM_CUDA(cudaMemcpy2DAsync(tot, 8, scan + np, 8 * n1, 8, 8, cudaMemcpyDeviceToHost, st));
     FARM_CUDA(cudaStreamSynchronize(st));
     const uint64_t totP = tot[0], totStatus = tot[1], totOff = tot[2], totH = tot[3], totV = tot[4], totCol = tot[5],
                    totRow = tot[6];
@@ -2700,11 +2853,14 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
     FARM_TRY(s->s[S_ROWY].ensure(8 * totRow + 16));
     FARM_TRY(s->s[S_COLXF].ensure(16 * totCol + 16));
     FARM_TRY(s->s[S_ROWYF].ensure(16 * totRow + 16));
-    FARM_CUDA(cudaMemsetAsync(s->d_status.p, 0, totStatus + 16, st));
-    FARM_CUDA(cudaMemsetAsync(s->d_areas.p, 0, 8 * totP + 16, st));
-    FARM_CUDA(cudaMemsetAsync(s->d_offset.p, 0, 4 * totOff + 16, st));
-    FARM_CUDA(cudaMemsetAsync(s->d_hoff.p, 0, 4 * totH + 16, st));
-    FARM_CUDA(cudaMemsetAsync(s->d_voff.p, 0, 4 * totV + 16, st));
+    {
+        // every buffer's room is a multiple of 16 bytes past its entries
+        ZeroArgs z{{s->d_status.as<uint4>(), s->d_areas.as<uint4>(), s->d_offset.as<uint4>(), s->d_hoff.as<uint4>(),
+                    s->d_voff.as<uint4>()},
+                   {totStatus / 16 + 1, 8 * totP / 16 + 1, 4 * totOff / 16 + 1, 4 * totH / 16 + 1, 4 * totV / 16 + 1}};
+        k_zero<<<gb(totP), 256, 0, st>>>(z);
+        R.launches++;
+    }
     R.colx = s->s[S_COLX].as<double>();
     R.rowy = s->s[S_ROWY].as<double>();
     R.colf = s->s[S_COLXF].as<LineF>();
@@ -2727,6 +2883,7 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
     s->rtot.status_bytes = totStatus;
 
     // ---- phase 1: per-polygon totals size the sequence and node arrays
+    SmallInfo info{};
     {
         StoreView sv = s->view();
         FARM_TRY(s->s[S_TMP_B].ensure(3 * 8 * n1 + 16));
@@ -2742,9 +2899,9 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
             // polygons whose edges meet [e0, e0 + n)
             uint32_t pa = 0, pb = np;
             {
-                const std::vector<uint64_t> &ho = R.hoff;
-                pa = (uint32_t)(std::upper_bound(ho.begin(), ho.end(), e0) - ho.begin() - 1);
-                pb = (uint32_t)(std::lower_bound(ho.begin(), ho.end(), e0 + n) - ho.begin());
+                const uint64_t *ho = R.hoff, *he = ho + n1;
+                pa = (uint32_t)(std::upper_bound(ho, he, e0) - ho - 1);
+                pb = (uint32_t)(std::lower_bound(ho, he, e0 + n) - ho);
                 if (pb > np) pb = np;
             }
             const uint32_t *perm = nullptr;
@@ -2754,41 +2911,56 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
                                                                    c16, ne, ovf); });
             R.launches++;
         }
-        int h_ovf = 1;
-        FARM_TRY(d2h(s, &h_ovf, ovf, 4));
-        R.counts_kept = h_ovf == 0;
         FARM_TRY(s->s[S_TMP_A].ensure(2 * 3 * 8 * n1 + 16));
         uint64_t *sz = s->s[S_TMP_A].as<uint64_t>(), *sc = sz + 3 * n1;
         k_tot_sizes<<<gb(n1), 256, 0, st>>>(tot3, R.hdr, np, sz);
         R.launches++;
-        for (int t = 0; t < 3; t++) FARM_TRY(excl_scan(s, sz + t * n1, sc + t * n1, n1));
-        k_set_node_bases<<<gb(np), 256, 0, st>>>(R.hdr, np, sz, sc);
+        FARM_TRY(scan_rows(R, sz, sc, n1, 3));
+        FARM_TRY(s->s[S_SMALLP].ensure(512 + 4ull * np + np + 16));
+        R.info = s->s[S_SMALLP].as<SmallInfo>();
+        static_assert(sizeof(SmallInfo) <= 512, "the list follows at 512");
+        R.list = reinterpret_cast<uint32_t *>(s->s[S_SMALLP].as<unsigned char>() + 512);
+        R.done = reinterpret_cast<uint8_t *>(R.list + np);
+        FARM_CUDA(cudaMemsetAsync(R.info, 0, sizeof(SmallInfo), st));
+        k_small_pick<<<gb(np), 256, 0, st>>>(R.hdr, np, sz, sc, R.doff, small_on(), ovf, R.list, R.done, R.info);
         R.launches++;
-        uint64_t tseq, th, tv;
-        FARM_TRY(d2h(s, &tseq, sc + np, 8));
-        FARM_TRY(d2h(s, &th, sc + n1 + np, 8));
-        FARM_TRY(d2h(s, &tv, sc + 2 * n1 + np, 8));
-        FARM_TRY(s->d_seq.ensure(8 * tseq + 16));
-        FARM_TRY(s->d_hnodes.ensure(8 * th + 16));
-        FARM_TRY(s->d_vnodes.ensure(8 * tv + 16));
-        s->tot_seq = tseq;
-        s->rtot.sequences = tseq;
-        s->rtot.hnodes = th;
-        s->rtot.vnodes = tv;
+        int h_ovf = 1;
+        FARM_CUDA(cudaMemcpyAsync(&h_ovf, ovf, 4, cudaMemcpyDeviceToHost, st));
+        FARM_CUDA(cudaMemcpyAsync(&info, R.info, sizeof info, cudaMemcpyDeviceToHost, st));
+        FARM_CUDA(cudaStreamSynchronize(st));
+        R.counts_kept = h_ovf == 0;
+        FARM_TRY(s->d_seq.ensure(8 * info.seq + 16));
+        FARM_TRY(s->d_hnodes.ensure(8 * info.hnodes + 16));
+        FARM_TRY(s->d_vnodes.ensure(8 * info.vnodes + 16));
+        s->tot_seq = info.seq;
+        s->rtot.sequences = info.seq;
+        s->rtot.hnodes = info.hnodes;
+        s->rtot.vnodes = info.vnodes;
     }
 
-    // ---- phase 2: chunks
-    std::vector<uint64_t> hscan(8 * n1);
-    std::vector<PolyHdr> hh(np);
-    FARM_CUDA(cudaMemcpyAsync(hscan.data(), scan, 8 * 8 * n1, cudaMemcpyDeviceToHost, st));
-    FARM_CUDA(cudaMemcpyAsync(hh.data(), R.hdr, sizeof(PolyHdr) * np, cudaMemcpyDeviceToHost, st));
-    FARM_CUDA(cudaStreamSynchronize(st));
-    const std::vector<uint64_t> &hoff = R.hoff;
+    // ---- phase 2, small polygons: a block each
+    if (info.n) {
+        FARM_TRY(raster_small(R, info));
+        FARM_CUDA(cudaMemcpyAsync(&info, R.info, sizeof info, cudaMemcpyDeviceToHost, st));
+        if (info.n == np) FARM_CUDA(cudaStreamSynchronize(st));  // else read with the headers below
+        s->rtot.chunks++;
+    }
+    const bool all_small = info.n == np && info.left == 0;
+
+    // ---- phase 2, the rest: chunks
+    std::vector<uint64_t> hscan(all_small ? 0 : 8 * n1);
+    std::vector<PolyHdr> hh(all_small ? 0 : np);
+    if (!all_small) {
+        FARM_CUDA(cudaMemcpyAsync(hscan.data(), scan, 8 * 8 * n1, cudaMemcpyDeviceToHost, st));
+        FARM_CUDA(cudaMemcpyAsync(hh.data(), R.hdr, sizeof(PolyHdr) * np, cudaMemcpyDeviceToHost, st));
+        FARM_CUDA(cudaStreamSynchronize(st));
+    }
+    const uint64_t *hoff = R.hoff;
     const uint64_t kChunkEdges = env_u64("FARM_CHUNK_EDGES", 1ull << 27);
     const uint64_t kChunkCross = env_u64("FARM_CHUNK_CROSS", 1ull << 27);
     const uint64_t kChunkPix = env_u64("FARM_CHUNK_PIX", 1ull << 27);
     uint32_t p = 0;
-    while (p < np) {
+    while (!all_small && p < np) {
         uint32_t q = p;
         uint64_t ce = 0, cc = 0, cp = 0;
         do {
@@ -2815,8 +2987,29 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
         ch.nrow = hscan[7 * n1 + q] - ch.row0;
         ch.hn0 = hh[p].hnode;
         ch.vn0 = hh[p].vnode;
+        ch.nhn = hh[q - 1].hnode + hh[q - 1].n_hnodes - ch.hn0;
+        ch.nvn = hh[q - 1].vnode + hh[q - 1].n_vnodes - ch.vn0;
+        ch.done = R.done;
         FARM_TRY(raster_chunk(R, ch));
         p = q;
+    }
+    if (info.n) {
+        s->rtot.crossings += info.crossings;
+        s->rtot.clip_x_points += info.clip_x;
+        s->rtot.clip_y_points += info.clip_y;
+    }
+    // ---- hierarchy
+    if (o->hierarchy) {
+        Chunk ch{};
+        ch.np = np;
+        FARM_TRY(s->s[S_TMP_B].ensure(4ull * 32 * np + 16));
+        uint32_t *fb = s->s[S_TMP_B].as<uint32_t>();
+        FARM_CUDA(cudaMemsetAsync(fb, 0xFF, 4ull * 32 * np, st));
+        for (int pass = 0; pass < 2; pass++)
+            k_merge<<<gb(32ull * np), 256, 0, st>>>(R.hdr, ch, s->d_status.as<uint8_t>(), s->d_areas.as<double>(),
+                                                    R.cc, pass, fb);
+        R.launches += 2;
+        FARM_CUDA(cudaGetLastError());
     }
     (void)totRow;
 
