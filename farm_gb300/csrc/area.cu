@@ -14,11 +14,12 @@
 // other polygon's raster, and flips at each crossing after it.
 //
 // Work: items are (pair, side, chunk of that side's edges), taken by persistent
-// warps from a global counter. A lane takes one edge: it finds its crossings
-// through the other polygon's raster (edge sequences of the BORDER pixels
-// around the edge, each crossing edge counted at its first listing), and adds
-// its signed inside length: the leaving parameters minus the entering ones,
-// plus the tail when it ends inside. Per-item
+// warps from a global counter. A lane holds one edge; the warp walks the window
+// of the other polygon's raster around all its edges together, queues the edges
+// listed there, and every lane tests its edge against each (each crossing edge
+// counted at its first listing). An edge's share is its signed inside length:
+// the leaving parameters minus the entering ones, plus the tail when it ends
+// inside. Per-item
 // partial sums are reduced per pair in a fixed order (deterministic results).
 // Coordinates are taken relative to the pair's source first vertex.
 // General position is assumed (no collinear overlaps, no crossing exactly at a
@@ -31,23 +32,20 @@
 #include <vector>
 
 #include "common.cuh"
+#include "segments.cuh"
 
 namespace farm {
 
-// The two tuning knobs of the area pass by size bucket (bucket b holds pairs
-// whose larger edge count has floor(log2) == b), chosen by farm_area_autotune:
-// c, the edges per work item (default 16), and w, the candidate-window size in
-// pixels above which an edge is searched by the whole warp instead of its own
-// lane (default 200).
+// The tuning knob of the area pass by size bucket (bucket b holds pairs whose
+// larger edge count has floor(log2) == b), chosen by farm_area_autotune: the
+// edges per work item (default 16).
 struct Chunks {
     uint16_t c[32];
-    uint16_t w[32];
     __host__ __device__ static int bucket(uint32_t es, uint32_t et) {
         uint32_t m = es > et ? es : et;
         return m ? 31 - clz32(m) : 0;
     }
     __host__ __device__ uint32_t of(uint32_t es, uint32_t et) const { return c[bucket(es, et)]; }
-    __host__ __device__ uint32_t wide_of(uint32_t es, uint32_t et) const { return w[bucket(es, et)]; }
     __host__ __device__ static int clz32(uint32_t x) {
 #ifdef __CUDA_ARCH__
         return __clz(x);
@@ -74,13 +72,25 @@ struct AreaArgs {
     int spread;                    // take items in a spread order (see k_area)
 };
 
+// A sum with the rounding errors of its additions (Knuth's TwoSum) beside it: an
+// edge's crossing parameters are added in the order its slices meet them, which
+// groups entering and leaving ones, so partial sums grow and would round.
+struct Sum2 {
+    double s = 0, e = 0;
+    __device__ __forceinline__ void add(double v) {
+        const double t = __dadd_rn(s, v), b = __dsub_rn(t, s);
+        e = __dadd_rn(e, __dadd_rn(__dsub_rn(s, __dsub_rn(t, b)), __dsub_rn(v, b)));
+        s = t;
+    }
+};
+
 __device__ __forceinline__ double cross2(double ax, double ay, double bx, double by) { return ax * by - ay * bx; }
 
-// Point-in-polygon of (px, py) for polygon H through its raster: a ray to the
-// right along the pixel row; the first non-BORDER pixel tells its side, edges
-// of BORDER pixels before it flip the parity (each edge counted in the pixel
-// whose x-range holds its crossing).
-__device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, double px, double py, int cc) {
+// Point-in-polygon of (px, py) for polygon H through its raster, by a warp: a
+// ray to the right along the pixel row; the first non-BORDER pixel tells its
+// side, edges of BORDER pixels before it flip the parity (each edge counted in
+// the pixel whose x-range holds its crossing).
+__device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, double px, double py, int cc, int lane) {
     if (px < H.mbr[0] || px > H.mbr[2] || py < H.mbr[1] || py > H.mbr[3]) return false;
     int row = offset_y(H.mbr, H.step_y, H.dimy, py);
     int col = offset_x(H.mbr, H.step_x, H.dimx, px);
@@ -95,169 +105,106 @@ __device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, double px, dou
         if (s != 1) return c == col ? (s == 2) : (odd ^ (s == 2));
         double x_lo = c == col ? -1e300 : H.mbr[0] + c * H.step_x;
         double x_hi = c == H.dimx - 1 ? 1e300 : H.mbr[0] + (c + 1) * H.step_x;
-        for (uint32_t q = off[pid]; q < off[pid + 1]; q++) {
+        bool flip = false;
+        for (uint32_t q = off[pid] + lane; q < off[pid + 1]; q += 32) {
             uint2 sq = seq[q];
             for (uint32_t k = 0; k < sq.y; k++) {
                 float2 a = r[sq.x + k], b = r[sq.x + k + 1];
                 if ((a.y > py) != (b.y > py)) {
                     double xi = (double)a.x + (py - a.y) * ((double)b.x - a.x) / ((double)b.y - a.y);
-                    if (xi > px && xi >= x_lo && xi < x_hi) odd = !odd;
+                    if (xi > px && xi >= x_lo && xi < x_hi) flip = !flip;
                 }
             }
         }
+        odd ^= __popc(__ballot_sync(0xffffffffu, flip)) & 1;
     }
     return odd;  // past the raster: outside, so the crossings decide
 }
 
-// The pixels of polygon O searched for edges that may cross segment
-// (x0, y0) -> (x1, y1): rows sy..ey of a one-pixel-padded window, and in each
-// row the columns row_cols gives.
-struct SegWin {
-    double x0, y0, x1, y1;
-    int sx, ex, sy, ey;
+// An edge in the other polygon's pixel units, with the rounding of those (the
+// differences are taken in double): m is far above it.
+struct EdgeUV {
+    float u0, v0, u1, v1, m;
 };
-
-__device__ __forceinline__ bool seg_window(const PolyHdr &O, double x0, double y0, double x1, double y1, SegWin &w) {
-    const double mnx = fmin(x0, x1), mxx = fmax(x0, x1), mny = fmin(y0, y1), mxy = fmax(y0, y1);
-    if (mxx < O.mbr[0] || mnx > O.mbr[2] || mxy < O.mbr[1] || mny > O.mbr[3]) return false;
-    w.x0 = x0;
-    w.y0 = y0;
-    w.x1 = x1;
-    w.y1 = y1;
-    w.sx = offset_x(O.mbr, O.step_x, O.dimx, mnx) - 1;
-    w.ex = offset_x(O.mbr, O.step_x, O.dimx, mxx) + 1;
-    w.sy = offset_y(O.mbr, O.step_y, O.dimy, mny) - 1;
-    w.ey = offset_y(O.mbr, O.step_y, O.dimy, mxy) + 1;
-    w.sx = w.sx < 0 ? 0 : w.sx;
-    w.sy = w.sy < 0 ? 0 : w.sy;
-    w.ex = w.ex >= O.dimx ? O.dimx - 1 : w.ex;
-    w.ey = w.ey >= O.dimy ? O.dimy - 1 : w.ey;
-    return true;
+__device__ __forceinline__ EdgeUV edge_uv(const PolyHdr &O, float2 P, float2 Q) {
+    const float sx = (float)O.step_x, sy = (float)O.step_y;
+    EdgeUV e;
+    e.u0 = (float)((double)P.x - O.mbr[0]) / sx;
+    e.v0 = (float)((double)P.y - O.mbr[1]) / sy;
+    e.u1 = (float)((double)Q.x - O.mbr[0]) / sx;
+    e.v1 = (float)((double)Q.y - O.mbr[1]) / sy;
+    e.m = 0.01f + 1e-6f * fmaxf(fmaxf(fabsf(e.u0), fabsf(e.u1)), fmaxf(fabsf(e.v0), fabsf(e.v1)));
+    return e;
 }
 
-// Columns xa..xb of window row y; false when the row holds none. Only the
-// columns the segment spans within rows y-1 .. y+1, one more on either side:
-// every pixel within a pixel of the segment's path, which holds every edge of
-// O that the segment crosses (an edge is listed in each pixel it passes
-// through, or, where the reference's walk cuts a grid corner, in the diagonal
-// neighbours).
-// Both for_candidate_edges and first_listing call it, so its products and sums
-// are explicit roundings: no contraction may differ between the two.
-__device__ __forceinline__ bool row_cols(const PolyHdr &O, const SegWin &w, int y, int &xa, int &xb) {
-    xa = w.sx;
-    xb = w.ex;
-    if (w.y1 != w.y0) {
-        const double ylo = __dadd_rn(O.mbr[1], __dmul_rn((double)(y - 1), O.step_y));
-        const double yhi = __dadd_rn(O.mbr[1], __dmul_rn((double)(y + 2), O.step_y));
-        const double dy = __dsub_rn(w.y1, w.y0);
-        double ta = __ddiv_rn(__dsub_rn(ylo, w.y0), dy), tb = __ddiv_rn(__dsub_rn(yhi, w.y0), dy);
-        if (ta > tb) {
-            const double tmp = ta;
-            ta = tb;
-            tb = tmp;
-        }
-        ta = ta < 0 ? 0 : ta;
-        tb = tb > 1 ? 1 : tb;
-        if (ta > tb) return false;
-        const double dx = __dsub_rn(w.x1, w.x0);
-        double xa_ = __dadd_rn(w.x0, __dmul_rn(ta, dx)), xb_ = __dadd_rn(w.x0, __dmul_rn(tb, dx));
-        if (xa_ > xb_) {
-            const double tmp = xa_;
-            xa_ = xb_;
-            xb_ = tmp;
-        }
-        const int ca = offset_x(O.mbr, O.step_x, O.dimx, xa_) - 1, cb = offset_x(O.mbr, O.step_x, O.dimx, xb_) + 1;
-        xa = ca > w.sx ? ca : w.sx;
-        xb = cb < w.ex ? cb : w.ex;
+// Columns of row y searched for edges that may cross edge e: those the edge
+// spans within rows y - 1 .. y + 1 and one more on either side, every pixel
+// within a pixel of its path. That holds every edge of O that it crosses (an
+// edge is listed in each pixel it passes through, or, where the reference's
+// walk cuts a grid corner, in the diagonal neighbours). lo > hi: none.
+__device__ __forceinline__ int2 edge_columns(const EdgeUV &e, int y, int dimx) {
+    const float a = (float)(y - 1) - e.m, b = (float)(y + 2) + e.m;
+    if (fmaxf(e.v0, e.v1) < a || fminf(e.v0, e.v1) > b) return make_int2(0x7fffffff, -1);
+    const float du = e.u1 - e.u0, dv = e.v1 - e.v0;
+    float t0 = 0.f, t1 = 1.f;
+    if (fabsf(dv) > e.m) {
+        const float p = (a - e.v0) / dv, q = (b - e.v0) / dv;
+        t0 = fmaxf(0.f, fminf(p, q));
+        t1 = fminf(1.f, fmaxf(p, q));
     }
-    return true;
+    const float p = e.u0 + t0 * du, q = e.u0 + t1 * du;
+    const float lo = floorf(fminf(p, q) - e.m) - 1.f, hi = floorf(fmaxf(p, q) + e.m) + 1.f;
+    const int l = lo > 0.f ? (lo < 2e9f ? (int)lo : 0x7fffffff) : 0;
+    const int h = hi < (float)(dimx - 1) ? (hi >= 0.f ? (int)hi : -1) : dimx - 1;
+    return l <= h ? make_int2(l, h) : make_int2(0x7fffffff, -1);
 }
 
-// Column ranges of the last kRowCache window rows the enumeration computed,
-// in a ring indexed by row & (kRowCache - 1) (an empty row is stored as
-// xa > xb), so that first_listing reads them instead of recomputing: the
-// earlier listings of an edge that crosses the segment lie within a few rows
-// of the current one, even when the window spans hundreds of rows.
-constexpr int kRowCache = 16;
-struct RowCache {
-    int2 r[kRowCache];
+// whether the edge has a length and its box meets O's
+__device__ __forceinline__ bool edge_meets(const PolyHdr &O, float2 P, float2 Q) {
+    return (P.x != Q.x || P.y != Q.y) && !(fmaxf(P.x, Q.x) < O.mbr[0] || fminf(P.x, Q.x) > O.mbr[2] ||
+                                           fmaxf(P.y, Q.y) < O.mbr[1] || fminf(P.y, Q.y) > O.mbr[3]);
+}
+
+// A group of up to 32 consecutive edges [first, first + n) of a ring, searched
+// together: the window's columns of row y are those between the first and the
+// last that any of them searches.
+struct Group {
+    const PolyHdr *O;
+    const float2 *ring;
+    uint32_t first, n;
+    int sy;
 };
-
-// Edges of polygon O listed by the BORDER pixels of window w, row by row, left
-// to right, sequence by sequence. Calls f(pixel, first column of its row,
-// sequence index, edge index); an edge listed by several of these pixels (or
-// sequences) comes once per listing. Pixel ids grow in this order (row-major).
-template <typename F>
-__device__ void for_candidate_edges(const StoreView &sv, const PolyHdr &O, const SegWin &w, int cc, RowCache &rc,
-                                    F f) {
-    const uint8_t *st = sv.status + O.st;
-    const uint32_t *off = sv.offset + O.off;
-    const uint2 *seq = sv.seq + O.seq;
-    for (int y = w.sy; y <= w.ey; y++) {
-        int xa, xb;
-        const bool ok = row_cols(O, w, y, xa, xb);
-        rc.r[y & (kRowCache - 1)] = ok ? make_int2(xa, xb) : make_int2(1, 0);
-        if (!ok) continue;
-        for (int x = xa; x <= xb; x++) {
-            const uint32_t pid = (uint32_t)(y * O.dimx + x);
-            if (show_status(st[pid], cc) != 1) continue;
-            for (uint32_t q = off[pid]; q < off[pid + 1]; q++) {
-                const uint2 sq = seq[q];
-                for (uint32_t k = 0; k < sq.y; k++) f(pid, xa, q, sq.x + k);
-            }
-        }
+constexpr int kRowCache = 256;  // a window's last rows, kept by row & (kRowCache - 1)
+constexpr int kQueueRows = 64;  // rows a queued edge may wait
+// the group's columns of a row that is no longer kept
+__device__ __noinline__ int2 group_columns(const Group &g, int y) {
+    int2 c = make_int2(0x7fffffff, -1);
+    for (uint32_t k = 0; k < g.n; k++) {
+        const float2 P = g.ring[g.first + k], Q = g.ring[g.first + k + 1];
+        if (!edge_meets(*g.O, P, Q)) continue;
+        const int2 e = edge_columns(edge_uv(*g.O, P, Q), y, g.O->dimx);
+        c.x = min(c.x, e.x);
+        c.y = max(c.y, e.y);
     }
+    return c;
 }
 
-// The same enumeration with the warp sharing one segment: every lane walks
-// the window in the same order (so each holds the same row cache), and the
-// candidate listings of each row — all sequences of all its pixels, in
-// order — are dealt to the lanes round robin; f runs for the lane's share.
-// A long edge across a dense polygon meets thousands of candidates, which a
-// single lane would otherwise test one after another.
-template <typename F>
-__device__ void for_candidate_edges_warp(const StoreView &sv, const PolyHdr &O, const SegWin &w, int cc,
-                                         RowCache &rc, int lane, F f) {
-    const uint8_t *st = sv.status + O.st;
-    const uint32_t *off = sv.offset + O.off;
-    const uint2 *seq = sv.seq + O.seq;
-    for (int y = w.sy; y <= w.ey; y++) {
-        int xa, xb;
-        const bool ok = row_cols(O, w, y, xa, xb);
-        rc.r[y & (kRowCache - 1)] = ok ? make_int2(xa, xb) : make_int2(1, 0);
-        if (!ok) continue;
-        uint32_t base = 0;  // listings of the row before the current sequence
-        for (int x = xa; x <= xb; x++) {
-            const uint32_t pid = (uint32_t)(y * O.dimx + x);
-            if (show_status(st[pid], cc) != 1) continue;
-            for (uint32_t q = off[pid]; q < off[pid + 1]; q++) {
-                const uint2 sq = seq[q];
-                // this lane's listings k of the sequence: (base + k) % 32 == lane
-                uint32_t k = (uint32_t)((lane - (int)(base & 31u) + 32) & 31);
-                for (; k < sq.y; k += 32) f(pid, xa, q, sq.x + k);
-                base += sq.y;
-            }
-        }
-    }
-}
-
-// Whether the listing of edge f met in pixel pid (sequence q, its row's first
-// column xa) is the first listing of f that for_candidate_edges meets: no
-// BORDER pixel of the window with a smaller id (an earlier row, or the same
-// row further left) lists f, and no earlier sequence of pid holds it. Each
-// edge that crosses the segment is then counted exactly once, whatever the
-// number of pixels listing it, with no per-edge memory. The pixels listing f
-// come from the edge -> pixel index (ascending ids, so the scan stops at pid),
-// and window membership from the rows the enumeration computed (or the same
-// row_cols for rows older than the cache), so both agree to the bit.
-__device__ bool first_listing(const StoreView &sv, const PolyHdr &O, const SegWin &w, int cc, const RowCache &rc,
-                              const uint64_t *ep_off, const uint32_t *ep_pix, uint32_t pid, int xa, uint32_t q,
-                              uint32_t f) {
-    const uint64_t g = O.ring + f;
+// Whether the listing of edge f in pixel pid (sequence q; lo: its row's first
+// column) is the first listing of f in the group's window: no BORDER pixel of
+// the window with a smaller id (an earlier row, or the same row further left)
+// lists f, and no earlier sequence of pid holds it. Each edge that crosses is
+// then counted exactly once, whatever the number of pixels listing it, with no
+// per-edge memory. The pixels listing f come from the edge -> pixel index
+// (ascending ids, so the scan stops at pid), window membership from the kept
+// rows (or the same function for older ones).
+__device__ bool first_listing(const StoreView &sv, const Group &g, const int2 *rows, const uint64_t *ep_off,
+                              const uint32_t *ep_pix, int cc, uint32_t pid, int lo, uint32_t q, uint32_t f) {
+    const PolyHdr &O = *g.O;
+    const uint64_t at = O.ring + f;
     const uint32_t dimx = (uint32_t)O.dimx;
     const int py = (int)(pid / dimx);
     int self = 0;
-    for (uint64_t i = ep_off[g], e = ep_off[g + 1]; i < e; i++) {
+    for (uint64_t i = ep_off[at], e = ep_off[at + 1]; i < e; i++) {
         const uint32_t r = ep_pix[i];
         if (r > pid) break;
         if (r == pid) {
@@ -265,21 +212,14 @@ __device__ bool first_listing(const StoreView &sv, const PolyHdr &O, const SegWi
             continue;
         }
         const int ry = (int)(r / dimx), rx = (int)(r - (uint32_t)ry * dimx);
-        if (ry < w.sy) continue;  // above the window
+        if (ry < g.sy) continue;  // above the window
         if (show_status(sv.status[O.st + r], cc) != 1) continue;
         if (ry == py) {
-            if (rx >= xa) return false;
+            if (rx >= lo) return false;
             continue;
         }
-        int cxa, cxb;
-        if (ry > py - kRowCache) {  // still in the ring (rows sy .. py were enumerated in order)
-            const int2 c = rc.r[ry & (kRowCache - 1)];
-            cxa = c.x;
-            cxb = c.y;
-        } else if (!row_cols(O, w, ry, cxa, cxb)) {
-            continue;
-        }
-        if (rx >= cxa && rx <= cxb) return false;
+        const int2 c = ry > py - (kRowCache - kQueueRows) ? rows[ry & (kRowCache - 1)] : group_columns(g, ry);
+        if (rx >= c.x && rx <= c.y) return false;
     }
     if (self > 1) {  // pid holds f in more than one sequence: the first counts
         const uint2 *seq = sv.seq + O.seq;
@@ -293,26 +233,6 @@ __device__ bool first_listing(const StoreView &sv, const PolyHdr &O, const SegWi
 
 // Crossing parameter t of segment p -> p + d with edge e of ring r, in [0, 1)
 // on both (half-open, so a crossing at a shared vertex counts once).
-// FP32 rejection ahead of crossing(): edge A->B lies strictly on one side of
-// the line through P->Q, or P->Q strictly on one side of the line through
-// A->B, by a margin of 1e-6 (~17 u32) times the orientation products'
-// magnitudes. That is far above the rounding of this test (~4 u32) and of
-// crossing()'s FP64 arithmetic, so such segments cannot cross and crossing()
-// would return false as well; only the candidates near a crossing pay for
-// FP64, which on GB300 issues at 1/64 of the FP32 rate.
-__device__ __forceinline__ bool apart32(float2 P, float2 Q, float2 A, float2 B) {
-    const float ex = Q.x - P.x, ey = Q.y - P.y;
-    const float ax = A.x - P.x, ay = A.y - P.y, bx = B.x - P.x, by = B.y - P.y;
-    const float oa = ex * ay - ey * ax, ob = ex * by - ey * bx;
-    const float ma = 1e-6f * (fabsf(ex * ay) + fabsf(ey * ax)), mb = 1e-6f * (fabsf(ex * by) + fabsf(ey * bx));
-    if ((oa > ma && ob > mb) || (oa < -ma && ob < -mb)) return true;
-    const float gx = B.x - A.x, gy = B.y - A.y;
-    const float px = P.x - A.x, py = P.y - A.y, qx = Q.x - A.x, qy = Q.y - A.y;
-    const float op = gx * py - gy * px, oq = gx * qy - gy * qx;
-    const float mp = 1e-6f * (fabsf(gx * py) + fabsf(gy * px)), mq = 1e-6f * (fabsf(gx * qy) + fabsf(gy * qx));
-    return (op > mp && oq > mq) || (op < -mp && oq < -mq);
-}
-
 __device__ __forceinline__ bool crossing(double px, double py, double dx, double dy, const float2 *r, uint32_t e,
                                          double ox, double oy, double &t, double &den) {
     float2 a = r[e], b = r[e + 1];
@@ -327,19 +247,8 @@ __device__ __forceinline__ bool crossing(double px, double py, double dx, double
     return t >= 0 && t < 1 && u >= 0 && u < 1;
 }
 
-// Default knobs: edges per item, and the window size (pixels) above which an
-// edge is searched by the whole warp (for_candidate_edges_warp) instead of
-// its own lane. FARM_AREA_WIDE_WINDOW overrides the window size of every
-// bucket.
-constexpr int kDefaultChunk = 16;
-constexpr int kDefaultWide = 200;
-
-static long wide_window_env() {
-    const char *v = getenv("FARM_AREA_WIDE_WINDOW");
-    if (!v || !*v) return 0;
-    const long x = strtol(v, nullptr, 10);
-    return x > 0 && x < 65536 ? x : 0;
-}
+constexpr int kDefaultChunk = 16;   // edges per item
+constexpr int kDefaultWide = 200;   // of the window table, which nothing reads any more
 
 // FARM_AREA_SPREAD=0 takes the items in pair order
 static int spread_items() {
@@ -348,9 +257,33 @@ static int spread_items() {
 }
 
 
-__global__ void __launch_bounds__(256) k_area(const StoreView sv, AreaArgs a) {
-    const int lane = threadIdx.x & 31;
+// What bounds it is instruction issue in the tests of edge pairs. A lane per
+// edge that walked its own window of pixels, sequences and listed edges kept 7
+// of 32 lanes busy and took two FP64 divisions per row and edge; consecutive
+// edges lie together, so the group's common window is little larger than each
+// edge's, and its listed edges, those whose box meets the group's, are queued
+// and tested by all lanes at once. A group of R < 32 edges is repeated over
+// floor(32 / R) slices of lanes, which share the queue. Row ranges are FP32
+// with a margin: they need only hold every crossing's listings, and the same
+// for all of an item. A pair of edges is rejected in FP32 when one lies
+// strictly on one side of the other's line by a margin far above the test's
+// rounding and crossing()'s, so only the pairs near a crossing reach FP64,
+// which GB300 issues at 1/64 of its FP32 rate.
+// 801 pairs of up to 20,000 vertices: 72 ms with a window per lane.
+constexpr int kAreaQueue = 64;
+struct AreaEntry {
+    float4 seg;  // the listed edge's ends
+    uint32_t f, pid, q;
+    int lo;      // first column of the row it was met in
+};
+__global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a) {
+    __shared__ int2 s_rows[8][kRowCache];
+    __shared__ AreaEntry s_queue[8][kAreaQueue];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int cc = sv.category_count;
+    int2 *rows = s_rows[wib];
+    AreaEntry *queue = s_queue[wib];
     unsigned long long my_tests = 0, my_cross = 0;
     for (;;) {
         const uint64_t n = *a.n;
@@ -361,7 +294,7 @@ __global__ void __launch_bounds__(256) k_area(const StoreView sv, AreaArgs a) {
         }
         unsigned long long it = 0;
         if (lane == 0) it = atomicAdd(a.next, 1ull);
-        it = __shfl_sync(0xffffffffu, it, 0);
+        it = __shfl_sync(full, it, 0);
         if (it >= nitems) break;
         // Items lie pair after pair, and the heavy pairs' items are each slow:
         // taken in that order, a heavy pair near the end leaves a tail. The
@@ -379,7 +312,6 @@ __global__ void __launch_bounds__(256) k_area(const StoreView sv, AreaArgs a) {
         const PolyHdr &T = sv.hdr[a.tgt_base + a.pairs[2 * p + 1]];
         uint32_t es = S.nv - 1, et = T.nv - 1;  // edges (the ring's last edge is the zero-length closing one)
         const uint32_t chunk = a.chunks.of(es, et);
-        const long wide_window = (long)a.chunks.wide_of(es, et);
         uint64_t cs = (es + chunk - 1) / chunk;
         bool side_t = rel >= cs;
         const PolyHdr &M = side_t ? T : S;  // the boundary integrated
@@ -392,91 +324,169 @@ __global__ void __launch_bounds__(256) k_area(const StoreView sv, AreaArgs a) {
         const double ox = o0.x, oy = o0.y;
         const double sign = a.orient[side_t ? a.tgt_base + a.pairs[2 * p + 1] : a.pairs[2 * p]];
         // state at the chunk's first vertex
-        bool in0 = false;
-        if (lane == 0) in0 = pip_raster(sv, O, mr[first].x, mr[first].y, cc);
-        in0 = __shfl_sync(0xffffffffu, in0, 0);
+        bool state = pip_raster(sv, O, mr[first].x, mr[first].y, cc, lane);
         double acc = 0;
-        bool state = in0;
         // a crossing leaves O when O's edge turns the way O's interior lies:
         // entering iff (d x g) has the opposite sign of O's orientation
         const double osign = a.orient[side_t ? a.pairs[2 * p] : a.tgt_base + a.pairs[2 * p + 1]];
+        const uint8_t *ost = sv.status + O.st;
+        const uint32_t *ooff = sv.offset + O.off;
+        const uint2 *oseq = sv.seq + O.seq;
         for (uint32_t b0 = first; b0 < last; b0 += 32) {
-            uint32_t e = b0 + lane;
-            bool valid = e < last;
-            double px = 0, py = 0, dx = 0, dy = 0;
-            double sum_t = 0;  // leaving t minus entering t
+            const uint32_t R = min(32u, last - b0), G = 32u / R, slice = (uint32_t)lane / R;
+            const uint32_t e = b0 + (uint32_t)lane % R;
+            const float2 P = mr[e], Q = mr[e + 1];
+            const double px = (double)P.x - ox, py = (double)P.y - oy;
+            const double dx = (double)Q.x - P.x, dy = (double)Q.y - P.y;
+            const bool active = slice < G && edge_meets(O, P, Q);
+            Sum2 sum_t;  // leaving t minus entering t
             int nc = 0;
-            float2 P = make_float2(0.f, 0.f), Q = P;
-            bool wide = false;
-            if (valid) {
-                P = mr[e];
-                Q = mr[e + 1];
-                px = (double)P.x - ox;
-                py = (double)P.y - oy;
-                dx = (double)Q.x - P.x;
-                dy = (double)Q.y - P.y;
-                SegWin w;
-                const bool has_w = (dx != 0 || dy != 0) && seg_window(O, P.x, P.y, Q.x, Q.y, w);
-                wide = has_w && (long)(w.ex - w.sx + 1) * (long)(w.ey - w.sy + 1) > wide_window;
-                if (has_w && !wide) {
-                    // an edge of O may be listed by several pixels: count it
-                    // at its first listing only (tested before the FP64
-                    // crossing, which then runs once per edge pair)
-                    RowCache rc;
-                    for_candidate_edges(sv, O, w, cc, rc, [&](uint32_t pid, int xa, uint32_t q, uint32_t f) {
-                        double t, den;
-                        if (apart32(P, Q, orr[f], orr[f + 1]) ||
-                            !first_listing(sv, O, w, cc, rc, a.ep_off, a.ep_pix, pid, xa, q, f))
-                            return;
-                        my_tests++;
-                        if (!crossing(px, py, dx, dy, orr, f, ox, oy, t, den)) return;
-                        nc++;
-                        sum_t += (osign * den > 0) ? t : -t;
-                    });
+            if (__any_sync(full, active)) {
+                const EdgeUV uv = edge_uv(O, P, Q);
+                // rows of the group's window, and its box
+                int ylo = 0x7fffffff, yhi = -1;
+                float bx0 = INFINITY, by0 = INFINITY, bx1 = -INFINITY, by1 = -INFINITY;
+                if (active) {
+                    const float lo = floorf(fminf(uv.v0, uv.v1) - uv.m) - 1.f;
+                    const float hi = floorf(fmaxf(uv.v0, uv.v1) + uv.m) + 1.f;
+                    ylo = lo > 0.f ? (int)fminf(lo, 2e9f) : 0;
+                    yhi = hi < (float)(O.dimy - 1) ? (int)hi : O.dimy - 1;
+                    bx0 = fminf(P.x, Q.x);
+                    bx1 = fmaxf(P.x, Q.x);
+                    by0 = fminf(P.y, Q.y);
+                    by1 = fmaxf(P.y, Q.y);
                 }
-            }
-            // edges with wide windows: the whole warp takes one at a time
-            for (unsigned wm = __ballot_sync(0xffffffffu, wide); wm; wm &= wm - 1) {
-                const int src = __ffs(wm) - 1;
-                const float2 Pw = make_float2(__shfl_sync(0xffffffffu, P.x, src), __shfl_sync(0xffffffffu, P.y, src));
-                const float2 Qw = make_float2(__shfl_sync(0xffffffffu, Q.x, src), __shfl_sync(0xffffffffu, Q.y, src));
-                const double pxw = (double)Pw.x - ox, pyw = (double)Pw.y - oy;
-                const double dxw = (double)Qw.x - Pw.x, dyw = (double)Qw.y - Pw.y;
-                SegWin ww;
-                seg_window(O, Pw.x, Pw.y, Qw.x, Qw.y, ww);  // the owner's window, recomputed identically
-                RowCache rc;
-                double st_l = 0;
-                int nc_l = 0;
-                for_candidate_edges_warp(sv, O, ww, cc, rc, lane, [&](uint32_t pid, int xa, uint32_t q, uint32_t f) {
-                    double t, den;
-                    if (apart32(Pw, Qw, orr[f], orr[f + 1]) ||
-                        !first_listing(sv, O, ww, cc, rc, a.ep_off, a.ep_pix, pid, xa, q, f))
-                        return;
-                    my_tests++;
-                    if (!crossing(pxw, pyw, dxw, dyw, orr, f, ox, oy, t, den)) return;
-                    nc_l++;
-                    st_l += (osign * den > 0) ? t : -t;
-                });
+                ylo = __reduce_min_sync(full, ylo);
+                yhi = __reduce_max_sync(full, yhi);
                 for (int o = 16; o; o >>= 1) {
-                    st_l += __shfl_xor_sync(0xffffffffu, st_l, o);
-                    nc_l += __shfl_xor_sync(0xffffffffu, nc_l, o);
+                    bx0 = fminf(bx0, __shfl_xor_sync(full, bx0, o));
+                    by0 = fminf(by0, __shfl_xor_sync(full, by0, o));
+                    bx1 = fmaxf(bx1, __shfl_xor_sync(full, bx1, o));
+                    by1 = fmaxf(by1, __shfl_xor_sync(full, by1, o));
                 }
-                if (lane == src) {
-                    sum_t = st_l;
-                    nc = nc_l;
+                const Group grp{&O, mr, b0, R, ylo};
+                // FP32 rejection: margins of 1e-6 (~17 u32) times the largest
+                // products a vertex of O can give
+                const float ex = Q.x - P.x, ey = Q.y - P.y;
+                const float ru = fmaxf(fabsf((float)O.mbr[0] - P.x), fabsf((float)O.mbr[2] - P.x));
+                const float rv = fmaxf(fabsf((float)O.mbr[1] - P.y), fabsf((float)O.mbr[3] - P.y));
+                const float ma = 1.1e-6f * (fabsf(ex) * rv + fabsf(ey) * ru);
+                const float rm = 1.1e-6f * (ru + rv + fabsf(ex) + fabsf(ey));
+                int qn = 0;
+                // the first m queued edges against every lane's edge
+                auto test = [&](int m) {
+                    unsigned hits = 0;
+                    if (active) {
+                        for (int j = (int)slice; j < m; j += (int)G) {
+                            const float4 s = queue[j].seg;
+                            const float U = s.x - P.x, V = s.y - P.y, U2 = s.z - P.x, V2 = s.w - P.y;
+                            const float oc = __fmaf_rn(ex, V, -(ey * U)), od = __fmaf_rn(ex, V2, -(ey * U2));
+                            const float gx = U2 - U, gy = V2 - V;
+                            const float op = __fmaf_rn(gy, U, -(gx * V));
+                            const float oq = op + __fmaf_rn(gx, ey, -(gy * ex));
+                            const float mb = rm * (fabsf(gx) + fabsf(gy));
+                            if (!(fminf(oc, od) > ma || fmaxf(oc, od) < -ma || fminf(op, oq) > mb ||
+                                  fmaxf(op, oq) < -mb))
+                                hits |= 1u << j;
+                        }
+                    }
+                    for (; hits; hits &= hits - 1) {
+                        const AreaEntry c = queue[__ffs(hits) - 1];
+                        if (!first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, c.pid, c.lo, c.q, c.f)) continue;
+                        double t, den;
+                        my_tests++;
+                        if (!crossing(px, py, dx, dy, orr, c.f, ox, oy, t, den)) continue;
+                        nc++;
+                        sum_t.add((osign * den > 0) ? t : -t);
+                    }
+                    __syncwarp();
+                };
+                for (int y = ylo; y <= yhi; y++) {
+                    int2 col = active ? edge_columns(uv, y, O.dimx) : make_int2(0x7fffffff, -1);
+                    col.x = __reduce_min_sync(full, col.x);
+                    col.y = __reduce_max_sync(full, col.y);
+                    if (lane == 0) rows[y & (kRowCache - 1)] = col;
+                    __syncwarp();
+                    for (int x0 = col.x; x0 <= col.y; x0 += 32) {
+                        // the row's BORDER pixels, their sequences, and these' edges, flattened
+                        const int x = x0 + lane;
+                        const uint32_t pid = (uint32_t)(y * O.dimx + x);
+                        uint32_t sq0 = 0, nsq = 0;
+                        if (x <= col.y && show_status(ost[pid], cc) == 1) {
+                            sq0 = ooff[pid];
+                            nsq = ooff[pid + 1] - sq0;
+                        }
+                        uint32_t tsq;
+                        const uint32_t xsq = warp_excl_scan(nsq, lane, tsq);
+                        for (uint32_t s0 = 0; s0 < tsq; s0 += 32) {
+                            const uint32_t si = s0 + lane;
+                            const int ow = warp_owner(xsq, si);
+                            const uint32_t q = __shfl_sync(full, sq0, ow) + (si - __shfl_sync(full, xsq, ow));
+                            const uint32_t qpid = __shfl_sync(full, pid, ow);
+                            const uint2 sq = si < tsq ? oseq[q] : make_uint2(0u, 0u);
+                            uint32_t te;
+                            const uint32_t xe = warp_excl_scan(sq.y, lane, te);
+                            for (uint32_t k0 = 0; k0 < te; k0 += 32) {
+                                const uint32_t k = k0 + lane;
+                                const int oe = warp_owner(xe, k);
+                                const uint32_t f = __shfl_sync(full, sq.x, oe) + (k - __shfl_sync(full, xe, oe));
+                                const uint32_t fq = __shfl_sync(full, q, oe), fpid = __shfl_sync(full, qpid, oe);
+                                bool in = false;
+                                float2 A = make_float2(0.f, 0.f), B = A;
+                                if (k < te) {
+                                    A = orr[f];
+                                    B = orr[f + 1];
+                                    in = !(fmaxf(A.x, B.x) < bx0 || fminf(A.x, B.x) > bx1 || fmaxf(A.y, B.y) < by0 ||
+                                           fminf(A.y, B.y) > by1);
+                                }
+                                const unsigned m = __ballot_sync(full, in);
+                                if (in)
+                                    queue[qn + __popc(m & ((1u << lane) - 1u))] =
+                                        AreaEntry{make_float4(A.x, A.y, B.x, B.y), f, fpid, fq, col.x};
+                                qn += __popc(m);
+                                __syncwarp();
+                                if (qn >= 32) {
+                                    test(32);
+                                    qn -= 32;
+                                    AreaEntry mv{};
+                                    if (lane < qn) mv = queue[32 + lane];
+                                    __syncwarp();
+                                    if (lane < qn) queue[lane] = mv;
+                                    __syncwarp();
+                                }
+                            }
+                        }
+                    }
+                    // a queued edge's listing test looks back from its own row, so
+                    // it may not wait while the ring of kept rows moves on
+                    if (qn && ((y - ylo) & (kQueueRows - 1)) == kQueueRows - 1) {
+                        test(qn);
+                        qn = 0;
+                    }
                 }
+                if (qn) test(qn);
+            }
+            // the slices' shares, in their order
+            Sum2 tot_t;
+            int tot_c = 0;
+            for (uint32_t k = 0; k < G; k++) {
+                const int src = (int)((uint32_t)lane % R + R * k);
+                tot_t.add(__shfl_sync(full, sum_t.s, src));
+                tot_t.e += __shfl_sync(full, sum_t.e, src);
+                tot_c += __shfl_sync(full, nc, src);
             }
             // parity of crossings of earlier edges of the chunk
-            unsigned odd = __ballot_sync(0xffffffffu, valid && (nc & 1));
-            bool s_here = state ^ (__popc(odd & ((1u << lane) - 1)) & 1);
+            const bool valid = (uint32_t)lane < R;
+            const unsigned odd = __ballot_sync(full, valid && (tot_c & 1));
+            const bool s_here = state ^ (__popc(odd & ((1u << lane) - 1)) & 1);
             if (valid) {
-                double len = sum_t + ((s_here ^ (nc & 1)) ? 1.0 : 0.0);
-                acc += cross2(px, py, dx, dy) * len;
+                tot_t.add((s_here ^ (tot_c & 1)) ? 1.0 : 0.0);
+                acc += cross2(px, py, dx, dy) * (tot_t.s + tot_t.e);
+                my_cross += (unsigned long long)tot_c;
             }
             state ^= (__popc(odd) & 1);
-            if (valid) my_cross += (unsigned long long)nc;
         }
-        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(full, acc, o);
         if (lane == 0) a.partial[it] = 0.5 * sign * acc;
     }
     if (my_tests) atomicAdd(&a.work[0], my_tests);
@@ -585,11 +595,7 @@ __global__ void k_area_reduce(const uint64_t *__restrict__ item_start, const uin
 
 static Chunks chunks_of(const farm_store *s) {
     Chunks c;
-    const long env_w = wide_window_env();
-    for (int b = 0; b < 32; b++) {
-        c.c[b] = (uint16_t)(s->area_chunk[b] > 0 ? s->area_chunk[b] : kDefaultChunk);
-        c.w[b] = (uint16_t)(env_w ? env_w : (s->area_wide[b] > 0 ? s->area_wide[b] : kDefaultWide));
-    }
+    for (int b = 0; b < 32; b++) c.c[b] = (uint16_t)(s->area_chunk[b] > 0 ? s->area_chunk[b] : kDefaultChunk);
     return c;
 }
 
@@ -969,12 +975,11 @@ extern "C" int farm_area_set_wide(farm_store *s, const int32_t *wide_by_bucket) 
 }
 
 // Autotuner: for every size bucket present in the sample (floor(log2) of a
-// pair's larger edge count), time the area pass on up to 2048 of its pairs,
-// first over the candidate chunk sizes 8..256 (edges per work item), then, at the
-// best chunk, over the candidate window thresholds (pixels above which an
-// edge is searched by the whole warp), and keep the fastest of each. One
-// untimed pass per bucket warms up. The store keeps both tables
-// (farm_area_set_chunks, farm_area_set_wide); they are also returned.
+// pair's larger edge count), time the area pass on up to 2048 of its pairs
+// over the candidate chunk sizes 8..256 (edges per work item) and keep the
+// fastest. One untimed pass per bucket warms up. The store keeps the table
+// (farm_area_set_chunks); it is also returned, with the window table, which
+// nothing reads any more (farm_area_set_wide), at its default.
 extern "C" int farm_area_autotune(farm_store *s, const uint32_t *pairs, uint64_t n, int mem, int32_t *chunk_out,
                                   int32_t *wide_out) {
     using namespace farm;
@@ -1010,23 +1015,14 @@ extern "C" int farm_area_autotune(farm_store *s, const uint32_t *pairs, uint64_t
         }
     }
     static const int32_t kChunkCand[] = {8, 16, 32, 64, 128, 256};
-    static const int32_t kWideCand[] = {24, 48, 200, 800};
-    int32_t saved_c[32], saved_w[32];
+    int32_t saved_c[32];
     memcpy(saved_c, s->area_chunk, sizeof saved_c);
-    memcpy(saved_w, s->area_wide, sizeof saved_w);
     int32_t best_c[32], best_w[32];
     memcpy(best_c, s->area_chunk, sizeof best_c);
     memcpy(best_w, s->area_wide, sizeof best_w);
-    auto restore = [&]() {
-        memcpy(s->area_chunk, saved_c, sizeof saved_c);
-        memcpy(s->area_wide, saved_w, sizeof saved_w);
-    };
-    // one pass of bucket b's pairs with chunk c and window w everywhere
-    auto timed = [&](int b, int32_t c, int32_t w, double *ms) -> int {
-        for (int q = 0; q < 32; q++) {
-            s->area_chunk[q] = c;
-            s->area_wide[q] = w;
-        }
+    // one pass of bucket b's pairs with chunk c everywhere
+    auto timed = [&](int b, int32_t c, double *ms) -> int {
+        for (int q = 0; q < 32; q++) s->area_chunk[q] = c;
         farm_stats stt;
         const int rc = intersection_area(s, byb[b].data(), byb[b].size() / 2, FARM_MEM_HOST, nullptr, &stt);
         *ms = stt.ms_total;
@@ -1035,29 +1031,21 @@ extern "C" int farm_area_autotune(farm_store *s, const uint32_t *pairs, uint64_t
     for (int b = 0; b < 32; b++) {
         if (byb[b].empty()) continue;
         double ms = 0, best_ms = 1e300;
-        int rc = timed(b, kDefaultChunk, kDefaultWide, &ms);  // warm-up
-        int32_t bc = kDefaultChunk, bw = kDefaultWide;
+        int rc = timed(b, kDefaultChunk, &ms);  // warm-up
+        int32_t bc = kDefaultChunk;
         for (int32_t c : kChunkCand) {
-            if (rc == FARM_OK) rc = timed(b, c, kDefaultWide, &ms);
+            if (rc == FARM_OK) rc = timed(b, c, &ms);
             if (rc == FARM_OK && ms < best_ms) {
                 best_ms = ms;
                 bc = c;
             }
         }
-        for (int32_t w : kWideCand) {
-            if (w == kDefaultWide) continue;  // timed above at bc
-            if (rc == FARM_OK) rc = timed(b, bc, w, &ms);
-            if (rc == FARM_OK && ms < best_ms) {
-                best_ms = ms;
-                bw = w;
-            }
-        }
         if (rc != FARM_OK) {
-            restore();
+            memcpy(s->area_chunk, saved_c, sizeof saved_c);
             return rc;
         }
         best_c[b] = bc;
-        best_w[b] = bw;
+        best_w[b] = kDefaultWide;
     }
     memcpy(s->area_chunk, best_c, sizeof best_c);
     memcpy(s->area_wide, best_w, sizeof best_w);

@@ -72,7 +72,7 @@ typedef struct farm_stats {
     uint64_t in_hits;        /* decided by an IN pixel overlap (intersect) */
     uint64_t border_pairs;   /* BORDER x BORDER pixel pairs examined (area: crossings counted) */
     uint64_t segment_tests;  /* segment-pair (or point-segment) evaluations (area: FP64 crossing tests) */
-    uint64_t fp64_rechecks;  /* within: edge-sequence pairs re-evaluated in FP64 after the FP32 pass;
+    uint64_t fp64_rechecks;  /* within: point-segment tests evaluated in FP64 after the FP32 screen;
                                 learned intersect: pairs refined exactly */
     double ms_total;         /* device time of the call (CUDA events) */
     double ms_stage[4];      /* raster, filter, refine, other */
@@ -80,7 +80,7 @@ typedef struct farm_stats {
     int32_t reserved;
     uint64_t src_window_pixels; /* source pixels in the target-MBR windows */
     uint64_t tgt_window_pixels; /* target pixels visited under non-OUT source pixels */
-    uint64_t sequence_pairs;    /* within: edge-sequence pairs evaluated (FP32 pass) */
+    uint64_t sequence_pairs;    /* within: edge-sequence pairs of the tested candidates */
 } farm_stats;
 
 const char *farm_last_error(void);
@@ -234,14 +234,13 @@ void farm_area_plan_destroy(farm_area_plan *p);
 /* Edges per area work item by size bucket b = floor(log2(larger edge count of
  * the pair)), 32 entries (0 = default 16). */
 int farm_area_set_chunks(farm_store *s, const int32_t *chunk_by_bucket);
-/* Candidate-window size (pixels of the other polygon's raster) above which an
- * edge is searched by the whole warp rather than its own lane, by size
- * bucket, 32 entries (0 = default 200). */
+/* Window sizes by size bucket, 32 entries (0 = default 200). They chose between
+ * two searches of an edge's candidates, which are one now: kept with the store,
+ * read by nothing. */
 int farm_area_set_wide(farm_store *s, const int32_t *wide_by_bucket);
 /* Per size bucket present in the sample (up to 2048 pairs each): time the
- * chunk sizes 8..256, then at the best chunk the window sizes 24..800, keep
- * the fastest of each in the store and return both tables (32 entries each;
- * either output may be NULL). */
+ * chunk sizes 8..256, keep the fastest in the store and return both tables (32
+ * entries each; either output may be NULL). */
 int farm_area_autotune(farm_store *s, const uint32_t *pairs, uint64_t n, int mem, int32_t *chunk_out,
                        int32_t *wide_out);
 
