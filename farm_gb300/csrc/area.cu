@@ -72,17 +72,10 @@ struct AreaArgs {
     int spread;                    // take items in a spread order (see k_area)
 };
 
-// A sum with the rounding errors of its additions (Knuth's TwoSum) beside it: an
-// edge's crossing parameters are added in the order its slices meet them, which
-// groups entering and leaving ones, so partial sums grow and would round.
-struct Sum2 {
-    double s = 0, e = 0;
-    __device__ __forceinline__ void add(double v) {
-        const double t = __dadd_rn(s, v), b = __dsub_rn(t, s);
-        e = __dadd_rn(e, __dadd_rn(__dsub_rn(s, __dsub_rn(t, b)), __dsub_rn(v, b)));
-        s = t;
-    }
-};
+// Crossing parameters are added as integers of 2^-60: exact, in any order and
+// over any lanes. Entering and leaving ones alternate along an edge, so their
+// signed sum lies in [-1, 1]; what partial sums carry beyond 64 bits falls off.
+constexpr double kParamScale = 1152921504606846976.0;  // 2^60
 
 __device__ __forceinline__ double cross2(double ax, double ay, double bx, double by) { return ax * by - ay * bx; }
 
@@ -276,14 +269,24 @@ struct AreaEntry {
     uint32_t f, pid, q;
     int lo;      // first column of the row it was met in
 };
+struct AreaHit {
+    uint32_t f, pid, q;
+    int lo;
+};
 __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a) {
     __shared__ int2 s_rows[8][kRowCache];
     __shared__ AreaEntry s_queue[8][kAreaQueue];
+    __shared__ AreaHit s_hit[8][kAreaQueue];
+    __shared__ uint8_t s_hedge[8][kAreaQueue];
+    __shared__ unsigned long long s_sum[8][32];
+    __shared__ uint32_t s_cnt[8][32];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int cc = sv.category_count;
     int2 *rows = s_rows[wib];
     AreaEntry *queue = s_queue[wib];
+    AreaHit *hit = s_hit[wib];  // pairs that may cross, until there are 32 for the FP64 test
+    uint8_t *hedge = s_hedge[wib];
     unsigned long long my_tests = 0, my_cross = 0;
     for (;;) {
         const uint64_t n = *a.n;
@@ -339,8 +342,10 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
             const double px = (double)P.x - ox, py = (double)P.y - oy;
             const double dx = (double)Q.x - P.x, dy = (double)Q.y - P.y;
             const bool active = slice < G && edge_meets(O, P, Q);
-            Sum2 sum_t;  // leaving t minus entering t
-            int nc = 0;
+            // per edge: leaving t minus entering t, crossings
+            s_sum[wib][lane] = 0ull;
+            s_cnt[wib][lane] = 0u;
+            __syncwarp();
             if (__any_sync(full, active)) {
                 const EdgeUV uv = edge_uv(O, P, Q);
                 // rows of the group's window, and its box
@@ -372,7 +377,27 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                 const float rv = fmaxf(fabsf((float)O.mbr[1] - P.y), fabsf((float)O.mbr[3] - P.y));
                 const float ma = 1.1e-6f * (fabsf(ex) * rv + fabsf(ey) * ru);
                 const float rm = 1.1e-6f * (ru + rv + fabsf(ex) + fabsf(ey));
-                int qn = 0;
+                int qn = 0, hn = 0;
+                // the first m pairs that may cross: FP64, a pair per lane
+                auto cross = [&](int m) {
+                    __syncwarp();
+                    if (lane < m) {
+                        const AreaHit c = hit[lane];
+                        if (first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, c.pid, c.lo, c.q, c.f)) {
+                            const uint32_t k = hedge[lane];
+                            const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
+                            double t, den;
+                            my_tests++;
+                            if (crossing((double)A.x - ox, (double)A.y - oy, (double)B.x - A.x, (double)B.y - A.y, orr,
+                                         c.f, ox, oy, t, den)) {
+                                const long long v = __double2ll_rn(t * kParamScale);
+                                atomicAdd(&s_sum[wib][k], (unsigned long long)(osign * den > 0 ? v : -v));
+                                atomicAdd(&s_cnt[wib][k], 1u);
+                            }
+                        }
+                    }
+                    __syncwarp();
+                };
                 // the first m queued edges against every lane's edge
                 auto test = [&](int m) {
                     unsigned hits = 0;
@@ -390,14 +415,30 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                                 hits |= 1u << j;
                         }
                     }
-                    for (; hits; hits &= hits - 1) {
-                        const AreaEntry c = queue[__ffs(hits) - 1];
-                        if (!first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, c.pid, c.lo, c.q, c.f)) continue;
-                        double t, den;
-                        my_tests++;
-                        if (!crossing(px, py, dx, dy, orr, c.f, ox, oy, t, den)) continue;
-                        nc++;
-                        sum_t.add((osign * den > 0) ? t : -t);
+                    for (unsigned any = __ballot_sync(full, hits != 0); any; any = __ballot_sync(full, hits != 0)) {
+                        if (hits) {
+                            const AreaEntry &c = queue[__ffs(hits) - 1];
+                            const int at = hn + __popc(any & ((1u << lane) - 1u));
+                            hit[at] = AreaHit{c.f, c.pid, c.q, c.lo};
+                            hedge[at] = (uint8_t)((uint32_t)lane % R);
+                            hits &= hits - 1;
+                        }
+                        hn += __popc(any);
+                        if (hn >= 32) {
+                            cross(32);
+                            hn -= 32;
+                            AreaHit mv{};
+                            uint8_t me_ = 0;
+                            if (lane < hn) {
+                                mv = hit[32 + lane];
+                                me_ = hedge[32 + lane];
+                            }
+                            __syncwarp();
+                            if (lane < hn) {
+                                hit[lane] = mv;
+                                hedge[lane] = me_;
+                            }
+                        }
                     }
                     __syncwarp();
                 };
@@ -459,32 +500,28 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                     }
                     // a queued edge's listing test looks back from its own row, so
                     // it may not wait while the ring of kept rows moves on
-                    if (qn && ((y - ylo) & (kQueueRows - 1)) == kQueueRows - 1) {
-                        test(qn);
+                    if (y == yhi || ((y - ylo) & (kQueueRows - 1)) == kQueueRows - 1) {
+                        if (qn) test(qn);
                         qn = 0;
+                        if (hn) cross(hn);
+                        hn = 0;
                     }
                 }
-                if (qn) test(qn);
             }
-            // the slices' shares, in their order
-            Sum2 tot_t;
-            int tot_c = 0;
-            for (uint32_t k = 0; k < G; k++) {
-                const int src = (int)((uint32_t)lane % R + R * k);
-                tot_t.add(__shfl_sync(full, sum_t.s, src));
-                tot_t.e += __shfl_sync(full, sum_t.e, src);
-                tot_c += __shfl_sync(full, nc, src);
-            }
+            __syncwarp();
             // parity of crossings of earlier edges of the chunk
             const bool valid = (uint32_t)lane < R;
+            const uint32_t tot_c = valid ? s_cnt[wib][lane] : 0u;
             const unsigned odd = __ballot_sync(full, valid && (tot_c & 1));
             const bool s_here = state ^ (__popc(odd & ((1u << lane) - 1)) & 1);
             if (valid) {
-                tot_t.add((s_here ^ (tot_c & 1)) ? 1.0 : 0.0);
-                acc += cross2(px, py, dx, dy) * (tot_t.s + tot_t.e);
+                const long long tail = (s_here ^ (tot_c & 1)) ? 1ll << 60 : 0ll;
+                const double len = (double)((long long)s_sum[wib][lane] + tail) * (1.0 / kParamScale);
+                acc += cross2(px, py, dx, dy) * len;
                 my_cross += (unsigned long long)tot_c;
             }
             state ^= (__popc(odd) & 1);
+            __syncwarp();
         }
         for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(full, acc, o);
         if (lane == 0) a.partial[it] = 0.5 * sign * acc;
