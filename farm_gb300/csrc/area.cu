@@ -224,20 +224,27 @@ __device__ bool first_listing(const StoreView &sv, const Group &g, const int2 *r
     return true;
 }
 
-// Crossing parameter t of segment p -> p + d with edge e of ring r, in [0, 1)
-// on both (half-open, so a crossing at a shared vertex counts once).
-__device__ __forceinline__ bool crossing(double px, double py, double dx, double dy, const float2 *r, uint32_t e,
-                                         double ox, double oy, double &t, double &den) {
-    float2 a = r[e], b = r[e + 1];
-    double ax = (double)a.x - ox, ay = (double)a.y - oy;
-    double gx = (double)b.x - a.x, gy = (double)b.y - a.y;
-    if (gx == 0 && gy == 0) return false;
+// Crossing parameter t of segment P -> Q with edge e of ring r, in [0, 1) on
+// both (half-open, so a crossing at a shared vertex counts once). The
+// differences of floats are taken in double; both parameters' ranges are
+// decided on numerator and denominator (n / d < 1 exactly when |n| < |d| of
+// the same sign, as doubles one ulp apart divide to less than 1), so that
+// only a crossing divides, once.
+__device__ __forceinline__ bool crossing(float2 P, float2 Q, const float2 *r, uint32_t e, double &t, double &den) {
+    const float2 a = r[e], b = r[e + 1];
+    const double dx = (double)Q.x - P.x, dy = (double)Q.y - P.y;
+    const double gx = (double)b.x - a.x, gy = (double)b.y - a.y;
     den = cross2(dx, dy, gx, gy);
     if (den == 0) return false;
-    double rx = ax - px, ry = ay - py;
-    t = cross2(rx, ry, gx, gy) / den;
-    double u = cross2(rx, ry, dx, dy) / den;
-    return t >= 0 && t < 1 && u >= 0 && u < 1;
+    const double rx = (double)a.x - P.x, ry = (double)a.y - P.y;
+    const double tn = cross2(rx, ry, gx, gy), un = cross2(rx, ry, dx, dy);
+    const double ad = fabs(den);
+    const bool neg = den < 0;
+    const bool t_in = fabs(tn) < ad && (tn == 0 || (tn < 0) == neg);
+    const bool u_in = fabs(un) < ad && (un == 0 || (un < 0) == neg);
+    if (!(t_in && u_in)) return false;
+    t = tn / den;
+    return true;
 }
 
 constexpr int kDefaultChunk = 16;   // edges per item
@@ -388,8 +395,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                             const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
                             double t, den;
                             my_tests++;
-                            if (crossing((double)A.x - ox, (double)A.y - oy, (double)B.x - A.x, (double)B.y - A.y, orr,
-                                         c.f, ox, oy, t, den)) {
+                            if (crossing(A, B, orr, c.f, t, den)) {
                                 const long long v = __double2ll_rn(t * kParamScale);
                                 atomicAdd(&s_sum[wib][k], (unsigned long long)(osign * den > 0 ? v : -v));
                                 atomicAdd(&s_cnt[wib][k], 1u);
