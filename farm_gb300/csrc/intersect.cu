@@ -314,10 +314,6 @@ int intersect_filter(farm_store *s, const uint32_t *dpairs, uint64_t n, uint8_t 
     return FARM_OK;
 }
 
-// Work order for the exact query: pairs by descending product of their
-// polygons' vertex counts, so that the heaviest pairs start first and the
-// pass does not end on a long pair that started last (longest-first
-// scheduling). Results are written by pair index, so the order is invisible.
 __global__ void k_pair_cost(const StoreView sv, const uint32_t *__restrict__ pairs, uint64_t n, uint64_t tgt_base,
                             uint32_t *__restrict__ key, uint32_t *__restrict__ idx) {
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
@@ -333,16 +329,15 @@ static bool pair_order_on() {
     return !(v && *v == '0');
 }
 
-static int pair_order(farm_store *s, const uint32_t *dpairs, uint64_t n, const uint32_t **order) {
+int pair_order(farm_store *s, const uint32_t *dpairs, uint64_t n, uint64_t tgt_base, const uint32_t **order) {
     *order = nullptr;
-    // up to a warp per pair all pairs start at once, in any order
-    if (n <= 16ull * sm_count() || n > 0xFFFFFFFFull) return FARM_OK;
+    if (n <= 16ull * sm_count() || n > 0xFFFFFFFFull || !pair_order_on()) return FARM_OK;
     cudaStream_t stream = s->stream;
     FARM_TRY(s->s[Q_PAIR_ORDER].ensure(16 * n + 64));
     uint32_t *key = s->s[Q_PAIR_ORDER].as<uint32_t>(), *key_s = key + n, *idx = key_s + n, *idx_s = idx + n;
     unsigned blocks = grid_for(n, 256);
     if (blocks > 16u * (unsigned)sm_count()) blocks = 16u * (unsigned)sm_count();
-    k_pair_cost<<<blocks, 256, 0, stream>>>(s->view(), dpairs, n, s->n_side[0], key, idx);
+    k_pair_cost<<<blocks, 256, 0, stream>>>(s->view(), dpairs, n, tgt_base, key, idx);
     FARM_CUDA(cudaGetLastError());
     s->launches++;
     size_t bytes = 0;
@@ -412,7 +407,7 @@ int intersect(farm_store *s, const uint32_t *pairs, uint64_t n, int mode, int me
     // (a smaller pool), 150,001 heavy pairs 26.8 / 26.8 / 24.2 ms.
     if (mode == FARM_MODE_EXACT && n) FARM_TRY(spill_pool(s, n, next + 8, 512.f, 4096.f, &sp));
     FARM_CUDA(cudaEventRecord(s->ev[6], stream));
-    if (mode == FARM_MODE_EXACT && pair_order_on()) FARM_TRY(pair_order(s, dpairs, n, &pv.order));
+    if (mode == FARM_MODE_EXACT) FARM_TRY(pair_order(s, dpairs, n, pv.tgt_base, &pv.order));
     const int blocks = query_blocks(n);
     if (mode == FARM_MODE_APPROX)
         k_intersect<K_APPROX><<<blocks, kWarpsPerBlock * 32, 0, stream>>>(sv, pv, next, dout, ctr, SpillPool{});

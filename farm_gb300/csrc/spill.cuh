@@ -114,4 +114,11 @@ __device__ __forceinline__ void spill_units(const SpillPool &sp, F f, D done) {
 // beyond. FARM_SPILL_BUDGET sets it.
 int spill_pool(farm_store *s, uint64_t n, unsigned long long *ctr, float few, float many, SpillPool *sp);
 
+// Work order of a pair list: by descending product of the polygons' vertex
+// counts, so that the heaviest pairs start first and the pass does not end on a
+// long pair that started last. Results are written by pair index, so the order
+// is invisible. *order is null (index order) for a list of up to a pair per
+// resident warp, whose pairs all start at once. FARM_PAIR_ORDER=0: index order.
+int pair_order(farm_store *s, const uint32_t *dpairs, uint64_t n, uint64_t tgt_base, const uint32_t **order);
+
 }  // namespace farm

@@ -381,6 +381,7 @@ enum : uint8_t { W_FALSE = 0, W_TRUE = 1, W_BADPOLY = 2 };
 
 struct WithinArgs {
     const uint32_t *pairs;
+    const uint32_t *order;  // pairs taken in this order, or index order
     uint64_t n;
     uint64_t tgt_base;
     double thr;
@@ -733,7 +734,10 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
     WithinTally my;
     for (;;) {
         unsigned long long pid = 0;
-        if (lane == 0) pid = atomicAdd(a.next, 1ull);
+        if (lane == 0) {
+            pid = atomicAdd(a.next, 1ull);
+            if (a.order && pid < a.n) pid = a.order[pid];
+        }
         pid = __shfl_sync(full, pid, 0);
         if (pid >= a.n) break;
         const PolyHdr &S = sv.hdr[a.pairs[2 * pid]];
@@ -1173,6 +1177,7 @@ int within(farm_store *s, const uint32_t *pairs, uint64_t n, double distance, in
         WithinArgs wa;
         wa.pairs = dpairs;
         wa.n = n;
+        FARM_TRY(pair_order(s, dpairs, n, tgt_base, &wa.order));
         wa.tgt_base = tgt_base;
         wa.thr = distance;
         wa.geo = geography != 0;
