@@ -179,10 +179,28 @@ inline unsigned grid_for(uint64_t n, unsigned block) {
 
 int sm_count();
 
+// Float bits mapped so that unsigned order is numeric order (-0 just before +0).
+__host__ __device__ inline uint32_t float_key(uint32_t u) { return (u & 0x80000000u) ? ~u : (u | 0x80000000u); }
+__host__ __device__ inline uint32_t float_unkey(uint32_t k) { return (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k; }
+
+// A polygon's vertex box from ring_boxes' keys, as the reference's loop leaves
+// it (vertex_sequence.cpp:152-168): Box.h:6-12's start values, float bias.
+__device__ inline void ring_box(const uint4 &k, double *m) {
+    const float lx = __uint_as_float(float_unkey(k.x)), ly = __uint_as_float(float_unkey(k.y));
+    const float hx = __uint_as_float(float_unkey(~k.z)), hy = __uint_as_float(float_unkey(~k.w));
+    const double bias = (double)1e-9f;
+    m[0] = fmin(100000.0, (double)lx) - bias;
+    m[1] = fmin(100000.0, (double)ly) - bias;
+    m[2] = fmax(-100000.0, (double)hx) + bias;
+    m[3] = fmax(-100000.0, (double)hy) + bias;
+}
+
 }  // namespace farm
 
 struct farm_store;
 namespace farm {
+// Vertex boxes of the store's polygons as order keys (ring_box) in box[n_poly].
+int ring_boxes(farm_store *s, uint4 *box);
 // FARM_EINVAL unless every pair's source index is below the source count and
 // its target index below the target count (the source count when self).
 // Device pairs are checked by a kernel (one synchronisation).
@@ -215,7 +233,8 @@ enum ScratchSlot : int {
     Q_AREA_EPOFF = 37,  // area: edge -> pixel index offsets (per ring position)
     Q_AREA_EPPIX = 38,  // area: edge -> pixel index entries
     Q_PAIR_ORDER = 39,  // intersect: the longest-first pair order
-    Q_SPILL = 48,       // intersect, contain: pixel pairs left to all warps
+    Q_SPILL = 48,       // intersect, contain, within: work left to all warps
+    Q_BOX = 51,         // vertex boxes (ring_boxes)
 };
 }  // namespace farm
 
@@ -239,7 +258,7 @@ struct farm_store {
     uint64_t tot_P = 0, tot_status = 0, tot_seq = 0;
     farm_raster_totals rtot = {};
     // scratch for the rasterizer and the queries
-    farm::DevBuf s[51];
+    farm::DevBuf s[52];
     farm::DevBuf cub_tmp;
     farm::DevBuf d_pairs, d_out, d_counters;
     farm::DevBuf d_check;  // pair-index validation counter

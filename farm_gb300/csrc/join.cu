@@ -8,12 +8,12 @@
 // (farm_host.cpp) computes that set on the host. Here it is computed from the
 // rings already in the store, so an end-to-end query needs no host join:
 //
-//   k_join_mbr     per polygon (a warp each): its MBR from the stored vertices,
-//                  the Box.h:6-12 start values and the float bias of
+//   k_ring_boxes,  per polygon: its MBR from the stored vertices, the
+//   k_join_mbr     Box.h:6-12 start values and the float bias of
 //                  vertex_sequence.cpp:152-168, as farm_mbr and k_header do;
 //   sort           sources by their low x (order-preserving 64-bit keys);
 //   k_join_width   the widest source box;
-//   k_join_count   per target (a thread each): the sources whose low x lies in
+//   k_join_count   per target (a warp each): the sources whose low x lies in
 //                  [q.lo.x - widest, q.hi.x] (q the widened target box), each
 //                  tested by the same closed-overlap comparisons as the host;
 //   scan, k_join_fill with the same loop, one 64-bit key per pair
@@ -34,35 +34,12 @@ __device__ __forceinline__ uint64_t jkey(double v) {  // order-preserving bits o
     return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
 
-// MBR (lx, ly, hx, hy) of polygons [p0, p0 + n) of the store, by warp.
-__global__ void k_join_mbr(const float2 *__restrict__ ring, const uint64_t *__restrict__ off, uint64_t p0, uint32_t n,
-                           double4 *__restrict__ mbr) {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t k = warp; k < n; k += nw) {
-        const uint64_t p = p0 + k;
-        const uint64_t b = off[p], e = off[p + 1];
-        const float2 *r = ring + b + 2ull * p;
-        const uint32_t m = (uint32_t)(e - b);
-        double lx = 100000.0, ly = 100000.0, hx = -100000.0, hy = -100000.0;
-        for (uint32_t j = lane; j < m; j += 32) {
-            const float2 q = r[j];
-            lx = fmin(lx, (double)q.x);
-            hx = fmax(hx, (double)q.x);
-            ly = fmin(ly, (double)q.y);
-            hy = fmax(hy, (double)q.y);
-        }
-        for (int o = 16; o; o >>= 1) {
-            lx = fmin(lx, __shfl_xor_sync(0xffffffffu, lx, o));
-            hx = fmax(hx, __shfl_xor_sync(0xffffffffu, hx, o));
-            ly = fmin(ly, __shfl_xor_sync(0xffffffffu, ly, o));
-            hy = fmax(hy, __shfl_xor_sync(0xffffffffu, hy, o));
-        }
-        if (lane == 0) {
-            const double bias = (double)1e-9f;
-            mbr[k] = make_double4(lx - bias, ly - bias, hx + bias, hy + bias);
-        }
+// MBRs (lx, ly, hx, hy) of n polygons from their vertex boxes.
+__global__ void k_join_mbr(const uint4 *__restrict__ box, uint32_t n, double4 *__restrict__ mbr) {
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        double m[4];
+        ring_box(box[k], m);
+        mbr[k] = make_double4(m[0], m[1], m[2], m[3]);
     }
 }
 
@@ -137,31 +114,36 @@ __device__ __forceinline__ bool overlap(const double4 &s, const double4 &q) {
     return !(s.x > q.z || q.x > s.z || s.y > q.w || q.y > s.w);
 }
 
+// A warp per target, lanes over its candidate sources.
 __global__ void k_join_count(JoinArgs a, uint64_t *__restrict__ cnt) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < a.nt; t += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < a.nt; t += (gridDim.x * blockDim.x) >> 5) {
         const double4 q = widen(a, a.tgt[t]);
         uint32_t lo, hi;
         cand_range(a, q, lo, hi);
-        uint64_t c = 0;
-        for (uint32_t k = lo; k < hi; k++) {
+        uint32_t c = 0;
+        for (uint32_t k = lo + lane; k < hi; k += 32) {
             const uint32_t s = a.sidx[k];
-            if (a.self && s == t) continue;
-            c += overlap(a.src[s], q);
+            c += !(a.self && s == t) && overlap(a.src[s], q);
         }
-        cnt[t] = c;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) cnt[t] = c;
     }
 }
 
 __global__ void k_join_fill(JoinArgs a, const uint64_t *__restrict__ start, uint64_t *__restrict__ out) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < a.nt; t += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < a.nt; t += (gridDim.x * blockDim.x) >> 5) {
         const double4 q = widen(a, a.tgt[t]);
         uint32_t lo, hi;
         cand_range(a, q, lo, hi);
         uint64_t at = start[t];
-        for (uint32_t k = lo; k < hi; k++) {
-            const uint32_t s = a.sidx[k];
-            if (a.self && s == t) continue;
-            if (overlap(a.src[s], q)) out[at++] = ((uint64_t)s << 32) | t;
+        for (uint32_t k0 = lo; k0 < hi; k0 += 32) {
+            const uint32_t k = k0 + lane, s = k < hi ? a.sidx[k] : 0u;
+            const bool in = k < hi && !(a.self && s == t) && overlap(a.src[s], q);
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) out[at + __popc(m & ((1u << lane) - 1u))] = ((uint64_t)s << 32) | t;
+            at += __popc(m);
         }
     }
 }
@@ -187,16 +169,15 @@ int mbr_join_gpu(farm_store *s, double expand, int geography, int self, uint32_t
     *n_out = 0;
     if (ns == 0 || nt == 0) return FARM_OK;
     cudaStream_t st = s->stream;
-    const uint64_t tfirst = self ? 0 : ns;
     // scratch (the query slots: the join runs between loading and querying)
     DevBuf &bm = s->s[Q_SCR0], &bk = s->s[Q_SCR1], &bc = s->s[Q_SCR2], &bo = s->s[Q_SCR3], &bt = s->s[Q_SCR4];
     FARM_TRY(bm.ensure(32 * (ns + nt) + 64));
     double4 *msrc = bm.as<double4>(), *mtgt = self ? msrc : msrc + ns;
-    k_join_mbr<<<grid_cap(32 * ns), 256, 0, st>>>(s->d_ring.as<float2>(), s->d_off.as<uint64_t>(), 0, (uint32_t)ns,
-                                                  msrc);
-    if (!self)
-        k_join_mbr<<<grid_cap(32 * nt), 256, 0, st>>>(s->d_ring.as<float2>(), s->d_off.as<uint64_t>(), tfirst,
-                                                      (uint32_t)nt, mtgt);
+    FARM_TRY(s->s[Q_BOX].ensure(sizeof(uint4) * s->n_poly));
+    FARM_TRY(ring_boxes(s, s->s[Q_BOX].as<uint4>()));
+    // both sides' boxes in one go: the targets' follow the sources'
+    k_join_mbr<<<grid_cap(self ? ns : ns + nt), 256, 0, st>>>(s->s[Q_BOX].as<uint4>(), (uint32_t)(self ? ns : ns + nt),
+                                                             msrc);
     // sources by low x
     FARM_TRY(bk.ensure(24 * (ns + 1) + 8 * 900 + 64));
     uint64_t *key = bk.as<uint64_t>(), *key_s = key + ns;
@@ -228,7 +209,7 @@ int mbr_join_gpu(farm_store *s, double expand, int geography, int self, uint32_t
     JoinArgs a{msrc, mtgt, key_s, idx_s, (uint32_t)ns, (uint32_t)nt, expand, geography, self, deg, wkey};
     FARM_TRY(bc.ensure(16 * (nt + 1) + 64));
     uint64_t *cnt = bc.as<uint64_t>(), *start = cnt + (nt + 1);
-    k_join_count<<<grid_cap(nt), 256, 0, st>>>(a, cnt);
+    k_join_count<<<grid_cap(32 * nt), 256, 0, st>>>(a, cnt);
     FARM_CUDA(cudaMemsetAsync(cnt + nt, 0, 8, st));
     {
         size_t bytes = 0;
@@ -239,7 +220,7 @@ int mbr_join_gpu(farm_store *s, double expand, int geography, int self, uint32_t
     uint64_t total = 0;
     FARM_CUDA(cudaMemcpyAsync(&total, start + nt, 8, cudaMemcpyDeviceToHost, st));
     FARM_CUDA(cudaStreamSynchronize(st));
-    s->launches += self ? 5 : 6;
+    s->launches += 4;
     *n_out = total;
     if (total > cap) {
         set_error("farm_mbr_join_gpu: " + std::to_string(total) + " candidate pairs exceed the buffer's " +
@@ -249,7 +230,7 @@ int mbr_join_gpu(farm_store *s, double expand, int geography, int self, uint32_t
     if (!total) return FARM_OK;
     FARM_TRY(bo.ensure(16 * total + 64));
     uint64_t *pk = bo.as<uint64_t>(), *pk_s = pk + total;
-    k_join_fill<<<grid_cap(nt), 256, 0, st>>>(a, start, pk);
+    k_join_fill<<<grid_cap(32 * nt), 256, 0, st>>>(a, start, pk);
     {
         size_t bytes = 0;
         FARM_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, bytes, pk, pk_s, (int64_t)total, 0, 64, st));

@@ -155,38 +155,16 @@ __device__ void layering(PolyHdr &h, const RasterParams &rp) {
     h.num_layers = (uint32_t)(high - low + 1);
 }
 
-// One warp per polygon: MBR (vertex_sequence.cpp:152-168), raster geometry.
-__global__ void k_header(const float2 *__restrict__ ring, const uint64_t *__restrict__ off, uint32_t npoly,
+// A thread per polygon: raster geometry from the vertex box.
+__global__ void k_header(const uint4 *__restrict__ box, const uint64_t *__restrict__ off, uint32_t npoly,
                          RasterParams rp, PolyHdr *__restrict__ hdr, uint64_t *__restrict__ sizes) {
-    uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t p = warp; p < npoly; p += nwarps) {
-        uint64_t b = off[p], e = off[p + 1];
-        const float2 *r = ring + b + 2ull * p;
-        uint32_t m = (uint32_t)(e - b);
-        double lx = 100000.0, ly = 100000.0, hx = -100000.0, hy = -100000.0;
-        for (uint32_t j = lane; j < m; j += 32) {
-            float2 q = r[j];
-            lx = fmin(lx, (double)q.x);
-            hx = fmax(hx, (double)q.x);
-            ly = fmin(ly, (double)q.y);
-            hy = fmax(hy, (double)q.y);
-        }
-        for (int o = 16; o; o >>= 1) {
-            lx = fmin(lx, __shfl_xor_sync(0xffffffffu, lx, o));
-            hx = fmax(hx, __shfl_xor_sync(0xffffffffu, hx, o));
-            ly = fmin(ly, __shfl_xor_sync(0xffffffffu, ly, o));
-            hy = fmax(hy, __shfl_xor_sync(0xffffffffu, hy, o));
-        }
-        if (lane == 0) {
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npoly; p += gridDim.x * blockDim.x) {
+        {
+            const uint64_t b = off[p], e = off[p + 1];
+            const uint32_t m = (uint32_t)(e - b);
             PolyHdr h;
             memset(&h, 0, sizeof h);
-            const double bias = (double)1e-9f;
-            h.mbr[0] = lx - bias;
-            h.mbr[1] = ly - bias;
-            h.mbr[2] = hx + bias;
-            h.mbr[3] = hy + bias;
+            ring_box(box[p], h.mbr);
             h.nv = m + 1;
             h.ring = b + 2ull * p;
             h.edge = b;
@@ -2836,7 +2814,9 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
     R.hdr = s->d_hdr.as<PolyHdr>();
     uint64_t *sizes = s->s[S_SIZES].as<uint64_t>(), *scan = s->s[S_SCAN].as<uint64_t>();
     R.scan = scan;
-    k_header<<<gb(32ull * np), 256, 0, st>>>(s->d_ring.as<float2>(), R.doff, np, rp, R.hdr, sizes);
+    FARM_TRY(s->s[Q_BOX].ensure(sizeof(uint4) * np));
+    FARM_TRY(ring_boxes(s, s->s[Q_BOX].as<uint4>()));
+    k_header<<<gb(2ull * np), 128, 0, st>>>(s->s[Q_BOX].as<uint4>(), R.doff, np, rp, R.hdr, sizes);
     R.launches++;
     FARM_TRY(scan_rows(R, sizes, scan, n1, 8));
     uint64_t tot[8];

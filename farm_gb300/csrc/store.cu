@@ -144,6 +144,57 @@ __global__ void k_pad_rings(const float2 *__restrict__ xy, const uint64_t *__res
     }
 }
 
+// Smallest and largest coordinates of every polygon, as keys: x, y of the
+// smallest, ~x, ~y of the largest, so that all four are minima and start as all
+// ones. A warp takes a tile of the padded rings, polygon after polygon, and
+// reduces in registers: a polygon of 100,000 vertices is 25 tiles, not the last
+// warp's 3,125 loads (37.6M vertices in 3,300 polygons: 1.2 ms with a warp per
+// polygon and its minima in FP64). NaN coordinates count for nothing, as in a
+// loop of minima. The padding repeats a polygon's first vertex.
+constexpr uint32_t kBoxTile = 4096;
+__global__ void k_ring_boxes(const float2 *__restrict__ ring, const uint64_t *__restrict__ off, uint32_t npoly,
+                             uint64_t total, uint4 *__restrict__ box) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, tiles = (total + kBoxTile - 1) / kBoxTile;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tiles; t += nw) {
+        const uint64_t v1 = min(total, (t + 1) * kBoxTile);
+        uint64_t v = t * kBoxTile;  // stored vertices
+        for (uint32_t p = find_segment(off, npoly, v); v < v1; p++) {
+            const uint64_t e = min(v1, off[p + 1]);
+            const float2 *r = ring + 2ull * p;
+            float lx = INFINITY, ly = INFINITY, hx = -INFINITY, hy = -INFINITY;
+            for (uint64_t k = v + lane; k < e; k += 32) {
+                const float2 q = r[k];
+                lx = fminf(lx, q.x);
+                hx = fmaxf(hx, q.x);
+                ly = fminf(ly, q.y);
+                hy = fmaxf(hy, q.y);
+            }
+            const uint32_t kx = __reduce_min_sync(0xffffffffu, float_key(__float_as_uint(lx)));
+            const uint32_t ky = __reduce_min_sync(0xffffffffu, float_key(__float_as_uint(ly)));
+            const uint32_t mx = __reduce_min_sync(0xffffffffu, ~float_key(__float_as_uint(hx)));
+            const uint32_t my = __reduce_min_sync(0xffffffffu, ~float_key(__float_as_uint(hy)));
+            if (lane < 4)
+                atomicMin(reinterpret_cast<uint32_t *>(box + p) + lane,
+                          lane == 0 ? kx : (lane == 1 ? ky : (lane == 2 ? mx : my)));
+            v = e;
+        }
+    }
+}
+
+int ring_boxes(farm_store *s, uint4 *box) {
+    FARM_CUDA(cudaMemsetAsync(box, 0xFF, sizeof(uint4) * s->n_poly, s->stream));
+    const uint64_t warps = (s->n_edges + kBoxTile - 1) / kBoxTile;
+    unsigned blocks = grid_for(32 * warps, 128);
+    const unsigned cap = 32u * (unsigned)sm_count();
+    if (blocks > cap) blocks = cap;
+    k_ring_boxes<<<blocks, 128, 0, s->stream>>>(s->d_ring.as<float2>(), s->d_off.as<uint64_t>(), (uint32_t)s->n_poly,
+                                               s->n_edges, box);
+    FARM_CUDA(cudaGetLastError());
+    s->launches++;
+    return FARM_OK;
+}
+
 }  // namespace farm
 
 using namespace farm;

@@ -128,21 +128,23 @@ class Store:
         given, else numpy. `cap` bounds the pairs (0: counted first)."""
         lib = self._lib
         n = C.c_uint64(0)
-        if cap <= 0:
-            rc = lib.farm_mbr_join_gpu(self._h, float(expand), int(geography), int(self_join), None, 0, MEM_HOST,
-                                       C.byref(n))
-            if rc not in (0, -4):
-                check_gpu(rc)
-            cap = int(n.value)
-        if device is not None:
-            import torch
-            out = torch.empty((max(cap, 1), 2), dtype=torch.int32, device=device)
-            check_gpu(lib.farm_mbr_join_gpu(self._h, float(expand), int(geography), int(self_join),
-                                             C.c_void_p(out.data_ptr()), cap, MEM_DEVICE, C.byref(n)))
-            return out[:n.value]
-        out = np.zeros((max(cap, 1), 2), dtype=np.uint32)
-        check_gpu(lib.farm_mbr_join_gpu(self._h, float(expand), int(geography), int(self_join),
-                                         C.c_void_p(out.ctypes.data), cap, MEM_HOST, C.byref(n)))
+        # without a bound, room for a few pairs per polygon first (untouched
+        # pages cost nothing), and the counted number if that overflows
+        room = cap if cap > 0 else min(16 * (self.n_source + self.n_target) + 1024, 1 << 22)
+        for _ in range(2):
+            if device is not None:
+                import torch
+                out = torch.empty((max(room, 1), 2), dtype=torch.int32, device=device)
+                ptr, mem = out.data_ptr(), MEM_DEVICE
+            else:
+                out = np.empty((max(room, 1), 2), dtype=np.uint32)
+                ptr, mem = out.ctypes.data, MEM_HOST
+            rc = lib.farm_mbr_join_gpu(self._h, float(expand), int(geography), int(self_join), C.c_void_p(ptr), room,
+                                       mem, C.byref(n))
+            if cap > 0 or rc != -4:
+                break
+            room = int(n.value)
+        check_gpu(rc)
         return out[:n.value]
 
     def intersect(self, pairs, mode: int = MODE_EXACT, out=None):
