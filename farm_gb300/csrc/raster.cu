@@ -2322,6 +2322,8 @@ static int raster_small(RasterCtx &R, const SmallInfo &info) {
     a.pix = (uint32_t)info.pix;
     a.lines = (uint32_t)info.lines;
     a.n = (uint32_t)info.n;
+    a.big = (uint32_t)info.big;
+    a.npoly = R.np;
     a.cert = R.cert;
     a.cc = R.cc;
     a.slice = small_scratch(a, nullptr, nullptr);

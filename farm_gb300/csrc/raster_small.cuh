@@ -22,13 +22,15 @@ constexpr uint32_t kSmallMany = 1024;  // polygons from which the narrow blocks 
 constexpr int kWalkBlocks64 = 8, kFillBlocks64 = 14, kBlocks256 = 2;  // resident per SM
 // A polygon is small up to these sizes: above them a block alone is slower
 // than the pipeline's whole chip, and the shared counters would not fit.
+constexpr uint32_t kSmallBig = 256;  // edges from which a small polygon is taken first
 constexpr uint32_t kSmallEdges = 2048, kSmallNodes = 8192, kSmallPix = 2048, kSmallLines = 512;
 
 // What the host needs to know of phase 1 (one copy): array totals, and the
 // small polygons' number and largest sizes, which size the scratch.
 struct SmallInfo {
     unsigned long long seq, hnodes, vnodes;  // totals over all polygons
-    unsigned long long n;                    // small polygons
+    unsigned long long n, big, rest;         // small polygons: all, those taken first, the others
+    unsigned long long next[2];              // the kernels' next polygons
     unsigned long long edges, cross, hn, vn, pix, lines;  // their largest
     unsigned long long left;                 // small polygons left to the pipeline (scratch too short)
     unsigned long long clip_x, clip_y, crossings;         // points and crossings of the small polygons
@@ -54,7 +56,7 @@ struct SmallArgs {
     uint64_t slice;  // scratch bytes per block
     uint32_t cap_e, cap_c, cap_h, cap_v, cap_x, cap_cp, cap_y, hash;
     uint32_t pix, lines;  // shared counters
-    uint32_t n;
+    uint32_t n, big, npoly;
     int cert, cc;
 };
 
@@ -119,29 +121,72 @@ __global__ void k_small_pick(PolyHdr *__restrict__ hdr, uint32_t npoly, const ui
         info->hnodes = sc[n1 + npoly];
         info->vnodes = sc[2 * n1 + npoly];
     }
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < npoly; p += gridDim.x * blockDim.x) {
-        PolyHdr &h = hdr[p];
-        h.seq = sc[p];
-        h.n_seq = (uint32_t)sz[p];
-        h.hnode = sc[n1 + p];
-        h.n_hnodes = (uint32_t)sz[n1 + p];
-        h.vnode = sc[2 * n1 + p];
-        h.n_vnodes = (uint32_t)sz[2 * n1 + p];
-        const uint64_t ne = off[p + 1] - off[p];
-        const uint32_t lines = (uint32_t)(h.dimx > h.dimy ? h.dimx : h.dimy) + 3;
-        const bool small = counts_ok && *ovf == 0 && ne <= kSmallEdges && sz[n1 + p] <= kSmallNodes &&
-                           sz[2 * n1 + p] <= kSmallNodes && sz[p] <= 2 * kSmallNodes && h.P <= kSmallPix &&
-                           lines <= kSmallLines;
-        done[p] = 0;
-        if (!small) continue;
-        list[atomicAdd(&info->n, 1ull)] = p;
-        atomicMax(&info->edges, (unsigned long long)ne);
-        atomicMax(&info->cross, (unsigned long long)sz[p]);
-        atomicMax(&info->hn, (unsigned long long)sz[n1 + p]);
-        atomicMax(&info->vn, (unsigned long long)sz[2 * n1 + p]);
-        atomicMax(&info->pix, (unsigned long long)h.P);
-        atomicMax(&info->lines, (unsigned long long)lines);
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < npoly; p0 += gridDim.x * blockDim.x) {
+        const uint32_t p = p0 + lane;
+        bool small = false;
+        uint32_t ne = 0, cross = 0, hn = 0, vn = 0, pix = 0, lines = 0;
+        if (p < npoly) {
+            PolyHdr &h = hdr[p];
+            h.seq = sc[p];
+            h.n_seq = (uint32_t)sz[p];
+            h.hnode = sc[n1 + p];
+            h.n_hnodes = (uint32_t)sz[n1 + p];
+            h.vnode = sc[2 * n1 + p];
+            h.n_vnodes = (uint32_t)sz[2 * n1 + p];
+            const uint64_t edges = off[p + 1] - off[p];
+            lines = (uint32_t)(h.dimx > h.dimy ? h.dimx : h.dimy) + 3;
+            small = counts_ok && *ovf == 0 && edges <= kSmallEdges && sz[n1 + p] <= kSmallNodes &&
+                    sz[2 * n1 + p] <= kSmallNodes && sz[p] <= 2 * kSmallNodes && h.P <= kSmallPix &&
+                    lines <= kSmallLines;
+            done[p] = 0;
+            ne = (uint32_t)edges;
+            cross = h.n_seq;
+            hn = h.n_hnodes;
+            vn = h.n_vnodes;
+            pix = h.P;
+        }
+        // the list from the front: larger polygons, from the back: the others
+        const unsigned any = __ballot_sync(full, small), front = __ballot_sync(full, small && ne >= kSmallBig);
+        if (!any) continue;
+        unsigned long long at_f = 0;
+        if (lane == 0) {
+            at_f = atomicAdd(&info->big, (unsigned long long)__popc(front));
+            atomicAdd(&info->n, (unsigned long long)__popc(any));
+        }
+        at_f = __shfl_sync(full, at_f, 0);
+        const unsigned back = any & ~front;
+        unsigned long long at_k = 0;
+        if (lane == 0 && back) at_k = atomicAdd(&info->rest, (unsigned long long)__popc(back));
+        at_k = __shfl_sync(full, at_k, 0);
+        const unsigned below = (1u << lane) - 1u;
+        if (small) {
+            if (ne >= kSmallBig) list[at_f + __popc(front & below)] = p;
+            else list[npoly - 1 - (at_k + __popc(back & below))] = p;
+        }
+        auto largest = [&](unsigned long long *to, uint32_t v) {
+            const uint32_t m = __reduce_max_sync(full, small ? v : 0u);
+            if (lane == 0) atomicMax(to, (unsigned long long)m);
+        };
+        largest(&info->edges, ne);
+        largest(&info->cross, cross);
+        largest(&info->hn, hn);
+        largest(&info->vn, vn);
+        largest(&info->pix, pix);
+        largest(&info->lines, lines);
     }
+}
+
+// The next polygon of a kernel, largest ones first: ~0 past the last.
+__device__ __forceinline__ uint32_t small_next(const SmallArgs &a, int which, uint32_t *shared) {
+    __syncthreads();  // the last polygon's shared arrays are done with
+    if (threadIdx.x == 0) {
+        const unsigned long long q = atomicAdd(&a.info->next[which], 1ull);
+        *shared = q >= a.n ? ~0u : (q < a.big ? a.list[q] : a.list[a.npoly - 1 - (q - a.big)]);
+    }
+    __syncthreads();
+    return *shared;
 }
 
 // exclusive scan over the block (several small counts may be packed in one
@@ -318,13 +363,14 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_walk(SmallArgs a) {
     __shared__ uint64_t sums[kWarps];
     __shared__ uint64_t sortb[kWarps][kLineMid];
     __shared__ int s_err;
+    __shared__ uint32_t s_next;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     SmallScratch s;
     small_scratch(a, a.scratch + blockIdx.x * a.slice, &s);
-    for (uint32_t q = blockIdx.x; q < a.n; q += gridDim.x) {
-        const uint32_t p = a.list[q];
+    for (;;) {
+        const uint32_t p = small_next(a, 0, &s_next);
+        if (p == ~0u) break;
         const PolyHdr &h = a.hdr[p];
-        __syncthreads();  // the last polygon's shared arrays are done with
         if (tid == 0) {
             s_err = h.err;
             a.done[p] = 1;
@@ -455,14 +501,15 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
     uint32_t *cnt = yst + a.lines + 1;     // lines x warps + 1
     __shared__ uint64_t sums[kWarps];
     __shared__ int s_full;
+    __shared__ uint32_t s_next;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     SmallScratch s;
     small_scratch(a, a.scratch + blockIdx.x * a.slice, &s);
-    for (uint32_t q = blockIdx.x; q < a.n; q += gridDim.x) {
-        const uint32_t p = a.list[q];
+    for (;;) {
+        const uint32_t p = small_next(a, 1, &s_next);
+        if (p == ~0u) break;
         const PolyHdr &h = a.hdr[p];
         if (h.err) continue;
-        __syncthreads();  // the last polygon's shared arrays are done with
         if (tid == 0) s_full = 0;
         __syncthreads();
         const float2 *r = a.sv.ring + h.ring;
