@@ -183,10 +183,11 @@ __device__ __noinline__ double pt_seg_dist(float2 p, float2 p1, float2 p2, bool 
 // constants below are about 3x wider, as c0 (the threshold, the third term
 // over the pair's largest coordinate) and k1 (the first); the relative term
 // is in the final comparison. A test that is not clearly at or past the
-// threshold is evaluated in FP64, so the answer is pt_seg_dist's.
+// threshold, nor clearly below it (c1), is evaluated in FP64, so the answer is
+// pt_seg_dist's.
 struct Near {
     double thr;
-    float c0, k1;
+    float c0, c1, k1;
 };
 constexpr float kScaleGeo = 111.5f;  // no degree is longer: 40076 / 360 km
 
@@ -198,6 +199,7 @@ __device__ __forceinline__ Near near_of(const PolyHdr &S, const PolyHdr &T, doub
     // the running minimum of the reference starts at 100000: any test is below a larger threshold
     w.thr = thr > 100000.0 ? (double)INFINITY : thr;
     w.c0 = (float)w.thr * 1.000001f + 5e-14f * (float)m * sc;
+    w.c1 = (float)w.thr * 0.999999f - 5e-14f * (float)m * sc;
     w.k1 = 4e-6f * sc;
     return w;
 }
@@ -233,21 +235,22 @@ __device__ __forceinline__ Seg make_seg(float2 p1, float2 p2) {
     return g;
 }
 
+// The FP32 screen: *may unless the distance is surely not below the threshold,
+// *sure when it surely is; e: the point's longitude entry.
 template <bool kGeo>
-__device__ __forceinline__ bool near_test(float2 p, const Seg &g, const Near &w, const float2 *tab, uint32_t &rechk) {
+__device__ __forceinline__ void screen(float2 p, float2 e, const Seg &g, const Near &w, bool &may, bool &sure) {
     const float A = __fsub_rn(p.x, g.p1.x), B = __fsub_rn(p.y, g.p1.y);
     const float t = __saturatef(__fmul_rn(__fmaf_rn(A, g.C, __fmul_rn(B, g.D)), g.inv));
     float dx = __fmaf_rn(-t, g.C, A), dy = __fmaf_rn(-t, g.D, B);
-    float lim = __fmaf_rn(w.k1, fabsf(A) + fabsf(B) + g.L, w.c0);
+    float err = __fmul_rn(w.k1, fabsf(A) + fabsf(B) + g.L);
     if (kGeo) {
-        const float2 e = tab[lat_index(p.y)];
-        lim = __fmaf_rn(fabsf(dx), e.y, lim);
+        err = __fmaf_rn(fabsf(dx), e.y, err);
         dx = __fmul_rn(dx, e.x);
         dy = __fmul_rn(dy, (float)(40076.0 / 360.0));
     }
-    if (__fmaf_rn(dx, dx, __fmul_rn(dy, dy)) > lim * lim * 1.00001f) return false;
-    rechk++;
-    return pt_seg_dist(p, g.p1, g.p2, kGeo) < w.thr;
+    const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy)), up = w.c0 + err, dn = w.c1 - err;
+    may |= !(d2 > up * up * 1.00001f);
+    sure |= dn > 0.f && d2 * 1.00001f < dn * dn;
 }
 
 // One side of a candidate pixel pair: its pixel's edge sequences.
@@ -265,114 +268,157 @@ __device__ __forceinline__ SeqSet seq_set(const StoreView &sv, const PolyHdr &h,
 // reads points [start, start + len) and the len - 1 segments between them
 // (segment_to_segment_within_batch). Over all sequence pairs of a pixel pair
 // that is every point of one side against every segment of the other.
-template <bool kGeo>
-__device__ __noinline__ bool points_near_segments(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
-                                     uint32_t &rechk) {
-    for (uint32_t i = G.a; i < G.b; i++) {
-        const uint2 e = G.seq[i];
-        if (e.y < 2) continue;
-        float2 p1 = G.ring[e.x];
-        for (uint32_t k = 1; k < e.y; k++) {
-            const float2 p2 = G.ring[e.x + k];
-            const Seg g = make_seg(p1, p2);
-            for (uint32_t j = P.a; j < P.b; j++) {
-                const uint2 f = P.seq[j];
-                if (f.y < 2) continue;
-                for (uint32_t q = 0; q < f.y; q++)
-                    if (near_test<kGeo>(P.ring[f.x + q], g, w, tab, rechk)) return true;
-            }
-            p1 = p2;
-        }
-    }
-    return false;
-}
 
-// The same with the warp on one pixel pair: segments over the lanes, points read by all.
+// Points staged per warp and side: (x, y, longitude entry), and those of them
+// that start a segment (to the next one).
+constexpr uint32_t kWPts = 128;
+struct WStage {
+    float4 pt[2][kWPts];
+    uint8_t seg[2][kWPts];
+    uint32_t nseg[2];
+};
+
+// The next chunk of a side's points, sequence after sequence (those of fewer
+// than 2 points skipped), into st->pt[side]: its length, 0 past the last.
+// (*g, *at): the group of 32 sequences and the point in it; a chunk that ends
+// inside a group is followed by one that starts with its last point.
 template <bool kGeo>
-__device__ __noinline__ bool points_near_segments_warp(const SeqSet &P, const SeqSet &G, const Near &w, const float2 *tab,
-                                          int lane, uint32_t &rechk) {
+__device__ uint32_t stage_points(const SeqSet &Q, WStage *st, int side, const float2 *tab, uint32_t *g, uint32_t *at,
+                                 int lane) {
     const unsigned full = 0xffffffffu;
-    for (uint32_t i0 = G.a; i0 < G.b; i0 += 32) {
-        const uint2 e = i0 + lane < G.b ? G.seq[i0 + lane] : make_uint2(0u, 0u);
-        const uint32_t mine = e.y >= 2 ? e.y - 1 : 0u;
+    for (; Q.a + *g < Q.b; *g += 32, *at = 0) {
+        const uint32_t i = Q.a + *g + lane;
+        const uint2 e = i < Q.b ? Q.seq[i] : make_uint2(0u, 0u);
+        const uint32_t mine = e.y >= 2 ? e.y : 0u;
         uint32_t incl = mine;
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t u = __shfl_up_sync(full, incl, o);
             if (lane >= o) incl += u;
         }
         const uint32_t total = __shfl_sync(full, incl, 31), excl = incl - mine;
-        for (uint32_t s0 = 0; s0 < total; s0 += 32) {
-            const uint32_t s = s0 + lane;
-            int owner = 0;
+        if (total == 0 || (*at && total - *at < 2)) continue;  // empty, or only the repeated point left
+        const uint32_t n = min(kWPts, total - *at);
+        uint32_t ns = 0;
+        __syncwarp();
+        for (uint32_t k0 = 0; k0 < n; k0 += 32) {
+            const uint32_t k = k0 + lane, f = *at + k;
+            int ow = 0;
             for (int b = 16; b; b >>= 1)
-                if (__shfl_sync(full, excl, owner + b) <= s) owner += b;
-            const uint32_t start = __shfl_sync(full, e.x, owner), ex = __shfl_sync(full, excl, owner);
-            const bool valid = s < total;
-            Seg g{};
-            if (valid) g = make_seg(G.ring[start + (s - ex)], G.ring[start + (s - ex) + 1]);
-            for (uint32_t j = P.a; j < P.b; j++) {
-                const uint2 f = P.seq[j];
-                if (f.y < 2) continue;
-                bool hit = false;
-                for (uint32_t q = 0; q < f.y && !hit; q++) {
-                    const float2 p = P.ring[f.x + q];
-                    if (valid) hit = near_test<kGeo>(p, g, w, tab, rechk);
-                }
-                if (__any_sync(full, hit)) return true;
+                if (__shfl_sync(full, excl, ow + b) <= f) ow += b;
+            const uint32_t start = __shfl_sync(full, e.x, ow), ex = __shfl_sync(full, excl, ow),
+                           len = __shfl_sync(full, mine, ow);
+            bool starts = false;
+            if (k < n) {
+                const float2 p = Q.ring[start + (f - ex)];
+                const float2 s = kGeo ? tab[lat_index(p.y)] : make_float2(1.f, 0.f);
+                st->pt[side][k] = make_float4(p.x, p.y, s.x, s.y);
+                starts = f - ex + 1 < len && k + 1 < n;
             }
+            const unsigned m = __ballot_sync(full, starts);
+            if (starts) st->seg[side][ns + __popc(m & ((1u << lane) - 1u))] = (uint8_t)k;
+            ns += __popc(m);
         }
+        if (lane == 0) st->nseg[side] = ns;
+        __syncwarp();
+        *at += n;
+        if (*at >= total) {
+            *g += 32;
+            *at = 0;
+        } else {
+            *at -= 1;
+        }
+        return n;
+    }
+    return 0;
+}
+
+// Staged segments of side gs against the np staged points of the other: a segment per lane, a group of R < 32 of them repeated over floor(32 /
+// R) slices of lanes that share the points.
+template <bool kGeo>
+__device__ bool staged_near(const WStage *st, int gs, uint32_t np, const Near &w, int lane, uint32_t &tests,
+                            uint32_t &rechk) {
+    const unsigned full = 0xffffffffu;
+    const float4 *pt = st->pt[gs ^ 1];
+    const uint32_t ns = st->nseg[gs];
+    for (uint32_t k0 = 0; k0 < ns; k0 += 32) {
+        const uint32_t R = min(32u, ns - k0);
+        const uint32_t G = 32u / R, slice = (uint32_t)lane / R;
+        const bool valid = slice < G;
+        Seg g{};
+        if (valid) {
+            const uint32_t at = st->seg[gs][k0 + (uint32_t)lane % R];
+            const float4 a = st->pt[gs][at], b = st->pt[gs][at + 1];
+            g = make_seg(make_float2(a.x, a.y), make_float2(b.x, b.y));
+        }
+        const uint32_t q = (np + G - 1) / G;
+        const uint32_t j0 = valid ? min(np, slice * q) : np, j1 = min(np, j0 + q);
+        tests += j1 - j0;
+        bool may = false, hit = false;
+#pragma unroll 4
+        for (uint32_t j = j0; j < j1; j++) {
+            const float4 p = pt[j];
+            screen<kGeo>(make_float2(p.x, p.y), make_float2(p.z, p.w), g, w, may, hit);
+        }
+        if (__any_sync(full, hit)) return true;
+        if (!__any_sync(full, may)) continue;
+        for (uint32_t j = j0; may && j < j1 && !hit; j++) {
+            const float4 p = pt[j];
+            bool here = false, sure = false;
+            screen<kGeo>(make_float2(p.x, p.y), make_float2(p.z, p.w), g, w, here, sure);
+            if (!here) continue;
+            rechk++;
+            hit = pt_seg_dist(make_float2(p.x, p.y), g.p1, g.p2, kGeo) < w.thr;
+        }
+        if (__any_sync(full, hit)) return true;
     }
     return false;
 }
 
-// Point-segment tests a lane takes on a candidate by itself; a larger one gets the warp.
-constexpr uint32_t kLaneTests = 1024;
+// One candidate by the warp: every point of one side against every segment of
+// the other, both ways.
+template <bool kGeo>
+__device__ __noinline__ bool warp_near(const SeqSet &A, const SeqSet &B, const Near &w, const float2 *tab, WStage *st,
+                                       int lane, uint32_t &tests, uint32_t &rechk) {
+    uint32_t ga = 0, ata = 0;
+    for (uint32_t na; (na = stage_points<kGeo>(A, st, 0, tab, &ga, &ata, lane)) != 0;) {
+        uint32_t gb = 0, atb = 0;
+        for (uint32_t nb; (nb = stage_points<kGeo>(B, st, 1, tab, &gb, &atb, lane)) != 0;)
+            if (staged_near<kGeo>(st, 0, nb, w, lane, tests, rechk) ||
+                staged_near<kGeo>(st, 1, na, w, lane, tests, rechk))
+                return true;
+    }
+    return false;
+}
 
 struct WithinTally {
     unsigned long long cand = 0, box = 0, tests = 0, rechk = 0, seqp = 0;
 };
 
-// Candidates (one per lane, valid lanes) against the threshold: the mask of
-// lanes whose pixel pair holds a point-segment distance below it.
-__device__ __noinline__ unsigned test_candidates(const StoreView &sv, const PolyHdr &S, const PolyHdr &T, bool valid, uint32_t id1,
-                                    uint32_t id2, const Near &w, bool geo, const float2 *tab, int lane,
-                                    WithinTally &my) {
+// Candidates (one per lane, valid lanes) against the threshold, the warp on one
+// at a time: the mask of lanes whose pixel pair holds a point-segment distance
+// below it. (A lane per candidate, its points read one by one, took 1.1x to 1.4x
+// the time: 32 lanes at 32 places wait for every load.)
+__device__ __noinline__ unsigned test_candidates(const StoreView &sv, const PolyHdr &S, const PolyHdr &T, bool valid,
+                                                 uint32_t id1, uint32_t id2, const Near &w, bool geo, const float2 *tab,
+                                                 WStage *stage, int lane, WithinTally &my) {
     const unsigned full = 0xffffffffu;
     SeqSet A{}, B{};
-    uint32_t tests = 0, rechk = 0;
     if (valid) {
         A = seq_set(sv, S, id1);
         B = seq_set(sv, T, id2);
-        uint32_t pa = 0, ga = 0, pb = 0, gb = 0;
-        for (uint32_t i = A.a; i < A.b; i++) {
-            const uint32_t y = A.seq[i].y;
-            if (y >= 2) pa += y, ga += y - 1;
-        }
-        for (uint32_t i = B.a; i < B.b; i++) {
-            const uint32_t y = B.seq[i].y;
-            if (y >= 2) pb += y, gb += y - 1;
-        }
-        tests = pa * gb + pb * ga;
-        my.tests += tests;
         my.seqp += (unsigned long long)(A.b - A.a) * (B.b - B.a);
     }
-    bool hit = false;
-    if (tests && tests <= kLaneTests) {
-        hit = geo ? points_near_segments<true>(B, A, w, tab, rechk) || points_near_segments<true>(A, B, w, tab, rechk)
-                  : points_near_segments<false>(B, A, w, tab, rechk) ||
-                        points_near_segments<false>(A, B, w, tab, rechk);
-    }
-    __syncwarp();
-    unsigned hits = __ballot_sync(full, hit);
-    for (unsigned m = __ballot_sync(full, tests > kLaneTests); m; m &= m - 1) {
+    uint32_t tests = 0, rechk = 0;
+    unsigned hits = 0;
+    for (unsigned m = __ballot_sync(full, valid); m; m &= m - 1) {
         const int src = __ffs(m) - 1;
-        const SeqSet a = seq_set(sv, S, __shfl_sync(full, id1, src)), b = seq_set(sv, T, __shfl_sync(full, id2, src));
-        const bool h = geo ? points_near_segments_warp<true>(b, a, w, tab, lane, rechk) ||
-                                 points_near_segments_warp<true>(a, b, w, tab, lane, rechk)
-                           : points_near_segments_warp<false>(b, a, w, tab, lane, rechk) ||
-                                 points_near_segments_warp<false>(a, b, w, tab, lane, rechk);
+        const SeqSet a{sv.seq + S.seq, sv.ring + S.ring, __shfl_sync(full, A.a, src), __shfl_sync(full, A.b, src)};
+        const SeqSet b{sv.seq + T.seq, sv.ring + T.ring, __shfl_sync(full, B.a, src), __shfl_sync(full, B.b, src)};
+        const bool h = geo ? warp_near<true>(a, b, w, tab, stage, lane, tests, rechk)
+                           : warp_near<false>(a, b, w, tab, stage, lane, tests, rechk);
         if (h) hits |= 1u << src;
     }
+    my.tests += tests;
     my.rechk += rechk;
     return hits;
 }
@@ -688,6 +734,13 @@ __device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id
     return 0;
 }
 
+struct WithinShared {
+    WStage stage[8];
+    Layer layers[8][2][kMaxLayers];
+    uint2 queue[8][kQueue];
+    float2 tab[900];  // longitude entries, geography only
+};
+
 // resident blocks of k_within per SM (its grid, and so its scratch)
 constexpr int kWithinBlocks = 2;
 // box pairs of a level above which its pixel sets are pruned first
@@ -704,23 +757,25 @@ constexpr uint32_t kPrunePairs = 256;
 // box than a max-distance already found: they can be in neither the smallest
 // max-distance nor a kept pair.
 //
-// Refinement: a lane per candidate (they have 28 point-segment tests on
-// average in configuration 3, far too few for a warp each), first the closest
-// one each lane met, then all, up to the budget; the rest is spilled.
+// Refinement: the candidates' points staged in shared memory, a segment per
+// lane; first the closest candidate each lane met, then all, up to the budget;
+// the rest is spilled.
 //
 // 60,001 pairs of configuration 3: 794 ms refinement and 55 ms descent with an
-// ordered refinement, a warp per pair.
+// ordered refinement, a warp per pair; 29 ms in all so (36 ms with a lane per
+// candidate and every hit confirmed in FP64).
 __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView sv, WithinArgs a) {
-    __shared__ uint2 queue[8][kQueue];
-    __shared__ Layer layers[8][2][kMaxLayers];
-    __shared__ float2 tab[900];
+    extern __shared__ __align__(16) unsigned char within_smem[];
+    WithinShared &sh = *reinterpret_cast<WithinShared *>(within_smem);
+    float2 *tab = sh.tab;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    WStage *stage = &sh.stage[wib];
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int cc = sv.category_count;
     const bool geo = a.geo;
-    uint2 *q = queue[wib];
-    Layer *LS = layers[wib][0], *LT = layers[wib][1];
+    uint2 *q = sh.queue[wib];
+    Layer *LS = sh.layers[wib][0], *LT = sh.layers[wib][1];
     if (geo)
         for (int k = threadIdx.x; k < 900; k += blockDim.x) tab[k] = lon_entry(k);
     const uint32_t cap = a.cap_pix, bw = (cap >> 5) + 1;
@@ -849,6 +904,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
             double mbd = INFINITY;
             for (Product p(ns, nt); p.next(lane, k1, k2, v);)
                 if (v && !(lv.max2(ss.fbox[k1], ts.fbox[k2], lv.sx(k1)) > m2_lim)) {
+                    my.rechk++;
                     const double md = exact_hi(fin, ss.p[k1], ts.p[k2]);
                     mbd = md < mbd ? md : mbd;
                 }
@@ -873,6 +929,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                 d = lv.dist(ss.fbox[k1], ts.fbox[k2], sx_);
                 if (lv.low(d, sx_) > lim_up) return false;
                 if (lv.high(d, sx_) < lim_dn) return true;
+                my.rechk++;
                 const double lo = exact_lo(fin, ss.p[k1], ts.p[k2]);
                 return !(lo > a.thr) && lo < mbd;
             };
@@ -964,7 +1021,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                     } else {
                         const uint2 c = k + lane < qn ? q[k + lane] : make_uint2(~0u, ~0u);
                         const bool ok = c.x != ~0u && !(know_last && c.x == last1 && c.y == last2);
-                        const unsigned hits = test_candidates(sv, S, T, ok, c.x, c.y, w, geo, tab, lane, my);
+                        const unsigned hits = test_candidates(sv, S, T, ok, c.x, c.y, w, geo, tab, stage, lane, my);
                         k += 32;
                         spent += 32;
                         if (hits == 0) continue;
@@ -989,14 +1046,12 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                         while (r == 2) {
                             // the running minimum still at its start value unless
                             // an earlier candidate holds a distance below it
-                            Near far = w;
-                            far.thr = 100000.0;
-                            far.c0 += 100100.f;
+                            const Near far = near_of(S, T, 100000.0, geo);
                             unsigned below = 0;
                             for (Product p(ns, nt); !below && p.next(lane, k1, k2, v);) {
                                 const bool ok = v && keep_pair(k1, k2, d) && !(ss.p[k1] == last1 && ts.p[k2] == last2);
                                 below = test_candidates(sv, S, T, ok, ok ? ss.p[k1] : 0, ok ? ts.p[k2] : 0, far, geo,
-                                                        tab, lane, my);
+                                                        tab, stage, lane, my);
                             }
                             r = below ? 0 : last_pair(fin, last1, last2, w.thr, &from, lane, my.rechk);
                         }
@@ -1049,8 +1104,10 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
 // slice by slice across the chunks (as spill_units, a lane per entry).
 __global__ void __launch_bounds__(256, 3) k_within_spill(const StoreView sv, WithinArgs a) {
     __shared__ float2 tab[900];
+    __shared__ WStage stages[8];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    WStage *stage = &stages[threadIdx.x >> 5];
     const unsigned long long n = min(a.sp.ctr[0], (unsigned long long)a.sp.cap);
     if (n == 0) return;
     if (a.geo)
@@ -1072,7 +1129,7 @@ __global__ void __launch_bounds__(256, 3) k_within_spill(const StoreView sv, Wit
         const PolyHdr &T = sv.hdr[a.tgt_base + a.pairs[2 * h.pid + 1]];
         const uint2 cd = e + lane < h.count ? a.sp.items[c * kQueue + e + lane] : make_uint2(~0u, 0u);
         const bool v = cd.x != ~0u;
-        if (test_candidates(sv, S, T, v, cd.x, cd.y, near_of(S, T, a.thr, a.geo), a.geo, tab, lane, my) && lane == 0) {
+        if (test_candidates(sv, S, T, v, cd.x, cd.y, near_of(S, T, a.thr, a.geo), a.geo, tab, stage, lane, my) && lane == 0) {
             a.sp.flag[h.head] = 1u;
             a.out[h.pid] = W_TRUE;
         }
@@ -1189,7 +1246,8 @@ int within(farm_store *s, const uint32_t *pairs, uint64_t n, double distance, in
         wa.next = ctr;
         wa.stats = ctr + 1;
         FARM_TRY(spill_pool(s, n, ctr + 8, 64.f, 512.f, &wa.sp));
-        k_within<<<(unsigned)blocks, 256, 0, stream>>>(s->view(), wa);
+        FARM_CUDA(cudaFuncSetAttribute(k_within, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WithinShared)));
+        k_within<<<(unsigned)blocks, 256, sizeof(WithinShared), stream>>>(s->view(), wa);
         FARM_CUDA(cudaGetLastError());
         FARM_CUDA(cudaEventRecord(s->ev[8], stream));
         k_within_spill<<<3 * sm_count(), 256, 0, stream>>>(s->view(), wa);

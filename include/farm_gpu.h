@@ -72,7 +72,7 @@ typedef struct farm_stats {
     uint64_t in_hits;        /* decided by an IN pixel overlap (intersect) */
     uint64_t border_pairs;   /* BORDER x BORDER pixel pairs examined (area: crossings counted) */
     uint64_t segment_tests;  /* segment-pair (or point-segment) evaluations (area: FP64 crossing tests) */
-    uint64_t fp64_rechecks;  /* within: point-segment tests evaluated in FP64 after the FP32 screen;
+    uint64_t fp64_rechecks;  /* within: box distances and point-segment tests taken in FP64 after the FP32 screens;
                                 learned intersect: pairs refined exactly */
     double ms_total;         /* device time of the call (CUDA events) */
     double ms_stage[4];      /* raster, filter, refine, other */
