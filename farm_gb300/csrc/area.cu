@@ -271,19 +271,16 @@ static int spread_items() {
 // which GB300 issues at 1/64 of its FP32 rate.
 // 801 pairs of up to 20,000 vertices: 72 ms with a window per lane.
 constexpr int kAreaQueue = 64;
-struct AreaEntry {
-    float4 seg;  // the listed edge's ends
+struct AreaListing {  // an edge met in a pixel of the window
     uint32_t f, pid, q;
-    int lo;      // first column of the row it was met in
-};
-struct AreaHit {
-    uint32_t f, pid, q;
-    int lo;
+    int lo;  // first column of the row it was met in
 };
 __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a) {
     __shared__ int2 s_rows[8][kRowCache];
-    __shared__ AreaEntry s_queue[8][kAreaQueue];
-    __shared__ AreaHit s_hit[8][kAreaQueue];
+    __shared__ AreaListing s_list[8][kAreaQueue];
+    __shared__ float4 s_seg[8][kAreaQueue];
+    __shared__ uint32_t s_edge[8][kAreaQueue];
+    __shared__ uint32_t s_hit[8][kAreaQueue];
     __shared__ uint8_t s_hedge[8][kAreaQueue];
     __shared__ unsigned long long s_sum[8][32];
     __shared__ uint32_t s_cnt[8][32];
@@ -291,8 +288,10 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int cc = sv.category_count;
     int2 *rows = s_rows[wib];
-    AreaEntry *queue = s_queue[wib];
-    AreaHit *hit = s_hit[wib];  // pairs that may cross, until there are 32 for the FP64 test
+    AreaListing *list = s_list[wib];  // listings, until there are 32 to look up
+    float4 *seg = s_seg[wib];         // the edges of first listings (ends, number), until there are 32 for the FP32 test
+    uint32_t *edge = s_edge[wib];
+    uint32_t *hit = s_hit[wib];       // pairs that may cross, until there are 32 for the FP64 test
     uint8_t *hedge = s_hedge[wib];
     unsigned long long my_tests = 0, my_cross = 0;
     for (;;) {
@@ -384,32 +383,30 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                 const float rv = fmaxf(fabsf((float)O.mbr[1] - P.y), fabsf((float)O.mbr[3] - P.y));
                 const float ma = 1.1e-6f * (fabsf(ex) * rv + fabsf(ey) * ru);
                 const float rm = 1.1e-6f * (ru + rv + fabsf(ex) + fabsf(ey));
-                int qn = 0, hn = 0;
+                int ln = 0, qn = 0, hn = 0;
                 // the first m pairs that may cross: FP64, a pair per lane
                 auto cross = [&](int m) {
                     __syncwarp();
                     if (lane < m) {
-                        const AreaHit c = hit[lane];
-                        if (first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, c.pid, c.lo, c.q, c.f)) {
-                            const uint32_t k = hedge[lane];
-                            const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
-                            double t, den;
-                            my_tests++;
-                            if (crossing(A, B, orr, c.f, t, den)) {
-                                const long long v = __double2ll_rn(t * kParamScale);
-                                atomicAdd(&s_sum[wib][k], (unsigned long long)(osign * den > 0 ? v : -v));
-                                atomicAdd(&s_cnt[wib][k], 1u);
-                            }
+                        const uint32_t k = hedge[lane], f = hit[lane];
+                        const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
+                        double t, den;
+                        my_tests++;
+                        if (crossing(A, B, orr, f, t, den)) {
+                            const long long v = __double2ll_rn(t * kParamScale);
+                            atomicAdd(&s_sum[wib][k], (unsigned long long)(osign * den > 0 ? v : -v));
+                            atomicAdd(&s_cnt[wib][k], 1u);
                         }
                     }
                     __syncwarp();
                 };
-                // the first m queued edges against every lane's edge
+                // the first m edges against every lane's edge
                 auto test = [&](int m) {
+                    __syncwarp();
                     unsigned hits = 0;
                     if (active) {
                         for (int j = (int)slice; j < m; j += (int)G) {
-                            const float4 s = queue[j].seg;
+                            const float4 s = seg[j];
                             const float U = s.x - P.x, V = s.y - P.y, U2 = s.z - P.x, V2 = s.w - P.y;
                             const float oc = __fmaf_rn(ex, V, -(ey * U)), od = __fmaf_rn(ex, V2, -(ey * U2));
                             const float gx = U2 - U, gy = V2 - V;
@@ -423,9 +420,8 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                     }
                     for (unsigned any = __ballot_sync(full, hits != 0); any; any = __ballot_sync(full, hits != 0)) {
                         if (hits) {
-                            const AreaEntry &c = queue[__ffs(hits) - 1];
                             const int at = hn + __popc(any & ((1u << lane) - 1u));
-                            hit[at] = AreaHit{c.f, c.pid, c.q, c.lo};
+                            hit[at] = edge[__ffs(hits) - 1];
                             hedge[at] = (uint8_t)((uint32_t)lane % R);
                             hits &= hits - 1;
                         }
@@ -433,17 +429,52 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                         if (hn >= 32) {
                             cross(32);
                             hn -= 32;
-                            AreaHit mv{};
-                            uint8_t me_ = 0;
+                            uint32_t mv = 0;
+                            uint8_t mk = 0;
                             if (lane < hn) {
                                 mv = hit[32 + lane];
-                                me_ = hedge[32 + lane];
+                                mk = hedge[32 + lane];
                             }
                             __syncwarp();
                             if (lane < hn) {
                                 hit[lane] = mv;
-                                hedge[lane] = me_;
+                                hedge[lane] = mk;
                             }
+                        }
+                    }
+                    __syncwarp();
+                };
+                // the first m listings: those that are their edge's first go on
+                auto look_up = [&](int m) {
+                    __syncwarp();
+                    uint32_t f = 0;
+                    bool keep = false;
+                    if (lane < m) {
+                        const AreaListing l = list[lane];
+                        f = l.f;
+                        keep = first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, l.pid, l.lo, l.q, f);
+                    }
+                    const unsigned kept = __ballot_sync(full, keep);
+                    if (keep) {
+                        const int at = qn + __popc(kept & ((1u << lane) - 1u));
+                        const float2 A = orr[f], B = orr[f + 1];
+                        seg[at] = make_float4(A.x, A.y, B.x, B.y);
+                        edge[at] = f;
+                    }
+                    qn += __popc(kept);
+                    if (qn >= 32) {
+                        test(32);
+                        qn -= 32;
+                        float4 mv = make_float4(0.f, 0.f, 0.f, 0.f);
+                        uint32_t mf = 0;
+                        if (lane < qn) {
+                            mv = seg[32 + lane];
+                            mf = edge[32 + lane];
+                        }
+                        __syncwarp();
+                        if (lane < qn) {
+                            seg[lane] = mv;
+                            edge[lane] = mf;
                         }
                     }
                     __syncwarp();
@@ -488,31 +519,30 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                                 }
                                 const unsigned m = __ballot_sync(full, in);
                                 if (in)
-                                    queue[qn + __popc(m & ((1u << lane) - 1u))] =
-                                        AreaEntry{make_float4(A.x, A.y, B.x, B.y), f, fpid, fq, col.x};
-                                qn += __popc(m);
+                                    list[ln + __popc(m & ((1u << lane) - 1u))] = AreaListing{f, fpid, fq, col.x};
+                                ln += __popc(m);
                                 __syncwarp();
-                                if (qn >= 32) {
-                                    test(32);
-                                    qn -= 32;
-                                    AreaEntry mv{};
-                                    if (lane < qn) mv = queue[32 + lane];
+                                if (ln >= 32) {
+                                    look_up(32);
+                                    ln -= 32;
+                                    AreaListing mv{};
+                                    if (lane < ln) mv = list[32 + lane];
                                     __syncwarp();
-                                    if (lane < qn) queue[lane] = mv;
+                                    if (lane < ln) list[lane] = mv;
                                     __syncwarp();
                                 }
                             }
                         }
                     }
-                    // a queued edge's listing test looks back from its own row, so
-                    // it may not wait while the ring of kept rows moves on
-                    if (y == yhi || ((y - ylo) & (kQueueRows - 1)) == kQueueRows - 1) {
-                        if (qn) test(qn);
-                        qn = 0;
-                        if (hn) cross(hn);
-                        hn = 0;
+                    // a listing is looked up from its own row, so it may not
+                    // wait while the ring of kept rows moves on
+                    if (ln && (y == yhi || ((y - ylo) & (kQueueRows - 1)) == kQueueRows - 1)) {
+                        look_up(ln);
+                        ln = 0;
                     }
                 }
+                if (qn) test(qn);
+                if (hn) cross(hn);
             }
             __syncwarp();
             // parity of crossings of earlier edges of the chunk
