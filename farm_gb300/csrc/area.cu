@@ -83,7 +83,11 @@ __device__ __forceinline__ double cross2(double ax, double ay, double bx, double
 // ray to the right along the pixel row; the first non-BORDER pixel tells its
 // side, edges of BORDER pixels before it flip the parity (each edge counted in
 // the pixel whose x-range holds its crossing).
-__device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, double px, double py, int cc, int lane) {
+// Where the ray meets an edge is decided in FP32 when the ends of the pixel and
+// the point are further off than its rounding (5 u of the edge's width and 2 u
+// of its coordinates), else in FP64.
+__device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, float2 pt, int cc, int lane) {
+    const double px = pt.x, py = pt.y;
     if (px < H.mbr[0] || px > H.mbr[2] || py < H.mbr[1] || py > H.mbr[3]) return false;
     int row = offset_y(H.mbr, H.step_y, H.dimy, py);
     int col = offset_x(H.mbr, H.step_x, H.dimx, px);
@@ -98,15 +102,24 @@ __device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, double px, dou
         if (s != 1) return c == col ? (s == 2) : (odd ^ (s == 2));
         double x_lo = c == col ? -1e300 : H.mbr[0] + c * H.step_x;
         double x_hi = c == H.dimx - 1 ? 1e300 : H.mbr[0] + (c + 1) * H.step_x;
+        const float lo = (float)fmax(px, x_lo), hi = (float)x_hi;
         bool flip = false;
         for (uint32_t q = off[pid] + lane; q < off[pid + 1]; q += 32) {
             uint2 sq = seq[q];
             for (uint32_t k = 0; k < sq.y; k++) {
-                float2 a = r[sq.x + k], b = r[sq.x + k + 1];
-                if ((a.y > py) != (b.y > py)) {
-                    double xi = (double)a.x + (py - a.y) * ((double)b.x - a.x) / ((double)b.y - a.y);
-                    if (xi > px && xi >= x_lo && xi < x_hi) flip = !flip;
+                const float2 a = r[sq.x + k], b = r[sq.x + k + 1];
+                if ((a.y > pt.y) == (b.y > pt.y)) continue;
+                const float dx = b.x - a.x, dy = b.y - a.y;
+                const float xf = a.x + (pt.y - a.y) / dy * dx;
+                const float m = 1e-6f * (fabsf(dx) + fabsf(a.x) + fabsf(b.x)) + 1.2e-38f;
+                const bool ok = fabsf(dy) < INFINITY;
+                if (ok && (xf < lo - m || xf > hi + m)) continue;
+                bool in = ok && xf > lo + m && xf < hi - m;
+                if (!in) {
+                    const double xi = (double)a.x + (py - a.y) * ((double)b.x - a.x) / ((double)b.y - a.y);
+                    in = xi > px && xi >= x_lo && xi < x_hi;
                 }
+                if (in) flip = !flip;
             }
         }
         odd ^= __popc(__ballot_sync(0xffffffffu, flip)) & 1;
@@ -114,18 +127,40 @@ __device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, double px, dou
     return odd;  // past the raster: outside, so the crossings decide
 }
 
-// An edge in the other polygon's pixel units, with the rounding of those (the
-// differences are taken in double): m is far above it.
+// The other polygon's box and pixel size, in FP32: the box's corner in two
+// parts, so that a difference from it is as good as one taken in FP64 and
+// rounded, and its sides rounded so that a float is outside of them exactly
+// when it is outside of the box.
+struct Frame {
+    float xh, xl, yh, yl, sx, sy;
+    float x0, y0, x1, y1;
+};
+__device__ __forceinline__ Frame frame_of(const PolyHdr &O) {
+    Frame f;
+    f.xh = (float)O.mbr[0];
+    f.xl = (float)(O.mbr[0] - f.xh);
+    f.yh = (float)O.mbr[1];
+    f.yl = (float)(O.mbr[1] - f.yh);
+    f.sx = (float)O.step_x;
+    f.sy = (float)O.step_y;
+    f.x0 = __double2float_ru(O.mbr[0]);
+    f.y0 = __double2float_ru(O.mbr[1]);
+    f.x1 = __double2float_rd(O.mbr[2]);
+    f.y1 = __double2float_rd(O.mbr[3]);
+    return f;
+}
+
+// An edge in the other polygon's pixel units, with the rounding of those: m is
+// far above it.
 struct EdgeUV {
     float u0, v0, u1, v1, m;
 };
-__device__ __forceinline__ EdgeUV edge_uv(const PolyHdr &O, float2 P, float2 Q) {
-    const float sx = (float)O.step_x, sy = (float)O.step_y;
+__device__ __forceinline__ EdgeUV edge_uv(const Frame &O, float2 P, float2 Q) {
     EdgeUV e;
-    e.u0 = (float)((double)P.x - O.mbr[0]) / sx;
-    e.v0 = (float)((double)P.y - O.mbr[1]) / sy;
-    e.u1 = (float)((double)Q.x - O.mbr[0]) / sx;
-    e.v1 = (float)((double)Q.y - O.mbr[1]) / sy;
+    e.u0 = ((P.x - O.xh) - O.xl) / O.sx;
+    e.v0 = ((P.y - O.yh) - O.yl) / O.sy;
+    e.u1 = ((Q.x - O.xh) - O.xl) / O.sx;
+    e.v1 = ((Q.y - O.yh) - O.yl) / O.sy;
     e.m = 0.01f + 1e-6f * fmaxf(fmaxf(fabsf(e.u0), fabsf(e.u1)), fmaxf(fabsf(e.v0), fabsf(e.v1)));
     return e;
 }
@@ -153,9 +188,9 @@ __device__ __forceinline__ int2 edge_columns(const EdgeUV &e, int y, int dimx) {
 }
 
 // whether the edge has a length and its box meets O's
-__device__ __forceinline__ bool edge_meets(const PolyHdr &O, float2 P, float2 Q) {
-    return (P.x != Q.x || P.y != Q.y) && !(fmaxf(P.x, Q.x) < O.mbr[0] || fminf(P.x, Q.x) > O.mbr[2] ||
-                                           fmaxf(P.y, Q.y) < O.mbr[1] || fminf(P.y, Q.y) > O.mbr[3]);
+__device__ __forceinline__ bool edge_meets(const Frame &O, float2 P, float2 Q) {
+    return (P.x != Q.x || P.y != Q.y) && !(fmaxf(P.x, Q.x) < O.x0 || fminf(P.x, Q.x) > O.x1 ||
+                                           fmaxf(P.y, Q.y) < O.y0 || fminf(P.y, Q.y) > O.y1);
 }
 
 // A group of up to 32 consecutive edges [first, first + n) of a ring, searched
@@ -172,10 +207,11 @@ constexpr int kQueueRows = 64;  // rows a queued edge may wait
 // the group's columns of a row that is no longer kept
 __device__ __noinline__ int2 group_columns(const Group &g, int y) {
     int2 c = make_int2(0x7fffffff, -1);
+    const Frame fr = frame_of(*g.O);
     for (uint32_t k = 0; k < g.n; k++) {
         const float2 P = g.ring[g.first + k], Q = g.ring[g.first + k + 1];
-        if (!edge_meets(*g.O, P, Q)) continue;
-        const int2 e = edge_columns(edge_uv(*g.O, P, Q), y, g.O->dimx);
+        if (!edge_meets(fr, P, Q)) continue;
+        const int2 e = edge_columns(edge_uv(fr, P, Q), y, g.O->dimx);
         c.x = min(c.x, e.x);
         c.y = max(c.y, e.y);
     }
@@ -282,7 +318,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
     __shared__ uint32_t s_edge[8][kAreaQueue];
     __shared__ uint32_t s_hit[8][kAreaQueue];
     __shared__ uint8_t s_hedge[8][kAreaQueue];
-    __shared__ unsigned long long s_sum[8][32];
+    __shared__ uint32_t s_lo[8][32], s_hi[8][32];
     __shared__ uint32_t s_cnt[8][32];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -333,27 +369,26 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
         const double ox = o0.x, oy = o0.y;
         const double sign = a.orient[side_t ? a.tgt_base + a.pairs[2 * p + 1] : a.pairs[2 * p]];
         // state at the chunk's first vertex
-        bool state = pip_raster(sv, O, mr[first].x, mr[first].y, cc, lane);
+        bool state = pip_raster(sv, O, mr[first], cc, lane);
         double acc = 0;
         // a crossing leaves O when O's edge turns the way O's interior lies:
         // entering iff (d x g) has the opposite sign of O's orientation
         const double osign = a.orient[side_t ? a.pairs[2 * p] : a.tgt_base + a.pairs[2 * p + 1]];
         const uint8_t *ost = sv.status + O.st;
+        const Frame frame = frame_of(O);
         const uint32_t *ooff = sv.offset + O.off;
         const uint2 *oseq = sv.seq + O.seq;
         for (uint32_t b0 = first; b0 < last; b0 += 32) {
             const uint32_t R = min(32u, last - b0), G = 32u / R, slice = (uint32_t)lane / R;
             const uint32_t e = b0 + (uint32_t)lane % R;
             const float2 P = mr[e], Q = mr[e + 1];
-            const double px = (double)P.x - ox, py = (double)P.y - oy;
-            const double dx = (double)Q.x - P.x, dy = (double)Q.y - P.y;
-            const bool active = slice < G && edge_meets(O, P, Q);
+            const bool active = slice < G && edge_meets(frame, P, Q);
             // per edge: leaving t minus entering t, crossings
-            s_sum[wib][lane] = 0ull;
+            s_lo[wib][lane] = s_hi[wib][lane] = 0u;
             s_cnt[wib][lane] = 0u;
             __syncwarp();
             if (__any_sync(full, active)) {
-                const EdgeUV uv = edge_uv(O, P, Q);
+                const EdgeUV uv = edge_uv(frame, P, Q);
                 // rows of the group's window, and its box
                 int ylo = 0x7fffffff, yhi = -1;
                 float bx0 = INFINITY, by0 = INFINITY, bx1 = -INFINITY, by1 = -INFINITY;
@@ -383,88 +418,158 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                 const float rv = fmaxf(fabsf((float)O.mbr[1] - P.y), fabsf((float)O.mbr[3] - P.y));
                 const float ma = 1.1e-6f * (fabsf(ex) * rv + fabsf(ey) * ru);
                 const float rm = 1.1e-6f * (ru + rv + fabsf(ex) + fabsf(ey));
+                // Rows, a row's BORDER pixels 32 at a time, their sequences 32 at a
+                // time, and these' edges 32 at a time, as one loop: each step takes
+                // the innermost that is left, and what is queued is worked off in
+                // one place (the kernel's code is larger than the instruction cache
+                // takes lightly; with a copy per use 40% of the stalls were on it).
                 int ln = 0, qn = 0, hn = 0;
-                // the first m pairs that may cross: FP64, a pair per lane
-                auto cross = [&](int m) {
-                    __syncwarp();
-                    if (lane < m) {
-                        const uint32_t k = hedge[lane], f = hit[lane];
-                        const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
-                        double t, den;
-                        my_tests++;
-                        if (crossing(A, B, orr, f, t, den)) {
-                            const long long v = __double2ll_rn(t * kParamScale);
-                            atomicAdd(&s_sum[wib][k], (unsigned long long)(osign * den > 0 ? v : -v));
-                            atomicAdd(&s_cnt[wib][k], 1u);
+                int y = ylo - 1, x0 = 0;
+                int2 col = make_int2(0, -1);
+                uint32_t s0 = 0, tsq = 0, k0 = 0, te = 0;
+                uint32_t pid = 0, sq0 = 0, xsq = 0, qq = 0, qpid = 0, xe = 0;
+                uint2 sq = make_uint2(0u, 0u);
+                for (bool end = false; !end;) {
+                    bool look_all = false;
+                    if (k0 < te) {
+                        const uint32_t k = k0 + lane;
+                        k0 += 32;
+                        const int oe = warp_owner(xe, k);
+                        const uint32_t f = __shfl_sync(full, sq.x, oe) + (k - __shfl_sync(full, xe, oe));
+                        const uint32_t fq = __shfl_sync(full, qq, oe), fpid = __shfl_sync(full, qpid, oe);
+                        bool in = false;
+                        if (k < te) {
+                            const float2 A = orr[f], B = orr[f + 1];
+                            in = !(fmaxf(A.x, B.x) < bx0 || fminf(A.x, B.x) > bx1 || fmaxf(A.y, B.y) < by0 ||
+                                   fminf(A.y, B.y) > by1);
+                        }
+                        const unsigned m = __ballot_sync(full, in);
+                        if (in) list[ln + __popc(m & ((1u << lane) - 1u))] = AreaListing{f, fpid, fq, col.x};
+                        ln += __popc(m);
+                        if (ln < 32) continue;
+                    } else if (s0 < tsq) {
+                        const uint32_t si = s0 + lane;
+                        s0 += 32;
+                        const int ow = warp_owner(xsq, si);
+                        qq = __shfl_sync(full, sq0, ow) + (si - __shfl_sync(full, xsq, ow));
+                        qpid = __shfl_sync(full, pid, ow);
+                        sq = si < tsq ? oseq[qq] : make_uint2(0u, 0u);
+                        xe = warp_excl_scan(sq.y, lane, te);
+                        k0 = 0;
+                        continue;
+                    } else if (x0 <= col.y) {
+                        const int x = x0 + lane;
+                        x0 += 32;
+                        pid = (uint32_t)(y * O.dimx + x);
+                        sq0 = 0;
+                        uint32_t nsq = 0;
+                        if (x <= col.y && show_status(ost[pid], cc) == 1) {
+                            sq0 = ooff[pid];
+                            nsq = ooff[pid + 1] - sq0;
+                        }
+                        xsq = warp_excl_scan(nsq, lane, tsq);
+                        s0 = 0;
+                        continue;
+                    } else {
+                        // a listing is looked up from its own row, so it may not
+                        // wait while the ring of kept rows moves on
+                        end = ++y > yhi;
+                        look_all = end || ((y - ylo) & (kQueueRows - 1)) == 0;
+                        if (!end) {
+                            col = active ? edge_columns(uv, y, O.dimx) : make_int2(0x7fffffff, -1);
+                            col.x = __reduce_min_sync(full, col.x);
+                            col.y = __reduce_max_sync(full, col.y);
+                            x0 = col.x;
+                            if (lane == 0) rows[y & (kRowCache - 1)] = col;
+                            if (!look_all || !ln) continue;
                         }
                     }
                     __syncwarp();
-                };
-                // the first m edges against every lane's edge
-                auto test = [&](int m) {
-                    __syncwarp();
-                    unsigned hits = 0;
-                    if (active) {
-                        for (int j = (int)slice; j < m; j += (int)G) {
-                            const float4 s = seg[j];
-                            const float U = s.x - P.x, V = s.y - P.y, U2 = s.z - P.x, V2 = s.w - P.y;
-                            const float oc = __fmaf_rn(ex, V, -(ey * U)), od = __fmaf_rn(ex, V2, -(ey * U2));
-                            const float gx = U2 - U, gy = V2 - V;
-                            const float op = __fmaf_rn(gy, U, -(gx * V));
-                            const float oq = op + __fmaf_rn(gx, ey, -(gy * ex));
-                            const float mb = rm * (fabsf(gx) + fabsf(gy));
-                            if (!(fminf(oc, od) > ma || fmaxf(oc, od) < -ma || fminf(op, oq) > mb ||
-                                  fmaxf(op, oq) < -mb))
-                                hits |= 1u << j;
+                    // 32 listings, or all: those that are their edge's first go on
+                    if (ln >= 32 || (look_all && ln)) {
+                        uint32_t f = 0;
+                        bool keep = false;
+                        if (lane < ln) {
+                            const AreaListing l = list[lane];
+                            f = l.f;
+                            keep = first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, l.pid, l.lo, l.q, f);
                         }
+                        const unsigned kept = __ballot_sync(full, keep);
+                        if (keep) {
+                            const int at = qn + __popc(kept & ((1u << lane) - 1u));
+                            const float2 A = orr[f], B = orr[f + 1];
+                            seg[at] = make_float4(A.x, A.y, B.x, B.y);
+                            edge[at] = f;
+                        }
+                        qn += __popc(kept);
+                        ln = max(ln - 32, 0);
+                        AreaListing mv{};
+                        if (lane < ln) mv = list[32 + lane];
+                        __syncwarp();
+                        if (lane < ln) list[lane] = mv;
+                        __syncwarp();
                     }
-                    for (unsigned any = __ballot_sync(full, hits != 0); any; any = __ballot_sync(full, hits != 0)) {
-                        if (hits) {
-                            const int at = hn + __popc(any & ((1u << lane) - 1u));
-                            hit[at] = edge[__ffs(hits) - 1];
-                            hedge[at] = (uint8_t)((uint32_t)lane % R);
-                            hits &= hits - 1;
-                        }
-                        hn += __popc(any);
-                        if (hn >= 32) {
-                            cross(32);
-                            hn -= 32;
-                            uint32_t mv = 0;
-                            uint8_t mk = 0;
-                            if (lane < hn) {
-                                mv = hit[32 + lane];
-                                mk = hedge[32 + lane];
+                    // 32 edges, at the end all, against every lane's edge; and 32
+                    // pairs that may cross, at the end all, in FP64, one per lane
+                    while (qn >= 32 || (end && (qn | hn))) {
+                        const int m = min(qn, 32);
+                        unsigned hits = 0;
+                        if (active) {
+                            for (int j = (int)slice; j < m; j += (int)G) {
+                                const float4 s = seg[j];
+                                const float U = s.x - P.x, V = s.y - P.y, U2 = s.z - P.x, V2 = s.w - P.y;
+                                const float oc = __fmaf_rn(ex, V, -(ey * U)), od = __fmaf_rn(ex, V2, -(ey * U2));
+                                const float gx = U2 - U, gy = V2 - V;
+                                const float op = __fmaf_rn(gy, U, -(gx * V));
+                                const float oq = op + __fmaf_rn(gx, ey, -(gy * ex));
+                                const float mb = rm * (fabsf(gx) + fabsf(gy));
+                                if (!(fminf(oc, od) > ma || fmaxf(oc, od) < -ma || fminf(op, oq) > mb ||
+                                      fmaxf(op, oq) < -mb))
+                                    hits |= 1u << j;
                             }
-                            __syncwarp();
-                            if (lane < hn) {
-                                hit[lane] = mv;
-                                hedge[lane] = mk;
-                            }
                         }
-                    }
-                    __syncwarp();
-                };
-                // the first m listings: those that are their edge's first go on
-                auto look_up = [&](int m) {
-                    __syncwarp();
-                    uint32_t f = 0;
-                    bool keep = false;
-                    if (lane < m) {
-                        const AreaListing l = list[lane];
-                        f = l.f;
-                        keep = first_listing(sv, grp, rows, a.ep_off, a.ep_pix, cc, l.pid, l.lo, l.q, f);
-                    }
-                    const unsigned kept = __ballot_sync(full, keep);
-                    if (keep) {
-                        const int at = qn + __popc(kept & ((1u << lane) - 1u));
-                        const float2 A = orr[f], B = orr[f + 1];
-                        seg[at] = make_float4(A.x, A.y, B.x, B.y);
-                        edge[at] = f;
-                    }
-                    qn += __popc(kept);
-                    if (qn >= 32) {
-                        test(32);
-                        qn -= 32;
+                        const int left = qn - m;
+                        unsigned any;
+                        do {
+                            any = __ballot_sync(full, hits != 0);
+                            if (hits) {
+                                const int at = hn + __popc(any & ((1u << lane) - 1u));
+                                hit[at] = edge[__ffs(hits) - 1];
+                                hedge[at] = (uint8_t)((uint32_t)lane % R);
+                                hits &= hits - 1;
+                            }
+                            hn += __popc(any);
+                            if (hn >= 32 || (end && !left && !any && hn)) {
+                                __syncwarp();
+                                if (lane < hn) {
+                                    const uint32_t k = hedge[lane], f = hit[lane];
+                                    const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
+                                    double t, den;
+                                    my_tests++;
+                                    if (crossing(A, B, orr, f, t, den)) {
+                                        const long long v = __double2ll_rn(t * kParamScale);
+                                        const unsigned long long w = (unsigned long long)(osign * den > 0 ? v : -v);
+                                        const uint32_t wl = (uint32_t)w;
+                                        const uint32_t old = atomicAdd(&s_lo[wib][k], wl);
+                                        atomicAdd(&s_hi[wib][k], (uint32_t)(w >> 32) + (old + wl < wl ? 1u : 0u));
+                                        atomicAdd(&s_cnt[wib][k], 1u);
+                                    }
+                                }
+                                hn = max(hn - 32, 0);
+                                uint32_t mv = 0;
+                                uint8_t mk = 0;
+                                if (lane < hn) {
+                                    mv = hit[32 + lane];
+                                    mk = hedge[32 + lane];
+                                }
+                                __syncwarp();
+                                if (lane < hn) {
+                                    hit[lane] = mv;
+                                    hedge[lane] = mk;
+                                }
+                            }
+                        } while (any);
+                        qn = left;
                         float4 mv = make_float4(0.f, 0.f, 0.f, 0.f);
                         uint32_t mf = 0;
                         if (lane < qn) {
@@ -476,73 +581,9 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                             seg[lane] = mv;
                             edge[lane] = mf;
                         }
-                    }
-                    __syncwarp();
-                };
-                for (int y = ylo; y <= yhi; y++) {
-                    int2 col = active ? edge_columns(uv, y, O.dimx) : make_int2(0x7fffffff, -1);
-                    col.x = __reduce_min_sync(full, col.x);
-                    col.y = __reduce_max_sync(full, col.y);
-                    if (lane == 0) rows[y & (kRowCache - 1)] = col;
-                    __syncwarp();
-                    for (int x0 = col.x; x0 <= col.y; x0 += 32) {
-                        // the row's BORDER pixels, their sequences, and these' edges, flattened
-                        const int x = x0 + lane;
-                        const uint32_t pid = (uint32_t)(y * O.dimx + x);
-                        uint32_t sq0 = 0, nsq = 0;
-                        if (x <= col.y && show_status(ost[pid], cc) == 1) {
-                            sq0 = ooff[pid];
-                            nsq = ooff[pid + 1] - sq0;
-                        }
-                        uint32_t tsq;
-                        const uint32_t xsq = warp_excl_scan(nsq, lane, tsq);
-                        for (uint32_t s0 = 0; s0 < tsq; s0 += 32) {
-                            const uint32_t si = s0 + lane;
-                            const int ow = warp_owner(xsq, si);
-                            const uint32_t q = __shfl_sync(full, sq0, ow) + (si - __shfl_sync(full, xsq, ow));
-                            const uint32_t qpid = __shfl_sync(full, pid, ow);
-                            const uint2 sq = si < tsq ? oseq[q] : make_uint2(0u, 0u);
-                            uint32_t te;
-                            const uint32_t xe = warp_excl_scan(sq.y, lane, te);
-                            for (uint32_t k0 = 0; k0 < te; k0 += 32) {
-                                const uint32_t k = k0 + lane;
-                                const int oe = warp_owner(xe, k);
-                                const uint32_t f = __shfl_sync(full, sq.x, oe) + (k - __shfl_sync(full, xe, oe));
-                                const uint32_t fq = __shfl_sync(full, q, oe), fpid = __shfl_sync(full, qpid, oe);
-                                bool in = false;
-                                float2 A = make_float2(0.f, 0.f), B = A;
-                                if (k < te) {
-                                    A = orr[f];
-                                    B = orr[f + 1];
-                                    in = !(fmaxf(A.x, B.x) < bx0 || fminf(A.x, B.x) > bx1 || fmaxf(A.y, B.y) < by0 ||
-                                           fminf(A.y, B.y) > by1);
-                                }
-                                const unsigned m = __ballot_sync(full, in);
-                                if (in)
-                                    list[ln + __popc(m & ((1u << lane) - 1u))] = AreaListing{f, fpid, fq, col.x};
-                                ln += __popc(m);
-                                __syncwarp();
-                                if (ln >= 32) {
-                                    look_up(32);
-                                    ln -= 32;
-                                    AreaListing mv{};
-                                    if (lane < ln) mv = list[32 + lane];
-                                    __syncwarp();
-                                    if (lane < ln) list[lane] = mv;
-                                    __syncwarp();
-                                }
-                            }
-                        }
-                    }
-                    // a listing is looked up from its own row, so it may not
-                    // wait while the ring of kept rows moves on
-                    if (ln && (y == yhi || ((y - ylo) & (kQueueRows - 1)) == kQueueRows - 1)) {
-                        look_up(ln);
-                        ln = 0;
+                        __syncwarp();
                     }
                 }
-                if (qn) test(qn);
-                if (hn) cross(hn);
             }
             __syncwarp();
             // parity of crossings of earlier edges of the chunk
@@ -550,12 +591,16 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
             const uint32_t tot_c = valid ? s_cnt[wib][lane] : 0u;
             const unsigned odd = __ballot_sync(full, valid && (tot_c & 1));
             const bool s_here = state ^ (__popc(odd & ((1u << lane) - 1)) & 1);
-            if (valid) {
-                const long long tail = (s_here ^ (tot_c & 1)) ? 1ll << 60 : 0ll;
-                const double len = (double)((long long)s_sum[wib][lane] + tail) * (1.0 / kParamScale);
-                acc += cross2(px, py, dx, dy) * len;
-                my_cross += (unsigned long long)tot_c;
+            const long long tail = (s_here ^ (tot_c & 1)) ? 1ll << 60 : 0ll;
+            const long long inside =
+                valid ? (long long)((unsigned long long)s_hi[wib][lane] << 32 | s_lo[wib][lane]) + tail : 0ll;
+            const float z = (P.x - P.x) + (P.y - P.y) + (Q.x - Q.x) + (Q.y - Q.y);  // NaN unless they are finite
+            if (__any_sync(full, inside != 0 || z != 0.f)) {  // a group outside adds nothing
+                const double px = (double)P.x - ox, py = (double)P.y - oy;
+                const double dx = (double)Q.x - P.x, dy = (double)Q.y - P.y;
+                if (valid) acc += cross2(px, py, dx, dy) * ((double)inside * (1.0 / kParamScale));
             }
+            my_cross += (unsigned long long)tot_c;
             state ^= (__popc(odd) & 1);
             __syncwarp();
         }
