@@ -16,8 +16,8 @@
 // Work: items are (pair, side, chunk of that side's edges), taken by persistent
 // warps from a global counter. A lane holds one edge; the warp walks the window
 // of the other polygon's raster around all its edges together, queues the edges
-// listed there, and every lane tests its edge against each (each crossing edge
-// counted at its first listing). An edge's share is its signed inside length:
+// listed there (each at its first listing), and every lane tests its edge
+// against each. An edge's share is its signed inside length:
 // the leaving parameters minus the entering ones, plus the tail when it ends
 // inside. Per-item
 // partial sums are reduced per pair in a fixed order (deterministic results).
@@ -55,6 +55,29 @@ struct Chunks {
     }
 };
 
+// Items whose window holds many listings are cut into parts for all warps (see
+// k_area). A chunk of the pool is such an item's state: the sums of its edges'
+// crossings so far, the side of its first vertex, and its parts.
+struct AreaSpill {
+    unsigned long long sum[32];
+    uint32_t cnt[32];
+    uint64_t item;
+    uint32_t state, parts, done;
+    uint32_t pad;
+};
+struct AreaPool {
+    AreaSpill *chunk = nullptr;
+    uint2 *unit = nullptr;              // chunk, part; kAreaParts per chunk
+    unsigned long long *ctr = nullptr;  // [0] chunks asked for, [1] units, [2] next unit; zeroed
+    uint32_t cap = 0;                   // chunks; 0: every item stays with its warp
+};
+constexpr uint32_t kAreaParts = 32;   // most parts of an item
+// Steps (32 sequences each) a warp takes of an item before it is cut, and of
+// its parts. 801 pairs of up to 20,000 vertices: 5.16 ms; 32 / 8 5.38, 128 / 8
+// 5.02, 64 / 4 5.36, 64 / 16 5.25 (6.7 to 9.8 where the pool is too small for
+// the items cut); 1,440 pairs of up to 1,024 vertices: 1.35 ms with each.
+constexpr uint32_t kAreaBudget = 64, kAreaShareSteps = 8;
+
 struct AreaArgs {
     const uint32_t *pairs;
     const uint64_t *n;           // pair count (device scalar)
@@ -70,6 +93,8 @@ struct AreaArgs {
     unsigned long long *overflow;  // [0] unused, [1] items beyond cap_items
     unsigned long long *work;      // [0] FP64 crossing tests, [1] crossings counted
     int spread;                    // take items in a spread order (see k_area)
+    AreaPool pool;
+    int rest;                      // the pool's parts instead of the items
 };
 
 // Crossing parameters are added as integers of 2^-60: exact, in any order and
@@ -78,54 +103,6 @@ struct AreaArgs {
 constexpr double kParamScale = 1152921504606846976.0;  // 2^60
 
 __device__ __forceinline__ double cross2(double ax, double ay, double bx, double by) { return ax * by - ay * bx; }
-
-// Point-in-polygon of (px, py) for polygon H through its raster, by a warp: a
-// ray to the right along the pixel row; the first non-BORDER pixel tells its
-// side, edges of BORDER pixels before it flip the parity (each edge counted in
-// the pixel whose x-range holds its crossing).
-// Where the ray meets an edge is decided in FP32 when the ends of the pixel and
-// the point are further off than its rounding (5 u of the edge's width and 2 u
-// of its coordinates), else in FP64.
-__device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, float2 pt, int cc, int lane) {
-    const double px = pt.x, py = pt.y;
-    if (px < H.mbr[0] || px > H.mbr[2] || py < H.mbr[1] || py > H.mbr[3]) return false;
-    int row = offset_y(H.mbr, H.step_y, H.dimy, py);
-    int col = offset_x(H.mbr, H.step_x, H.dimx, px);
-    const uint8_t *st = sv.status + H.st;
-    const uint32_t *off = sv.offset + H.off;
-    const uint2 *seq = sv.seq + H.seq;
-    const float2 *r = sv.ring + H.ring;
-    bool odd = false;
-    for (int c = col; c < H.dimx; c++) {
-        uint32_t pid = (uint32_t)(row * H.dimx + c);
-        int s = show_status(st[pid], cc);
-        if (s != 1) return c == col ? (s == 2) : (odd ^ (s == 2));
-        double x_lo = c == col ? -1e300 : H.mbr[0] + c * H.step_x;
-        double x_hi = c == H.dimx - 1 ? 1e300 : H.mbr[0] + (c + 1) * H.step_x;
-        const float lo = (float)fmax(px, x_lo), hi = (float)x_hi;
-        bool flip = false;
-        for (uint32_t q = off[pid] + lane; q < off[pid + 1]; q += 32) {
-            uint2 sq = seq[q];
-            for (uint32_t k = 0; k < sq.y; k++) {
-                const float2 a = r[sq.x + k], b = r[sq.x + k + 1];
-                if ((a.y > pt.y) == (b.y > pt.y)) continue;
-                const float dx = b.x - a.x, dy = b.y - a.y;
-                const float xf = a.x + (pt.y - a.y) / dy * dx;
-                const float m = 1e-6f * (fabsf(dx) + fabsf(a.x) + fabsf(b.x)) + 1.2e-38f;
-                const bool ok = fabsf(dy) < INFINITY;
-                if (ok && (xf < lo - m || xf > hi + m)) continue;
-                bool in = ok && xf > lo + m && xf < hi - m;
-                if (!in) {
-                    const double xi = (double)a.x + (py - a.y) * ((double)b.x - a.x) / ((double)b.y - a.y);
-                    in = xi > px && xi >= x_lo && xi < x_hi;
-                }
-                if (in) flip = !flip;
-            }
-        }
-        odd ^= __popc(__ballot_sync(0xffffffffu, flip)) & 1;
-    }
-    return odd;  // past the raster: outside, so the crossings decide
-}
 
 // The other polygon's box and pixel size, in FP32: the box's corner in two
 // parts, so that a difference from it is as good as one taken in FP64 and
@@ -150,10 +127,61 @@ __device__ __forceinline__ Frame frame_of(const PolyHdr &O) {
     return f;
 }
 
+// Point-in-polygon of a vertex for polygon H through its raster, by a warp: a
+// ray to the right along the pixel row; the first non-BORDER pixel tells its
+// side, edges of BORDER pixels before it flip the parity (each edge counted in
+// the pixel whose x-range holds its crossing). The pixel and the crossing are
+// decided in FP32 when the pixel's ends and the point are further off than the
+// rounding (10 u of the box's coordinates at most), else in FP64.
+__device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, const Frame &fr, float2 pt, int cc, int lane) {
+    if (pt.x < fr.x0 || pt.x > fr.x1 || pt.y < fr.y0 || pt.y > fr.y1) return false;
+    const float u = ((pt.x - fr.xh) - fr.xl) / fr.sx, v = ((pt.y - fr.yh) - fr.yl) / fr.sy;
+    int col = (int)u, row = (int)v;
+    const float fu = u - (float)col, fv = v - (float)row, mu = 1e-4f + 1e-6f * u, mv = 1e-4f + 1e-6f * v;
+    if (!(fu > mu && fu < 1.f - mu && col < H.dimx)) col = offset_x(H.mbr, H.step_x, H.dimx, pt.x);
+    if (!(fv > mv && fv < 1.f - mv && row < H.dimy)) row = offset_y(H.mbr, H.step_y, H.dimy, pt.y);
+    const uint8_t *st = sv.status + H.st;
+    const uint32_t *off = sv.offset + H.off;
+    const uint2 *seq = sv.seq + H.seq;
+    const float2 *r = sv.ring + H.ring;
+    const float m = 1e-6f * (fabsf(fr.x0) + fabsf(fr.x1)) + 1.2e-38f;
+    bool odd = false;
+    for (int c = col; c < H.dimx; c++) {
+        const uint32_t pid = (uint32_t)(row * H.dimx + c);
+        const int s = show_status(st[pid], cc);
+        if (s != 1) return c == col ? (s == 2) : (odd ^ (s == 2));
+        const float lo = c == col ? pt.x : fmaxf(pt.x, fr.xh + (float)c * fr.sx);
+        const float hi = c == H.dimx - 1 ? INFINITY : fr.xh + (float)(c + 1) * fr.sx;
+        bool flip = false;
+        for (uint32_t q = off[pid] + lane; q < off[pid + 1]; q += 32) {
+            const uint2 sq = seq[q];
+            for (uint32_t k = 0; k < sq.y; k++) {
+                const float2 a = r[sq.x + k], b = r[sq.x + k + 1];
+                if ((a.y > pt.y) == (b.y > pt.y)) continue;
+                const float dx = b.x - a.x, dy = b.y - a.y;
+                const float xf = a.x + (pt.y - a.y) / dy * dx;
+                const bool ok = fabsf(dy) < INFINITY;
+                if (ok && (xf < lo - m || xf > hi + m)) continue;
+                bool in = ok && xf > lo + m && xf < hi - m;
+                if (!in) {
+                    const double x_lo = c == col ? -1e300 : H.mbr[0] + c * H.step_x;
+                    const double x_hi = c == H.dimx - 1 ? 1e300 : H.mbr[0] + (c + 1) * H.step_x;
+                    const double xi = (double)a.x + ((double)pt.y - a.y) * ((double)b.x - a.x) / ((double)b.y - a.y);
+                    in = xi > (double)pt.x && xi >= x_lo && xi < x_hi;
+                }
+                if (in) flip = !flip;
+            }
+        }
+        odd ^= __popc(__ballot_sync(0xffffffffu, flip)) & 1;
+    }
+    return odd;  // past the raster: outside, so the crossings decide
+}
+
 // An edge in the other polygon's pixel units, with the rounding of those: m is
 // far above it.
 struct EdgeUV {
     float u0, v0, u1, v1, m;
+    float per_row;  // 1 / (v1 - v0), 0 when that is within m
 };
 __device__ __forceinline__ EdgeUV edge_uv(const Frame &O, float2 P, float2 Q) {
     EdgeUV e;
@@ -162,6 +190,7 @@ __device__ __forceinline__ EdgeUV edge_uv(const Frame &O, float2 P, float2 Q) {
     e.u1 = ((Q.x - O.xh) - O.xl) / O.sx;
     e.v1 = ((Q.y - O.yh) - O.yl) / O.sy;
     e.m = 0.01f + 1e-6f * fmaxf(fmaxf(fabsf(e.u0), fabsf(e.u1)), fmaxf(fabsf(e.v0), fabsf(e.v1)));
+    e.per_row = fabsf(e.v1 - e.v0) > e.m ? 1.f / (e.v1 - e.v0) : 0.f;
     return e;
 }
 
@@ -173,10 +202,10 @@ __device__ __forceinline__ EdgeUV edge_uv(const Frame &O, float2 P, float2 Q) {
 __device__ __forceinline__ int2 edge_columns(const EdgeUV &e, int y, int dimx) {
     const float a = (float)(y - 1) - e.m, b = (float)(y + 2) + e.m;
     if (fmaxf(e.v0, e.v1) < a || fminf(e.v0, e.v1) > b) return make_int2(0x7fffffff, -1);
-    const float du = e.u1 - e.u0, dv = e.v1 - e.v0;
+    const float du = e.u1 - e.u0;
     float t0 = 0.f, t1 = 1.f;
-    if (fabsf(dv) > e.m) {
-        const float p = (a - e.v0) / dv, q = (b - e.v0) / dv;
+    if (e.per_row != 0.f) {
+        const float p = (a - e.v0) * e.per_row, q = (b - e.v0) * e.per_row;
         t0 = fmaxf(0.f, fminf(p, q));
         t1 = fminf(1.f, fmaxf(p, q));
     }
@@ -242,13 +271,9 @@ __device__ bool first_listing(const StoreView &sv, const Group &g, const int2 *r
         }
         const int ry = (int)(r / dimx), rx = (int)(r - (uint32_t)ry * dimx);
         if (ry < g.sy) continue;  // above the window
-        if (show_status(sv.status[O.st + r], cc) != 1) continue;
-        if (ry == py) {
-            if (rx >= lo) return false;
-            continue;
-        }
-        const int2 c = ry > py - (kRowCache - kQueueRows) ? rows[ry & (kRowCache - 1)] : group_columns(g, ry);
-        if (rx >= c.x && rx <= c.y) return false;
+        int2 c = make_int2(lo, 0x7fffffff);
+        if (ry != py) c = ry > py - (kRowCache - kQueueRows) ? rows[ry & (kRowCache - 1)] : group_columns(g, ry);
+        if (rx >= c.x && rx <= c.y && show_status(sv.status[O.st + r], cc) == 1) return false;
     }
     if (self > 1) {  // pid holds f in more than one sequence: the first counts
         const uint2 *seq = sv.seq + O.seq;
@@ -261,29 +286,36 @@ __device__ bool first_listing(const StoreView &sv, const Group &g, const int2 *r
 }
 
 // Crossing parameter t of segment P -> Q with edge e of ring r, in [0, 1) on
-// both (half-open, so a crossing at a shared vertex counts once). The
-// differences of floats are taken in double; both parameters' ranges are
-// decided on numerator and denominator (n / d < 1 exactly when |n| < |d| of
-// the same sign, as doubles one ulp apart divide to less than 1), so that
-// only a crossing divides, once.
-__device__ __forceinline__ bool crossing(float2 P, float2 Q, const float2 *r, uint32_t e, double &t, double &den) {
+// both (half-open, so a crossing at a shared vertex counts once); known: that
+// they cross is certain, only t is wanted. The differences of floats are taken
+// in double; both parameters' ranges are decided on numerator and denominator
+// (n / d < 1 exactly when |n| < |d| of the same sign, as doubles one ulp apart
+// divide to less than 1), so that only a crossing divides, once.
+__device__ __forceinline__ bool crossing(float2 P, float2 Q, const float2 *r, uint32_t e, bool known, double &t,
+                                         double &den) {
     const float2 a = r[e], b = r[e + 1];
     const double dx = (double)Q.x - P.x, dy = (double)Q.y - P.y;
     const double gx = (double)b.x - a.x, gy = (double)b.y - a.y;
     den = cross2(dx, dy, gx, gy);
-    if (den == 0) return false;
     const double rx = (double)a.x - P.x, ry = (double)a.y - P.y;
-    const double tn = cross2(rx, ry, gx, gy), un = cross2(rx, ry, dx, dy);
-    const double ad = fabs(den);
-    const bool neg = den < 0;
-    const bool t_in = fabs(tn) < ad && (tn == 0 || (tn < 0) == neg);
-    const bool u_in = fabs(un) < ad && (un == 0 || (un < 0) == neg);
-    if (!(t_in && u_in)) return false;
+    const double tn = cross2(rx, ry, gx, gy);
+    if (!known) {
+        if (den == 0) return false;
+        const double un = cross2(rx, ry, dx, dy), ad = fabs(den);
+        const bool neg = den < 0;
+        const bool t_in = fabs(tn) < ad && (tn == 0 || (tn < 0) == neg);
+        const bool u_in = fabs(un) < ad && (un == 0 || (un < 0) == neg);
+        if (!(t_in && u_in)) return false;
+    }
     t = tn / den;
     return true;
 }
 
-constexpr int kDefaultChunk = 16;   // edges per item
+// Edges per item: one group, a lane each. 801 pairs of up to 20,000 vertices: 7.7
+// ms with 8, 5.2 with 16, 4.5 with 24, 4.0 with 32; 1,440 pairs of up to 1,024
+// vertices 1.55 / 1.38 / 1.41 / 1.37 ms. Larger items repeat no walk either, but
+// are not cut.
+constexpr int kDefaultChunk = 32;
 constexpr int kDefaultWide = 200;   // of the window table, which nothing reads any more
 
 // FARM_AREA_SPREAD=0 takes the items in pair order
@@ -293,24 +325,66 @@ static int spread_items() {
 }
 
 
-// What bounds it is instruction issue in the tests of edge pairs. A lane per
-// edge that walked its own window of pixels, sequences and listed edges kept 7
-// of 32 lanes busy and took two FP64 divisions per row and edge; consecutive
-// edges lie together, so the group's common window is little larger than each
-// edge's, and its listed edges, those whose box meets the group's, are queued
-// and tested by all lanes at once. A group of R < 32 edges is repeated over
-// floor(32 / R) slices of lanes, which share the queue. Row ranges are FP32
+// What bounds it is instruction issue and the latency of the look-ups, then
+// FP64, which GB300 issues at 1/64 of its FP32 rate. A lane per edge that
+// walked its own window of pixels, sequences and listed edges kept 7 of 32
+// lanes busy and took two FP64 divisions per row and edge; consecutive edges
+// lie together, so the group's common window is little larger than each
+// edge's, and its listings go through three queues, each worked off 32 at a
+// time by all lanes: listings whose edge's box meets the group's (are they the
+// edge's first?), the edges of first listings (FP32 test with every lane's
+// edge), and the pairs that may cross (FP64). A group of R < 32 edges is
+// repeated over floor(32 / R) slices of lanes in the test. Row ranges are FP32
 // with a margin: they need only hold every crossing's listings, and the same
 // for all of an item. A pair of edges is rejected in FP32 when one lies
 // strictly on one side of the other's line by a margin far above the test's
-// rounding and crossing()'s, so only the pairs near a crossing reach FP64,
-// which GB300 issues at 1/64 of its FP32 rate.
-// 801 pairs of up to 20,000 vertices: 72 ms with a window per lane.
+// rounding and crossing()'s, and known to cross when both lie on either side
+// by it.
+//
+// Items differ by three orders of magnitude: half of them take under 10 us,
+// while an edge of a small polygon can have most of a large one in its window
+// (20,000 listings, 5 ms, twice the whole pass's share of a warp). So an item
+// is cut after kAreaBudget steps; a second launch takes the parts, each every
+// parts-th step of the same walk, adds its integer sums to the item's, and the
+// last one finishes the item: the same bits however it is cut.
+// 801 pairs of up to 20,000 vertices: 72 ms with a window per lane, 10.0 ms
+// with the look-up after the tests, 6.2 ms without cutting, 4.3 ms so.
 constexpr int kAreaQueue = 64;
 struct AreaListing {  // an edge met in a pixel of the window
     uint32_t f, pid, q;
     int lo;  // first column of the row it was met in
 };
+// the warp's share of an item
+struct AreaShare {
+    AreaSpill *sp;         // the item's chunk, if it is in the pool
+    uint32_t own, stride;  // its steps: own, own + stride, ...
+    uint32_t left;         // some of the item is left to others
+};
+
+// The rest of the warp's item to the pool: false when that is full.
+__device__ __noinline__ bool area_spill(const AreaPool &pool, AreaShare *sh, uint64_t item, bool state, float rest,
+                                        int lane) {
+    unsigned long long c = 0, u = 0;
+    if (lane == 0) c = atomicAdd(&pool.ctr[0], 1ull);
+    c = __shfl_sync(0xffffffffu, c, 0);
+    if (c >= pool.cap) return false;
+    AreaSpill *sp = &pool.chunk[c];
+    const uint32_t parts = 1u + min(kAreaParts - 1u, (uint32_t)(rest / (float)kAreaShareSteps));
+    if (lane == 0) {
+        sp->item = item;
+        sp->state = state;
+        sp->parts = parts;
+        sp->done = 0;
+        u = atomicAdd(&pool.ctr[1], (unsigned long long)parts);
+        sh->sp = sp;
+        sh->left = 1;
+    }
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (lane < (int)parts) pool.unit[u + lane] = make_uint2((uint32_t)c, (uint32_t)lane);
+    __syncwarp();
+    return true;
+}
+
 __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a) {
     __shared__ int2 s_rows[8][kRowCache];
     __shared__ AreaListing s_list[8][kAreaQueue];
@@ -320,6 +394,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
     __shared__ uint8_t s_hedge[8][kAreaQueue];
     __shared__ uint32_t s_lo[8][32], s_hi[8][32];
     __shared__ uint32_t s_cnt[8][32];
+    __shared__ AreaShare s_share[8];
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int cc = sv.category_count;
@@ -338,8 +413,19 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
             break;
         }
         unsigned long long it = 0;
-        if (lane == 0) it = atomicAdd(a.next, 1ull);
+        if (lane == 0) it = atomicAdd(a.rest ? &a.pool.ctr[2] : a.next, 1ull);
         it = __shfl_sync(full, it, 0);
+        AreaShare *share = &s_share[wib];
+        if (a.rest) {
+            if (it >= a.pool.ctr[1]) break;
+            const uint2 u = a.pool.unit[it];
+            AreaSpill *sp = &a.pool.chunk[u.x];
+            it = sp->item;
+            if (lane == 0) *share = AreaShare{sp, kAreaBudget + u.y, sp->parts, 0u};
+        } else if (lane == 0) {
+            *share = AreaShare{nullptr, 0u, 1u, 0u};
+        }
+        __syncwarp();
         if (it >= nitems) break;
         // Items lie pair after pair, and the heavy pairs' items are each slow:
         // taken in that order, a heavy pair near the end leaves a tail. The
@@ -347,7 +433,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
         // nitems: a bijection), which spreads every pair's items over the
         // pass. Each item writes its own partial, and the per-pair reduction
         // runs in item order, so the results do not depend on this order.
-        if (a.spread) {
+        if (a.spread && !a.rest) {
             const uint64_t P = (nitems % 1000003ull) ? 1000003ull : 999983ull;
             it = (unsigned long long)((it * P) % nitems);
         }
@@ -368,14 +454,16 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
         const float2 o0 = sv.ring[S.ring];
         const double ox = o0.x, oy = o0.y;
         const double sign = a.orient[side_t ? a.tgt_base + a.pairs[2 * p + 1] : a.pairs[2 * p]];
+        const Frame frame = frame_of(O);
         // state at the chunk's first vertex
-        bool state = pip_raster(sv, O, mr[first], cc, lane);
+        bool state = a.rest ? share->sp->state != 0 : pip_raster(sv, O, frame, mr[first], cc, lane);
+        // only a single group's sums can be left to the pool
+        const uint32_t limit = !a.rest && a.pool.cap && last - first <= 32 ? kAreaBudget : 0xffffffffu;
         double acc = 0;
         // a crossing leaves O when O's edge turns the way O's interior lies:
         // entering iff (d x g) has the opposite sign of O's orientation
-        const double osign = a.orient[side_t ? a.pairs[2 * p] : a.tgt_base + a.pairs[2 * p + 1]];
+        const bool inner_left = a.orient[side_t ? a.pairs[2 * p] : a.tgt_base + a.pairs[2 * p + 1]] > 0;
         const uint8_t *ost = sv.status + O.st;
-        const Frame frame = frame_of(O);
         const uint32_t *ooff = sv.offset + O.off;
         const uint2 *oseq = sv.seq + O.seq;
         for (uint32_t b0 = first; b0 < last; b0 += 32) {
@@ -424,6 +512,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                 // one place (the kernel's code is larger than the instruction cache
                 // takes lightly; with a copy per use 40% of the stalls were on it).
                 int ln = 0, qn = 0, hn = 0;
+                uint32_t step = 0, turn = share->own;
                 int y = ylo - 1, x0 = 0;
                 int2 col = make_int2(0, -1);
                 uint32_t s0 = 0, tsq = 0, k0 = 0, te = 0;
@@ -447,9 +536,15 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                         if (in) list[ln + __popc(m & ((1u << lane) - 1u))] = AreaListing{f, fpid, fq, col.x};
                         ln += __popc(m);
                         if (ln < 32) continue;
+                    } else if (s0 < tsq && step == limit &&
+                               area_spill(a.pool, share, it, state,
+                                          (float)step / (float)(y - ylo + 1) * (float)(yhi - y + 1), lane)) {
+                        end = look_all = true;
                     } else if (s0 < tsq) {
                         const uint32_t si = s0 + lane;
                         s0 += 32;
+                        if (step++ != turn) continue;
+                        turn += share->stride;
                         const int ow = warp_owner(xsq, si);
                         qq = __shfl_sync(full, sq0, ow) + (si - __shfl_sync(full, xsq, ow));
                         qpid = __shfl_sync(full, pid, ow);
@@ -513,7 +608,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                     // pairs that may cross, at the end all, in FP64, one per lane
                     while (qn >= 32 || (end && (qn | hn))) {
                         const int m = min(qn, 32);
-                        unsigned hits = 0;
+                        unsigned hits = 0, known = 0;  // known: both ends clearly on either side, of both
                         if (active) {
                             for (int j = (int)slice; j < m; j += (int)G) {
                                 const float4 s = seg[j];
@@ -526,6 +621,9 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                                 if (!(fminf(oc, od) > ma || fmaxf(oc, od) < -ma || fminf(op, oq) > mb ||
                                       fmaxf(op, oq) < -mb))
                                     hits |= 1u << j;
+                                if (fminf(oc, od) < -ma && fmaxf(oc, od) > ma && fminf(op, oq) < -mb &&
+                                    fmaxf(op, oq) > mb)
+                                    known |= 1u << j;
                             }
                         }
                         const int left = qn - m;
@@ -534,21 +632,22 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                             any = __ballot_sync(full, hits != 0);
                             if (hits) {
                                 const int at = hn + __popc(any & ((1u << lane) - 1u));
-                                hit[at] = edge[__ffs(hits) - 1];
-                                hedge[at] = (uint8_t)((uint32_t)lane % R);
+                                const int j = __ffs(hits) - 1;
+                                hit[at] = edge[j];
+                                hedge[at] = (uint8_t)((uint32_t)lane % R | (known >> j & 1u) << 5);
                                 hits &= hits - 1;
                             }
                             hn += __popc(any);
                             if (hn >= 32 || (end && !left && !any && hn)) {
                                 __syncwarp();
                                 if (lane < hn) {
-                                    const uint32_t k = hedge[lane], f = hit[lane];
+                                    const uint32_t h = hedge[lane], k = h & 31u, f = hit[lane];
                                     const float2 A = mr[b0 + k], B = mr[b0 + k + 1];
                                     double t, den;
                                     my_tests++;
-                                    if (crossing(A, B, orr, f, t, den)) {
+                                    if (crossing(A, B, orr, f, (h & 32u) != 0, t, den)) {
                                         const long long v = __double2ll_rn(t * kParamScale);
-                                        const unsigned long long w = (unsigned long long)(osign * den > 0 ? v : -v);
+                                        const unsigned long long w = (unsigned long long)((den > 0) == inner_left ? v : -v);
                                         const uint32_t wl = (uint32_t)w;
                                         const uint32_t old = atomicAdd(&s_lo[wib][k], wl);
                                         atomicAdd(&s_hi[wib][k], (uint32_t)(w >> 32) + (old + wl < wl ? 1u : 0u));
@@ -586,6 +685,30 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                 }
             }
             __syncwarp();
+            if (AreaSpill *sp = share->sp) {
+                // its sums to the pool; the last part takes all of them
+                const unsigned long long v = (unsigned long long)s_hi[wib][lane] << 32 | s_lo[wib][lane];
+                if (share->left) {
+                    sp->sum[lane] = v;
+                    sp->cnt[lane] = s_cnt[wib][lane];
+                    continue;
+                }
+                if (s_cnt[wib][lane]) {
+                    atomicAdd(&sp->sum[lane], v);
+                    atomicAdd(&sp->cnt[lane], s_cnt[wib][lane]);
+                }
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) share->left = atomicAdd(&sp->done, 1u) + 1u != share->stride;
+                __syncwarp();
+                if (share->left) continue;
+                __threadfence();
+                const unsigned long long tot = __ldcg(&sp->sum[lane]);
+                s_lo[wib][lane] = (uint32_t)tot;
+                s_hi[wib][lane] = (uint32_t)(tot >> 32);
+                s_cnt[wib][lane] = __ldcg(&sp->cnt[lane]);
+                __syncwarp();
+            }
             // parity of crossings of earlier edges of the chunk
             const bool valid = (uint32_t)lane < R;
             const uint32_t tot_c = valid ? s_cnt[wib][lane] : 0u;
@@ -604,6 +727,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
             state ^= (__popc(odd) & 1);
             __syncwarp();
         }
+        if (share->left) continue;
         for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(full, acc, o);
         if (lane == 0) a.partial[it] = 0.5 * sign * acc;
     }
@@ -784,7 +908,22 @@ struct AreaBufs {
     size_t scan_bytes;
     double *out;
     Chunks chunks;
+    AreaPool pool;
 };
+
+// The pool's memory: a chunk per eight items (one in 14 of 801 pairs of up to
+// 20,000 vertices is cut). Without it (an allocation that fails) every item
+// stays with its warp.
+static AreaPool area_pool(DevBuf &b, uint64_t items, unsigned long long *ctr) {
+    AreaPool p;
+    const uint64_t cap = std::min<uint64_t>(32768, std::max<uint64_t>(512, items / 8));
+    if (b.ensure(cap * (sizeof(AreaSpill) + kAreaParts * sizeof(uint2)) + 64) != FARM_OK) return p;
+    p.chunk = b.as<AreaSpill>();
+    p.unit = reinterpret_cast<uint2 *>(p.chunk + cap);
+    p.ctr = ctr;
+    p.cap = (uint32_t)cap;
+    return p;
+}
 
 static int scan_bytes(uint64_t cap, size_t *bytes) {
     FARM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, *bytes, (const uint64_t *)nullptr, (uint64_t *)nullptr,
@@ -803,7 +942,7 @@ static int area_items(farm_store *s, const AreaBufs &b, cudaStream_t st) {
 }
 
 static int area_compute(farm_store *s, const AreaBufs &b, cudaStream_t st) {
-    FARM_CUDA(cudaMemsetAsync(b.ctr, 0, 40, st));
+    FARM_CUDA(cudaMemsetAsync(b.ctr, 0, 64, st));
     AreaArgs aa{b.pairs,
                 b.n,
                 s->n_side[0],
@@ -817,9 +956,16 @@ static int area_compute(farm_store *s, const AreaBufs &b, cudaStream_t st) {
                 b.ctr,
                 b.ctr + 1,
                 b.ctr + 3,
-                spread_items()};
+                spread_items(),
+                b.pool,
+                0};
     k_area<<<sm_count() * 8, 256, 0, st>>>(s->view(), aa);
     FARM_CUDA(cudaGetLastError());
+    if (b.pool.cap) {
+        aa.rest = 1;
+        k_area<<<sm_count() * 3, 256, 0, st>>>(s->view(), aa);
+        FARM_CUDA(cudaGetLastError());
+    }
     unsigned blocks = (unsigned)((b.cap_pairs + 255) / 256);
     if (blocks > 4096) blocks = 4096;
     if (!blocks) blocks = 1;
@@ -883,6 +1029,7 @@ int intersection_area(farm_store *s, const uint32_t *pairs, uint64_t n, int mem,
     FARM_CUDA(cudaStreamSynchronize(stream));
     FARM_TRY(part.ensure(8 * nitems + 64));
     b.partial = part.as<double>();
+    b.pool = area_pool(s->s[Q_SPILL], nitems, ctr + 5);
     b.cap_items = nitems;
     FARM_TRY(area_compute(s, b, stream));
     FARM_CUDA(cudaEventRecord(s->ev[7], stream));
@@ -890,7 +1037,7 @@ int intersection_area(farm_store *s, const uint32_t *pairs, uint64_t n, int mem,
     unsigned long long work[2] = {0, 0};
     FARM_CUDA(cudaMemcpyAsync(work, ctr + 3, 16, cudaMemcpyDeviceToHost, stream));
     FARM_CUDA(cudaStreamSynchronize(stream));
-    s->launches += 4;
+    s->launches += b.pool.cap ? 5 : 4;
     if (st) {
         memset(st, 0, sizeof *st);
         st->pairs = n;
@@ -900,7 +1047,7 @@ int intersection_area(farm_store *s, const uint32_t *pairs, uint64_t n, int mem,
         cudaEventElapsedTime(&ms, s->ev[6], s->ev[7]);
         st->ms_total = ms;
         st->ms_stage[2] = ms;
-        st->kernel_launches = 4;
+        st->kernel_launches = b.pool.cap ? 5 : 4;
     }
     return FARM_OK;
 }
@@ -926,7 +1073,7 @@ extern "C" int farm_intersection_area(farm_store *s, const uint32_t *pairs, uint
 struct farm_area_plan {
     farm_store *s = nullptr;
     uint64_t cap_pairs = 0, cap_items = 0, epoch = 0;
-    farm::DevBuf pairs, n, cnt, start, partial, ctr, tmp, out;
+    farm::DevBuf pairs, n, cnt, start, partial, ctr, tmp, out, pool;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
 };
@@ -936,7 +1083,7 @@ void plan_free(farm_area_plan *p) {
     if (!p) return;
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->graph) cudaGraphDestroy(p->graph);
-    for (farm::DevBuf *b : {&p->pairs, &p->n, &p->cnt, &p->start, &p->partial, &p->ctr, &p->tmp, &p->out})
+    for (farm::DevBuf *b : {&p->pairs, &p->n, &p->cnt, &p->start, &p->partial, &p->ctr, &p->tmp, &p->out, &p->pool})
         b->release();
     delete p;
 }
@@ -965,7 +1112,7 @@ extern "C" int farm_area_plan_create(farm_store *s, uint64_t max_pairs, uint64_t
     if (rc == FARM_OK) rc = p->cnt.ensure(8 * (max_pairs + 1) + 64);
     if (rc == FARM_OK) rc = p->start.ensure(8 * (max_pairs + 1) + 64);
     if (rc == FARM_OK) rc = p->partial.ensure(8 * max_items + 64);
-    if (rc == FARM_OK) rc = p->ctr.ensure(64);
+    if (rc == FARM_OK) rc = p->ctr.ensure(128);
     if (rc == FARM_OK) rc = p->out.ensure(8 * max_pairs + 64);
     if (rc == FARM_OK) rc = scan_bytes(max_pairs, &b.scan_bytes);
     if (rc == FARM_OK) rc = p->tmp.ensure(b.scan_bytes + 64);
@@ -989,6 +1136,7 @@ extern "C" int farm_area_plan_create(farm_store *s, uint64_t max_pairs, uint64_t
     b.scan_tmp = p->tmp.p;
     b.out = p->out.as<double>();
     b.chunks = chunks_of(s);
+    b.pool = area_pool(p->pool, max_items, b.ctr + 5);
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
         plan_free(p);
@@ -1040,7 +1188,7 @@ extern "C" int farm_area_plan_run(farm_area_plan *p, const uint32_t *pairs, uint
     FARM_CUDA(cudaMemcpyAsync(flags, p->ctr.p, 40, cudaMemcpyDeviceToHost, st));
     if (n) FARM_CUDA(cudaMemcpyAsync(out, p->out.p, 8 * n, k_out, st));
     FARM_CUDA(cudaStreamSynchronize(st));
-    s->launches += 3;
+    s->launches += p->pool.cap ? 4 : 3;
     if (flags[2]) {
         set_error("farm_area_plan_run: the batch needs more work items than the plan's capacity of " +
                   std::to_string(p->cap_items));

@@ -233,7 +233,7 @@ enum ScratchSlot : int {
     Q_AREA_EPOFF = 37,  // area: edge -> pixel index offsets (per ring position)
     Q_AREA_EPPIX = 38,  // area: edge -> pixel index entries
     Q_PAIR_ORDER = 39,  // intersect: the longest-first pair order
-    Q_SPILL = 48,       // intersect, contain, within: work left to all warps
+    Q_SPILL = 48,       // intersect, contain, within, area: work left to all warps
     Q_BOX = 51,         // vertex boxes (ring_boxes)
 };
 }  // namespace farm

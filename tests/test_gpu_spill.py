@@ -67,3 +67,26 @@ def test_gpu_within_spilled_candidates_match_oracle(gpu_lib, monkeypatch, seed, 
     assert found == int(exp.sum())
     exp = np.array([O.within_heuristic(RS[s], RS[t], distance, geo) for s, t in pairs], np.uint8)
     assert np.array_equal(apx, exp), f"{int((apx != exp).sum())} of {len(exp)} differ (-a)"
+
+
+@pytest.mark.parametrize("chunk", [1, 16, 32, 33])  # items of more than 32 edges are not cut
+@pytest.mark.parametrize("seed,s_lo,s_hi,t_lo,t_hi,vpr", [(91, 8, 40, 9000, 14000, 10), (92, 600, 1500, 3000, 6000, 64),
+                                                          (93, 2000, 3000, 2000, 3000, 10)])
+def test_gpu_area_cut_items_match_oracle(gpu_lib, seed, s_lo, s_hi, t_lo, t_hi, vpr, chunk):
+    S = P.generate(P.StarParams(dom_hi=2.0, r_lo=1.0, n_lo=s_lo, n_hi=s_hi), seed, 3)
+    T = P.generate(P.StarParams(dom_hi=2.0, r_lo=1.0, n_lo=t_lo, n_hi=t_hi), seed + 1, 3)
+    pairs = np.ascontiguousarray(P.mbr_join(S.mbrs(), T.mbrs()), np.uint32)
+    assert len(pairs)
+    with Store() as st:
+        st.load_sets(S, T)
+        st.rasterize(vpr=vpr)
+        st.area_set_chunks([chunk] * 32)
+        out = st.intersection_area(pairs)
+        plan = st.area_plan(max_pairs=len(pairs), max_items=2 * 3 * (s_hi + t_hi) * 3)
+        assert np.array_equal(plan.run(pairs), out)
+        plan.close()
+    for k, (s, t) in enumerate(pairs):
+        exp = O.intersection_area(S.ring(s), T.ring(t))
+        a = max(0.5 * abs(np.sum(r[:-1, 0] * r[1:, 1] - r[1:, 0] * r[:-1, 1]))
+                for r in (S.ring(s).astype(np.float64), T.ring(t).astype(np.float64)))
+        assert abs(out[k] - exp) <= 1e-9 * exp + 1e-14 * a, (k, s, t, out[k], exp)
