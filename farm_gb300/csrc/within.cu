@@ -283,7 +283,7 @@ struct WStage {
 // (*g, *at): the group of 32 sequences and the point in it; a chunk that ends
 // inside a group is followed by one that starts with its last point.
 template <bool kGeo>
-__device__ uint32_t stage_points(const SeqSet &Q, WStage *st, int side, const float2 *tab, uint32_t *g, uint32_t *at,
+__device__ __noinline__ uint32_t stage_points(const SeqSet &Q, WStage *st, int side, const float2 *tab, uint32_t *g, uint32_t *at,
                                  int lane) {
     const unsigned full = 0xffffffffu;
     for (; Q.a + *g < Q.b; *g += 32, *at = 0) {
@@ -354,7 +354,7 @@ __device__ bool staged_near(const WStage *st, int gs, uint32_t np, const Near &w
         const uint32_t j0 = valid ? min(np, slice * q) : np, j1 = min(np, j0 + q);
         tests += j1 - j0;
         bool may = false, hit = false;
-#pragma unroll 4
+#pragma unroll 1
         for (uint32_t j = j0; j < j1; j++) {
             const float4 p = pt[j];
             screen<kGeo>(make_float2(p.x, p.y), make_float2(p.z, p.w), g, w, may, hit);
@@ -382,10 +382,11 @@ __device__ __noinline__ bool warp_near(const SeqSet &A, const SeqSet &B, const N
     uint32_t ga = 0, ata = 0;
     for (uint32_t na; (na = stage_points<kGeo>(A, st, 0, tab, &ga, &ata, lane)) != 0;) {
         uint32_t gb = 0, atb = 0;
+#pragma unroll 1
         for (uint32_t nb; (nb = stage_points<kGeo>(B, st, 1, tab, &gb, &atb, lane)) != 0;)
-            if (staged_near<kGeo>(st, 0, nb, w, lane, tests, rechk) ||
-                staged_near<kGeo>(st, 1, na, w, lane, tests, rechk))
-                return true;
+#pragma unroll 1
+            for (int side = 0; side < 2; side++)
+                if (staged_near<kGeo>(st, side, side ? na : nb, w, lane, tests, rechk)) return true;
     }
     return false;
 }
@@ -410,6 +411,7 @@ __device__ __noinline__ unsigned test_candidates(const StoreView &sv, const Poly
     }
     uint32_t tests = 0, rechk = 0;
     unsigned hits = 0;
+#pragma unroll 1
     for (unsigned m = __ballot_sync(full, valid); m; m &= m - 1) {
         const int src = __ffs(m) - 1;
         const SeqSet a{sv.seq + S.seq, sv.ring + S.ring, __shfl_sync(full, A.a, src), __shfl_sync(full, A.b, src)};
@@ -515,6 +517,7 @@ __device__ __forceinline__ void set_bit(uint32_t *bits, uint32_t id) { atomicOr(
 __device__ __noinline__ uint32_t compact_bits(uint32_t *bits, uint32_t nbits, uint32_t *list, int lane) {
     uint32_t nw = (nbits + 31) >> 5;
     uint32_t total = 0;
+#pragma unroll 1
     for (uint32_t w0 = 0; w0 < nw; w0 += 32) {
         uint32_t w = w0 + lane;
         uint32_t word = w < nw ? bits[w] : 0u;
@@ -543,6 +546,7 @@ __device__ __noinline__ uint32_t compact_bits(uint32_t *bits, uint32_t nbits, ui
 __device__ __noinline__ uint32_t next_set(const PolyHdr &h, const uint8_t *status, const Layer &g, const Layer *pg, uint32_t nq,
                              SideScratch &sc, int lane, int cc) {
     const uint8_t *st = status + h.st + g.offset;
+#pragma unroll 1
     for (uint32_t k = lane; k < nq; k += 32) {
         uint32_t id = sc.q[k];
         if (pg) {
@@ -555,7 +559,9 @@ __device__ __noinline__ uint32_t next_set(const PolyHdr &h, const uint8_t *statu
             int sy = offset_y(g.mbr, g.step_y, g.dimy, b.lo1 + 1e-6);
             int ex = offset_x(g.mbr, g.step_x, g.dimx, b.hi0 - 1e-6);
             int ey = offset_y(g.mbr, g.step_y, g.dimy, b.hi1 - 1e-6);
+#pragma unroll 1
             for (int x = sx; x <= ex; x++)
+#pragma unroll 1
                 for (int y = sy; y <= ey; y++) {
                     uint32_t c = (uint32_t)(y * g.dimx + x);
                     if (show_status(st[c], cc) == 1) set_bit(sc.bits, c);
@@ -601,12 +607,12 @@ struct Product {
 // the coordinate, so a box distance computed from them is off by at most
 // slack(k1) plus 4e-6 of itself; max-distances use the reference's own float
 // corners and are off by 4e-6 of themselves (scales and squares).
+template <bool kGeo>
 struct Level {
     float ex, ey;  // coordinate roundings, x and y
-    bool geo;
     const float *lon;
-    __device__ __forceinline__ float sx(uint32_t k1) const { return geo ? lon[k1] : 1.f; }
-    __device__ __forceinline__ float sy() const { return geo ? (float)(40076.0 / 360.0) : 1.f; }
+    __device__ __forceinline__ float sx(uint32_t k1) const { return kGeo ? lon[k1] : 1.f; }
+    __device__ __forceinline__ float sy() const { return kGeo ? (float)(40076.0 / 360.0) : 1.f; }
     __device__ __forceinline__ float slack(float sx_) const { return 1.5f * (ex * sx_ + ey * sy()); }
     __device__ __forceinline__ float dist(const float4 &a, const float4 &t, float sx_) const {
         const float dx = fmaxf(0.f, fmaxf(t.x - a.z, a.x - t.z)) * sx_;
@@ -629,9 +635,11 @@ __device__ __forceinline__ float warp_min(float v) {
 }
 
 // Keep the pixels of a side whose box may lie within `cut` of box bb.
-__device__ __noinline__ uint32_t prune_side(SideScratch &sc, uint32_t n, const float4 &bb, const Level &lv, bool source,
-                               float sx_low, float cut, int lane) {
+template <bool kGeo>
+__device__ __noinline__ uint32_t prune_side(SideScratch &sc, uint32_t n, const float4 &bb, const Level<kGeo> &lv,
+                                            bool source, float sx_low, float cut, int lane) {
     uint32_t at = 0;
+#pragma unroll 1
     for (uint32_t b = 0; b < n; b += 32) {
         const uint32_t k = b + lane;
         bool keep = false;
@@ -641,16 +649,16 @@ __device__ __noinline__ uint32_t prune_side(SideScratch &sc, uint32_t n, const f
         if (k < n) {
             id = sc.p[k];
             fb = sc.fbox[k];
-            if (source && lv.geo) lo = sc.lon[k];
-            const float sx_ = source ? (lv.geo ? lo : 1.f) : sx_low;
-            keep = !(lv.low(lv.dist(fb, bb, sx_), source ? sx_ : (lv.geo ? kScaleGeo : 1.f)) > cut);
+            if (source && kGeo) lo = sc.lon[k];
+            const float sx_ = source ? (kGeo ? lo : 1.f) : sx_low;
+            keep = !(lv.low(lv.dist(fb, bb, sx_), source ? sx_ : (kGeo ? kScaleGeo : 1.f)) > cut);
         }
         const unsigned m = __ballot_sync(0xffffffffu, keep);
         if (keep) {
             const uint32_t w = at + __popc(m & ((1u << lane) - 1));
             sc.p[w] = id;
             sc.fbox[w] = fb;
-            if (source && lv.geo) sc.lon[w] = lo;
+            if (source && kGeo) sc.lon[w] = lo;
         }
         at += __popc(m);
         __syncwarp();
@@ -706,8 +714,10 @@ __device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id
                                       unsigned long long &rechk) {
     const SeqSet A = seq_set(*f.sv, *f.S, id1), B = seq_set(*f.sv, *f.T, id2);
     uint32_t at = 0;
+#pragma unroll 1
     for (uint32_t ia = A.a; ia < A.b; ia++) {
         const uint2 e1 = A.seq[ia];
+#pragma unroll 1
         for (uint32_t jb = B.a; jb < B.b; jb++) {
             const uint2 e2 = B.seq[jb];
             if (e1.y < 2 || e2.y < 2) continue;
@@ -715,6 +725,7 @@ __device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id
             (*from)++;
             const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
             double m = 1.7976931348623157e308;
+#pragma unroll 1
             for (uint32_t k = lane; k < n1 + n2; k += 32) {
                 const uint32_t r = k < n1 ? k : k - n1, len = k < n1 ? e1.y - 1 : e2.y - 1;
                 const uint32_t pi = r / len, si = r % len;
@@ -764,6 +775,7 @@ constexpr uint32_t kPrunePairs = 256;
 // 60,001 pairs of configuration 3: 794 ms refinement and 55 ms descent with an
 // ordered refinement, a warp per pair; 29 ms in all so (36 ms with a lane per
 // candidate and every hit confirmed in FP64).
+template <bool kGeo>
 __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView sv, WithinArgs a) {
     extern __shared__ __align__(16) unsigned char within_smem[];
     WithinShared &sh = *reinterpret_cast<WithinShared *>(within_smem);
@@ -773,10 +785,11 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
     WStage *stage = &sh.stage[wib];
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int cc = sv.category_count;
-    const bool geo = a.geo;
+    constexpr bool geo = kGeo;
     uint2 *q = sh.queue[wib];
     Layer *LS = sh.layers[wib][0], *LT = sh.layers[wib][1];
     if (geo)
+#pragma unroll 1
         for (int k = threadIdx.x; k < 900; k += blockDim.x) tab[k] = lon_entry(k);
     const uint32_t cap = a.cap_pix, bw = (cap >> 5) + 1;
     uint32_t *wbase = a.scratch + warp * a.scratch_words;
@@ -784,6 +797,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
     uint32_t *base = wbase + 9ull * cap;
     SideScratch ss{base, base + bw, base + bw + cap, fboxes, reinterpret_cast<float *>(wbase + 8ull * cap)};
     SideScratch ts{base + bw + 2 * cap, base + 2 * bw + 2 * cap, base + 2 * bw + 3 * cap, fboxes + cap, nullptr};
+#pragma unroll 1
     for (uint32_t w = lane; w < bw; w += 32) ss.bits[w] = ts.bits[w] = 0u;
     __syncthreads();
     WithinTally my;
@@ -808,7 +822,9 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
         const uint32_t sL = S.num_layers - 1, tL = T.num_layers - 1;
         // initial queue: every layer-0 pixel pair (Ideal.cpp:2483-2488)
         uint32_t nqs = (uint32_t)(LS[0].dimx * LS[0].dimy), nqt = (uint32_t)(LT[0].dimx * LT[0].dimy);
+#pragma unroll 1
         for (uint32_t k = lane; k < nqs; k += 32) ss.q[k] = k;
+#pragma unroll 1
         for (uint32_t k = lane; k < nqt; k += 32) ts.q[k] = k;
         __syncwarp();
         uint32_t i = 0, j = 0;
@@ -831,6 +847,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
             uint32_t nt = next_set(T, sv.status, gt, t_next ? &LT[j - 1] : nullptr, nqt, ts, lane, cc);
             if (ns == 0 || nt == 0) break;
             if (lane == 0) my.box += (uint64_t)ns * nt;
+#pragma unroll 1
             for (uint32_t k = lane; k < ns; k += 32) {
                 const Box b = layer_box(gs, (int)ss.p[k]);
                 ss.fbox[k] = box_corners_f(b);
@@ -841,20 +858,21 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                     ss.lon[k] = c_inv_deg_lon_f[idx < 0 || idx >= 900 ? 899 : idx];
                 }
             }
+#pragma unroll 1
             for (uint32_t k = lane; k < nt; k += 32) ts.fbox[k] = box_corners_f(layer_box(gt, (int)ts.p[k]));
             __syncwarp();
             const float4 sbb = make_float4((float)gs.mbr[0], (float)gs.mbr[1], (float)(gs.mbr[0] + gs.dimx * gs.step_x),
                                            (float)(gs.mbr[1] + gs.dimy * gs.step_y));
             const float4 tbb = make_float4((float)gt.mbr[0], (float)gt.mbr[1], (float)(gt.mbr[0] + gt.dimx * gt.step_x),
                                            (float)(gt.mbr[1] + gt.dimy * gt.step_y));
-            Level lv;
+            Level<kGeo> lv;
             lv.ex = 2.4e-7f * (fmaxf(fabsf(sbb.x), fabsf(sbb.z)) + fmaxf(fabsf(tbb.x), fabsf(tbb.z)));
             lv.ey = 2.4e-7f * (fmaxf(fabsf(sbb.y), fabsf(sbb.w)) + fmaxf(fabsf(tbb.y), fabsf(tbb.w)));
-            lv.geo = geo;
             lv.lon = ss.lon;
             float sx_low = 1.f;  // the smallest longitude scale of the source pixels
             if (geo) {
                 sx_low = INFINITY;
+#pragma unroll 1
                 for (uint32_t k = lane; k < ns; k += 32) sx_low = fminf(sx_low, ss.lon[k]);
                 sx_low = warp_min(sx_low);
             }
@@ -864,6 +882,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                 // S's: the smallest max-distance of either is a first cut
                 float best = INFINITY;
                 uint32_t bk = 0;
+#pragma unroll 1
                 for (uint32_t k = lane; k < ns; k += 32) {
                     const float d = lv.dist(ss.fbox[k], tbb, lv.sx(k));
                     if (d < best) best = d, bk = k;
@@ -874,6 +893,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                 const float near_sx = lv.sx(bk);
                 best = INFINITY;
                 bk = 0;
+#pragma unroll 1
                 for (uint32_t k = lane; k < nt; k += 32) {
                     const float d = lv.dist(ts.fbox[k], sbb, sx_low);
                     if (d < best) best = d, bk = k;
@@ -882,7 +902,9 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                 bk = __shfl_sync(full, bk, __ffs(__ballot_sync(full, best == w)) - 1);
                 const float4 near_t = ts.fbox[bk];
                 float ub2 = INFINITY;
+#pragma unroll 1
                 for (uint32_t k = lane; k < nt; k += 32) ub2 = fminf(ub2, lv.max2(near_s, ts.fbox[k], near_sx));
+#pragma unroll 1
                 for (uint32_t k = lane; k < ns; k += 32) ub2 = fminf(ub2, lv.max2(ss.fbox[k], near_t, lv.sx(k)));
                 const float cut = sqrtf(warp_min(ub2)) * 1.00001f;
                 ns = prune_side(ss, ns, tbb, lv, true, sx_low, cut, lane);
@@ -989,10 +1011,12 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
             Product all(ns, nt);
             __syncwarp();
             for (;;) {
+#pragma unroll 1
                 for (int k = 0; k < qn && !yes;) {
                     bool check_last = false;
                     if (may_spill && (float)spent >= a.sp.budget) {
                         if (know_last) {
+#pragma unroll 1
                             for (int e = k + lane; e < qn; e += 32)
                                 if (q[e].x == last1 && q[e].y == last2) q[e].x = ~0u;
                             __syncwarp();
@@ -1075,6 +1099,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
         }
         // leave the scratch bitmaps clean for the next pair
         __syncwarp();
+#pragma unroll 1
         for (uint32_t w = lane; w < bw; w += 32) {
             ss.bits[w] = 0u;
             ts.bits[w] = 0u;
@@ -1111,6 +1136,7 @@ __global__ void __launch_bounds__(256, 3) k_within_spill(const StoreView sv, Wit
     const unsigned long long n = min(a.sp.ctr[0], (unsigned long long)a.sp.cap);
     if (n == 0) return;
     if (a.geo)
+#pragma unroll 1
         for (int k = threadIdx.x; k < 900; k += blockDim.x) tab[k] = lon_entry(k);
     __syncthreads();
     const unsigned long long total = n * ((a.sp.ctr[2] + 31) / 32);
@@ -1150,6 +1176,7 @@ __global__ void __launch_bounds__(256, 3) k_within_spill(const StoreView sv, Wit
 __global__ void k_within_cap(const PolyHdr *__restrict__ hdr, uint32_t npoly, unsigned long long *__restrict__ most) {
     const int lane = threadIdx.x & 31;
     unsigned long long mine = 0;
+#pragma unroll 1
     for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < npoly; p += (gridDim.x * blockDim.x) >> 5) {
         const PolyHdr &h = hdr[p];
         if (h.err || lane >= (int)h.num_layers) continue;
@@ -1246,8 +1273,9 @@ int within(farm_store *s, const uint32_t *pairs, uint64_t n, double distance, in
         wa.next = ctr;
         wa.stats = ctr + 1;
         FARM_TRY(spill_pool(s, n, ctr + 8, 64.f, 512.f, &wa.sp));
-        FARM_CUDA(cudaFuncSetAttribute(k_within, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WithinShared)));
-        k_within<<<(unsigned)blocks, 256, sizeof(WithinShared), stream>>>(s->view(), wa);
+        const auto kernel = wa.geo ? k_within<true> : k_within<false>;
+        FARM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(WithinShared)));
+        kernel<<<(unsigned)blocks, 256, sizeof(WithinShared), stream>>>(s->view(), wa);
         FARM_CUDA(cudaGetLastError());
         FARM_CUDA(cudaEventRecord(s->ev[8], stream));
         k_within_spill<<<3 * sm_count(), 256, 0, stream>>>(s->view(), wa);
