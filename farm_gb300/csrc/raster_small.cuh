@@ -11,6 +11,10 @@
 //
 // 11,000 polygons of 16..1,024 vertices (configuration 1): phase 2 took
 // 3.3 ms of device time and 160 launches.
+//
+// Loops are not unrolled: most run once or twice per thread, and what the
+// warps wait for then is instruction fetch (kernels of 96 and 88 KB unrolled,
+// 66 and 63 KB so: 3.17 -> 2.96 ms for that join as a whole).
 #pragma once
 
 // Two kernels: the walk (sequences, nodes) needs 128 registers a thread, the
@@ -123,6 +127,7 @@ __global__ void k_small_pick(PolyHdr *__restrict__ hdr, uint32_t npoly, const ui
     }
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+#pragma unroll 1
     for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < npoly; p0 += gridDim.x * blockDim.x) {
         const uint32_t p = p0 + lane;
         bool small = false;
@@ -217,6 +222,7 @@ template <int NT>
 __device__ void small_prefix(uint32_t *c, uint32_t n, uint64_t *sums) {
     uint64_t run = 0;
     __syncthreads();
+#pragma unroll 1
     for (uint32_t b = 0; b < n; b += NT) {
         const uint32_t i = b + threadIdx.x;
         const uint64_t v = i < n ? c[i] : 0u;
@@ -272,7 +278,9 @@ __device__ void small_sort_line(double *v, uint32_t n, uint64_t *buf, int lane) 
     if (n < 2) return;
     if (n <= 32) {
         uint64_t k = (uint32_t)lane < n ? dkey(v[lane]) : ~0ull;
+#pragma unroll 1
         for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll 1
             for (int j = size >> 1; j > 0; j >>= 1) {
                 const uint64_t o = __shfl_xor_sync(0xffffffffu, k, j);
                 const bool up = (lane & size) == 0, lower = (lane & j) == 0;
@@ -287,12 +295,17 @@ __device__ void small_sort_line(double *v, uint32_t n, uint64_t *buf, int lane) 
     uint64_t *key = sm ? buf : reinterpret_cast<uint64_t *>(v);
     uint32_t N = 64;
     while (N < n) N <<= 1;
+#pragma unroll 1
     for (uint32_t i = lane; i < n; i += 32) key[i] = dkey(v[i]);
     if (sm)
+#pragma unroll 1
         for (uint32_t i = n + lane; i < N; i += 32) key[i] = ~0ull;
     __syncwarp();
+#pragma unroll 1
     for (uint32_t k = 2; k <= N; k <<= 1)
+#pragma unroll 1
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll 1
             for (uint32_t i = lane; i < N; i += 32) {
                 // ascending runs only: the first step of a merge pairs i with its mirror
                 const uint32_t ixj = j == (k >> 1) ? (i ^ (k - 1)) : (i ^ j);
@@ -306,6 +319,7 @@ __device__ void small_sort_line(double *v, uint32_t n, uint64_t *buf, int lane) 
             }
             __syncwarp();
         }
+#pragma unroll 1
     for (uint32_t i = lane; i < n; i += 32) v[i] = dval(key[i]);
     __syncwarp();
 }
@@ -315,6 +329,7 @@ __device__ void small_sort_line(double *v, uint32_t n, uint64_t *buf, int lane) 
 template <typename Key, typename Put>
 __device__ __forceinline__ void small_stable(uint32_t i0, uint32_t n, uint32_t *cur, uint32_t step, int lane, Key key,
                                              Put put) {
+#pragma unroll 1
     for (uint32_t b = i0; b < n; b += 32) {
         const uint32_t i = b + lane;
         const unsigned act = __ballot_sync(0xffffffffu, i < n);
@@ -339,12 +354,15 @@ __device__ __forceinline__ void small_bucket(uint32_t n, uint32_t nb, uint32_t *
                                              Key key, Put put, Before before) {
     constexpr uint32_t W = NT / 32;
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
+#pragma unroll 1
     for (uint32_t k = tid; k < nb * W; k += NT) cnt[k] = 0;
     __syncthreads();
     const uint32_t part = ((n + W - 1) / W + 31) & ~31u;
     const uint32_t i0 = min(n, warp * part), i1 = min(n, i0 + part);
+#pragma unroll 1
     for (uint32_t i = i0 + (tid & 31); i < i1; i += 32) atomicAdd(&cnt[key(i) * W + warp], 1u);
     small_prefix<NT>(cnt, nb * W, sums);
+#pragma unroll 1
     for (uint32_t b = tid; b <= nb; b += NT) start[b] = cnt[b * W];
     __syncthreads();
     before();
@@ -388,6 +406,7 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_walk(SmallArgs a) {
         // have any, fewer than half, are listed first, so that the lanes that
         // walk do so together. Packed: crossings, h-nodes, v-nodes, edges.
         uint64_t run = 0;
+#pragma unroll 1
         for (uint32_t b = 0; b < ne; b += NT) {
             const uint32_t e = b + tid;
             uint64_t c = 0, total;
@@ -406,6 +425,7 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_walk(SmallArgs a) {
         __syncthreads();
         const uint32_t nC = (uint32_t)(run & 0xFFFF), nH = (uint32_t)((run >> 16) & 0xFFFF),
                        nV = (uint32_t)((run >> 32) & 0xFFFF), nW = (uint32_t)(run >> 48);
+#pragma unroll 1
         for (uint32_t i = tid; i < nW; i += NT) {
             const uint64_t at = s.wa[i];
             const uint32_t e = s.we[i];
@@ -431,10 +451,12 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_walk(SmallArgs a) {
         uint32_t *offs = a.offset + h.off;
         uint2 *seq = a.seq + h.seq;
         if (nC == 0) {  // one sequence covering the ring (Ideal.cpp:523-529)
+#pragma unroll 1
             for (uint32_t i = tid; i < h.P; i += NT) offs[i] = i ? 1u : 0u;
             if (tid == 0) seq[0] = make_uint2(0u, h.nv);
         } else {
             const uint32_t wrap = s.ct[nC - 1];
+#pragma unroll 1
             for (uint32_t c = tid; c < nC; c += NT)
                 if (s.cf[c + 1 == nC ? 0 : c + 1] != s.ct[c]) atomicMin(&s_err, FARM_EASSERT);
             small_bucket<NT>(
@@ -451,22 +473,27 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_walk(SmallArgs a) {
                     }
                 },
                 [&]() {
+#pragma unroll 1
                     for (uint32_t i = tid; i < h.P; i += NT) offs[i] = start[i] + (i > wrap ? 1u : 0u);
                 });
         }
         if (tid == 0) offs[h.P] = h.n_seq;
         __syncthreads();
         // ---- grid-line nodes (process_intersection), horizontal then vertical
+#pragma unroll 1
         for (int vert = 0; vert < 2; vert++) {
             const uint32_t n = vert ? nV : nH, dim = (uint32_t)(vert ? dimx : dimy);
             const uint32_t *line = vert ? s.vl : s.hl;
             const double *val = vert ? s.vv : s.hv;
             double *out = vert ? a.vnodes + h.vnode : a.hnodes + h.hnode;
             uint32_t *lo = vert ? a.voff + h.vline : a.hoff + h.hline;
+#pragma unroll 1
             for (uint32_t i = tid; i <= dim + 2; i += NT) linec[i] = 0;
             __syncthreads();
+#pragma unroll 1
             for (uint32_t i = tid; i < n; i += NT) atomicAdd(&linec[line[i]], 1u);
             small_prefix<NT>(linec, dim + 2, sums);
+#pragma unroll 1
             for (uint32_t l = tid; l < dim + 2; l += NT) {
                 const uint32_t st = linec[l];
                 uint32_t v = linec[l + 1] != st ? st : 0u;
@@ -474,8 +501,10 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_walk(SmallArgs a) {
                 lo[l] = v;
             }
             __syncthreads();
+#pragma unroll 1
             for (uint32_t i = tid; i < n; i += NT) out[atomicAdd(&linec[line[i]], 1u)] = val[i];
             __syncthreads();  // linec[l] is now line l's end
+#pragma unroll 1
             for (uint32_t l = warp; l < dim + 2; l += kWarps) {
                 const uint32_t b = l ? linec[l - 1] : 0u;
                 small_sort_line(out + b, linec[l] - b, sortb[warp], lane);
@@ -517,11 +546,13 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
         const int dimx = h.dimx, dimy = h.dimy;
         // ---- scanline
         uint8_t *st = a.status + h.st;
+#pragma unroll 1
         for (int y = 1 + warp; y < dimy; y += kWarps)
             scan_row(h, st + (uint64_t)y * dimx, a.hoff[h.hline + y], a.hoff[h.hline + y + 1], a.hnodes + h.hnode, a.cc,
                      lane);
         // ---- column clip: points in edge order, counted, then written
         uint32_t nX = 0;
+#pragma unroll 1
         for (uint32_t b = 0; b < ne && !s_full; b += NT) {
             const uint32_t e = b + tid;
             uint32_t m = 0;
@@ -541,6 +572,7 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
             // by column, in clip order
             uint32_t hash = 64;
             while (hash < 2 * nX) hash <<= 1;
+#pragma unroll 1
             for (uint32_t i = tid; i < hash; i += NT) s.tab[i] = ~0u;
             small_bucket<NT>(
                 nX, ncols, cnt, linec, sums, [&](uint32_t i) { return s.xc[i]; },
@@ -568,9 +600,11 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
                 return t;
             };
             // xc keeps each point's slot from here on
+#pragma unroll 1
             for (uint32_t i = tid; i < nX; i += NT) s.xc[i] = slot_of(i, true);
             __syncthreads();
             bool small = false;
+#pragma unroll 1
             for (uint32_t i = tid; i < nX; i += NT) {
                 const bool d = *(volatile uint32_t *)&s.tab[s.xc[i]] != i;
                 s.drop[i] = d;
@@ -580,9 +614,11 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
                 // first copies near an axis, where points closer than 1e-9 count
                 // as equal: the reference's sequential rule, a column per warp
                 // (the indices of the column's small points go to xc)
+#pragma unroll 1
                 for (uint32_t c = warp; c < ncols; c += kWarps) {
                     const uint32_t b = linec[c], e = linec[c + 1];
                     uint32_t m = 0;
+#pragma unroll 1
                     for (uint32_t i0 = b; i0 < e; i0 += 32) {
                         const uint32_t i = i0 + lane;
                         const bool v = i < e && !s.drop[i] && small_pt(s.sp[i]);
@@ -591,9 +627,11 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
                         m += __popc(bm);
                     }
                     __syncwarp();
+#pragma unroll 1
                     for (uint32_t i = 1; i < m; i++) {
                         const float2 me = s.sp[s.xc[b + i]];
                         bool eq = false;
+#pragma unroll 1
                         for (uint32_t j = lane; j < i; j += 32) {
                             const uint32_t o = s.xc[b + j];
                             eq |= !s.drop[o] && pt_eq(s.sp[o], me);
@@ -605,9 +643,11 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
             }
             __syncthreads();
             // column polygons: kept points in order plus the closing copy of the first
+#pragma unroll 1
             for (uint32_t c = warp; c < ncols; c += kWarps) {
                 const uint32_t b = linec[c], e = linec[c + 1];
                 uint32_t m = 0;
+#pragma unroll 1
                 for (uint32_t i0 = b; i0 < e; i0 += 32)
                     m += __popc(__ballot_sync(0xffffffffu, i0 + lane < e && !s.drop[i0 + lane]));
                 if (lane == 0) cpst[c] = m ? m + 1 : 0u;
@@ -617,10 +657,12 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
             __syncthreads();
         }
         if (!s_full) {
+#pragma unroll 1
             for (uint32_t c = warp; c < ncols; c += kWarps) {
                 const uint32_t b = linec[c], e = linec[c + 1], at = cpst[c];
                 uint32_t m = 0;
                 float2 f0 = make_float2(0.f, 0.f);
+#pragma unroll 1
                 for (uint32_t i0 = b; i0 < e; i0 += 32) {
                     const uint32_t i = i0 + lane;
                     const bool v = i < e && !s.drop[i];
@@ -642,12 +684,14 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
                     s.cpc[at + m] = c;
                 }
             }
+#pragma unroll 1
             for (uint32_t i = tid; i <= h.P; i += NT) pixc[i] = 0;
             __syncthreads();
         }
         // ---- cell clip: points in column-polygon order, counted, then written
         const uint32_t nCP = s_full ? 0u : cpst[ncols];
         uint32_t nY = 0;
+#pragma unroll 1
         for (uint32_t b = 0; b < nCP && !s_full; b += NT) {
             const uint32_t j = b + tid;
             uint32_t m = 0, c = 0;
@@ -674,24 +718,29 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
                 atomicAdd(&a.info->crossings, 0ull - (unsigned long long)(h.n_seq > 1 ? h.n_seq - 1 : 0));
             }
             // the scanline's classes go back to the walk's border marks, as phase 1 left them
+#pragma unroll 1
             for (uint32_t i = tid; i < h.P; i += NT) st[i] = st[i] == 1 ? 1 : 0;
             continue;
         }
         // by cell: a column's points stably by row (as k_cell_bucket)
         const int nrows = h.nrows;
+#pragma unroll 1
         for (uint32_t c = warp; c < ncols; c += kWarps) {
             if (cpst[c + 1] == cpst[c]) continue;
             // the column's last point: the next non-empty column's first
             uint32_t e = nY;
+#pragma unroll 1
             for (uint32_t d = c + 1; d < ncols; d++)
                 if (cpst[d + 1] != cpst[d]) {
                     e = yst[d];
                     break;
                 }
             const uint32_t b = yst[c];
+#pragma unroll 1
             for (uint32_t i = b + lane; i < e; i += 32) atomicAdd(&pixc[s.yr[i] * dimx + c], 1u);
             __syncwarp();
             uint32_t base = 0;
+#pragma unroll 1
             for (int r0 = 0; r0 < nrows; r0 += 32) {
                 const int rr = r0 + lane;
                 const uint32_t v = rr < nrows ? pixc[rr * dimx + c] : 0u;
@@ -710,6 +759,7 @@ __global__ void __launch_bounds__(NT, kBlocks) k_small_fill(SmallArgs a) {
         }
         __syncthreads();
         // ---- cell areas and classes (pixc[id] is now the end of the cell's points in its column)
+#pragma unroll 1
         for (uint32_t id = tid; id < h.P; id += NT) {
             const uint32_t x = id % (uint32_t)dimx, y = id / (uint32_t)dimx;
             if (x >= ncols || y >= (uint32_t)nrows || cpst[x + 1] == cpst[x]) continue;
