@@ -146,6 +146,7 @@ __device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, const Frame &f
     const float2 *r = sv.ring + H.ring;
     const float m = 1e-6f * (fabsf(fr.x0) + fabsf(fr.x1)) + 1.2e-38f;
     bool odd = false;
+#pragma unroll 1
     for (int c = col; c < H.dimx; c++) {
         const uint32_t pid = (uint32_t)(row * H.dimx + c);
         const int s = show_status(st[pid], cc);
@@ -153,8 +154,10 @@ __device__ bool pip_raster(const StoreView &sv, const PolyHdr &H, const Frame &f
         const float lo = c == col ? pt.x : fmaxf(pt.x, fr.xh + (float)c * fr.sx);
         const float hi = c == H.dimx - 1 ? INFINITY : fr.xh + (float)(c + 1) * fr.sx;
         bool flip = false;
+#pragma unroll 1
         for (uint32_t q = off[pid] + lane; q < off[pid + 1]; q += 32) {
             const uint2 sq = seq[q];
+#pragma unroll 1
             for (uint32_t k = 0; k < sq.y; k++) {
                 const float2 a = r[sq.x + k], b = r[sq.x + k + 1];
                 if ((a.y > pt.y) == (b.y > pt.y)) continue;
@@ -237,6 +240,7 @@ constexpr int kQueueRows = 64;  // rows a queued edge may wait
 __device__ __noinline__ int2 group_columns(const Group &g, int y) {
     int2 c = make_int2(0x7fffffff, -1);
     const Frame fr = frame_of(*g.O);
+#pragma unroll 1
     for (uint32_t k = 0; k < g.n; k++) {
         const float2 P = g.ring[g.first + k], Q = g.ring[g.first + k + 1];
         if (!edge_meets(fr, P, Q)) continue;
@@ -262,6 +266,7 @@ __device__ bool first_listing(const StoreView &sv, const Group &g, const int2 *r
     const uint32_t dimx = (uint32_t)O.dimx;
     const int py = (int)(pid / dimx);
     int self = 0;
+#pragma unroll 1
     for (uint64_t i = ep_off[at], e = ep_off[at + 1]; i < e; i++) {
         const uint32_t r = ep_pix[i];
         if (r > pid) break;
@@ -277,6 +282,7 @@ __device__ bool first_listing(const StoreView &sv, const Group &g, const int2 *r
     }
     if (self > 1) {  // pid holds f in more than one sequence: the first counts
         const uint2 *seq = sv.seq + O.seq;
+#pragma unroll 1
         for (uint32_t p = sv.offset[O.off + pid]; p < q; p++) {
             const uint2 sq = seq[p];
             if (f >= sq.x && f - sq.x < sq.y) return false;
@@ -348,7 +354,10 @@ static int spread_items() {
 // parts-th step of the same walk, adds its integer sums to the item's, and the
 // last one finishes the item: the same bits however it is cut.
 // 801 pairs of up to 20,000 vertices: 72 ms with a window per lane, 10.0 ms
-// with the look-up after the tests, 6.2 ms without cutting, 4.3 ms so.
+// with the look-up after the tests, 6.2 ms without cutting, 4.3 ms so, 3.7 ms
+// with groups of 32 edges. Loops are not unrolled: most run once or twice, and
+// in the first launch a warp waits for instruction fetch more than for anything
+// else (77 KB unrolled, 70 KB so: 3.87 -> 3.68 ms).
 constexpr int kAreaQueue = 64;
 struct AreaListing {  // an edge met in a pixel of the window
     uint32_t f, pid, q;
@@ -466,6 +475,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
         const uint8_t *ost = sv.status + O.st;
         const uint32_t *ooff = sv.offset + O.off;
         const uint2 *oseq = sv.seq + O.seq;
+#pragma unroll 1
         for (uint32_t b0 = first; b0 < last; b0 += 32) {
             const uint32_t R = min(32u, last - b0), G = 32u / R, slice = (uint32_t)lane / R;
             const uint32_t e = b0 + (uint32_t)lane % R;
@@ -518,6 +528,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                 uint32_t s0 = 0, tsq = 0, k0 = 0, te = 0;
                 uint32_t pid = 0, sq0 = 0, xsq = 0, qq = 0, qpid = 0, xe = 0;
                 uint2 sq = make_uint2(0u, 0u);
+#pragma unroll 1
                 for (bool end = false; !end;) {
                     bool look_all = false;
                     if (k0 < te) {
@@ -610,6 +621,7 @@ __global__ void __launch_bounds__(256, 3) k_area(const StoreView sv, AreaArgs a)
                         const int m = min(qn, 32);
                         unsigned hits = 0, known = 0;  // known: both ends clearly on either side, of both
                         if (active) {
+#pragma unroll 1
                             for (int j = (int)slice; j < m; j += (int)G) {
                                 const float4 s = seg[j];
                                 const float U = s.x - P.x, V = s.y - P.y, U2 = s.z - P.x, V2 = s.w - P.y;
