@@ -359,11 +359,12 @@ static int query_blocks(uint64_t n) {
 int spill_pool(farm_store *s, uint64_t n, unsigned long long *ctr, float few, float many, SpillPool *sp) {
     const uint32_t cap = (uint32_t)(n < 4096 ? 4096 : (n > 65536 ? 65536 : n));
     DevBuf &b = s->s[Q_SPILL];
-    FARM_TRY(b.ensure((uint64_t)cap * (kQueue * sizeof(uint2) + sizeof(SpillChunk) + 4) + 64));
+    sp->ctr = ctr;
+    // without memory for a pool every pair stays with its warp
+    if (b.ensure((uint64_t)cap * (kQueue * sizeof(uint2) + sizeof(SpillChunk) + 4) + 64) != FARM_OK) return FARM_OK;
     sp->items = b.as<uint2>();
     sp->chunk = reinterpret_cast<SpillChunk *>(sp->items + (uint64_t)cap * kQueue);
     sp->flag = reinterpret_cast<uint32_t *>(sp->chunk + cap);
-    sp->ctr = ctr;
     sp->cap = cap;
     const char *v = getenv("FARM_SPILL_BUDGET");
     sp->budget = v && *v ? (float)atof(v) : (n <= 16ull * sm_count() ? few : many);
