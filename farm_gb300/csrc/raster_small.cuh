@@ -10,7 +10,7 @@
 // in a scratch slice per block, which stays in L1/L2.
 //
 // 11,000 polygons of 16..1,024 vertices (configuration 1): phase 2 took
-// 3.3 ms of device time and 160 launches.
+// 3.3 ms of device time and 160 launches, 1.5 ms and a dozen so.
 //
 // Loops are not unrolled: most run once or twice per thread, and what the
 // warps wait for then is instruction fetch (kernels of 96 and 88 KB unrolled,

@@ -150,9 +150,9 @@ __global__ void k_pad_rings(const float2 *__restrict__ xy, const uint64_t *__res
 // reduces in registers: a polygon of 100,000 vertices is 98 tiles, not the last
 // warp's 3,125 loads (37.6M vertices in 3,300 polygons: 1.2 ms with a warp per
 // polygon and its minima in FP64). A tile is 32 loads a lane, one chain: tiles
-// of 4,096 left a store of 160 polygons to a few warps (a join of 40
-// and 120 polygons: 689 us with them, 647 us with these). NaN coordinates count for nothing, as in a
-// loop of minima. The padding repeats a polygon's first vertex.
+// of 4,096 left a store of 160 polygons to a few warps (a join of 40 and 120
+// polygons: 689 us with them, 647 us with these). NaN coordinates count for
+// nothing, as in a loop of minima. The padding repeats a polygon's first vertex.
 constexpr uint32_t kBoxTile = 1024;
 __global__ void k_ring_boxes(const float2 *__restrict__ ring, const uint64_t *__restrict__ off, uint32_t npoly,
                              uint64_t total, uint4 *__restrict__ box) {

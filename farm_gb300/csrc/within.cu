@@ -26,8 +26,8 @@
 // which FP32 with an error bound decides for all but a few.
 //
 // Kernels: k_within (one warp per pair) descends, tests the finest level's
-// candidates a lane each, and spills what is past its budget; k_within_spill
-// tests those over all warps.
+// candidates one after the other, and spills what is past its budget;
+// k_within_spill tests those over all warps.
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -332,8 +332,9 @@ __device__ __noinline__ uint32_t stage_points(const SeqSet &Q, WStage *st, int s
     return 0;
 }
 
-// Staged segments of side gs against the np staged points of the other: a segment per lane, a group of R < 32 of them repeated over floor(32 /
-// R) slices of lanes that share the points.
+// Staged segments of side gs against the np staged points of the other: a
+// segment per lane, a group of R < 32 of them repeated over floor(32 / R)
+// slices of lanes that share the points.
 template <bool kGeo>
 __device__ bool staged_near(const WStage *st, int gs, uint32_t np, const Near &w, int lane, uint32_t &tests,
                             uint32_t &rechk) {
@@ -774,7 +775,9 @@ constexpr uint32_t kPrunePairs = 256;
 //
 // 60,001 pairs of configuration 3: 794 ms refinement and 55 ms descent with an
 // ordered refinement, a warp per pair; 29 ms in all so (36 ms with a lane per
-// candidate and every hit confirmed in FP64).
+// candidate and every hit confirmed in FP64). What was left waited for
+// instruction fetch more than for anything else: short loops are not unrolled
+// and each metric has a kernel of its own (223 -> 150 KB of code, 26 ms).
 template <bool kGeo>
 __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView sv, WithinArgs a) {
     extern __shared__ __align__(16) unsigned char within_smem[];
