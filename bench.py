@@ -189,7 +189,7 @@ FP32_NOMINAL = 128 * 152 * 2.07e9
 # figure times the step's units.
 TRAFFIC_PER_UNIT = {
     "edge_walk": 199.0,   # bytes per edge (k_walk_tot + k_walk_fill): 42.6 GB / 2.14e8 edges
-    "refine": 6621.8,     # bytes per candidate pair (k_intersect): 174.3 MB / 26,320 pairs
+    "refine": 6621.8,     # bytes per candidate pair (k_intersect, before the spill pool): 174.3 MB / 26,320 pairs
 }
 
 
@@ -224,7 +224,7 @@ def rooflines(rt: dict, qs: dict, n_pairs: float, stage: dict, steps: int, peaks
     cell clip (count + emit): FP64, 4 flops per emitted clip point;
     column clip: FP64, 2 flops per emitted point;
     cell areas: FP64, 4 flops per clip point (shoelace term + accumulation);
-    filter + refine (k_intersect): FP32, 28 flops per segment-pair test in the
+    filter + refine (k_intersect, k_refine_spill): FP32, 28 flops per segment-pair test in the
       reference's order with its early exit (counted by the oracle on the
       parity sample and scaled to the step; the GPU's own test count is
       reported beside it); its HBM bytes per filter_bytes();
@@ -284,7 +284,7 @@ def rooflines(rt: dict, qs: dict, n_pairs: float, stage: dict, steps: int, peaks
     dom = dict(cand[name])
     dom["kernel"] = {"edge_walk": "k_walk_tot + k_walk_fill", "cell_clip": "k_clipy (count + emit)",
                      "column_clip": "k_clipx (count + emit)", "cell_area": "k_cells",
-                     "refine": "k_intersect (filter + refine)"}[name]
+                     "refine": "k_intersect + k_refine_spill (filter + refine)"}[name]
     units = {"edge_walk": rt["vertices"] / steps, "refine": n_pairs / steps}
     tpu = TRAFFIC_PER_UNIT.get(name)
     dom["traffic"] = tpu * units[name] if tpu and name in units else None
