@@ -90,3 +90,23 @@ def test_gpu_area_cut_items_match_oracle(gpu_lib, seed, s_lo, s_hi, t_lo, t_hi, 
         a = max(0.5 * abs(np.sum(r[:-1, 0] * r[1:, 1] - r[1:, 0] * r[:-1, 1]))
                 for r in (S.ring(s).astype(np.float64), T.ring(t).astype(np.float64)))
         assert abs(out[k] - exp) <= 1e-9 * exp + 1e-14 * a, (k, s, t, out[k], exp)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 257, 20001])  # parts of a warp, of a block, several blocks
+@pytest.mark.parametrize("n_lo,n_hi,vpr", [(8, 60, 4), (16, 4000, 10), (2000, 4000, 2000)])
+def test_gpu_contain_points_flattened_match_oracle(gpu_lib, n_lo, n_hi, vpr, n):
+    # pixels of a few edges to thousands, points on vertices, near them and anywhere
+    S = P.generate(P.StarParams(dom_hi=3.0, n_lo=n_lo, n_hi=n_hi), 95, 7)
+    rng = np.random.default_rng(n)
+    pts = rng.uniform(-0.5, 3.5, (n, 2)).astype(np.float32)
+    on = rng.integers(0, len(S.xy), n)
+    pts = np.where((rng.random(n) < 0.5)[:, None], S.xy[on], pts).astype(np.float32)
+    pairs = np.stack([rng.integers(0, 7, n), rng.permutation(n)], 1).astype(np.uint32)
+    RS = O.rasterize_set(S, vpr)
+    with Store() as st:
+        st.load(0, S.off, S.xy)
+        st.rasterize(vpr=vpr)
+        out, found = st.contain_points(pts, pairs)
+    exp = O.contain_points_many(RS, pts, pairs)
+    assert np.array_equal(out, exp), f"{int((out != exp).sum())} of {n} differ"
+    assert found == int(np.asarray(exp).sum())
