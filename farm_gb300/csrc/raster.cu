@@ -2926,7 +2926,13 @@ int rasterize(farm_store *s, const farm_raster_opts *o, int *launches) {
         s->rtot.vnodes = info.vnodes;
     }
 
-    // ---- phase 2, small polygons: a block each
+    // ---- phase 2, small polygons: a block each, when all are. The pipeline's
+    // launches and waits are there for one polygon as for many, and blocks
+    // before it only add to them: joins of 1,911 polygons of up to 4,145
+    // vertices 5.48 ms with the small ones taken out, 4.59 ms without; 400 of up
+    // to 4,000 3.27 / 2.79; 5,000 of up to 8,000 12.6 / 12.3; 3,300 of up to
+    // 100,000 73.4 / 72.8.
+    if (info.n < np) info.n = 0;
     if (info.n) {
         FARM_TRY(raster_small(R, info));
         FARM_CUDA(cudaMemcpyAsync(&info, R.info, sizeof info, cudaMemcpyDeviceToHost, st));

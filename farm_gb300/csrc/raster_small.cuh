@@ -24,8 +24,11 @@
 // one is then the whole wait.
 constexpr uint32_t kSmallMany = 1024;  // polygons from which the narrow blocks are taken
 constexpr int kWalkBlocks64 = 8, kFillBlocks64 = 14, kBlocks256 = 2;  // resident per SM
-// A polygon is small up to these sizes: above them a block alone is slower
-// than the pipeline's whole chip, and the shared counters would not fit.
+// A polygon is small up to these sizes (twice the edges and nodes for blocks of
+// 256 threads): above them a block alone is slower than the pipeline's whole
+// chip, and the shared counters would not fit. Joins of 400 polygons of up to
+// 4,000 vertices 2.19 ms so, 2.79 ms by the pipeline; 1,000 at -v 64 3.05 / 4.02;
+// 10,000 of up to 2,000 4.32 / 6.64.
 constexpr uint32_t kSmallBig = 256;  // edges from which a small polygon is taken first
 constexpr uint32_t kSmallEdges = 2048, kSmallNodes = 8192, kSmallPix = 2048, kSmallLines = 512;
 
@@ -127,6 +130,7 @@ __global__ void k_small_pick(PolyHdr *__restrict__ hdr, uint32_t npoly, const ui
     }
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    const uint32_t wide = npoly < kSmallMany ? 2 : 1;  // blocks of 256 threads
 #pragma unroll 1
     for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < npoly; p0 += gridDim.x * blockDim.x) {
         const uint32_t p = p0 + lane;
@@ -142,8 +146,8 @@ __global__ void k_small_pick(PolyHdr *__restrict__ hdr, uint32_t npoly, const ui
             h.n_vnodes = (uint32_t)sz[2 * n1 + p];
             const uint64_t edges = off[p + 1] - off[p];
             lines = (uint32_t)(h.dimx > h.dimy ? h.dimx : h.dimy) + 3;
-            small = counts_ok && *ovf == 0 && edges <= kSmallEdges && sz[n1 + p] <= kSmallNodes &&
-                    sz[2 * n1 + p] <= kSmallNodes && sz[p] <= 2 * kSmallNodes && h.P <= kSmallPix &&
+            small = counts_ok && *ovf == 0 && edges <= wide * kSmallEdges && sz[n1 + p] <= wide * kSmallNodes &&
+                    sz[2 * n1 + p] <= wide * kSmallNodes && sz[p] <= 2 * wide * kSmallNodes && h.P <= kSmallPix &&
                     lines <= kSmallLines;
             done[p] = 0;
             ne = (uint32_t)edges;

@@ -38,6 +38,8 @@ def _comb(teeth):
 
 CASES = {
     "edges": lambda: [_star(n, n) for n in (2046, 2047, 2048, 2049, 1300)],
+    "edges_few": lambda: [_star(n, n) for n in (4094, 4095, 2500)],
+    "edges_over": lambda: [_star(n, n) for n in (4097, 100)],
     "tiny": lambda: [_star(n, n) for n in (3, 3, 4, 5, 7, 31, 32, 33, 127, 128, 129, 257)],
     "mixed": lambda: [_star(n, n) for n in (20, 5000, 40, 9000, 300, 2500, 16)],
     "axes": lambda: [_star(n, n, c, r) for n, c, r in
