@@ -707,51 +707,52 @@ __device__ __noinline__ CandKey cand_key(const Finest &f, uint32_t id1, uint32_t
     return c;
 }
 
-// The sequence pairs of candidate (id1, id2), the last in order, from the
-// *from-th on (skipped ones not counted): 1 when the next one holds a distance
-// below the threshold, 0 when it ends the search (its minimum is below the
-// running minimum's start value, or there is none), 2 when it does neither.
-__device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id2, double thr, uint32_t *from, int lane,
-                                      unsigned long long &rechk) {
-    const SeqSet A = seq_set(*f.sv, *f.S, id1), B = seq_set(*f.sv, *f.T, id2);
-    uint32_t at = 0;
-#pragma unroll 1
-    for (uint32_t ia = A.a; ia < A.b; ia++) {
-        const uint2 e1 = A.seq[ia];
-#pragma unroll 1
-        for (uint32_t jb = B.a; jb < B.b; jb++) {
-            const uint2 e2 = B.seq[jb];
-            if (e1.y < 2 || e2.y < 2) continue;
-            if (at++ < *from) continue;
-            (*from)++;
-            const uint32_t n1 = e2.y * (e1.y - 1), n2 = e1.y * (e2.y - 1);
-            double m = 1.7976931348623157e308;
-#pragma unroll 1
-            for (uint32_t k = lane; k < n1 + n2; k += 32) {
-                const uint32_t r = k < n1 ? k : k - n1, len = k < n1 ? e1.y - 1 : e2.y - 1;
-                const uint32_t pi = r / len, si = r % len;
-                const float2 *pr = k < n1 ? B.ring + e2.x : A.ring + e1.x;
-                const float2 *gr = k < n1 ? A.ring + e1.x : B.ring + e2.x;
-                const double d = pt_seg_dist(pr[pi], gr[si], gr[si + 1], f.geo);
-                m = m < d ? m : d;
-            }
-            for (int o = 16; o; o >>= 1) {
-                const double v = __shfl_xor_sync(0xffffffffu, m, o);
-                m = m < v ? m : v;
-            }
-            if (lane == 0) rechk += n1 + n2;
-            return m < thr ? 1 : (m < 100000.0 ? 0 : 2);
-        }
-    }
-    return 0;
-}
-
 struct WithinShared {
     WStage stage[8];
     Layer layers[8][2][kMaxLayers];
     uint2 queue[8][kQueue];
     float2 tab[900];  // longitude entries, geography only
 };
+
+// The sequence pairs of candidate (id1, id2), the last in order, from the
+// *from-th on (skipped ones not counted): 1 when the next one holds a distance
+// below the threshold, 0 when it ends the search (its minimum is below the
+// running minimum's start value, or there is none), 2 when it does neither.
+// Both questions are the staged tests' of one sequence against one, so no
+// product of two lengths is formed (a single-pixel polygon's sequence is its
+// whole ring, and two of 46,342 vertices make 2^32 tests).
+template <bool kGeo>
+__device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id2, double thr, uint32_t *from, int lane,
+                                      WithinTally &my) {
+    extern __shared__ __align__(16) unsigned char within_smem[];
+    WithinShared &sh = *reinterpret_cast<WithinShared *>(within_smem);
+    WStage *stage = &sh.stage[threadIdx.x >> 5];
+    SeqSet A = seq_set(*f.sv, *f.S, id1), B = seq_set(*f.sv, *f.T, id2);
+    const uint32_t b0 = B.a, b1 = B.b;
+    uint32_t at = 0;
+#pragma unroll 1
+    for (const uint32_t a1 = A.b; A.a < a1; A.a++) {
+#pragma unroll 1
+        for (B.a = b0; B.a < b1; B.a++) {
+            if (A.seq[A.a].y < 2 || B.seq[B.a].y < 2) continue;
+            if (at++ < *from) continue;
+            (*from)++;
+            A.b = A.a + 1;
+            B.b = B.a + 1;
+            uint32_t tests = 0, rechk = 0;
+            int r = 1;
+#pragma unroll 1
+            for (bool near = false; !near && r >= 0; r -= !near) {
+                near = warp_near<kGeo>(A, B, near_of(*f.S, *f.T, r ? thr : 100000.0, kGeo), sh.tab, stage, lane, tests,
+                                       rechk);
+            }
+            my.tests += tests;
+            my.rechk += rechk;
+            return r < 0 ? 2 : r;
+        }
+    }
+    return 0;
+}
 
 // resident blocks of k_within per SM (its grid, and so its scratch)
 constexpr int kWithinBlocks = 2;
@@ -1069,8 +1070,9 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                     if (check_last) {
                         know_last = true;
                         uint32_t from = 0;
-                        int r = last_pair(fin, last1, last2, w.thr, &from, lane, my.rechk);
-                        while (r == 2) {
+                        int r;
+#pragma unroll 1
+                        while ((r = last_pair<kGeo>(fin, last1, last2, w.thr, &from, lane, my)) == 2) {
                             // the running minimum still at its start value unless
                             // an earlier candidate holds a distance below it
                             const Near far = near_of(S, T, 100000.0, geo);
@@ -1080,7 +1082,7 @@ __global__ void __launch_bounds__(256, kWithinBlocks) k_within(const StoreView s
                                 below = test_candidates(sv, S, T, ok, ok ? ss.p[k1] : 0, ok ? ts.p[k2] : 0, far, geo,
                                                         tab, stage, lane, my);
                             }
-                            r = below ? 0 : last_pair(fin, last1, last2, w.thr, &from, lane, my.rechk);
+                            if (below) break;
                         }
                         yes = r == 1;
                     }
