@@ -208,6 +208,16 @@ int check_pairs(farm_store *s, const uint32_t *pairs, uint64_t n, int mem, bool 
 // Book a loaded side's offsets (h from 0, n + 1 entries) and room for its
 // padded rings; *ring_first: the float2 index of the side's first ring.
 int stage_side(farm_store *s, int side, std::vector<uint64_t> h, uint64_t *ring_first);
+// Empty a staged side again, and for one whose load does not get to the end:
+void unstage_side(farm_store *s, int side);
+struct StagedSide {
+    farm_store *s;
+    int side;
+    bool loaded = false;
+    ~StagedSide() {
+        if (!loaded) unstage_side(s, side);
+    }
+};
 // The same with explicit bounds: first index below n_first, second below
 // n_second; the names label the two counts in the message.
 int check_pair_limits(farm_store *s, const uint32_t *pairs, uint64_t n, int mem, uint64_t n_first,

@@ -167,6 +167,7 @@ extern "C" int farm_store_load_dt(farm_store *s, int side, const char *path, int
     for (uint64_t k = 0; k < n; k++) h[k + 1] = h[k] + rec_m[keep[k]];
     uint64_t ring_first = 0;
     FARM_TRY(stage_side(s, side, h, &ring_first));
+    StagedSide staged{s, side};
 
     // pass 2: chunks of consecutive polygons, each at most one staging buffer
     // of padded rings (a larger single polygon gets a buffer of its own size)
@@ -206,6 +207,7 @@ extern "C" int farm_store_load_dt(farm_store *s, int side, const char *path, int
         k0 = k1;
     }
     FARM_CUDA(cudaStreamSynchronize(s->stream));
+    staged.loaded = true;
     if (n_out) *n_out = n;
     return FARM_OK;
 }

@@ -312,41 +312,74 @@ namespace farm {
 // ring array, where polygon p's ring starts at cat[p] + 2p (the source side
 // first, so a target side appends in place when it fits). *ring_first gets
 // the float2 index of this side's first ring. The device offsets are copied
-// from s->h_cat, which stays valid until the next call.
+// from s->h_cat, which stays valid until the next call. Without memory for the
+// buffers the store stays as it was.
 int stage_side(farm_store *s, int side, std::vector<uint64_t> h, uint64_t *ring_first) {
     const uint64_t n = h.size() - 1;
+    // a new source side drops any target side
+    const uint64_t n0 = side == 0 ? n : s->n_side[0], n1 = side == 0 ? 0 : n;
+    const std::vector<uint64_t> &h0 = side == 0 ? h : s->h_off[0];
+    const uint64_t t0 = h0[n0], t1 = n1 ? h[n1] : 0;
+    std::vector<uint64_t> cat(n0 + n1 + 1);
+    for (uint64_t k = 0; k <= n0; k++) cat[k] = h0[k];
+    for (uint64_t k = 1; k <= n1; k++) cat[n0 + k] = t0 + h[k];
+    const uint64_t total = t0 + t1;
+    const size_t need = (total + 2 * (n0 + n1)) * sizeof(float2) + 64, off_bytes = cat.size() * 8;
+    DevBuf nr, no;
+    if (need > s->d_ring.cap) FARM_TRY(nr.ensure(need + need / 8));
+    if (off_bytes > s->d_off.cap) {
+        const int rc = no.ensure(off_bytes);
+        if (rc != FARM_OK) {
+            nr.release();
+            return rc;
+        }
+    }
     s->rasterized = false;
-    if (side == 0) {  // a new source side drops any target side
+    s->h_off[side] = std::move(h);
+    s->n_side[side] = n;
+    if (side == 0) {
         s->n_side[1] = 0;
         s->h_off[1].clear();
     }
-    s->h_off[side] = std::move(h);
-    s->n_side[side] = n;
-    const uint64_t n0 = s->n_side[0], n1 = s->n_side[1];
-    const uint64_t t0 = s->h_off[0][n0], t1 = n1 ? s->h_off[1][n1] : 0;
-    std::vector<uint64_t> &cat = s->h_cat;
-    cat.assign(n0 + n1 + 1, 0);
-    for (uint64_t k = 0; k <= n0; k++) cat[k] = s->h_off[0][k];
-    for (uint64_t k = 1; k <= n1; k++) cat[n0 + k] = t0 + s->h_off[1][k];
-    const uint64_t total = t0 + t1;
-    const size_t need = (total + 2 * (n0 + n1)) * sizeof(float2) + 64;
-    if (need > s->d_ring.cap) {
-        DevBuf nr;
-        FARM_TRY(nr.ensure(need + need / 8));
-        if (side == 1 && s->d_ring.p)
-            FARM_CUDA(cudaMemcpyAsync(nr.p, s->d_ring.p, (t0 + 2 * n0) * sizeof(float2), cudaMemcpyDeviceToDevice,
-                                      s->stream));
-        FARM_CUDA(cudaStreamSynchronize(s->stream));
-        s->d_ring.release();
-        s->d_ring = nr;
-        nr.p = nullptr;
-    }
-    FARM_TRY(s->d_off.ensure((n0 + n1 + 1) * 8));
-    FARM_CUDA(cudaMemcpyAsync(s->d_off.p, cat.data(), (n0 + n1 + 1) * 8, cudaMemcpyHostToDevice, s->stream));
-    *ring_first = side == 0 ? 0 : t0 + 2 * n0;
+    s->h_cat = std::move(cat);
     s->n_poly = n0 + n1;
     s->n_edges = total;
+    cudaError_t e = cudaSuccess;
+    if (nr.p) {
+        if (side == 1 && s->d_ring.p)
+            e = cudaMemcpyAsync(nr.p, s->d_ring.p, (t0 + 2 * n0) * sizeof(float2), cudaMemcpyDeviceToDevice, s->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+        s->d_ring.release();
+        s->d_ring = nr;
+    }
+    if (no.p) {
+        s->d_off.release();
+        s->d_off = no;
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(s->d_off.p, s->h_cat.data(), off_bytes, cudaMemcpyHostToDevice, s->stream);
+    if (e != cudaSuccess) {
+        unstage_side(s, 0);
+        return cuda_fail(e, "loading a side's offsets");
+    }
+    *ring_first = side == 0 ? 0 : t0 + 2 * n0;
     return FARM_OK;
+}
+
+// A load that failed after stage_side: the side is empty again (the source
+// side takes the target side with it), so that no later call takes the
+// half-loaded rings for polygons.
+void unstage_side(farm_store *s, int side) {
+    s->rasterized = false;
+    for (int k = side; k < 2; k++) {
+        s->n_side[k] = 0;
+        s->h_off[k].clear();
+    }
+    const uint64_t n0 = s->n_side[0];
+    s->h_cat.resize(n0 + 1);
+    s->h_cat[0] = 0;
+    s->n_poly = n0;
+    s->n_edges = s->h_cat[n0];
 }
 
 }  // namespace farm
@@ -384,15 +417,16 @@ int farm_store_load(farm_store *s, int side, uint64_t n, const uint64_t *off, co
     const uint64_t o0 = h[0];
     for (auto &v : h) v -= o0;
     const uint64_t side_total = h[n];
+    // the padding kernel reads whole (x, y) pairs: 8-byte loads
+    if (mem == FARM_MEM_DEVICE && (reinterpret_cast<uintptr_t>(xy + 2 * o0) & 7u)) {
+        set_error("farm_store_load: device vertices must start on an 8-byte boundary");
+        return FARM_EINVAL;
+    }
     uint64_t ring_first = 0;
     FARM_TRY(stage_side(s, side, std::move(h), &ring_first));
+    StagedSide staged{s, side};
     const float2 *src;
     if (mem == FARM_MEM_DEVICE) {
-        // the padding kernel reads whole (x, y) pairs: 8-byte loads
-        if (reinterpret_cast<uintptr_t>(xy + 2 * o0) & 7u) {
-            set_error("farm_store_load: device vertices must start on an 8-byte boundary");
-            return FARM_EINVAL;
-        }
         src = reinterpret_cast<const float2 *>(xy) + o0;
     } else {
         // Pinned host memory is read by the padding kernel itself over the
@@ -428,6 +462,7 @@ int farm_store_load(farm_store *s, int side, uint64_t n, const uint64_t *off, co
         s->launches++;
     }
     FARM_CUDA(cudaStreamSynchronize(s->stream));
+    staged.loaded = true;
     return FARM_OK;
 }
 
