@@ -335,6 +335,7 @@ int stage_side(farm_store *s, int side, std::vector<uint64_t> h, uint64_t *ring_
         }
     }
     s->rasterized = false;
+    s->raster_epoch++;  // area plans hold the former rings' addresses
     s->h_off[side] = std::move(h);
     s->n_side[side] = n;
     if (side == 0) {
