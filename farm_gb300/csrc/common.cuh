@@ -170,6 +170,12 @@ __device__ inline uint32_t find_segment(const uint64_t *starts, uint32_t n, uint
     return lo;
 }
 
+// Pair k of a list. Two 4-byte loads: a caller's device list is uint32 values
+// and may start at any of them.
+__device__ __forceinline__ uint2 load_pair(const uint32_t *pairs, uint64_t k) {
+    return make_uint2(pairs[2 * k], pairs[2 * k + 1]);
+}
+
 inline unsigned grid_for(uint64_t n, unsigned block) {
     uint64_t g = (n + block - 1) / block;
     if (g < 1) g = 1;

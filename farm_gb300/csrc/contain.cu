@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(32 * kPointWarps)
         PointPixel w{0u, 0u, 0.f, false};
         const uint2 *seq = nullptr;
         if (k < n) {
-            const uint2 pq = reinterpret_cast<const uint2 *>(pairs)[k];
+            const uint2 pq = load_pair(pairs, k);
             const PolyHdr &H = sv.hdr[side_base + pq.x];
             if (H.err) {
                 v = 3;

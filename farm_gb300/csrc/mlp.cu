@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kScoreThreads, 1)
                 *reinterpret_cast<__nv_bfloat16 *>(xr + (k >> 3) * tc::kLBO + (k & 7) * 2) = v;
             };
             if (r0 + r < n) {
-                const uint2 pq = reinterpret_cast<const uint2 *>(pairs)[r0 + r];
+                const uint2 pq = load_pair(pairs, r0 + r);
                 pair_features(sv, sv.hdr[pq.x], sv.hdr[tgt_base + pq.y], lut, cc, lane, put);
             } else {
                 for (int k = lane; k < kInPad; k += 32) put(k, __float2bfloat16_rn(0.f));

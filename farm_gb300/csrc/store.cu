@@ -74,7 +74,7 @@ __global__ void k_check_pairs(const uint32_t *__restrict__ pairs, uint64_t n, ui
                               unsigned long long *__restrict__ bad) {
     unsigned long long mine = 0;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (uint64_t)gridDim.x * blockDim.x) {
-        const uint2 p = reinterpret_cast<const uint2 *>(pairs)[k];
+        const uint2 p = load_pair(pairs, k);
         mine += (p.x >= n_src) | (p.y >= n_tgt);
     }
     if (mine) atomicAdd(bad, mine);
