@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(256) k_head(const __nv_bfloat16 *__restrict__ 
             const int j = lane + 32 * t;
             const float e = r < n ? d * w[t] * gelu_grad(Z2[r * kHid + j]) : 0.f;
             dZ2[r * kHid + j] = __float2bfloat16_rn(e);
-            g3[t] += d * h[t];
+            if (d != 0) g3[t] += d * h[t];  // padding may hold anything, infinities and NaN too
             g2[t] += e;
         }
     }
