@@ -1,8 +1,8 @@
 """Small polygons a block each, by path: a store of 1,024 or more (the 64-thread
-kernels) up to the sizes that count as small, one polygon over them, and
-polygons whose points outgrow the scratch beside others whose do not. Rasters
-byte for byte the pipeline's, a sample of them the oracle's; the path is told
-by the launches and the chunks."""
+kernels) up to the sizes that count as small, one polygon over them, polygons
+whose points outgrow the scratch beside others whose do not, and scratch for a
+part of the blocks or for none. Rasters byte for byte the pipeline's, a sample
+of them the oracle's; the path is told by the launches and the chunks."""
 import numpy as np
 import pytest
 
@@ -93,3 +93,24 @@ def test_gpu_points_beyond_the_scratch(gpu_lib, monkeypatch, n, teeth):
     _same(mixed, pipe)
     if not any(r["err"] for r in pipe):
         assert tm == tp
+
+
+@pytest.mark.parametrize("n", [200, 1100])
+def test_gpu_scratch_for_some_blocks_or_none(gpu_lib, monkeypatch, n):
+    ps = _set(_many()[:n])
+    full, lf, _, tf = _run(monkeypatch, ps, 10, False)
+    pipe, lp, _, _ = _run(monkeypatch, ps, 10, False, FARM_RASTER_SMALL="0")
+    none, ln, cn, tn = _run(monkeypatch, ps, 10, False, FARM_SMALL_SCRATCH="1")
+    assert ln == lp and cn == 1
+    _same(none, pipe)
+    # a slice is the same for every bound: find one that lets some of the blocks through
+    for bits in range(20, 36):
+        some, ls, cs, ts = _run(monkeypatch, ps, 10, False, FARM_SMALL_SCRATCH=str(1 << bits))
+        assert cs == 1 and ls in (lf, lp)
+        if ls == lf:
+            break
+    else:
+        pytest.fail("no bound lets the blocks through")
+    _same(some, full)
+    if not any(r["err"] for r in full):
+        assert ts == tf == tn
