@@ -740,12 +740,12 @@ __device__ __noinline__ int last_pair(const Finest &f, uint32_t id1, uint32_t id
             A.b = A.a + 1;
             B.b = B.a + 1;
             uint32_t tests = 0, rechk = 0;
-            int r = 1;
+            int r = 1;  // below the threshold (1), or else below the start value (0)?
 #pragma unroll 1
-            for (bool near = false; !near && r >= 0; r -= !near) {
-                near = warp_near<kGeo>(A, B, near_of(*f.S, *f.T, r ? thr : 100000.0, kGeo), sh.tab, stage, lane, tests,
-                                       rechk);
-            }
+            for (; r >= 0; r--)
+                if (warp_near<kGeo>(A, B, near_of(*f.S, *f.T, r ? thr : 100000.0, kGeo), sh.tab, stage, lane, tests,
+                                    rechk))
+                    break;
             my.tests += tests;
             my.rechk += rechk;
             return r < 0 ? 2 : r;
