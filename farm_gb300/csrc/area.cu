@@ -15,12 +15,13 @@
 //
 // Work: items are (pair, side, chunk of that side's edges), taken by persistent
 // warps from a global counter. A lane holds one edge; the warp walks the window
-// of the other polygon's raster around all its edges together, queues the edges
-// listed there (each at its first listing), and every lane tests its edge
-// against each. An edge's share is its signed inside length:
-// the leaving parameters minus the entering ones, plus the tail when it ends
-// inside. Per-item
-// partial sums are reduced per pair in a fixed order (deterministic results).
+// of the other polygon's raster around all its edges together and queues the
+// edges listed there whose box meets the group's (each at its first listing);
+// the lanes test their edges against the queued ones, a group of fewer than 32
+// edges in slices that share the queue. An edge's share is its signed inside
+// length: the leaving parameters minus the entering ones, plus the tail when it
+// ends inside. Per-item partial sums are reduced per pair in a fixed order
+// (deterministic results).
 // Coordinates are taken relative to the pair's source first vertex.
 // General position is assumed (no collinear overlaps, no crossing exactly at a
 // vertex); crossings at a shared vertex are counted once by half-open ranges.
@@ -38,7 +39,7 @@ namespace farm {
 
 // The tuning knob of the area pass by size bucket (bucket b holds pairs whose
 // larger edge count has floor(log2) == b), chosen by farm_area_autotune: the
-// edges per work item (default 16).
+// edges per work item (default 32).
 struct Chunks {
     uint16_t c[32];
     __host__ __device__ static int bucket(uint32_t es, uint32_t et) {
@@ -98,8 +99,9 @@ struct AreaArgs {
 };
 
 // Crossing parameters are added as integers of 2^-60: exact, in any order and
-// over any lanes. Entering and leaving ones alternate along an edge, so their
-// signed sum lies in [-1, 1]; what partial sums carry beyond 64 bits falls off.
+// over any lanes. Entering and leaving ones alternate along an edge where the
+// other ring is simple, so their signed sum lies in [-1, 1]; what partial sums
+// carry beyond 64 bits falls off.
 constexpr double kParamScale = 1152921504606846976.0;  // 2^60
 
 __device__ __forceinline__ double cross2(double ax, double ay, double bx, double by) { return ax * by - ay * bx; }
@@ -356,8 +358,9 @@ static int spread_items() {
 // 801 pairs of up to 20,000 vertices: 72 ms with a window per lane, 10.0 ms
 // with the look-up after the tests, 6.2 ms without cutting, 4.3 ms so, 3.7 ms
 // with groups of 32 edges. Loops are not unrolled: most run once or twice, and
-// in the first launch a warp waits for instruction fetch more than for anything
-// else (77 KB unrolled, 70 KB so: 3.87 -> 3.68 ms).
+// the code is larger than the instruction cache takes lightly (77 KB unrolled,
+// 70 KB so: 3.87 -> 3.68 ms). What a warp of the first launch waits for then is
+// the look-ups' loads, with FP64 busy 44% of the time.
 constexpr int kAreaQueue = 64;
 struct AreaListing {  // an edge met in a pixel of the window
     uint32_t f, pid, q;

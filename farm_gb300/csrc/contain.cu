@@ -2,7 +2,8 @@
 // its GPU form, query_contain.cu, is commented out and never launched).
 //
 //   farm_contain_points: does polygon p hold point q (Ideal::contain(Point &),
-//     Ideal.cpp:1101-1157). One thread per (polygon, point) pair: the MBR test
+//     Ideal.cpp:1101-1157). One lane per (polygon, point) pair up to its pixel,
+//     the BORDER pixels' edges over all lanes of the warp: the MBR test
 //     (box::contain, Box.cpp:65-70), the pixel's class, and for a BORDER pixel
 //     the parity of the pixel's edges whose FP32 crossing abscissa lies in
 //     [x, the pixel's right border] plus the nodes below y on the grid line at

@@ -1,5 +1,5 @@
-// Work sharing for the pair kernels (intersect, contain): pixel pairs that a
-// warp leaves to all warps.
+// Work sharing for the pair kernels (intersect, contain, within): pixel pairs
+// that a warp leaves to all warps.
 //
 // A persistent warp per candidate pair is the cheapest way through a list of
 // light pairs, but a pair of two heavy polygons has up to 10^6 times a light

@@ -125,7 +125,7 @@ class Store:
                  cap: int = 0):
         """Candidate pairs of the loaded sides computed on the GPU (uint32
         [k, 2], ascending (source, target)): a CUDA tensor when `device` is
-        given, else numpy. `cap` bounds the pairs (0: counted first)."""
+        given, else numpy. `cap` bounds the pairs (0: no bound)."""
         lib = self._lib
         n = C.c_uint64(0)
         # without a bound, room for a few pairs per polygon first (untouched

@@ -225,22 +225,24 @@ int farm_tc_gemm_test(const void *A, const void *B, float *C, int M, int N, int 
  * up to max_pairs pairs in and replays the graph (results as
  * farm_intersection_area). max_items bounds the batch's work items: each pair
  * has ceil(edges_s / chunk) + ceil(edges_t / chunk) of them (chunk per size
- * bucket, 16 by default); a batch needing more fails with FARM_EOVERFLOW.
- * A plan is tied to the store's current rasterization. */
+ * bucket, 32 by default); a batch needing more fails with FARM_EOVERFLOW.
+ * A plan is tied to the store's current rasterization: after a load or another
+ * rasterization it refuses to run. */
 typedef struct farm_area_plan farm_area_plan;
 int farm_area_plan_create(farm_store *s, uint64_t max_pairs, uint64_t max_items, farm_area_plan **out);
 int farm_area_plan_run(farm_area_plan *p, const uint32_t *pairs, uint64_t n, int mem, double *out, farm_stats *st);
 void farm_area_plan_destroy(farm_area_plan *p);
 /* Edges per area work item by size bucket b = floor(log2(larger edge count of
- * the pair)), 32 entries (0 = default 16). */
+ * the pair)), 32 entries (0 = default 32). */
 int farm_area_set_chunks(farm_store *s, const int32_t *chunk_by_bucket);
 /* Window sizes by size bucket, 32 entries (0 = default 200). They chose between
- * two searches of an edge's candidates, which are one now: kept with the store,
- * read by nothing. */
+ * two searches of an edge's candidates, which are one now: kept with the store
+ * and reported by farm_area_autotune, without effect on any result or time. */
 int farm_area_set_wide(farm_store *s, const int32_t *wide_by_bucket);
 /* Per size bucket present in the sample (up to 2048 pairs each): time the
  * chunk sizes 8..256, keep the fastest in the store and return both tables (32
- * entries each; either output may be NULL). */
+ * entries each; either output may be NULL; the window table has its default at
+ * the sample's buckets). */
 int farm_area_autotune(farm_store *s, const uint32_t *pairs, uint64_t n, int mem, int32_t *chunk_out,
                        int32_t *wide_out);
 
