@@ -189,7 +189,6 @@ FP32_NOMINAL = 128 * 152 * 2.07e9
 # figure times the step's units.
 TRAFFIC_PER_UNIT = {
     "edge_walk": 199.0,   # bytes per edge (k_walk_tot + k_walk_fill): 42.6 GB / 2.14e8 edges
-    "refine": 6621.8,     # bytes per candidate pair (k_intersect, before the spill pool): 174.3 MB / 26,320 pairs
 }
 
 
@@ -285,9 +284,8 @@ def rooflines(rt: dict, qs: dict, n_pairs: float, stage: dict, steps: int, peaks
     dom["kernel"] = {"edge_walk": "k_walk_tot + k_walk_fill", "cell_clip": "k_clipy (count + emit)",
                      "column_clip": "k_clipx (count + emit)", "cell_area": "k_cells",
                      "refine": "k_intersect + k_refine_spill (filter + refine)"}[name]
-    units = {"edge_walk": rt["vertices"] / steps, "refine": n_pairs / steps}
     tpu = TRAFFIC_PER_UNIT.get(name)
-    dom["traffic"] = tpu * units[name] if tpu and name in units else None
+    dom["traffic"] = tpu * rt["vertices"] / steps if tpu else None
     dom["traffic_note"] = ("ncu dram bytes per unit on a 400-strip case x units per step "
                            "(profiles/dram_traffic_small_strip.md)" if dom["traffic"] else
                            "no ncu capture of this kernel's DRAM bytes")
