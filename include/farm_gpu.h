@@ -93,7 +93,9 @@ void farm_store_destroy(farm_store *s);
 /* Load one side's rings (side 0 = source, 1 = target). Rings in the host
  * layout of farm_host.h: off[n+1] (vertex offsets), xy float32 pairs with the
  * closing copy included, exactly as a .dt record stores them. mem says where
- * off/xy live (FARM_MEM_HOST or FARM_MEM_DEVICE). Replaces both sides' data.
+ * off/xy live (FARM_MEM_HOST or FARM_MEM_DEVICE). Replaces that side's rings;
+ * a load of side 0 drops side 1. A call that is refused or finds no memory for
+ * the rings leaves the store as it was.
  * xy holds the off[n] - off[0] vertices that the offsets describe. Host
  * vertices in pinned (page-locked) memory at an 8-byte boundary are read by
  * the device over the host link with no staging copy; others are staged
